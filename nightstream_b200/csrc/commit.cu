@@ -99,16 +99,7 @@ PPEntry* pp_lookup(int device, uint64_t m) {
 int launch_commit(neo_gpu_ctx* ctx, const int8_t* d_digits, uint32_t n_vec, uint64_t m, uint64_t* d_out, int digits) {
     PPEntry* pp = pp_lookup(ctx->device, m);
     if (!pp || !pp->kappa) return ctx->fail(NEO_ERR_ARG, "commit: PP not loaded for this m");
-    if (pp->tc) {
-        // tensor-core path (commit_tc.cu); scratch for every form the call may take
-        uint32_t g, k, kb;
-        size_t need = 0;
-        if (digits != TC_DIGITS_ANY) need = tc_scratch_bytes(n_vec, m, true, pp->kappa, &g, &k, &kb);
-        if (digits != TC_DIGITS_SMALL) need = std::max(need, tc_scratch_bytes(n_vec, m, false, pp->kappa, &g, &k, &kb));
-        void* scratch = nullptr;
-        NEO_CK(ctx, ctx_scratch(ctx, need, &scratch));
-        return launch_commit_tc(ctx, pp, d_digits, n_vec, d_out, (uint8_t*)scratch, ctx->d_err, digits);
-    }
+    if (pp->tc) return launch_commit_tc(ctx, pp, d_digits, n_vec, d_out, digits);  // kappa <= 16: the tensor cores (commit_tc.cu)
     const uint32_t kappa = pp->kappa;
     // pick a chunking that fills the GPU: ~4 blocks per SM in total
     uint32_t target_blocks = 148 * 8;
@@ -152,7 +143,7 @@ int pp_slot(neo_gpu_ctx* ctx, uint32_t kappa, uint64_t m, PPEntry** out) {
 // (byte limbs, pre-swizzled tiles) when the shape allows it.
 int pp_finish(neo_gpu_ctx* ctx, PPEntry* pp, uint32_t kappa) {
     pp->kappa = kappa;
-    if (kappa <= 16 && pp->m % 2 == 0) return tc_pp_prepare(ctx, pp);
+    if (kappa <= 16) return tc_pp_prepare(ctx, pp);
     if (pp->d_pp_limbs) { cudaFree(pp->d_pp_limbs); pp->d_pp_limbs = nullptr; }
     return NEO_OK;
 }

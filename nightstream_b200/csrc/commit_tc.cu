@@ -1,63 +1,60 @@
 // commit_tc.cu -- Ajtai commitment as an exact int8 tensor-core GEMM (tcgen05).
 //
-// c_i(X) = sum_j M[i][j](X) z_j(X) mod Phi_81 (crates/neo-ajtai/src/commit.rs:679-744).
-// Phi_81 divides X^81 - 1, so the product is taken mod X^81 - 1 (a length-81
-// cyclic convolution whose matrix entries are the raw PP coefficients) and
-// folded back with X^54 = -X^27 - 1.  As a GEMM:
+// c_i(X) = sum_j M[i][j](X) z_j(X) mod Phi_81 (crates/neo-ajtai/src/commit.rs:679-744),
+// as a GEMM of PP byte limbs and windows of one short sequence per column:
 //
-//   D[(i,l)][(v,r)] = sum_{j, s<64} A[(i,l)][(j,s)] * B[(v,r)][(j,s)]
-//   A[(i,l)][(j,s)] = byte l of M[i][j][s]  (u8; 0 for s >= 54)
-//   B[(v,r)][(j,s)] = z_{v,j}[(r - s) mod 81] (s8; z[x] = 0 for x >= 54)
-//   c'_{v,i}[r] = sum_l 2^(8l) D[(i,l)][(v,r)]  (mod q), r < 81
+//   D[(i,l)][(v,o)] = sum_{j, s<64} A[(i,l)][(j,s)] G_{v,j}[o + s]
+//   A[(i,l)][(j,s)] = byte l of M[i][j][s]  (u8; 0 for s >= 54 and j = m, the pad of an odd m)
 //
-// M = 128 = kappa * 8 rows, K = 64 m (s padded to 64 so one 128-byte K block
-// holds exactly two columns j), N = 81 per vector.  Accumulation is int32 in
-// TMEM; a CTA covers at most 512 K blocks, so |D| <= 255*128*65536 < 2^31 for
-// any int8 digit: no overflow.  CTAs split K and groups of NV vectors; a second
-// kernel sums the int32 partials, recombines limbs mod q and folds 81 -> 54.
+// M = 128 = kappa * 8 rows, K = 64 per column (one 128-byte K block holds
+// exactly two columns).  Two forms of the sequence G (s8):
 //
-// A tiles are stored in HBM already in the 128B-swizzled K-major UMMA layout
-// (16 KB per K block, contiguous) and fetched with one cp.async.bulk each.
+//  * Small digits (|z| <= 63): [X^r] X^s z mod Phi_81 is h(r - s) for r >= 27 and
+//    -h(r - 27 - s) for r < 27, where h has period 81 and
+//      h(x) = -z[x + 27] (-27 <= x < 0),  z[x] - z[x + 27] (0 <= x < 27),  z[x] (27 <= x < 54)
+//    (X^54 = -X^27 - 1, X^81 = 1 mod Phi_81).  So the 54 output rows are the
+//    windows o = 0..53 of G[w] = h(80 - w): row r = 80 - o for o >= 27, and
+//    r = 26 - o with the finished sum negated for o < 27.  64 rows and
+//    128 sequence bytes per vector, 7 chunks of 16 bytes per phase.
+//  * Any int8 digit (cyclic): the product mod X^81 - 1, G[w] = z[(80 - w) mod 81]
+//    (z[x] = 0 for x >= 54), rows o = 0..80, output row 80 - o, folded 81 -> 54
+//    with X^54 = -X^27 - 1 when the sum is finished.  96 rows and 160 bytes per
+//    vector, 9 chunks.
 //
-// B is never materialised row by row.  With F_{v,j}[w] = z_{v,j}[(80 - w) mod 81]
-// (160 bytes per column, precomputed) the B row of output r is the window
-// F[r' + s], s < 64, with r' = 80 - r.  Writing r' = 16a + 8h + b, that window
-// is the 16-byte-aligned chunks a + k (k < 4) of the phase sequence
-// G_p[x] = F[x + p], p = 8h + b.  So the builders write, per column, the 16
-// phase sequences as 9 chunks of 16 bytes laid out [chunk][h][v][b] (9 KB),
-// and a no-swizzle K-major descriptor with 8-row-group stride 128 B and
-// K-chunk stride NV*256 B walks all rows (a, h, v, b) of all NV vectors: row
-// group g = (2a + h) NV + v sits at g*128 and its K chunk k at
-// (a + k) NV 256 = g-part + k*LBO.  Rows r' < 88 per vector (44 groups,
-// N = 256 + 96); r' in [81, 88) are computed and discarded.
+// Accumulation is int32 in TMEM; a CTA covers at most 512 K blocks, so
+// |D| <= 255*128*65536 < 2^31: no overflow.  CTAs split K and groups of NV
+// vectors.
+//
+// B is never materialised row by row.  Writing o = 16a + 8h + b, the window of
+// row o is the 16-byte-aligned chunks a + k (k < 4) of the phase sequence
+// G_p[x] = G[x + p], p = 8h + b.  So the builders write, per column, the 16
+// phases as chunks laid out [chunk][h][v][b][16 B], and a no-swizzle K-major
+// descriptor with 8-row-group stride 128 B and K-chunk stride LBO = NV*256 B
+// walks all rows (a, h, v, b): row group g = (2a + h) NV + v sits at g*128 and
+// its K chunk k at (a + k) LBO.
+//
+// One launch per call.  Warp roles of a CTA: a bulk-copy producer (A tiles,
+// stored in HBM in the 128B-swizzled K-major layout, 16 KB per K block), the
+// MMA issuer, four builder warps that are the epilogue later, and two
+// transposer warps that read the digit rows (16 to 64 columns at a time) and write
+// G straight into shared memory.  The epilogue recombines the 8 limbs of every
+// (i, column) mod q in registers and adds the value's 32-bit halves into 64-bit
+// accumulators in L2 (exact and order-free); the last CTA of a vector group
+// (ticket) reduces them, writes the commitments and leaves the accumulators zero.
+//
+// What bounds it, and what it measured, stands at commit_win_kernel.
 #include "internal.cuh"
+#include <algorithm>
 
 namespace {
 
-constexpr int TC_NV = 4;                    // vectors per CTA
-constexpr int TC_NPAD = 352;                // MMA N total: 44 groups of 8 rows, r' < 88 per vector
-constexpr int TC_N0 = 256, TC_N1 = TC_NPAD - 256;  // two MMAs per K step (N = 256, 96)
-constexpr int TC_ASTAGES = 6;               // A tiles + F sequences ring (bulk copies run ahead)
-constexpr int TC_BSTAGES = 4;               // B phase buffers ring (built by threads, overlaps MMA)
 constexpr int TC_A_BYTES = 128 * 128;       // 16 KB
-constexpr int TC_BCHUNKS = 9;               // 16-byte K chunks per column: a + k, a <= 5, k < 4
-constexpr int TC_BCOL_BYTES = TC_BCHUNKS * TC_NV * 256;  // [chunk][h][v][b][16 B] = 9 KB per column
-constexpr int TC_B_BYTES = 2 * TC_BCOL_BYTES;            // two columns per K block: 18 KB
-constexpr int TC_BLBO = TC_NV * 256;        // K-direction core-matrix stride (bytes)
-constexpr int TC_BSBO = 128;                // N-direction 8-row-group stride (bytes)
-constexpr int TC_FBYTES = 160;              // F sequence length (10 x 16 B)
-constexpr int TC_F_STAGE = TC_NV * 2 * TC_FBYTES;  // NV x 2 columns x 160 B
-constexpr int TC_SMEM_BYTES = TC_ASTAGES * (TC_A_BYTES + TC_F_STAGE) + TC_BSTAGES * TC_B_BYTES;
-constexpr int TC_BUILDERS = 256;            // 8 builder warps
-constexpr int TC_THREADS = 64 + TC_BUILDERS;  // warp0 producer, warp1 MMA, warps2-9 B build (2-5 epilogue)
+constexpr int TC_BUILDERS = 128;            // warps 2..5: B builders, then the epilogue (one TMEM lane group each)
+constexpr int TC_TRANSPOSERS = 64;          // warps 6, 7
 constexpr int TC_MAX_KB = 512;              // K blocks per CTA (int32 overflow bound)
+constexpr uint32_t TC_MIN_KB = 4;           // K blocks per CTA worth a CTA of its own (m = 2^10: 2 and 4 14.6 us, 8 16.7)
 constexpr uint32_t TC_SPIN_LIMIT = 1u << 22;       // wait attempts (each suspends at most a hardware limit)
 constexpr uint64_t TC_WAIT_NS = 500ull * 1000 * 1000;  // 0.5 s of global time per wait
-
-static_assert(TC_B_BYTES % 1024 == 0 && TC_A_BYTES % 1024 == 0, "stage buffers stay 1024-byte aligned");
-static_assert(TC_SMEM_BYTES + 1024 + 256 <= 232448, "shared memory budget");
-static_assert(TC_NPAD % 16 == 0 && TC_N1 % 16 == 0 && TC_N1 >= 16, "MMA N constraints (M=128)");
-static_assert(TC_N0 == 32 * 8, "the first MMA covers row groups 0..31");
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -122,12 +119,12 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
 }
 
 // UMMA shared-memory descriptor: K-major, no swizzle: 8-row x 16-byte core
-// matrices, LBO between core matrices along K, SBO between 8-row groups.
-__device__ __forceinline__ uint64_t ns_desc(uint32_t saddr) {
+// matrices, `lbo` bytes between core matrices along K, 128 between 8-row groups.
+__device__ __forceinline__ uint64_t ns_desc(uint32_t saddr, uint32_t lbo) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((TC_BLBO >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((TC_BSBO >> 4) & 0x3FFF) << 32;
+    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
+    d |= (uint64_t)((128 >> 4) & 0x3FFF) << 32;
     d |= (uint64_t)1 << 46;  // descriptor version (sm_100); layout bits 61-63 = 0: no swizzle
     return d;
 }
@@ -160,7 +157,8 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 // coefficients s = 8g..8g+7 of M[i][2kb+jj] (one coalesced 64-byte run),
 // splits them into 8 byte planes l and stores each 8-byte piece at row
 // (i, l), K offset 64 jj + 8g of the swizzled tile in shared memory; the
-// 16 KB tile then goes out as 1024 contiguous 16-byte stores.
+// 16 KB tile then goes out as 1024 contiguous 16-byte stores.  The last K
+// block of an odd m has zeros in place of its second column.
 __global__ void __launch_bounds__(256) pp_limbs_kernel(const uint64_t* __restrict__ pp, uint32_t kappa, uint64_t m,
                                                        uint8_t* __restrict__ ppl) {
     __shared__ __align__(16) uint8_t tile[TC_A_BYTES];
@@ -171,7 +169,7 @@ __global__ void __launch_bounds__(256) pp_limbs_kernel(const uint64_t* __restric
 #pragma unroll
     for (int e = 0; e < 8; e++) {
         const uint32_t s_ = g * 8 + e;
-        w[e] = (i < kappa && s_ < NEO_D) ? pp[((uint64_t)i * m + kb * 2 + jj) * NEO_D + s_] : 0;
+        w[e] = (i < kappa && s_ < NEO_D && kb * 2 + jj < m) ? pp[((uint64_t)i * m + kb * 2 + jj) * NEO_D + s_] : 0;
     }
     const uint32_t k = jj * 64 + g * 8;  // K byte offset of this 8-byte piece
 #pragma unroll
@@ -189,406 +187,251 @@ __global__ void __launch_bounds__(256) pp_limbs_kernel(const uint64_t* __restric
     for (int q = 0; q < TC_A_BYTES / 16 / 256; q++) dst[t + 256 * q] = src[t + 256 * q];
 }
 
-// prep: F[v][j][w] = z_{v,j}[(80 - w) mod 81] (0 for indices >= 54), w < 160
-__global__ void f_seq_kernel(const int8_t* __restrict__ digits, uint32_t n_vec, uint64_t m, uint8_t* __restrict__ F) {
-    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (tid >= (uint64_t)n_vec * m) return;
-    const uint64_t v = tid / m, j = tid % m;
-    int8_t z[NEO_D];
-    const int8_t* zv = digits + v * NEO_D * m + j;
-#pragma unroll
-    for (int x = 0; x < NEO_D; x++) z[x] = zv[(uint64_t)x * m];
-    uint32_t w32[TC_FBYTES / 4];
-#pragma unroll
-    for (int q = 0; q < TC_FBYTES / 4; q++) {
-        uint32_t word = 0;
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-            int w = q * 4 + b;
-            int x = w <= 80 ? 80 - w : 161 - w;
-            uint8_t byte = (x >= 0 && x < NEO_D) ? (uint8_t)z[x] : 0;
-            word |= (uint32_t)byte << (8 * b);
-        }
-        w32[q] = word;
-    }
-    uint4* dst = reinterpret_cast<uint4*>(F + tid * TC_FBYTES);
-#pragma unroll
-    for (int q = 0; q < TC_FBYTES / 16; q++) dst[q] = make_uint4(w32[4 * q], w32[4 * q + 1], w32[4 * q + 2], w32[4 * q + 3]);
-}
 
 // ---------------------------------------------------------------------------
-// main GEMM kernel
+// main kernel
 // ---------------------------------------------------------------------------
 struct TcArgs {
-    const uint8_t* ppl;     // pre-swizzled limb tiles
-    const uint8_t* F;       // [n_vec][m][144]
-    int32_t* partial;       // [n_cta][128][TC_NPAD]
-    uint32_t* err;          // error flag (timeouts)
+    const uint8_t* ppl;        // pre-swizzled limb tiles
+    const int8_t* digits;      // [n_vec][54][m]
+    const uint8_t* G;          // not fused: [n_groups][n_kb] records
+    unsigned long long* acc;   // [n_groups][2][16][NPAD] sums acc0, acc1 (zero between calls)
+    uint32_t* tickets;         // [n_groups] (zero between calls)
+    uint64_t* out;             // [n_vec][kappa][54]
+    uint32_t* err;             // error word (timeouts)
+    uint32_t* bad;             // small form: bit 16 set when a sequence entry leaves int8
+    const uint32_t* only_if;   // null, or the whole launch does nothing while *only_if is zero
     uint64_t m;
-    uint32_t n_vec, n_groups, n_ksplit, kb_per_cta, n_kb;
+    uint32_t n_vec, kappa, n_groups, n_ksplit, kb_per_cta, n_kb;
 };
 
-__global__ void __launch_bounds__(TC_THREADS, 1) commit_tc_kernel(const TcArgs a) {
+// Shapes of one form (CYC: any int8 digit) at NV vectors per CTA.  FUSED: the
+// CTA's transposer warps make G from the digits; else win_seq_kernel made it.
+template <int NV, bool CYC, bool FUSED>
+struct Win {
+    static constexpr int OUT = CYC ? 81 : NEO_D;        // windows that make outputs
+    static constexpr int BLOCKS = CYC ? 6 : 4;          // 16-row blocks per vector
+    static constexpr int NCH = BLOCKS + 3;              // 16-byte chunks of a phase
+    static constexpr int SEQ = CYC ? 160 : 128;         // bytes of G
+    // MMA N: whole 8-row groups up to the last output (56 or 88 rows a vector), in 16s
+    static constexpr int NPAD = ((OUT + 7) / 8 * 8 * NV + 15) / 16 * 16;
+    static constexpr uint32_t LBO = 2 * NV * 128;       // K-direction core-matrix stride
+    static constexpr int BCOL = NCH * LBO;              // B bytes per column
+    static constexpr int B_BYTES = 2 * BCOL;            // two columns per K block
+    // two CTAs per SM: while one waits on its rings the other issues MMAs (one
+    // CTA with 6 vectors, N = 2 x 192 and rings of 6 / 4 took 320 us where 4
+    // vectors and two CTAs took 298: 12 vectors at m = 2^16)
+    static constexpr int CTAS = 2;
+    static constexpr int THREADS = 256;                 // 8 warps: two per TMEM lane group in the epilogue
+    static constexpr int TILE = TC_TRANSPOSERS / NV;    // fused: columns per G tile, one (column, vector) per transposer thread
+    static constexpr int KPT = FUSED ? TILE / 2 : 1;    // K blocks per G buffer
+    // strides of a vector and of a column in a G buffer.  Odd counts of 16 bytes
+    // between vectors: the builders' word loads (lanes = vectors, phases) fall
+    // on distinct banks; fused also between columns, for the transposers'
+    // 16-byte stores (lanes = columns).  Else a K block's record is one copy.
+    static constexpr int VP = FUSED ? SEQ + 16 : 2 * SEQ + 16;
+    static constexpr int CP = FUSED ? NV * VP + (NV == 1 ? 0 : 16) : SEQ;
+    static constexpr int G_BYTES = FUSED ? TILE * CP : NV * VP;
+    // WPK builder warps make one K block: lanes (warp, sub, v, b) share its four
+    // (column, half of the chunks) tasks
+    static constexpr int WPK = NV == 4 ? (FUSED ? 4 : 2) : 1;
+    static constexpr int SUB = 4 / NV;
+    static constexpr int TASKS = 4 / (SUB * WPK);       // per lane
+    static constexpr int CPP = (NCH + 1) / 2;           // chunks per task
+    static constexpr int BSTAGES = NV == 4 ? (FUSED ? 2 : 3) : 4;
+    static constexpr int ASTAGES = NV == 2 && CYC ? 3 : 4;
+    // groups of warps that build: at most BSTAGES, so that a warp waiting for a B
+    // buffer has seen that buffer's use before the last one end (phase parities
+    // stay unambiguous)
+    static constexpr int NB = TC_BUILDERS / 32 / WPK;
+    static constexpr int GSTAGES = FUSED ? 2 : 4;
+    static constexpr int SMEM = ASTAGES * TC_A_BYTES + BSTAGES * B_BYTES + GSTAGES * G_BYTES;
+    static constexpr int DYN = SMEM + 1024 /*alignment*/ + 256 /*barriers*/;
+    static constexpr uint32_t TMEM_COLS = NPAD <= 64 ? 64 : (NPAD <= 128 ? 128 : 256);
+    static_assert(NPAD <= 256 && NPAD % 16 == 0, "one MMA per K step (M = 128: N <= 256, N % 16 == 0)");
+    static_assert(B_BYTES % 128 == 0 && G_BYTES % 16 == 0 && (VP / 16) % 2 == 1 && (!FUSED || (CP / 16) % 2 == 1), "alignment");
+    static_assert((OUT + 7) / 8 % 2 == 1, "an odd count of 8-row groups: the last chunk is read at h = 0 only");
+    static_assert(NB <= BSTAGES && TASKS >= 1, "builder warps");
+    static_assert(FUSED ? KPT >= BSTAGES : GSTAGES > BSTAGES, "a G buffer's last use is over when a B buffer is free");
+    static_assert((2 * (ASTAGES + BSTAGES + GSTAGES) + 1) * 8 + 4 <= 256, "barrier space");
+    static_assert(DYN + 64 + 1024 <= 233472 / CTAS, "shared memory of the resident CTAs");
+    static_assert(TMEM_COLS * CTAS <= 512, "TMEM columns of the resident CTAs");
+};
+
+// One digit; volatile keeps a batch of loads together in program order.  Rows
+// are m bytes apart, and lines of L1 would be claimed for 16 bytes each: .cg.
+__device__ __forceinline__ int ld_digit(const int8_t* p) {
+    int v;
+    asm volatile("ld.global.cg.s8 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
+// acc0 + 2^32 acc1 mod q of one (i, column): sums of signed terms below 2^35
+__device__ __forceinline__ uint64_t acc_value(unsigned long long acc0, unsigned long long acc1) {
+    const uint64_t h = gl::from_i64((long long)acc1);
+    return gl::add(gl::from_i64((long long)acc0), gl::reduce128(h << 32, h >> 32));
+}
+
+template <bool CYC>
+__device__ __forceinline__ void build_sequence(const int (&z)[NEO_D], uint4* dst, bool& bad) {
+    constexpr int SEQ = CYC ? 160 : 128;
+#pragma unroll
+    for (int q = 0; q < SEQ / 16; q++) {
+        uint32_t w4[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            uint32_t word = 0;
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const int w = q * 16 + e * 4 + b;
+                int g = 0;  // entries no output reads (A is zero for s >= 54) stay zero
+                if constexpr (CYC) {
+                    const int x = w <= 80 ? 80 - w : 161 - w;
+                    g = x >= 0 && x < NEO_D ? z[x] : 0;
+                } else {
+                    g = w < 27 ? -z[26 - w]
+                      : w < 54 ? z[80 - w]
+                      : w < 81 ? z[80 - w] - z[107 - w]
+                      : w < 108 ? -z[107 - w] : 0;
+                    if (w >= 54 && w < 81) bad |= g > 127 || g < -127;   // g and -g fit int8
+                    if (w < 54) bad |= z[w] == -128;                      // and so does -z
+                }
+                word |= (uint32_t)(uint8_t)(int8_t)g << (8 * b);
+            }
+            w4[e] = word;
+        }
+        dst[q] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+    }
+}
+
+// Entry w of G of four columns as one word (byte c = column c), from four-column
+// words of the digit rows.
+__device__ __forceinline__ uint32_t seq_word(const uint32_t (&z)[NEO_D], int w) {
+    return w < 27 ? __vneg4(z[26 - w])
+         : w < 54 ? z[80 - w]
+         : w < 81 ? __vsub4(z[80 - w], z[107 - w])
+         : w < 108 ? __vneg4(z[107 - w]) : 0;
+}
+
+// G of every (vector, column), one record of NV * VP bytes per (vector group, K
+// block) so that the GEMM fetches it with one copy: vector v, column jj at
+// v VP + jj SEQ.  A block makes 128 columns of one vector, four per thread
+// (V4: digit rows in aligned 4-byte words; else byte loads): a warp reads whole
+// 128-byte lines, the sequences are staged in shared memory and written in runs
+// of 2 SEQ bytes.
+constexpr int SEQ_COLS = 128, SEQ_T = SEQ_COLS / 4;
+template <bool V4>
+__global__ void __launch_bounds__(SEQ_T) win_seq_kernel(const int8_t* __restrict__ digits, uint64_t m, uint32_t n_kb,
+                                                        uint8_t* __restrict__ G, uint32_t* __restrict__ bad_flag) {
+    using S = Win<4, false, false>;
+    constexpr int NV = 4;
+    constexpr int PITCH = S::SEQ + 16;  // per column; a thread's four columns are SEQ_T apart in the stage
+    __shared__ __align__(16) uint8_t s_out[SEQ_COLS * PITCH];
+    const uint32_t v = blockIdx.y, tid = threadIdx.x;
+    const uint64_t j0 = (uint64_t)blockIdx.x * SEQ_COLS, j = j0 + 4 * tid;
+    const int8_t* zv = digits + (uint64_t)v * NEO_D * m;
+    uint32_t z[NEO_D];
+    if constexpr (V4) {  // m % 4 == 0: a word is inside the row or past it
+        const int8_t* zp = zv + (j < m ? j : 0);
+#pragma unroll
+        for (int x = 0; x < NEO_D; x++) z[x] = __ldg(reinterpret_cast<const uint32_t*>(zp + (uint64_t)x * m));
+#pragma unroll
+        for (int x = 0; x < NEO_D; x++) z[x] = j < m ? z[x] : 0;
+    } else {
+#pragma unroll
+        for (int x = 0; x < NEO_D; x++) {
+            uint32_t w = 0;
+#pragma unroll
+            for (int c = 0; c < 4; c++) {  // past the row (and the pad of an odd m's last K block): zero
+                const uint32_t d = j + c < m ? (uint8_t)__ldg(zv + (uint64_t)x * m + j + c) : 0u;
+                w |= d << (8 * c);
+            }
+            z[x] = w;
+        }
+    }
+    // a digit of -128, or a difference that leaves int8 or whose negative does
+    uint32_t bad = 0;
+#pragma unroll
+    for (int x = 0; x < NEO_D; x++) bad |= __vcmpeq4(z[x], 0x80808080u);
+#pragma unroll
+    for (int x = 0; x < 27; x++) {
+        const uint32_t d = __vsub4(z[x], z[x + 27]);
+        bad |= ((z[x] ^ z[x + 27]) & (z[x] ^ d)) & 0x80808080u;  // signed overflow
+        bad |= __vcmpeq4(d, 0x80808080u);
+    }
+    if (bad) atomicOr(bad_flag, 1u << 16);
+#pragma unroll
+    for (int q = 0; q < S::SEQ / 16; q++) {
+        uint32_t o[4][4];  // [column][word]
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int w = 16 * q + 4 * e;
+            const uint32_t a = seq_word(z, w), b = seq_word(z, w + 1), c = seq_word(z, w + 2), d = seq_word(z, w + 3);
+            const uint32_t ab0 = __byte_perm(a, b, 0x5140), ab1 = __byte_perm(a, b, 0x7362);
+            const uint32_t cd0 = __byte_perm(c, d, 0x5140), cd1 = __byte_perm(c, d, 0x7362);
+            o[0][e] = __byte_perm(ab0, cd0, 0x5410);
+            o[1][e] = __byte_perm(ab0, cd0, 0x7632);
+            o[2][e] = __byte_perm(ab1, cd1, 0x5410);
+            o[3][e] = __byte_perm(ab1, cd1, 0x7632);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++)  // column 4 tid + c at stage row c SEQ_T + tid: a store's lanes on distinct banks
+            *reinterpret_cast<uint4*>(s_out + (c * SEQ_T + tid) * PITCH + q * 16) = make_uint4(o[c][0], o[c][1], o[c][2], o[c][3]);
+    }
+    __syncwarp();
+    constexpr uint32_t CH = S::SEQ / 16;
+    const uint64_t kb0 = j0 / 2;
+    const uint32_t cols = 2 * (uint32_t)min((uint64_t)SEQ_COLS / 2, n_kb - kb0);
+    uint8_t* out = G + ((uint64_t)(v / NV) * n_kb + kb0) * (NV * S::VP) + (v % NV) * S::VP;
+#pragma unroll 4
+    for (uint32_t e = tid; e < cols * CH; e += SEQ_T) {
+        const uint32_t c = e / CH, q = e % CH;
+        *reinterpret_cast<uint4*>(out + (uint64_t)(c / 2) * (NV * S::VP) + (c & 1) * S::SEQ + q * 16) =
+            *reinterpret_cast<const uint4*>(s_out + ((c & 3) * SEQ_T + (c >> 2)) * PITCH + q * 16);
+    }
+}
+static_assert(SEQ_T == 32, "win_seq_kernel: one warp, synchronised as one");
+
+// What bounds it.  One vector: HBM (537 MB of tiles at m = 2^16: 88 us = 6.1 TB/s;
+// before, with separate sequence and reduce launches and 112-byte sequences per
+// half of the rows, 127 us).  Groups of four: shared memory.  Per K block the MMAs
+// read 352 wavefronts of 128 bytes, the builders store 91 and load 68, the A tile
+// and G arrive with 136, against 478 cycles of MMA (N = 224; MMAs alone reach 4.5
+// POPS): 12 ternary vectors at m = 2^16 take 290 us (361 before), of which the
+// sequence launch 33; m = 2^14 85 (119), m = 2^10 23 (43).  Windows of one
+// 81-periodic sequence need 7 chunks a phase where one sequence per half of the
+// rows needed 10.  One launch instead of four: 1 vector at m = 2^10 10.4 us (26).
+// Any digit: 5 vectors at m = 10006 49 us (94); an odd m, which ran on CUDA cores,
+// 1 vector at m = 5001 19 us (806).
+template <int NV, bool CYC, bool FUSED>
+__global__ void __launch_bounds__(Win<NV, CYC, FUSED>::THREADS, Win<NV, CYC, FUSED>::CTAS)
+commit_win_kernel(const __grid_constant__ TcArgs a) {
+    using S = Win<NV, CYC, FUSED>;
+    if (a.only_if && __ldcg(a.only_if) == 0) return;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // 1024-align the tile buffers (dynamic smem base alignment is not guaranteed)
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* sA = smem;                                        // [ASTAGES][16 KB]
-    uint8_t* sB = sA + TC_ASTAGES * TC_A_BYTES;                // [BSTAGES][18 KB]
-    uint8_t* sF = sB + TC_BSTAGES * TC_B_BYTES;                // [ASTAGES][1280 B]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sF + TC_ASTAGES * TC_F_STAGE);
-    uint64_t* full_a = bars;                                   // [ASTAGES] A tile + F landed
-    uint64_t* empty_a = bars + TC_ASTAGES;                     // [ASTAGES] MMAs done reading the A tile
-    uint64_t* full_b = bars + 2 * TC_ASTAGES;                  // [BSTAGES] B tile built
-    uint64_t* empty_b = full_b + TC_BSTAGES;                   // [BSTAGES] MMAs done reading the B tile
-    uint64_t* done = empty_b + TC_BSTAGES;                     // [1]
+    uint8_t* sB = sA + S::ASTAGES * TC_A_BYTES;                // [BSTAGES][B_BYTES]
+    uint8_t* sG = sB + S::BSTAGES * S::B_BYTES;                // [GSTAGES][G_BYTES]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sG + S::GSTAGES * S::G_BYTES);
+    uint64_t* full_a = bars;                                   // A tile landed
+    uint64_t* empty_a = full_a + S::ASTAGES;                   // MMAs done reading the A tile
+    uint64_t* full_b = empty_a + S::ASTAGES;                   // B phases built
+    uint64_t* empty_b = full_b + S::BSTAGES;                   // MMAs done reading the B phases
+    uint64_t* full_g = empty_b + S::BSTAGES;                   // G buffer written
+    uint64_t* empty_g = full_g + S::GSTAGES;                   // builders done reading the G buffer
+    uint64_t* done = empty_g + S::GSTAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     __shared__ int s_abort;
+    __shared__ bool s_last;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t cta = blockIdx.x;
-    const uint32_t group = cta % a.n_groups, ks = cta / a.n_groups;
+    const uint32_t group = blockIdx.x % a.n_groups, ks = blockIdx.x / a.n_groups;
     const uint32_t kb0 = ks * a.kb_per_cta;
     const uint32_t kb1 = min(a.n_kb, kb0 + a.kb_per_cta);
     const uint32_t nkb = kb1 > kb0 ? kb1 - kb0 : 0;
-    const uint32_t nvalid = min((uint32_t)TC_NV, a.n_vec - group * TC_NV);  // vectors of this group
-
-    if (threadIdx.x == 0) {
-        s_abort = 0;
-        for (int s = 0; s < TC_ASTAGES; s++) {
-            mbar_init(&full_a[s], 1);
-            mbar_init(&empty_a[s], 1);
-        }
-        for (int s = 0; s < TC_BSTAGES; s++) {
-            mbar_init(&full_b[s], TC_BUILDERS / 32);
-            mbar_init(&empty_b[s], 1);
-        }
-        mbar_init(done, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = *tmem_slot;
-
-    if (warp == 0) {
-        // ---- producer: A tiles and F sequences ----
-        if (lane == 0) {
-            for (uint32_t it = 0; it < nkb; it++) {
-                const int s = it % TC_ASTAGES;
-                const uint32_t ph = (it / TC_ASTAGES) & 1;
-                if (it >= TC_ASTAGES && !mbar_wait(&empty_a[s], ph ^ 1)) { atomicOr(a.err, 1u); s_abort = 1; break; }
-                if (s_abort) break;
-                const uint64_t kb = kb0 + it;
-                mbar_expect_tx(&full_a[s], TC_A_BYTES + nvalid * 2 * TC_FBYTES);
-                bulk_g2s(sA + s * TC_A_BYTES, a.ppl + kb * TC_A_BYTES, TC_A_BYTES, &full_a[s]);
-                // F sequences of columns 2kb, 2kb+1 for each vector of the group (288 contiguous bytes)
-                for (uint32_t vl = 0; vl < nvalid; vl++)
-                    bulk_g2s(sF + s * TC_F_STAGE + vl * 2 * TC_FBYTES,
-                             a.F + ((uint64_t)(group * TC_NV + vl) * a.m + kb * 2) * TC_FBYTES, 2 * TC_FBYTES, &full_a[s]);
-            }
-        }
-    } else if (warp == 1) {
-        // ---- MMA issuer ----
-        if (lane == 0) {
-            const uint32_t id0 = idesc_i8(TC_N0), id1 = idesc_i8(TC_N1);
-            for (uint32_t it = 0; it < nkb; it++) {
-                const int sa = it % TC_ASTAGES, sb = it % TC_BSTAGES;
-                if (!mbar_wait(&full_a[sa], (it / TC_ASTAGES) & 1) || !mbar_wait(&full_b[sb], (it / TC_BSTAGES) & 1)) {
-                    atomicOr(a.err, 2u);
-                    s_abort = 1;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;");
-                const uint32_t a0 = smem_u32(sA + sa * TC_A_BYTES), b0 = smem_u32(sB + sb * TC_B_BYTES);
-#pragma unroll
-                for (int k = 0; k < 4; k++) {  // 4 x 32-byte K steps: column k/2, s in [32(k%2), 32(k%2)+32)
-                    const uint64_t ad = sw128_desc(a0 + 32 * k);
-                    const uint32_t acc = (it > 0 || k > 0) ? 1u : 0u;
-                    const uint32_t bcol = b0 + (k >> 1) * TC_BCOL_BYTES + (k & 1) * 2 * TC_BLBO;
-                    mma_i8(tmem, ad, ns_desc(bcol), id0, acc);
-                    mma_i8(tmem + TC_N0, ad, ns_desc(bcol + 32 * TC_BSBO), id1, acc);
-                }
-                mma_commit(&empty_a[sa]);  // tiles free once these MMAs complete
-                mma_commit(&empty_b[sb]);
-            }
-            mma_commit(done);
-        }
-    } else {
-        // ---- B builders (warps 2..9) ----
-        // thread (part, column jj, vector vl, phase p = 8h + b) writes chunks c of
-        // G_p: chunk c = F[16c + p, 16c + p + 16) at [jj][c][h][vl][b]; part 0 the
-        // chunks 0..4, part 1 the chunks 5..8 (warp-uniform)
-        const int bt = threadIdx.x - 64;
-        const int p = bt & 15, vl = (bt >> 4) & 3, jj = (bt >> 6) & 1, part = bt >> 7;
-        for (uint32_t it = 0; it < nkb; it++) {
-            const int sa = it % TC_ASTAGES, sb = it % TC_BSTAGES;
-            // F of this K block has landed, and the MMAs of K block it - BSTAGES released the B buffer;
-            // lane 0 waits for the warp, so every exit from this loop is warp-uniform
-            uint32_t st = 0;  // 0 go, 1 timed out, 2 another role aborted
-            if (lane == 0) {
-                if (!mbar_wait(&full_a[sa], (it / TC_ASTAGES) & 1) ||
-                    (it >= TC_BSTAGES && !mbar_wait(&empty_b[sb], ((it / TC_BSTAGES) & 1) ^ 1)))
-                    st = 1;
-                else if (s_abort)
-                    st = 2;
-            }
-            st = __shfl_sync(0xffffffffu, st, 0);
-            if (st == 1 && lane == 0) {
-                atomicOr(a.err, 4u);
-                s_abort = 1;
-            }
-            if (st) break;
-            uint8_t* dstB = sB + sb * TC_B_BYTES;
-            const uint8_t* srcF = sF + sa * TC_F_STAGE;
-            if ((uint32_t)vl < nvalid) {
-                const int c0 = part ? 5 : 0;
-                const int o = 16 * c0 + p;  // first F byte of this thread's chunks
-                const uint32_t* src = reinterpret_cast<const uint32_t*>(srcF + (vl * 2 + jj) * TC_FBYTES + (o & ~3));
-                const uint32_t sh = 8 * (o & 3);
-                uint8_t* dst = dstB + jj * TC_BCOL_BYTES + c0 * TC_BLBO + (p >> 3) * (TC_NV * 128) + vl * 128 + (p & 7) * 16;
-                uint32_t w[21];
-                if (part == 0) {  // 5 chunks: words [o/4, o/4 + 21) <= byte 96 of the 160-byte F
-#pragma unroll
-                    for (int q = 0; q < 21; q++) w[q] = src[q];
-#pragma unroll
-                    for (int c = 0; c < 5; c++)
-                        *reinterpret_cast<uint4*>(dst + c * TC_BLBO) =
-                            make_uint4(__funnelshift_r(w[4 * c], w[4 * c + 1], sh), __funnelshift_r(w[4 * c + 1], w[4 * c + 2], sh),
-                                       __funnelshift_r(w[4 * c + 2], w[4 * c + 3], sh), __funnelshift_r(w[4 * c + 3], w[4 * c + 4], sh));
-                } else {  // 4 chunks: words [o/4, o/4 + 17) end exactly at byte 160
-#pragma unroll
-                    for (int q = 0; q < 17; q++) w[q] = src[q];
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        *reinterpret_cast<uint4*>(dst + c * TC_BLBO) =
-                            make_uint4(__funnelshift_r(w[4 * c], w[4 * c + 1], sh), __funnelshift_r(w[4 * c + 1], w[4 * c + 2], sh),
-                                       __funnelshift_r(w[4 * c + 2], w[4 * c + 3], sh), __funnelshift_r(w[4 * c + 3], w[4 * c + 4], sh));
-                }
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full_b[sb]);
-        }
-        // ---- epilogue (warps 2..5 cover TMEM lane groups 2, 3, 0, 1): TMEM -> int32 partials ----
-        uint32_t okw = 0;  // lane 0 waits for the warp
-        if (lane == 0) okw = (nkb > 0 && !s_abort && mbar_wait(done, 0)) ? 1u : 0u;
-        const bool ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
-        if (nkb > 0 && !ok && warp < 6) atomicOr(a.err, 8u);
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const int lg = warp & 3;  // TMEM lane group this warp may access
-        const int row = lg * 32 + lane;
-        int32_t* dst = a.partial + ((uint64_t)cta * 128 + row) * TC_NPAD;
-        for (int c0 = 0; c0 < (warp < 6 ? TC_NPAD : 0); c0 += 16) {
-            uint32_t v[16];
-            const uint32_t taddr = tmem + ((uint32_t)(lg * 32) << 16) + (uint32_t)c0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                : "r"(taddr));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (ok) {
-#pragma unroll
-                for (int q = 0; q < 16; q += 4)
-                    *reinterpret_cast<int4*>(dst + c0 + q) = make_int4((int)v[q], (int)v[q + 1], (int)v[q + 2], (int)v[q + 3]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 16; q += 4) *reinterpret_cast<int4*>(dst + c0 + q) = make_int4(0, 0, 0, 0);
-            }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    if (warp == 1) {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
-    }
-}
-
-// c'_{v,i}[r] = sum_{ks} sum_l 2^(8l) D[ks][(i,l)][(v,r)] mod q, then fold 81 -> 54.
-// One block per (vector group, i): thread (col, half) sums the int32 partials
-// of TMEM column col over its half of the K splits for the 8 limb rows
-// (reads coalesced along the 352 columns), the halves meet in shared memory,
-// then each column is recombined mod q, mapped back to (v, r) and folded.
-constexpr int RED_THREADS = TC_NPAD * 2;
-__global__ void __launch_bounds__(RED_THREADS) commit_tc_reduce_kernel(const int32_t* __restrict__ partial,
-                                                                       uint32_t n_groups, uint32_t n_ksplit,
-                                                                       uint32_t kappa, uint32_t n_vec,
-                                                                       uint64_t* __restrict__ out) {
-    const uint32_t group = blockIdx.x / kappa, i = blockIdx.x % kappa;
-    const int col = threadIdx.x % TC_NPAD, half = threadIdx.x / TC_NPAD;
-    __shared__ int64_t s_acc[TC_NPAD][8];
-    __shared__ uint64_t s_c[TC_NV][81];
-    int64_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const uint32_t ks0 = half ? n_ksplit / 2 : 0, ks1 = half ? n_ksplit : n_ksplit / 2;
-    for (uint32_t ks = ks0; ks < ks1; ks++) {
-        const int32_t* p = partial + ((uint64_t)(ks * n_groups + group) * 128 + i * 8) * TC_NPAD + col;
-#pragma unroll
-        for (int l = 0; l < 8; l++) acc[l] += p[(uint64_t)l * TC_NPAD];
-    }
-    if (half) {
-#pragma unroll
-        for (int l = 0; l < 8; l++) s_acc[col][l] = acc[l];
-    }
-    __syncthreads();
-    if (!half) {
-        uint64_t c = 0;
-#pragma unroll
-        for (int l = 0; l < 8; l++) c = gl::add(c, gl::mul(gl::from_i64(acc[l] + s_acc[col][l]), 1ULL << (8 * l)));
-        // column -> row group g = (2a + h) NV + v, row b; r' = 16a + 8h + b, r = 80 - r'
-        const int g = col >> 3, b = col & 7;
-        const int v = g % TC_NV, h = (g / TC_NV) & 1, a = g / (2 * TC_NV);
-        const int rp = 16 * a + 8 * h + b;
-        if (rp <= 80) s_c[v][80 - rp] = c;
-    }
-    __syncthreads();
-    for (int x = threadIdx.x; x < TC_NV * NEO_D; x += blockDim.x) {
-        const int v = x / NEO_D, r = x % NEO_D;
-        const uint32_t vg = group * TC_NV + v;
-        if (vg < n_vec)
-            out[((uint64_t)vg * kappa + i) * NEO_D + r] = gl::sub(s_c[v][r], r >= 27 ? s_c[v][r + 27] : s_c[v][r + 54]);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Small-digit form: the product taken mod Phi_81 directly.
-//
-// For digits |z| <= 63 the rotation matrix of z mod Phi_81 itself fits int8:
-// [X^r] X^s z(X) mod Phi_81 = z[r-s] - z[r+27-s]                 (r >= 27)
-//                             z[r-s] - z[r+54-s] + z[r+81-s]      (r < 27)
-// (X^54 = -X^27 - 1 and X^81 = 1 mod Phi_81; z[x] = 0 outside [0, 54)), and
-// at most two of the terms are nonzero for any (r, s).  With r' = 58 - r for
-// the rows r >= 27 and r' = 31 - r for the rows r < 27 (r' < 32, rows r' < 5
-// computed and discarded), row r is the window [r', r' + 64) of one of two
-// sequences per (vector, column):
-//   H_0[w] = z[58 - w] - z[85 - w],   H_1[w] = z[31 - w] - z[85 - w] + z[112 - w].
-// So the B operand keeps the phase-sequence layout of the cyclic form with
-// 64 rows per vector instead of 88: N = 64 NV, one MMA per 32-byte K step
-// (A read once), 1.40x the algorithmic MACs instead of 1.93x, and the output
-// needs no 81 -> 54 fold.  Row groups g = ((2a + h) 2 + seq) NV + v, r' =
-// 16a + 8h + b; phase chunks [chunk][h][seq][v][b][16 B], chunk < 5.
-constexpr int P8_HSEQ = 112;            // bytes per window sequence (w < 95 used)
-constexpr int P8_FBYTES = 2 * P8_HSEQ;  // both sequences of one (vector, column)
-
-template <int NV>
-struct P8 {
-    static constexpr int NPAD = 64 * NV;        // MMA N
-    static constexpr int LBO = 4 * NV * 128;    // K-direction core-matrix stride
-    static constexpr int BCOL = 5 * LBO;        // B bytes per column
-    static constexpr int B_BYTES = 2 * BCOL;    // two columns per K block
-    static constexpr int F_STAGE = NV * 2 * P8_FBYTES;
-    // (column, vector, seq, phase pair) for NV <= 4; at least the 4 epilogue warps
-    static constexpr int BUILDERS = 128;
-    static_assert(NV <= 4, "one builder thread per (column, vector, seq, phase pair)");
-    static constexpr int THREADS = 64 + BUILDERS;
-    // groups of 4 vectors run two CTAs per SM (3 A stages, 2 B buffers each):
-    // while one waits on its rings the other issues MMAs (0.47 instead of
-    // 0.52 ms for 12 planes at m = 2^16); a single vector keeps one CTA with
-    // deeper rings
-    static constexpr int CTAS = NV == 4 ? 2 : 1;
-    static constexpr int ASTAGES = CTAS == 2 ? 3 : 6, BSTAGES = CTAS == 2 ? 2 : 4;
-    static constexpr int SMEM = ASTAGES * (TC_A_BYTES + F_STAGE) + BSTAGES * B_BYTES;
-    static constexpr uint32_t TMEM_COLS = NPAD <= 64 ? 64 : (NPAD <= 128 ? 128 : 256);
-    static_assert(NPAD <= 256 && NPAD % 16 == 0, "one MMA per K step (M = 128: N <= 256, N % 16 == 0)");
-    static_assert(B_BYTES % 1024 == 0, "B stages stay 1024-byte aligned");
-    static_assert(SMEM + 1024 + 256 <= 232448 / CTAS - 1024 * (CTAS - 1), "shared memory budget");
-    static_assert(TMEM_COLS * CTAS <= 512, "TMEM columns of the resident CTAs");
-};
-
-__device__ __forceinline__ uint64_t ns_desc_lbo(uint32_t saddr, uint32_t lbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((TC_BSBO >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
-
-// z[x], 0 outside [0, 54) (x is a compile-time constant after unrolling)
-__device__ __forceinline__ int zat(const int (&z)[NEO_D], int x) { return (x >= 0 && x < NEO_D) ? z[x] : 0; }
-
-// prep: the two window sequences of every (vector, column); a digit pair whose
-// window entry leaves int8 sets bit 16 of *err (the caller then takes the
-// cyclic form, or reports the error).  A block's 128 outputs are contiguous
-// (28 KB), so each thread writes its 224 bytes into shared memory (pitch 240 B:
-// an odd count of 16-byte chunks keeps a store phase on eight bank groups) and
-// the block copies them out with consecutive 16-byte stores.
-constexpr int P8_SEQ_THREADS = 128;
-constexpr int P8_SEQ_PITCH = P8_FBYTES + 16;
-__global__ void __launch_bounds__(P8_SEQ_THREADS) p8_seq_kernel(const int8_t* __restrict__ digits, uint32_t n_vec,
-                                                                uint64_t m, uint8_t* __restrict__ F,
-                                                                uint32_t* __restrict__ err) {
-    __shared__ __align__(16) uint8_t s_out[P8_SEQ_THREADS * P8_SEQ_PITCH];
-    const uint64_t total = (uint64_t)n_vec * m;
-    const uint64_t base = (uint64_t)blockIdx.x * P8_SEQ_THREADS;
-    const uint64_t tid = base + threadIdx.x;
-    if (tid < total) {
-        const uint64_t v = tid / m, j = tid % m;
-        int z[NEO_D];
-        const int8_t* zv = digits + v * NEO_D * m + j;
-#pragma unroll
-        for (int x = 0; x < NEO_D; x++) z[x] = zv[(uint64_t)x * m];
-        uint4* dst = reinterpret_cast<uint4*>(s_out + threadIdx.x * P8_SEQ_PITCH);
-        bool bad = false;
-#pragma unroll
-        for (int seq = 0; seq < 2; seq++) {
-#pragma unroll
-            for (int q = 0; q < P8_HSEQ / 16; q++) {
-                uint32_t w4[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    uint32_t word = 0;
-#pragma unroll
-                    for (int b = 0; b < 4; b++) {
-                        const int w = q * 16 + e * 4 + b;
-                        const int h = seq == 0 ? zat(z, 58 - w) - zat(z, 85 - w)
-                                               : zat(z, 31 - w) - zat(z, 85 - w) + zat(z, 112 - w);
-                        bad |= h < -128 || h > 127;
-                        word |= (uint32_t)(uint8_t)(int8_t)h << (8 * b);
-                    }
-                    w4[e] = word;
-                }
-                dst[seq * (P8_HSEQ / 16) + q] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
-            }
-        }
-        if (bad) atomicOr(err, 1u << 16);
-    }
-    __syncthreads();
-    const uint32_t cnt = (uint32_t)min((uint64_t)P8_SEQ_THREADS, total - base);
-    constexpr uint32_t CH = P8_FBYTES / 16;  // 14 chunks per output
-    uint4* out = reinterpret_cast<uint4*>(F + base * P8_FBYTES);
-    for (uint32_t k = threadIdx.x; k < cnt * CH; k += P8_SEQ_THREADS)
-        out[k] = *reinterpret_cast<const uint4*>(s_out + (k / CH) * P8_SEQ_PITCH + (k % CH) * 16);
-}
-
-template <int NV>
-__global__ void __launch_bounds__(P8<NV>::THREADS, P8<NV>::CTAS) commit_p8_kernel(const TcArgs a) {
-    using S = P8<NV>;
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* sA = smem;                                  // [ASTAGES][16 KB]
-    uint8_t* sB = sA + S::ASTAGES * TC_A_BYTES;          // [BSTAGES][B_BYTES]
-    uint8_t* sF = sB + S::BSTAGES * S::B_BYTES;          // [ASTAGES][F_STAGE]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sF + S::ASTAGES * S::F_STAGE);
-    uint64_t* full_a = bars;
-    uint64_t* empty_a = bars + S::ASTAGES;
-    uint64_t* full_b = bars + 2 * S::ASTAGES;
-    uint64_t* empty_b = full_b + S::BSTAGES;
-    uint64_t* done = empty_b + S::BSTAGES;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
-    __shared__ int s_abort;
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t cta = blockIdx.x;
-    const uint32_t group = cta % a.n_groups, ks = cta / a.n_groups;
-    const uint32_t kb0 = ks * a.kb_per_cta;
-    const uint32_t kb1 = min(a.n_kb, kb0 + a.kb_per_cta);
-    const uint32_t nkb = kb1 > kb0 ? kb1 - kb0 : 0;
-    const uint32_t nvalid = min((uint32_t)NV, a.n_vec - group * NV);
+    const uint32_t nvalid = min((uint32_t)NV, a.n_vec - group * NV);  // vectors of this group
 
     if (threadIdx.x == 0) {
         s_abort = 0;
@@ -597,8 +440,12 @@ __global__ void __launch_bounds__(P8<NV>::THREADS, P8<NV>::CTAS) commit_p8_kerne
             mbar_init(&empty_a[s], 1);
         }
         for (int s = 0; s < S::BSTAGES; s++) {
-            mbar_init(&full_b[s], S::BUILDERS / 32);
+            mbar_init(&full_b[s], S::WPK);
             mbar_init(&empty_b[s], 1);
+        }
+        for (int s = 0; s < S::GSTAGES; s++) {
+            mbar_init(&full_g[s], FUSED ? TC_TRANSPOSERS / 32 : 1);
+            mbar_init(&empty_g[s], S::KPT * S::WPK);
         }
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -612,25 +459,27 @@ __global__ void __launch_bounds__(P8<NV>::THREADS, P8<NV>::CTAS) commit_p8_kerne
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tmem_slot;
+    // a role's wait, by lane 0 for its warp so that every exit is warp-uniform:
+    // 0 go, 1 timed out, 2 another role aborted
+    auto warp_wait = [&](bool go) -> uint32_t {
+        uint32_t st = go ? (s_abort ? 2u : 0u) : 1u;
+        return __shfl_sync(0xffffffffu, st, 0);
+    };
 
     if (warp == 0) {
-        // ---- producer: A tiles and window sequences ----
+        // ---- producer: A tiles ----
         if (lane == 0) {
             for (uint32_t it = 0; it < nkb; it++) {
                 const int s = it % S::ASTAGES;
                 const uint32_t ph = (it / S::ASTAGES) & 1;
                 if (it >= S::ASTAGES && !mbar_wait(&empty_a[s], ph ^ 1)) { atomicOr(a.err, 1u); s_abort = 1; break; }
                 if (s_abort) break;
-                const uint64_t kb = kb0 + it;
-                mbar_expect_tx(&full_a[s], TC_A_BYTES + nvalid * 2 * P8_FBYTES);
-                bulk_g2s(sA + s * TC_A_BYTES, a.ppl + kb * TC_A_BYTES, TC_A_BYTES, &full_a[s]);
-                for (uint32_t vl = 0; vl < nvalid; vl++)  // columns 2kb, 2kb+1 of vector vl: 448 contiguous bytes
-                    bulk_g2s(sF + s * S::F_STAGE + vl * 2 * P8_FBYTES,
-                             a.F + ((uint64_t)(group * NV + vl) * a.m + kb * 2) * P8_FBYTES, 2 * P8_FBYTES, &full_a[s]);
+                mbar_expect_tx(&full_a[s], TC_A_BYTES);
+                bulk_g2s(sA + s * TC_A_BYTES, a.ppl + (uint64_t)(kb0 + it) * TC_A_BYTES, TC_A_BYTES, &full_a[s]);
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer: one M = 128, N = 64 NV MMA per 32-byte K step ----
+        // ---- MMA issuer: one M = 128, N = NPAD MMA per 32-byte K step ----
         if (lane == 0) {
             const uint32_t id = idesc_i8(S::NPAD);
             for (uint32_t it = 0; it < nkb; it++) {
@@ -644,90 +493,174 @@ __global__ void __launch_bounds__(P8<NV>::THREADS, P8<NV>::CTAS) commit_p8_kerne
                 const uint32_t a0 = smem_u32(sA + sa * TC_A_BYTES), b0 = smem_u32(sB + sb * S::B_BYTES);
 #pragma unroll
                 for (int k = 0; k < 4; k++) {  // column k/2, s in [32(k%2), 32(k%2)+32): chunks 2(k%2), 2(k%2)+1
-                    const uint32_t acc = (it > 0 || k > 0) ? 1u : 0u;
                     const uint32_t bcol = b0 + (k >> 1) * S::BCOL + (k & 1) * 2 * S::LBO;
-                    mma_i8(tmem, sw128_desc(a0 + 32 * k), ns_desc_lbo(bcol, S::LBO), id, acc);
+                    mma_i8(tmem, sw128_desc(a0 + 32 * k), ns_desc(bcol, S::LBO), id, (it > 0 || k > 0) ? 1u : 0u);
                 }
-                mma_commit(&empty_a[sa]);
+                mma_commit(&empty_a[sa]);  // tiles free once these MMAs complete
                 mma_commit(&empty_b[sb]);
             }
             mma_commit(done);
         }
-    } else {
-        // ---- B builders: thread (column jj, vector v, seq, b < 8) writes the
-        // chunks c < 5 of both phases p = b + 8h (h = 0, 1), G_p = H_seq[16c + p,
-        // 16c + p + 16), at [jj][c][h][seq][v][b]; the two phases share the
-        // words [b/4, b/4 + 23) of the sequence, read once.  A warp covers two
-        // (jj, v) pairs and both sequences, so each store phase writes whole
-        // 128-byte rows and the loads touch eight distinct words ----
-        const int bt = threadIdx.x - 64;
-        const int b = bt & 7, seq = (bt >> 3) & 1, combo = bt >> 4;
-        const int v = combo % NV, jj = combo / NV;
-        const bool active = jj < 2 && (uint32_t)v < nvalid;
-        for (uint32_t it = 0; it < nkb; it++) {
-            const int sb = it % S::BSTAGES;
-            uint32_t st = 0;  // 0 go, 1 timed out, 2 another role aborted (lane 0 waits for the warp)
-            if (lane == 0) {
-                const int sa = it % S::ASTAGES;
-                if (!mbar_wait(&full_a[sa], (it / S::ASTAGES) & 1) ||
-                    (it >= S::BSTAGES && !mbar_wait(&empty_b[sb], ((it / S::BSTAGES) & 1) ^ 1)))
-                    st = 1;
-                else if (s_abort)
-                    st = 2;
+    } else if (!FUSED && warp >= 2 + TC_BUILDERS / 32) {
+        // ---- second producer: the records of G (one thread of the last two warps) ----
+        if (lane == 0 && warp == 2 + TC_BUILDERS / 32) {
+            for (uint32_t it = 0; it < nkb; it++) {
+                const int s = it % S::GSTAGES;
+                if (it >= S::GSTAGES && !mbar_wait(&empty_g[s], ((it / S::GSTAGES) & 1) ^ 1)) { atomicOr(a.err, 0x20u); s_abort = 1; break; }
+                if (s_abort) break;
+                mbar_expect_tx(&full_g[s], S::G_BYTES);
+                bulk_g2s(sG + s * S::G_BYTES, a.G + ((uint64_t)group * a.n_kb + kb0 + it) * S::G_BYTES, S::G_BYTES, &full_g[s]);
             }
-            st = __shfl_sync(0xffffffffu, st, 0);
+        }
+    } else if (FUSED && warp >= 2 + TC_BUILDERS / 32) {
+        // ---- transposers: thread (column, vector) of a G tile ----
+        const int tt = threadIdx.x - 64 - TC_BUILDERS;
+        const int col = tt % S::TILE, v = tt / S::TILE;
+        const int8_t* zv = a.digits + (uint64_t)(group * NV + v) * NEO_D * a.m;
+        const uint32_t nt = (nkb + S::KPT - 1) / S::KPT;
+        bool bad = false;
+        for (uint32_t t = 0; t < nt; t++) {
+            const int sg = t & 1;
+            const uint64_t j = 2ull * (kb0 + t * S::KPT) + col;
+            const bool live = (uint32_t)v < nvalid && j < a.m && j < 2ull * kb1;
+            // all 54 loads are issued here, in flight together and across the wait
+            // (a thread without a column reads column 0 and drops it)
+            const int8_t* zp = live ? zv + j : a.digits;
+            int z[NEO_D];
+#pragma unroll
+            for (int x = 0; x < NEO_D; x++) z[x] = ld_digit(zp + (uint64_t)x * a.m);
+            bool go = true;
+            if (lane == 0 && t >= 2) go = mbar_wait(&empty_g[sg], ((t >> 1) & 1) ^ 1);
+            const uint32_t st = warp_wait(go);
+            if (st == 1 && lane == 0) {
+                atomicOr(a.err, 0x20u);
+                s_abort = 1;
+            }
+            if (st) break;
+#pragma unroll
+            for (int x = 0; x < NEO_D; x++) z[x] = live ? z[x] : 0;
+            build_sequence<CYC>(z, reinterpret_cast<uint4*>(sG + sg * S::G_BYTES + col * S::CP + v * S::VP), bad);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full_g[sg]);
+        }
+        if (!CYC && bad) atomicOr(a.bad, 1u << 16);
+    } else {
+        // ---- B builders: WPK warps make every NB-th K block, so that NB are in
+        // the making.  Lane (sub, v, b < 8), task (column jj, half of
+        // the chunks): CPP chunks of both phases p = b + 8h, G_p = G[16c + p,
+        // 16c + p + 16), at [jj][c][h][v][b]; the phases share the words read
+        // once.  A warp's stores fill whole 128-byte rows ----
+        const int b = lane & 7, v = (lane >> 3) % NV, sub = lane / (8 * NV);
+        const uint32_t sh = 8 * (b & 3);
+        for (uint32_t it = (warp - 2) / S::WPK; it < nkb; it += S::NB) {
+            const int sb = it % S::BSTAGES;
+            const uint32_t t = it / S::KPT, kt = it % S::KPT;  // G buffer and the K block in it
+            const int sg = t % S::GSTAGES;
+            bool go = true;
+            if (lane == 0) {
+                // empty_b first: once the MMAs of K block it - BSTAGES are done, every
+                // earlier use of G buffer sg is over (GSTAGES > BSTAGES), so its phase
+                // parity cannot be mistaken for the one before the last
+                if (it >= S::BSTAGES) go = mbar_wait(&empty_b[sb], ((it / S::BSTAGES) & 1) ^ 1);
+                if (go) go = mbar_wait(&full_g[sg], (t / S::GSTAGES) & 1);
+            }
+            const uint32_t st = warp_wait(go);
             if (st == 1 && lane == 0) {
                 atomicOr(a.err, 4u);
                 s_abort = 1;
             }
             if (st) break;
-            if (active) {
-                const int sa = it % S::ASTAGES;
-                const uint32_t* src = reinterpret_cast<const uint32_t*>(sF + sa * S::F_STAGE + (v * 2 + jj) * P8_FBYTES +
-                                                                        seq * P8_HSEQ) + (b >> 2);
-                uint32_t w[23];  // bytes < 96 of the 112-byte sequence
 #pragma unroll
-                for (int q = 0; q < 23; q++) w[q] = src[q];
-                const uint32_t sh = 8 * (b & 3);
-                uint8_t* dst = sB + sb * S::B_BYTES + jj * S::BCOL + seq * (NV * 128) + v * 128 + b * 16;
+            for (int task = 0; task < S::TASKS; task++) {
+                const int tk = (task * S::WPK + (warp - 2) % S::WPK) * S::SUB + sub, jj = tk & 1, c0 = (tk >> 1) * S::CPP;
+                const uint32_t* src = reinterpret_cast<const uint32_t*>(sG + sg * S::G_BYTES + (2 * kt + jj) * S::CP +
+                                                                        v * S::VP + 16 * c0) + (b >> 2);
+                uint32_t w[4 * S::CPP + 3];
 #pragma unroll
-                for (int h = 0; h < 2; h++)
+                for (int q = 0; q < 4 * S::CPP + 3; q++) w[q] = src[q];
+                uint8_t* dst = sB + sb * S::B_BYTES + jj * S::BCOL + c0 * S::LBO + v * 128 + b * 16;
 #pragma unroll
-                    for (int c = 0; c < 5; c++) {
+                for (int c = 0; c < S::CPP; c++) {
+                    if (c0 + c >= S::NCH) break;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        if (h && c0 + c >= S::NCH - 1) break;  // the last 16-row block has its first 8 rows only
                         const int o = 4 * c + 2 * h;
-                        *reinterpret_cast<uint4*>(dst + h * (2 * NV * 128) + c * S::LBO) =
+                        *reinterpret_cast<uint4*>(dst + h * (NV * 128) + c * S::LBO) =
                             make_uint4(__funnelshift_r(w[o], w[o + 1], sh), __funnelshift_r(w[o + 1], w[o + 2], sh),
                                        __funnelshift_r(w[o + 2], w[o + 3], sh), __funnelshift_r(w[o + 3], w[o + 4], sh));
                     }
+                }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full_b[sb]);
+            if (lane == 0) {
+                mbar_arrive(&full_b[sb]);
+                mbar_arrive(&empty_g[sg]);
+            }
         }
-        // ---- epilogue (warps 2..5 cover TMEM lane groups 2, 3, 0, 1) ----
-        uint32_t okw = 0;
-        if (lane == 0) okw = (nkb > 0 && !s_abort && mbar_wait(done, 0)) ? 1u : 0u;
-        const bool ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
-        if (nkb > 0 && !ok && warp < 6) atomicOr(a.err, 8u);
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        const int lg = warp & 3;
-        const int row = lg * 32 + lane;
-        int32_t* dst = a.partial + ((uint64_t)cta * 128 + row) * S::NPAD;
-        for (int c0 = 0; c0 < (warp < 6 ? S::NPAD : 0); c0 += 16) {
-            uint32_t v16[16];
-            const uint32_t taddr = tmem + ((uint32_t)(lg * 32) << 16) + (uint32_t)c0;
+    }
+    // ---- epilogue, every warp: lane group warp & 3, every other 32 columns.  Lane
+    // (i, l) holds limb row l of output row i; three exchange steps turn 8 columns
+    // of 8 limbs into one column per lane, as L + 2^32 H with L and H the sums of
+    // its low and high four limbs (|.| < 2^56) ----
+    uint32_t okw = 0;  // lane 0 waits for the warp
+    if (lane == 0) okw = (nkb > 0 && !s_abort && mbar_wait(done, 0)) ? 1u : 0u;
+    const bool ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
+    if (nkb > 0 && !ok && lane == 0) atomicOr(a.err, 8u);
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    {
+        const int lg = warp & 3;  // TMEM lane group this warp may access
+        const uint32_t i = (uint32_t)(lg * 4 + (lane >> 3));
+        const bool u4 = lane & 4, u2 = lane & 2, u1 = lane & 1;
+        const int col8 = (u2 ? 4 : 0) + (u1 ? 2 : 0) + (u4 ? 1 : 0);  // the lane's column of each eight
+        unsigned long long* acc0 = a.acc + ((uint64_t)group * 32 + i) * S::NPAD + col8;
+        unsigned long long* acc1 = acc0 + 16 * S::NPAD;
+        constexpr uint32_t STEPS = (S::NPAD + 31) / 32;  // TMEM is allocated past the last whole 32 columns
+        for (uint32_t step = warp >> 2; step < (ok ? STEPS : 0); step += 2) {
+            // CTAs start at different columns, so that they do not all add to the same lines at once
+            const int cb = (int)((step + ks) % STEPS * 32);
+            uint32_t x[32];
+            const uint32_t taddr = tmem + ((uint32_t)(lg * 32) << 16) + (uint32_t)cb;
             asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                : "=r"(v16[0]), "=r"(v16[1]), "=r"(v16[2]), "=r"(v16[3]), "=r"(v16[4]), "=r"(v16[5]), "=r"(v16[6]),
-                  "=r"(v16[7]), "=r"(v16[8]), "=r"(v16[9]), "=r"(v16[10]), "=r"(v16[11]), "=r"(v16[12]), "=r"(v16[13]),
-                  "=r"(v16[14]), "=r"(v16[15])
+                "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+                "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+                : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]),
+                  "=r"(x[8]), "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15]),
+                  "=r"(x[16]), "=r"(x[17]), "=r"(x[18]), "=r"(x[19]), "=r"(x[20]), "=r"(x[21]), "=r"(x[22]), "=r"(x[23]),
+                  "=r"(x[24]), "=r"(x[25]), "=r"(x[26]), "=r"(x[27]), "=r"(x[28]), "=r"(x[29]), "=r"(x[30]), "=r"(x[31])
                 : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int q = 0; q < 16; q += 4)
-                *reinterpret_cast<int4*>(dst + c0 + q) =
-                    ok ? make_int4((int)v16[q], (int)v16[q + 1], (int)v16[q + 2], (int)v16[q + 3]) : make_int4(0, 0, 0, 0);
+            for (int q = 0; q < 4; q++) {
+                const uint32_t* y = x + 8 * q;
+                long long s4[4], s2[2];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {  // limbs l, l + 2
+                    const int keep = (int)(u2 ? y[c + 4] : y[c]);
+                    const int got = __shfl_xor_sync(0xffffffffu, (int)(u2 ? y[c] : y[c + 4]), 2);
+                    s4[c] = (long long)(u2 ? got : keep) + (long long)(u2 ? keep : got) * 65536;
+                }
+#pragma unroll
+                for (int c = 0; c < 2; c++) {  // limbs l, l + 1 (and l + 2, l + 3)
+                    const long long keep = u1 ? s4[c + 2] : s4[c];
+                    const long long got = __shfl_xor_sync(0xffffffffu, u1 ? s4[c] : s4[c + 2], 1);
+                    s2[c] = (u1 ? got : keep) + (u1 ? keep : got) * 256;
+                }
+                const long long keep = u4 ? s2[1] : s2[0];
+                const long long got = __shfl_xor_sync(0xffffffffu, u4 ? s2[0] : s2[1], 4);
+                const long long L = u4 ? got : keep, H = u4 ? keep : got;
+                const int g = cb / 8 + q, vv = g % NV, ah = g / NV;  // row group (a, h), vector
+                // L + 2^32 H with 2^64 = 2^32 - 1: (L_lo - H_hi) + 2^32 (L_hi + H_lo + H_hi)
+                if ((uint32_t)vv < nvalid && 8 * ah + col8 < S::OUT && i < a.kappa) {
+                    const long long hh = H >> 32;
+                    atomicAdd(acc0 + 8 * g, (unsigned long long)((L & 0xFFFFFFFFll) - hh));
+                    atomicAdd(acc1 + 8 * g, (unsigned long long)((L >> 32) + (H & 0xFFFFFFFFll) + hh));
+                }
+            }
         }
+        __threadfence();
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -735,83 +668,151 @@ __global__ void __launch_bounds__(P8<NV>::THREADS, P8<NV>::CTAS) commit_p8_kerne
         asm volatile("tcgen05.fence::after_thread_sync;");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(S::TMEM_COLS));
     }
-}
-
-// c_{v,i}[r] = sum_{ks} sum_l 2^(8l) D[ks][(i,l)][col] mod q for the column
-// col of row r (no fold: the small-digit form computes mod Phi_81 directly).
-// Block (group·kappa + i, y) sums the K splits [y n/S, (y+1) n/S) of row i
-// (its two halves take alternate splits) into int64 slice sums; the last block
-// of a row (ticket) adds the S slices and reduces mod q.  With S slices per row
-// the grid fills the GPU even for a single vector (kappa rows).
-template <int NV>
-__global__ void __launch_bounds__(2 * P8<NV>::NPAD) commit_p8_reduce_kernel(const int32_t* __restrict__ partial,
-                                                                            uint32_t n_groups, uint32_t n_ksplit,
-                                                                            uint32_t kappa, uint32_t n_vec,
-                                                                            int64_t* __restrict__ slices,
-                                                                            uint32_t* __restrict__ tickets,
-                                                                            uint64_t* __restrict__ out) {
-    constexpr int NP = P8<NV>::NPAD;
-    const uint32_t row = blockIdx.x, S = gridDim.y, y = blockIdx.y;
-    const uint32_t group = row / kappa, i = row % kappa;
-    const int col = threadIdx.x % NP, half = threadIdx.x / NP;
-    __shared__ int64_t s_acc[NP][8];
-    __shared__ bool s_last;
-    int64_t acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const uint32_t ks0 = (uint32_t)((uint64_t)y * n_ksplit / S), ks1 = (uint32_t)((uint64_t)(y + 1) * n_ksplit / S);
-    for (uint32_t ks = ks0 + half; ks < ks1; ks += 2) {
-        const int32_t* pp = partial + ((uint64_t)(ks * n_groups + group) * 128 + i * 8) * NP + col;
-#pragma unroll
-        for (int l = 0; l < 8; l++) acc[l] += pp[(uint64_t)l * NP];
-    }
-    if (half) {
-#pragma unroll
-        for (int l = 0; l < 8; l++) s_acc[col][l] = acc[l];
-    }
-    __syncthreads();
-    int64_t* mine = slices + ((uint64_t)row * S + y) * 8 * NP;
-    if (!half) {
-#pragma unroll
-        for (int l = 0; l < 8; l++) mine[l * NP + col] = acc[l] + s_acc[col][l];
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicInc(tickets + row, S - 1) == S - 1;
+    if (threadIdx.x == 0) s_last = atomicInc(a.tickets + group, a.n_ksplit - 1) == a.n_ksplit - 1;
     __syncthreads();
     if (!s_last) return;
+    // ---- the group's last CTA: outputs, then zero accumulators for the next call.
+    // 64 threads per (vector, row i), one output row each; the loads of 4 pairs
+    // are in flight together ----
     __threadfence();
-    // last block: half h adds the slices y = h, h + 2, ...
+    unsigned long long* ga = a.acc + (uint64_t)group * 32 * S::NPAD;
+    const int r = threadIdx.x & 63;
+    if (r < NEO_D) {
+        // windows of output r: the small form's one, the cyclic form's two (folded)
+        const int o1 = CYC || r >= 27 ? 80 - r : 26 - r, o2 = r >= 27 ? 53 - r : 26 - r;
+        const unsigned long long* p1 = ga + 8 * ((o1 >> 3) * NV) + (o1 & 7);
+        const unsigned long long* p2 = ga + 8 * ((o2 >> 3) * NV) + (o2 & 7);
+        const uint32_t pairs = nvalid * 16;
+        for (uint32_t e0 = threadIdx.x >> 6; e0 < pairs; e0 += 16) {
+            unsigned long long w[4][CYC ? 4 : 2];
 #pragma unroll
-    for (int l = 0; l < 8; l++) acc[l] = 0;
-    for (uint32_t yy = half; yy < S; yy += 2) {
-        const int64_t* sl = slices + ((uint64_t)row * S + yy) * 8 * NP + col;
+            for (int u = 0; u < 4; u++) {
+                const uint32_t e = min(e0 + 4 * u, pairs - 1), off = (e & 15) * S::NPAD + (e >> 4) * 8;
+                w[u][0] = __ldcg(p1 + off);
+                w[u][1] = __ldcg(p1 + off + 16 * S::NPAD);
+                if constexpr (CYC) {
+                    w[u][2] = __ldcg(p2 + off);
+                    w[u][3] = __ldcg(p2 + off + 16 * S::NPAD);
+                }
+            }
 #pragma unroll
-        for (int l = 0; l < 8; l++) acc[l] += __ldcg(sl + l * NP);
+            for (int u = 0; u < 4; u++) {
+                const uint32_t e = e0 + 4 * u, i = e & 15, v = e >> 4;
+                uint64_t c = acc_value(w[u][0], w[u][1]);
+                if constexpr (CYC) c = gl::sub(c, acc_value(w[u][2], w[u][3]));
+                else if (r < 27) c = gl::neg(c);
+                if (e < pairs && i < a.kappa) a.out[((uint64_t)(group * NV + v) * a.kappa + i) * NEO_D + r] = c;
+            }
+        }
     }
     __syncthreads();
-    if (half) {
-#pragma unroll
-        for (int l = 0; l < 8; l++) s_acc[col][l] = acc[l];
-    }
-    __syncthreads();
-    if (half) return;
-    uint64_t c = 0;
-#pragma unroll
-    for (int l = 0; l < 8; l++) c = gl::add(c, gl::mul(gl::from_i64(acc[l] + s_acc[col][l]), 1ULL << (8 * l)));
-    const int g = col >> 3, b = col & 7;
-    const int v = g % NV, seq = (g / NV) & 1, h = (g / (2 * NV)) & 1, aa = g / (4 * NV);
-    const int rp = 16 * aa + 8 * h + b;
-    const uint32_t vg = group * NV + v;
-    if (rp >= 5 && vg < n_vec) out[((uint64_t)vg * kappa + i) * NEO_D + (seq ? 31 - rp : 58 - rp)] = c;
+    for (uint32_t e = threadIdx.x; e < 16 * S::NPAD; e += S::THREADS) reinterpret_cast<ulonglong2*>(ga)[e] = make_ulonglong2(0, 0);
 }
+
+// The context's commitment workspace: accumulators and tickets that every
+// launch finds and leaves zero, and the digit-check flag.
+int commit_ws(neo_gpu_ctx* ctx, uint32_t n_groups, size_t acc_words, TcArgs* a, uint32_t** flag) {
+    if (n_groups > ctx->commit_groups || acc_words > ctx->commit_words) {
+        const uint32_t groups = std::max<uint32_t>({n_groups, ctx->commit_groups, 16});
+        const size_t words = std::max(acc_words, ctx->commit_words);
+        const size_t bytes = 256 + ((size_t)groups * 4 + 255) / 256 * 256 + words * 8;
+        const bool pooled = g_alloc_stream == ctx->stream;
+        if (ctx->commit_buf) {
+            if (pooled) {
+                cudaFreeAsync(ctx->commit_buf, ctx->stream);
+            } else {
+                cudaStreamSynchronize(ctx->stream);
+                cudaFree(ctx->commit_buf);
+            }
+            ctx->commit_buf = nullptr;
+            ctx->commit_groups = 0;
+            ctx->commit_words = 0;
+        }
+        void* p = nullptr;
+        NEO_CK(ctx, pooled ? cudaMallocAsync(&p, bytes, ctx->stream) : cudaMalloc(&p, bytes));
+        ctx->commit_buf = p;
+        NEO_CK(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
+        ctx->commit_groups = groups;
+        ctx->commit_words = words;
+    }
+    uint8_t* p = reinterpret_cast<uint8_t*>(ctx->commit_buf);
+    *flag = reinterpret_cast<uint32_t*>(p);
+    a->tickets = reinterpret_cast<uint32_t*>(p + 256);
+    a->acc = reinterpret_cast<unsigned long long*>(p + 256 + ((size_t)ctx->commit_groups * 4 + 255) / 256 * 256);
+    return NEO_OK;
+}
+
+// K blocks per CTA up to which a group of four small-digit vectors is fused: one
+// launch less, but the transposers read the digit rows 16 bytes at a time, which
+// costs more than win_seq_kernel once that hides behind enough K blocks (12
+// vectors: m = 2^14 98.6 us fused, 96.6 apart; 2^16 306 and 291).  One and two
+// vectors, and any digits, are fused at every size (1 vector at m = 2^16: 91 us
+// fused, 104 apart).
+constexpr uint32_t FUSED_KB = 64;
+
+template <int NV, bool CYC, bool FUSED>
+int launch_gemm(neo_gpu_ctx* ctx, const TcArgs& a) {
+    using S = Win<NV, CYC, FUSED>;
+    static SmemLimit limit;
+    NEO_CK(ctx, limit.at_least(commit_win_kernel<NV, CYC, FUSED>, S::DYN));
+    commit_win_kernel<NV, CYC, FUSED><<<a.n_groups * a.n_ksplit, S::THREADS, S::DYN, ctx->stream>>>(a);
+    NEO_LAUNCHED(ctx);
+    return NEO_OK;
+}
+
+template <int NV, bool CYC>
+int launch_win(neo_gpu_ctx* ctx, TcArgs a) {
+    a.n_groups = (a.n_vec + NV - 1) / NV;
+    // whole waves of 148 SMs x the CTAs one SM holds, at most TC_MAX_KB K
+    // blocks per CTA and not fewer than TC_MIN_KB: a CTA with less does not pay
+    // for its launch, its sums and its ticket
+    uint32_t n_ksplit;
+    for (uint32_t waves = 1;; waves++) {
+        n_ksplit = std::max(1u, (148 * Win<NV, CYC, true>::CTAS * waves) / a.n_groups);
+        n_ksplit = std::min(n_ksplit, (a.n_kb + TC_MIN_KB - 1) / TC_MIN_KB);
+        if ((a.n_kb + n_ksplit - 1) / n_ksplit <= TC_MAX_KB) break;
+    }
+    a.kb_per_cta = (a.n_kb + n_ksplit - 1) / n_ksplit;
+    a.n_ksplit = (a.n_kb + a.kb_per_cta - 1) / a.kb_per_cta;
+    if constexpr (NV == 4 && !CYC) {
+        if (a.kb_per_cta > FUSED_KB) {
+            void* G = nullptr;
+            NEO_CK(ctx, ctx_scratch(ctx, (size_t)a.n_groups * a.n_kb * Win<4, false, false>::G_BYTES, &G));
+            uint8_t* g = reinterpret_cast<uint8_t*>(G);
+            a.G = g;
+            const dim3 grid((a.n_kb + SEQ_COLS / 2 - 1) / (SEQ_COLS / 2), a.n_vec);
+            if (a.m % 4 == 0 && reinterpret_cast<uintptr_t>(a.digits) % 4 == 0)
+                win_seq_kernel<true><<<grid, SEQ_T, 0, ctx->stream>>>(a.digits, a.m, a.n_kb, g, a.bad);
+            else
+                win_seq_kernel<false><<<grid, SEQ_T, 0, ctx->stream>>>(a.digits, a.m, a.n_kb, g, a.bad);
+            NEO_LAUNCHED(ctx);
+            return launch_gemm<4, false, false>(ctx, a);
+        }
+    }
+    return launch_gemm<NV, CYC, true>(ctx, a);
+}
+
+// Vectors per CTA.  Small digits: 4 (N = 256) reads each A tile from shared
+// memory once per four vectors; one or two vectors alone take their own size
+// instead of padding.  Any digit: 2 (N = 192), the most that leaves TMEM and
+// shared memory for two CTAs per SM.
+int launch_small(neo_gpu_ctx* ctx, const TcArgs& a) {
+    if (a.n_vec == 1) return launch_win<1, false>(ctx, a);
+    if (a.n_vec == 2) return launch_win<2, false>(ctx, a);
+    return launch_win<4, false>(ctx, a);
+}
+int launch_any(neo_gpu_ctx* ctx, const TcArgs& a) {
+    return a.n_vec == 1 ? launch_win<1, true>(ctx, a) : launch_win<2, true>(ctx, a);
+}
+size_t acc_words(uint32_t n_vec) { return ((size_t)n_vec + 3) / 4 * 4 * 32 * 96; }  // both forms: at most 96 rows a vector
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
 int tc_pp_prepare(neo_gpu_ctx* ctx, PPEntry* pp) {
     if (pp->kappa * 8 > 128) return ctx->fail(NEO_ERR_UNSUPPORTED, "tensor-core commit: kappa <= 16");
-    if (pp->m % 2) return ctx->fail(NEO_ERR_UNSUPPORTED, "tensor-core commit: m must be even");
     pp->tc = false;
-    const uint64_t n_kb = pp->m / 2;
+    const uint64_t n_kb = (pp->m + 1) / 2;
     if (!pp->d_pp_limbs) NEO_CK(ctx, cudaMalloc(&pp->d_pp_limbs, n_kb * TC_A_BYTES));  // size depends on m only
     pp_limbs_kernel<<<(unsigned)n_kb, 256, 0, ctx->stream>>>(pp->d_pp, pp->kappa, pp->m, pp->d_pp_limbs);
     NEO_LAUNCHED(ctx);
@@ -820,124 +821,28 @@ int tc_pp_prepare(neo_gpu_ctx* ctx, PPEntry* pp) {
     return NEO_OK;
 }
 
-// Vectors per CTA: the cyclic form runs groups of 4; the small-digit form
-// runs a single vector alone (the MCS commitment: N = 64, no padding
-// vectors) and groups of 4 otherwise.
-static uint32_t tc_nv(uint32_t n_vec, bool small) { return small && n_vec == 1 ? 1 : 4; }
-
-// K-split slices per row of the small-digit reduce: about two blocks per SM
-static uint32_t p8_slices(uint32_t n_groups, uint32_t kappa, uint32_t n_ksplit) {
-    const uint32_t rows = n_groups * kappa;
-    uint32_t s = (2 * 148 + rows - 1) / rows;
-    return std::max(1u, std::min(s, n_ksplit));
-}
-
-size_t tc_scratch_bytes(uint32_t n_vec, uint64_t m, bool small, uint32_t kappa, uint32_t* n_groups_out,
-                        uint32_t* n_ksplit_out, uint32_t* kb_per_cta_out) {
-    const uint32_t nv = tc_nv(n_vec, small);
-    const uint32_t n_groups = (n_vec + nv - 1) / nv;
-    const uint32_t n_kb = (uint32_t)(m / 2);
-    // fill whole waves of 148 SMs (1 CTA per SM), at most TC_MAX_KB K blocks per CTA
-    uint32_t waves = 1, n_ksplit;
-    for (;; waves++) {
-        // n_groups * n_ksplit <= whole waves of 148 SMs x the CTAs one SM holds
-        n_ksplit = (148 * (small && nv == 4 ? P8<4>::CTAS : 1) * waves) / n_groups;
-        if (n_ksplit == 0) n_ksplit = 1;
-        if (n_ksplit > n_kb) n_ksplit = n_kb;
-        if ((n_kb + n_ksplit - 1) / n_ksplit <= TC_MAX_KB) break;
-    }
-    const uint32_t kb_per_cta = (n_kb + n_ksplit - 1) / n_ksplit;
-    n_ksplit = (n_kb + kb_per_cta - 1) / kb_per_cta;
-    *n_groups_out = n_groups;
-    *n_ksplit_out = n_ksplit;
-    *kb_per_cta_out = kb_per_cta;
-    const size_t fb = small ? P8_FBYTES : TC_FBYTES, npad = small ? 64 * nv : TC_NPAD;
-    size_t f_bytes = (size_t)n_vec * m * fb + 64;
-    size_t p_bytes = (size_t)n_groups * n_ksplit * 128 * npad * 4;
-    // small form: the reduce's int64 slice sums and one ticket per row
-    size_t r_bytes = small ? (size_t)n_groups * kappa * p8_slices(n_groups, kappa, n_ksplit) * 8 * npad * 8 +
-                                 (((size_t)n_groups * kappa * 4 + 255) & ~size_t(255))
-                           : 0;
-    return ((f_bytes + 255) & ~size_t(255)) + p_bytes + r_bytes + 256 /*flag*/ + 256;
-}
-
-template <int NV>
-static int launch_p8(neo_gpu_ctx* ctx, const TcArgs& a, uint32_t kappa, uint8_t* red, uint64_t* d_out) {
-    using S = P8<NV>;
-    const size_t smem = S::SMEM + 1024 /*align*/ + 256 /*barriers*/;
-    static SmemLimit limit;
-    NEO_CK(ctx, limit.at_least(commit_p8_kernel<NV>, smem));
-    const uint32_t rows = a.n_groups * kappa, ns = p8_slices(a.n_groups, kappa, a.n_ksplit);
-    int64_t* slices = reinterpret_cast<int64_t*>(red);
-    uint32_t* tickets = reinterpret_cast<uint32_t*>(red + (size_t)rows * ns * 8 * S::NPAD * 8);
-    NEO_CK(ctx, cudaMemsetAsync(tickets, 0, (size_t)rows * 4, ctx->stream));
-    commit_p8_kernel<NV><<<a.n_groups * a.n_ksplit, S::THREADS, smem, ctx->stream>>>(a);
-    NEO_LAUNCHED(ctx);
-    commit_p8_reduce_kernel<NV><<<dim3(rows, ns), 2 * S::NPAD, 0, ctx->stream>>>(
-        a.partial, a.n_groups, a.n_ksplit, kappa, a.n_vec, slices, tickets, d_out);
-    NEO_LAUNCHED(ctx);
-    return NEO_OK;
-}
-
 int launch_commit_tc(neo_gpu_ctx* ctx, const PPEntry* pp, const int8_t* d_digits, uint32_t n_vec, uint64_t* d_out,
-                     uint8_t* scratch, uint32_t* d_err, int digits) {
-    const uint64_t m = pp->m;
-    TcArgs a;
+                     int digits) {
+    TcArgs a{};
     a.ppl = pp->d_pp_limbs;
-    a.err = d_err;
-    a.m = m;
+    a.digits = d_digits;
+    a.out = d_out;
+    a.err = ctx->d_err;
+    a.m = pp->m;
     a.n_vec = n_vec;
-    a.n_kb = (uint32_t)(m / 2);
-    if (digits != TC_DIGITS_ANY) {
-        // small-digit form; for digits of unknown size the window sequences are
-        // built first and checked (one synchronisation), falling back to the
-        // cyclic form when an entry leaves int8
-        uint32_t n_groups, n_ksplit, kb_per_cta;
-        const size_t need = tc_scratch_bytes(n_vec, m, true, pp->kappa, &n_groups, &n_ksplit, &kb_per_cta);
-        uint8_t* F = scratch;
-        const size_t f_end = ((size_t)n_vec * m * P8_FBYTES + 64 + 255) & ~size_t(255);
-        uint32_t* flag = reinterpret_cast<uint32_t*>(scratch + need - 512);
-        const bool known = digits == TC_DIGITS_SMALL;
-        if (!known) NEO_CK(ctx, cudaMemsetAsync(flag, 0, 4, ctx->stream));
-        p8_seq_kernel<<<ceil_div((uint64_t)n_vec * m, P8_SEQ_THREADS), P8_SEQ_THREADS, 0, ctx->stream>>>(
-            d_digits, n_vec, m, F, known ? d_err : flag);
-        NEO_LAUNCHED(ctx);
-        bool ok = true;
-        if (!known) {
-            uint32_t h_flag = 0;
-            NEO_CK(ctx, ctx_d2h(ctx, &h_flag, flag, 4));
-            NEO_CK(ctx, ctx_sync(ctx));
-            ok = h_flag == 0;
-        }
-        if (ok) {
-            a.F = F;
-            a.partial = reinterpret_cast<int32_t*>(scratch + f_end);
-            a.n_groups = n_groups;
-            a.n_ksplit = n_ksplit;
-            a.kb_per_cta = kb_per_cta;
-            uint8_t* red = scratch + f_end + (size_t)n_groups * n_ksplit * 128 * 64 * tc_nv(n_vec, true) * 4;
-            return tc_nv(n_vec, true) == 1 ? launch_p8<1>(ctx, a, pp->kappa, red, d_out)
-                                           : launch_p8<4>(ctx, a, pp->kappa, red, d_out);
-        }
-    }
-    uint32_t n_groups, n_ksplit, kb_per_cta;
-    tc_scratch_bytes(n_vec, m, false, pp->kappa, &n_groups, &n_ksplit, &kb_per_cta);
-    uint8_t* F = scratch;
-    int32_t* partial = reinterpret_cast<int32_t*>(scratch + (((size_t)n_vec * m * TC_FBYTES + 64 + 255) & ~size_t(255)));
-    f_seq_kernel<<<ceil_div((uint64_t)n_vec * m, 128), 128, 0, ctx->stream>>>(d_digits, n_vec, m, F);
-    NEO_LAUNCHED(ctx);
-    a.F = F;
-    a.partial = partial;
-    a.n_groups = n_groups;
-    a.n_ksplit = n_ksplit;
-    a.kb_per_cta = kb_per_cta;
-    const size_t smem = TC_SMEM_BYTES + 1024 /*align*/ + 256 /*barriers*/;
-    static SmemLimit limit;
-    NEO_CK(ctx, limit.at_least(commit_tc_kernel, smem));
-    commit_tc_kernel<<<n_groups * n_ksplit, TC_THREADS, smem, ctx->stream>>>(a);
-    NEO_LAUNCHED(ctx);
-    commit_tc_reduce_kernel<<<n_groups * pp->kappa, RED_THREADS, 0, ctx->stream>>>(partial, n_groups, n_ksplit,
-                                                                                     pp->kappa, n_vec, d_out);
-    NEO_LAUNCHED(ctx);
-    return NEO_OK;
+    a.kappa = pp->kappa;
+    a.n_kb = (uint32_t)((pp->m + 1) / 2);
+    uint32_t* flag = nullptr;
+    if (int rc = commit_ws(ctx, (n_vec + (n_vec > 1)) / (n_vec > 1 ? 2 : 1), acc_words(n_vec), &a, &flag)) return rc;
+    if (digits == TC_DIGITS_ANY) return launch_any(ctx, a);
+    // the caller's promise covers an even m, and a broken one is reported; else
+    // a digit that leaves the small form's range has the second launch redo the
+    // commitment in the general form (it ends at once when there was none)
+    const bool promised = digits == TC_DIGITS_SMALL && pp->m % 2 == 0;
+    a.bad = promised ? ctx->d_err : flag;
+    if (!promised) NEO_CK(ctx, cudaMemsetAsync(flag, 0, 4, ctx->stream));
+    if (int rc = launch_small(ctx, a)) return rc;
+    if (promised) return NEO_OK;
+    a.only_if = flag;
+    return launch_any(ctx, a);
 }

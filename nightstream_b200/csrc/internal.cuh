@@ -23,6 +23,10 @@ struct neo_gpu_ctx {
     uint32_t* d_err = nullptr;       // device error word (bounded-wait timeouts); 0 = ok
     void* scratch = nullptr;         // growable per-context scratch (stream-ordered use)
     size_t scratch_bytes = 0;
+    // tensor-core commitment workspace (commit_tc.cu): accumulators and tickets, zero between calls
+    void* commit_buf = nullptr;
+    uint32_t commit_groups = 0;
+    size_t commit_words = 0;
     // the last chi table a memory oracle built (the time-lane oracles of a
     // step share their point): key = ell then the point's words
     void* chi_cache = nullptr;
@@ -73,7 +77,7 @@ struct PPEntry {
     uint64_t m = 0;
     uint32_t kappa = 0;
     uint64_t* d_pp = nullptr;       // [kappa][m][54] canonical u64
-    uint8_t* d_pp_limbs = nullptr;  // tensor-core tiles: [m/2][128 rows][128 B], pre-swizzled
+    uint8_t* d_pp_limbs = nullptr;  // tensor-core tiles: [ceil(m/2)][128 rows][128 B], pre-swizzled
     bool tc = false;                // d_pp_limbs holds the tiles of the current d_pp
 };
 PPEntry* pp_lookup(int device, uint64_t m);
@@ -205,16 +209,14 @@ int launch_zrows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t R, uint64_t m, ui
 // What the caller knows about the digits of a commitment: any int8
 // (TC_DIGITS_ANY: the cyclic tensor-core form), |digit| <= 63 by construction
 // (TC_DIGITS_SMALL: the small-digit form, a violation is reported through the
-// device error word), or nothing (TC_DIGITS_CHECK: the small-digit form after
-// one device check, else the cyclic form).
+// device error word), or nothing (TC_DIGITS_CHECK: the small-digit form, redone in
+// the cyclic form on the device when a digit turned out too large).
 enum { TC_DIGITS_ANY = 0, TC_DIGITS_SMALL = 1, TC_DIGITS_CHECK = 2 };
 int launch_commit(neo_gpu_ctx* ctx, const int8_t* d_digits, uint32_t n_vec, uint64_t m, uint64_t* d_out,
                   int digits = TC_DIGITS_CHECK);
 int tc_pp_prepare(neo_gpu_ctx* ctx, PPEntry* pp);
-size_t tc_scratch_bytes(uint32_t n_vec, uint64_t m, bool small, uint32_t kappa, uint32_t* n_groups,
-                        uint32_t* n_ksplit, uint32_t* kb_per_cta);
 int launch_commit_tc(neo_gpu_ctx* ctx, const PPEntry* pp, const int8_t* d_digits, uint32_t n_vec, uint64_t* d_out,
-                     uint8_t* scratch, uint32_t* d_err, int digits);
+                     int digits);
 // reads and clears the device error word (synchronizes the stream)
 int check_device_error(neo_gpu_ctx* ctx);
 
