@@ -1119,17 +1119,24 @@ extern "C" int neo_gpu_addr_lookup_weights(neo_gpu_ctx* ctx, uint32_t ell, const
 // TwistWriteCheckAddrOracleSparseTime, twist_oracle.rs:1259-1642).
 //
 // The reference replays a HashMap memory over the time-ordered events every
-// round.  Here the events are compacted once into arrays; the memory value a
-// query event i sees at address block idx is
-//     init_tab[idx] + Σ_{j < i, wa_j >> bit = idx} inc_j·hw_j·wpw_j,
-// where init_tab is the initial memory folded on its low address bits (the
-// reference's init prefix weights are exactly that fold).  One thread per
-// query event sums the earlier writes from shared-memory tiles.  Degree 2:
-// values at x = 0, 1, 2 are reduced and interpolated on the host.
+// round.  Here the reads and writes are items in time order, and the memory
+// value a query item i sees at address block idx of round `bit` is
+//     init_tab[idx] + Σ_{j < i, addr_j >> bit = idx} d_j,
+// d_j = inc_j·hw_j·(address weight of the bound bits), init_tab the initial
+// memory folded on its low address bits (the reference's init prefix weights
+// are exactly that fold).  The items are kept sorted by (addr >> (bit + 1),
+// time): the two blocks a query interpolates between are then one run, and the
+// sums over its earlier writes are two prefix sums within the run.  A stable
+// radix sort makes the order of round 0; a fold merges each pair of sibling
+// runs by time.  Degree 2: values at x = 0, 1, 2, interpolated on the host.
+// (One thread per query summing every earlier write of its block took 653 us a
+// round at 2^14 events, each a read and a write, and 12.6 us at 2^10; now
+// 12.5 and 11.)
 // ===========================================================================
 namespace {
 
-constexpr int TA_T = 64;
+constexpr int TA_T = 64;     // build blocks
+constexpr int TE_T = 256;    // items per evaluation block
 
 __device__ __forceinline__ uint32_t addr_bits_at(const K* bits, uint64_t L, uint32_t A, uint64_t t) {
     uint32_t a = 0;
@@ -1140,16 +1147,21 @@ __device__ __forceinline__ uint32_t addr_bits_at(const K* bits, uint64_t L, uint
     return a;
 }
 
-// event flags: read kind: has_read | has_write nonzero; write kind: has_write nonzero
+// An item's sort key: write flag (read kind only) : address (30 bits) : item index (time order).
+__device__ __forceinline__ uint64_t ta_key(uint32_t write, uint32_t addr, uint32_t idx) {
+    return ((uint64_t)write << 63) | ((uint64_t)addr << 32) | idx;
+}
+__device__ __forceinline__ uint32_t ta_addr(uint64_t key) { return (uint32_t)(key >> 32) & 0x7FFFFFFFu; }
+
+// items per build block: kind 0 one for has_read != 0 and one for has_write != 0, kind 1 one for has_write != 0
 __global__ void ta_count_kernel(const K* __restrict__ hr, const K* __restrict__ hw, uint64_t L, uint32_t* __restrict__ counts) {
     __shared__ uint32_t s_cnt;
     if (threadIdx.x == 0) s_cnt = 0;
     __syncthreads();
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    bool f = false;
-    if (t < L) f = !gl::kiszero(hw[t]) || (hr && !gl::kiszero(hr[t]));
-    unsigned bal = __ballot_sync(0xffffffffu, f);
-    if ((threadIdx.x & 31) == 0 && bal) atomicAdd(&s_cnt, (uint32_t)__popc(bal));
+    const bool w = t < L && !gl::kiszero(hw[t]), r = t < L && hr && !gl::kiszero(hr[t]);
+    const int n = __popc(__ballot_sync(0xffffffffu, w)) + __popc(__ballot_sync(0xffffffffu, r));
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&s_cnt, (uint32_t)n);
     __syncthreads();
     if (threadIdx.x == 0) counts[blockIdx.x] = s_cnt;
 }
@@ -1160,174 +1172,374 @@ struct TaBuild {
     uint32_t ell, A;
     uint64_t L;
     const uint32_t* offs;   // exclusive prefix of the per-block counts
-    // outputs [E]
-    K *eq, *ehr, *erv, *ehw, *einc, *ewv;
-    uint32_t *era, *ewa;
+    // outputs [N]
+    uint64_t* key;
+    K *wt;                  // query weight χ·has (kind 0: reads; kind 1) or write delta inc·has_write (kind 0: writes)
+    K *kc;                  // a query's constant: rv, or wv − inc
+    K *d;                   // kind 1: write delta
 };
 
 __global__ void ta_build_kernel(const TaBuild a) {
     __shared__ uint32_t s_warp[TA_T / 32];
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    bool f = false;
-    if (t < a.L) f = !gl::kiszero(a.hw[t]) || (a.hr && !gl::kiszero(a.hr[t]));
+    const K hw = t < a.L ? a.hw[t] : gl::kzero(), hr = t < a.L && a.hr ? a.hr[t] : gl::kzero();
+    const bool w = !gl::kiszero(hw), r = !gl::kiszero(hr);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned bal = __ballot_sync(0xffffffffu, f);
-    if (lane == 0) s_warp[warp] = __popc(bal);
+    const unsigned bw = __ballot_sync(0xffffffffu, w), br = __ballot_sync(0xffffffffu, r);
+    if (lane == 0) s_warp[warp] = __popc(bw) + __popc(br);
     __syncthreads();
-    uint32_t before = 0;
-    for (int w = 0; w < warp; w++) before += s_warp[w];
-    before += __popc(bal & ((1u << lane) - 1));
-    if (!f) return;
-    const uint32_t e = a.offs[blockIdx.x] + before;
+    if (!w && !r) return;
+    uint32_t n = a.offs[blockIdx.x];
+    for (int i = 0; i < warp; i++) n += s_warp[i];
+    const unsigned lt = (1u << lane) - 1;
+    n += __popc(bw & lt) + __popc(br & lt);
     // χ_{r_cycle}(t)
     K chi = gl::kone();
-    for (uint32_t i = 0; i < a.ell; i++) {
-        K ri = a.r_cycle[i];
-        chi = gl::kmul(chi, ((t >> i) & 1) ? ri : gl::ksub(gl::kone(), ri));
+    if (r || !a.hr)
+        for (uint32_t i = 0; i < a.ell; i++) {
+            K ri = a.r_cycle[i];
+            chi = gl::kmul(chi, ((t >> i) & 1) ? ri : gl::ksub(gl::kone(), ri));
+        }
+    const K delta = w ? gl::kmul(a.inc[t], hw) : gl::kzero();
+    if (!a.hr) {
+        a.key[n] = ta_key(0, addr_bits_at(a.wa, a.L, a.A, t), n);
+        a.wt[n] = gl::kmul(chi, hw);
+        a.kc[n] = gl::ksub(a.wv[t], a.inc[t]);
+        a.d[n] = delta;
+        return;
     }
-    a.eq[e] = chi;
-    K hw = a.hw[t];
-    a.ehw[e] = hw;
-    a.einc[e] = a.inc[t];
-    const bool has_w = !gl::kiszero(hw);
-    if (a.hr) {
-        K hr = a.hr[t];
-        a.ehr[e] = hr;
-        a.erv[e] = a.rv[t];
-        a.era[e] = gl::kiszero(hr) ? 0u : addr_bits_at(a.ra, a.L, a.A, t);
-        a.ewa[e] = has_w ? addr_bits_at(a.wa, a.L, a.A, t) : 0u;
-    } else {
-        a.ewv[e] = a.wv[t];
-        a.ewa[e] = addr_bits_at(a.wa, a.L, a.A, t);
+    if (r) {  // a step's read comes before its write
+        a.key[n] = ta_key(0, addr_bits_at(a.ra, a.L, a.A, t), n);
+        a.wt[n] = gl::kmul(chi, hr);
+        a.kc[n] = a.rv[t];
+        n++;
+    }
+    if (w) {
+        a.key[n] = ta_key(1, addr_bits_at(a.wa, a.L, a.A, t), n);
+        a.wt[n] = delta;
     }
 }
 
-// one round of the address lane: a block (query block x, event block y) adds
-// the earlier writes of event block y to its queries' memory values
-struct TaEval {
-    int kind;  // 0 read, 1 write
-    uint32_t E, bit;
-    const K *eq, *hr, *rv, *hw, *inc, *wv, *rpw, *wpw;
-    const uint32_t *ra, *wa;
-    const K* init_tab;  // folded initial memory, >= 2 entries
-    K* partials;        // [3][gridDim.x * gridDim.y]
-    K* out;             // the round's values at x = 0, 1, 2 (the last block sums the partials)
-    unsigned int* ticket;
-};
+// ---- stable radix sort of the items by 8 address bits (least significant first) ----
+constexpr int RS_T = 256, RS_PER = 8, RS_TILE = RS_T * RS_PER;
 
-// grid.x: query events i in tiles of TA_T; grid.y: earlier-event chunks j of
-// TA_T.  The contribution is linear in the memory value, so each chunk adds
-// w·af(x)·(±its partial memory value) and chunk 0 adds the initial memory and
-// the constant terms; the reduction sums all blocks.
-__global__ void __launch_bounds__(TA_T) ta_eval_kernel(const TaEval a) {
-    __shared__ uint32_t s_key[TA_T];
-    __shared__ K s_d[TA_T];
-    __shared__ K s_red[3][TA_T / 32];
-    const uint32_t i = blockIdx.x * TA_T + threadIdx.x;
-    const uint32_t i_end = min(a.E, blockIdx.x * TA_T + TA_T);
-    const uint32_t j0 = blockIdx.y * TA_T;
-    bool q = false;
-    uint32_t addr = 0;
-    if (i < a.E) {
-        if (a.kind == 0) { q = !gl::kiszero(a.hr[i]); addr = a.ra[i]; }
-        else { q = !gl::kiszero(a.hw[i]); addr = a.wa[i]; }
+__global__ void __launch_bounds__(RS_T) rs_hist_kernel(const uint64_t* __restrict__ key, uint32_t N, int shift,
+                                                       uint32_t n_tiles, uint32_t* __restrict__ hist) {
+    __shared__ uint32_t s_h[256];
+    s_h[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t base = blockIdx.x * RS_TILE;
+#pragma unroll
+    for (int i = 0; i < RS_PER; i++) {
+        const uint32_t p = base + i * RS_T + threadIdx.x;
+        if (p < N) atomicAdd(&s_h[(ta_addr(key[p]) >> shift) & 255], 1u);
     }
-    const uint32_t base = a.bit >= 31 ? 0u : ((addr >> (a.bit + 1)) << 1);
-    K v0 = gl::kzero(), v1 = gl::kzero();
-    if (q && blockIdx.y == 0) {
-        v0 = a.init_tab[base];
-        v1 = a.init_tab[base + 1];
-    }
-    bool any = blockIdx.y == 0;
-    if (j0 < i_end) {  // block-uniform: some query of this block has earlier events in the chunk
-        const uint32_t j = j0 + threadIdx.x;
-        if (j < a.E) {
-            // the write event's key (its address block at this bit) and delta
-            // inc * has_write * address weight; no write: a key nothing matches
-            const K h = a.hw[j];
-            const bool w = !gl::kiszero(h);
-            s_key[threadIdx.x] = !w ? 0xFFFFFFFFu : (a.bit >= 32 ? 0u : (a.wa[j] >> a.bit));
-            s_d[threadIdx.x] = w ? gl::kmul(gl::kmul(a.inc[j], h), a.wpw[j]) : gl::kzero();
+    __syncthreads();
+    hist[(uint64_t)threadIdx.x * n_tiles + blockIdx.x] = s_h[threadIdx.x];
+}
+
+// exclusive scan of n counters, in place, one block
+__global__ void __launch_bounds__(1024) rs_scan_kernel(uint32_t* __restrict__ h, uint64_t n) {
+    __shared__ uint32_t s_w[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint64_t base = 0; base < n; base += 4096) {
+        const uint64_t i0 = base + 4 * (uint64_t)threadIdx.x;
+        uint32_t v[4], s = 0;
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            v[e] = i0 + e < n ? h[i0 + e] : 0;
+            s += v[e];
+        }
+        uint32_t inc = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (lane == 31) s_w[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t x = s_w[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += u;
+            }
+            s_w[lane] = x;  // inclusive
         }
         __syncthreads();
-        if (q && i > j0) {
-            const uint32_t jn = i - j0 < TA_T ? i - j0 : TA_T;
-            any = true;
-            for (uint32_t u = 0; u < jn; u++) {
-                const uint32_t k = s_key[u];
-                if (k == base) v0 = gl::kadd(v0, s_d[u]);
-                else if (k == base + 1) v1 = gl::kadd(v1, s_d[u]);
-            }
-        }
-    }
-    K c[3] = {gl::kzero(), gl::kzero(), gl::kzero()};
-    if (q && any) {
-        const bool b = a.bit < 32 && ((addr >> a.bit) & 1);
-        K w = a.kind == 0 ? gl::kmul(gl::kmul(a.eq[i], a.hr[i]), a.rpw[i]) : gl::kmul(gl::kmul(a.eq[i], a.hw[i]), a.wpw[i]);
-        K dv = gl::ksub(v1, v0);
-        K vx = v0;
+        uint32_t run = carry + (warp ? s_w[warp - 1] : 0) + inc - s;
 #pragma unroll
-        for (int x = 0; x < 3; x++) {
-            K af = b ? gl::kfq((uint64_t)x) : gl::kfq(gl::sub(1, (uint64_t)x));
-            K term;
-            if (blockIdx.y == 0) term = a.kind == 0 ? gl::ksub(vx, a.rv[i]) : gl::ksub(gl::ksub(a.wv[i], vx), a.inc[i]);
-            else term = a.kind == 0 ? vx : gl::kneg(vx);
-            c[x] = gl::kmul(gl::kmul(w, af), term);
-            vx = gl::kadd(vx, dv);
+        for (int e = 0; e < 4; e++) {
+            if (i0 + e < n) h[i0 + e] = run;
+            run += v[e];
         }
+        carry += s_w[31];
+        __syncthreads();
     }
+}
+
+// A warp owns RS_PER * 32 consecutive items and walks them in order, so equal
+// digits keep their order: rank among the warp's earlier items of the digit.
+__global__ void __launch_bounds__(RS_T) rs_scatter_kernel(const uint64_t* __restrict__ key, uint32_t N, int shift,
+                                                          uint32_t n_tiles, const uint32_t* __restrict__ offs,
+                                                          uint64_t* __restrict__ out) {
+    __shared__ uint32_t s_cnt[RS_T / 32][256];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int x = 0; x < 3; x++) {
-        K v = c[x];
+    for (int w = 0; w < RS_T / 32; w++) s_cnt[w][threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t base = blockIdx.x * RS_TILE + warp * (RS_PER * 32);
+    uint64_t k[RS_PER];
+    uint32_t rank[RS_PER];
+#pragma unroll
+    for (int i = 0; i < RS_PER; i++) {
+        const uint32_t p = base + i * 32 + lane;
+        k[i] = p < N ? key[p] : 0;
+        const uint32_t d = p < N ? (ta_addr(k[i]) >> shift) & 255 : 256;  // past the end: a digit of its own
+        const unsigned same = __match_any_sync(0xffffffffu, d);
+        const uint32_t before = d < 256 ? s_cnt[warp][d] : 0;
+        rank[i] = before + __popc(same & ((1u << lane) - 1));
+        __syncwarp();
+        if (d < 256 && lane == __ffs(same) - 1) s_cnt[warp][d] = before + __popc(same);
+        __syncwarp();
+    }
+    __syncthreads();
+    {   // first slot of (warp, digit): thread = digit
+        uint32_t run = offs[(uint64_t)threadIdx.x * n_tiles + blockIdx.x];
+#pragma unroll
+        for (int w = 0; w < RS_T / 32; w++) {
+            const uint32_t c = s_cnt[w][threadIdx.x];
+            s_cnt[w][threadIdx.x] = run;
+            run += c;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RS_PER; i++) {
+        const uint32_t p = base + i * 32 + lane;
+        if (p < N) out[s_cnt[warp][(ta_addr(k[i]) >> shift) & 255] + rank[i]] = k[i];
+    }
+}
+
+// ---- one round ----
+struct TaEval {
+    int kind;  // 0 read, 1 write
+    uint32_t N, bit;
+    const uint64_t* key;    // sorted by (addr >> (bit + 1), item)
+    const K *wt, *kc, *d;
+    const K* init_tab;      // folded initial memory, >= 2 entries
+    K* recs;                // [gridDim.x][TA_REC]
+    uint32_t* heads;        // [gridDim.x] 1: a run starts inside the block
+    K* out;                 // the round's values at x = 0, 1, 2
+    unsigned int* ticket;
+};
+constexpr int TA_REC = 8;   // S0..S2, U0..U2, T0, T1
+
+// Blocks of TE_T sorted items.  A query's contribution at x = 0, 1, 2 is w times
+//   child 0:  v0 − k,  0,  −(2 v1 − v0 − k);   child 1:  0,  v1 − k,  2 (2 v1 − v0 − k)
+// (negated for the write check), with v0, v1 the initial values plus the prefix
+// sums of its run.  For a run that began in an earlier block the block leaves the
+// factors U of the two sums carried in (S0 += U0 c0, S1 += U1 c1, S2 += U2 (2 c1
+// − c0)) and its own last run's sums T; the last block to finish (ticket, no
+// waits) scans the carries over the blocks and adds everything up.
+__global__ void __launch_bounds__(TE_T) ta_eval_kernel(const TaEval a) {
+    __shared__ K s_e[2][TE_T];              // exclusive prefix sums over the block (children 0, 1)
+    __shared__ K s_w[2][TE_T / 32];
+    __shared__ int s_h[TE_T / 32];
+    __shared__ K s_red[TE_T / 32][6];
+    __shared__ bool s_last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t p = blockIdx.x * TE_T + tid;
+    const bool live = p < a.N;
+    const uint64_t key = live ? a.key[p] : ~0ull;
+    const uint32_t addr = ta_addr(key), idx = (uint32_t)key, seg = addr >> (a.bit + 1);
+    const int child = (addr >> a.bit) & 1;
+    bool head = p == 0;
+    if (live && p) head = (ta_addr(a.key[p - 1]) >> (a.bit + 1)) != seg;
+    const bool is_q = live && (a.kind == 1 || !(key >> 63)), is_w = live && (a.kind == 1 || (key >> 63));
+    const K w = live ? a.wt[idx] : gl::kzero();
+    const K dl = !is_w ? gl::kzero() : a.kind == 1 ? a.d[idx] : w;
+    K kc = gl::kzero(), i0 = gl::kzero(), i1 = gl::kzero();
+    if (is_q) {
+        kc = a.kc[idx];
+        i0 = a.init_tab[2 * (uint64_t)seg];
+        i1 = a.init_tab[2 * (uint64_t)seg + 1];
+    }
+    // inclusive scans of the two children's deltas and of the last head's position
+    K x0 = child ? gl::kzero() : dl, x1 = child ? dl : gl::kzero();
+    const K own0 = x0, own1 = x1;
+    int h = live && head ? tid : -1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        K n0, n1;
+        n0.re = __shfl_up_sync(0xffffffffu, x0.re, o); n0.im = __shfl_up_sync(0xffffffffu, x0.im, o);
+        n1.re = __shfl_up_sync(0xffffffffu, x1.re, o); n1.im = __shfl_up_sync(0xffffffffu, x1.im, o);
+        const int hh = __shfl_up_sync(0xffffffffu, h, o);
+        if (lane >= o) {
+            x0 = gl::kadd(x0, n0);
+            x1 = gl::kadd(x1, n1);
+            h = max(h, hh);
+        }
+    }
+    if (lane == 31) { s_w[0][warp] = x0; s_w[1][warp] = x1; s_h[warp] = h; }
+    __syncthreads();
+    K b0 = gl::kzero(), b1 = gl::kzero(), t0 = gl::kzero(), t1 = gl::kzero();  // before this warp; the block's total
+    int last_head = -1;
+#pragma unroll 1
+    for (int i = 0; i < TE_T / 32; i++) {
+        if (i == warp) { b0 = t0; b1 = t1; h = max(h, last_head); }
+        t0 = gl::kadd(t0, s_w[0][i]);
+        t1 = gl::kadd(t1, s_w[1][i]);
+        last_head = max(last_head, s_h[i]);
+    }
+    const K e0 = gl::kadd(b0, gl::ksub(x0, own0)), e1 = gl::kadd(b1, gl::ksub(x1, own1));
+    s_e[0][tid] = e0;
+    s_e[1][tid] = e1;
+    __syncthreads();
+    const bool open = h < 0;
+    K c[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) c[i] = gl::kzero();
+    if (is_q) {
+        const K v0 = gl::kadd(i0, open ? e0 : gl::ksub(e0, s_e[0][h])), v1 = gl::kadd(i1, open ? e1 : gl::ksub(e1, s_e[1][h]));
+        const K w2 = child ? gl::kdbl(w) : gl::kneg(w);
+        const K near = gl::kmul(w, gl::ksub(child ? v1 : v0, kc));
+        c[0] = child ? gl::kzero() : near;
+        c[1] = child ? near : gl::kzero();
+        c[2] = gl::kmul(w2, gl::ksub(gl::ksub(gl::kdbl(v1), v0), kc));
+        if (open) {
+            c[3] = child ? gl::kzero() : w;
+            c[4] = child ? w : gl::kzero();
+            c[5] = w2;
+        }
+    }
+    const bool any_open = __syncthreads_or(is_q && open);
+    const int nc = any_open ? 6 : 3;
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        if (i >= nc) break;
+        K v = c[i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = gl::kadd(v, shfl_xor_km(v, o));
-        if (lane == 0) s_red[x][warp] = v;
+        if (lane == 0) s_red[warp][i] = v;
     }
     __syncthreads();
-    const uint64_t nb = (uint64_t)gridDim.x * gridDim.y;
-    if (threadIdx.x < 3) {
-        K s = gl::kzero();
-        for (int w = 0; w < TA_T / 32; w++) s = gl::kadd(s, s_red[threadIdx.x][w]);
-        a.partials[(uint64_t)threadIdx.x * nb + (uint64_t)blockIdx.y * gridDim.x + blockIdx.x] = s;
+    K* rec = a.recs + (uint64_t)blockIdx.x * TA_REC;
+    if (tid < 6) {
+        K v = gl::kzero();
+        if (tid < nc)
+            for (int i = 0; i < TE_T / 32; i++) v = gl::kadd(v, s_red[i][tid]);
+        rec[tid] = v;
+    } else if (tid < 8) {
+        const int ch = tid - 6;
+        const K tot = ch ? t1 : t0;
+        rec[tid] = last_head < 0 ? tot : gl::ksub(tot, s_e[ch][last_head]);
+    } else if (tid == 8) {
+        a.heads[blockIdx.x] = last_head >= 0;
     }
-    // the last block to finish sums the partials (ticket, no waits)
     __threadfence();
     __syncthreads();
-    __shared__ unsigned int s_last;
-    if (threadIdx.x == 0) s_last = atomicInc(a.ticket, (unsigned int)(nb - 1)) == nb - 1;
+    if (tid == 0) s_last = atomicInc(a.ticket, gridDim.x - 1) == gridDim.x - 1;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // the points x < 3 split over the block's warps, side by side
-    for (int x = warp; x < 3; x += TA_T / 32) {
-        K v = gl::kzero();
-#pragma unroll 4
-        for (uint64_t b = lane; b < nb; b += 32) {
-            const ulonglong2 u = __ldcg(reinterpret_cast<const ulonglong2*>(a.partials + (uint64_t)x * nb + b));
-            v = gl::kadd(v, gl::kmk(u.x, u.y));
+    // carries: inclusive segmented scan of (T0, T1, head) over the blocks, TE_T at a time
+    auto ldk = [](const K* q) {
+        const ulonglong2 u = __ldcg(reinterpret_cast<const ulonglong2*>(q));
+        return gl::kmk(u.x, u.y);
+    };
+    K sum[3] = {gl::kzero(), gl::kzero(), gl::kzero()};
+    K in0 = gl::kzero(), in1 = gl::kzero();  // carried into this batch of blocks
+    __shared__ K s_c[2][TE_T];
+    __shared__ uint32_t s_f[TE_T];
+    for (uint32_t base = 0; base < gridDim.x; base += TE_T) {
+        const uint32_t blk = base + tid;
+        const bool on = blk < gridDim.x;
+        const K* r = a.recs + (uint64_t)(on ? blk : 0) * TA_REC;
+        K y0 = on ? ldk(r + 6) : gl::kzero(), y1 = on ? ldk(r + 7) : gl::kzero();
+        uint32_t f = on ? __ldcg(a.heads + blk) : 0;
+        if (tid == 0 && !f) { y0 = gl::kadd(y0, in0); y1 = gl::kadd(y1, in1); }
+        const uint32_t live_n = min((uint32_t)TE_T, gridDim.x - base);
+        for (uint32_t o = 1; o < live_n; o <<= 1) {
+            s_c[0][tid] = y0; s_c[1][tid] = y1; s_f[tid] = f;
+            __syncthreads();
+            if ((uint32_t)tid >= o && !f) {
+                y0 = gl::kadd(y0, s_c[0][tid - o]);
+                y1 = gl::kadd(y1, s_c[1][tid - o]);
+                f = s_f[tid - o];
+            }
+            __syncthreads();
         }
+        s_c[0][tid] = y0; s_c[1][tid] = y1;
+        __syncthreads();
+        const K c0 = tid ? s_c[0][tid - 1] : in0, c1 = tid ? s_c[1][tid - 1] : in1;
+        if (on) {
+            sum[0] = gl::kadd(sum[0], gl::kadd(ldk(r), gl::kmul(ldk(r + 3), c0)));
+            sum[1] = gl::kadd(sum[1], gl::kadd(ldk(r + 1), gl::kmul(ldk(r + 4), c1)));
+            sum[2] = gl::kadd(sum[2], gl::kadd(ldk(r + 2), gl::kmul(ldk(r + 5), gl::ksub(gl::kdbl(c1), c0))));
+        }
+        in0 = s_c[0][TE_T - 1];
+        in1 = s_c[1][TE_T - 1];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        K v = sum[i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = gl::kadd(v, shfl_xor_km(v, o));
-        if (lane == 0) a.out[x] = v;
+        if (lane == 0) s_red[warp][i] = v;
+    }
+    __syncthreads();
+    if (tid < 3) {
+        K v = gl::kzero();
+        for (int i = 0; i < TE_T / 32; i++) v = gl::kadd(v, s_red[i][tid]);
+        a.out[tid] = a.kind == 0 ? v : gl::kneg(v);
     }
 }
 
-// One round's fold of the address lane: threads j < E fold the events'
-// address weights by the bound bit, the next `half` fold the initial-memory
-// table on its low address bit.
-__global__ void ta_fold_kernel(const uint32_t* __restrict__ ra, const uint32_t* __restrict__ wa, K* __restrict__ rpw,
-                               K* __restrict__ wpw, uint32_t E, uint32_t bit, K r, int kind, const K* __restrict__ tab,
-                               K* __restrict__ tab_out, uint64_t half) {
+// One fold of the address lane: item j's weights by its own bit, the
+// initial-memory table on its low address bit, and the items' order from
+// (addr >> (bit + 1), item) to (addr >> (bit + 2), item): an item moves by the
+// sibling run's items that come before it in time.
+struct TaFold {
+    uint32_t N, bit;
+    int kind;
+    K r;
+    const uint64_t* key;
+    uint64_t* key_out;
+    K *wt, *d;
+    const K* tab;
+    K* tab_out;
+    uint64_t half;
+};
+__global__ void __launch_bounds__(256) ta_fold_kernel(const TaFold a) {
     const uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (j < E) {
-        const K omr = gl::ksub(gl::kone(), r);
-        if (kind == 0) rpw[j] = gl::kmul(rpw[j], ((ra[j] >> bit) & 1) ? r : omr);
-        wpw[j] = gl::kmul(wpw[j], ((wa[j] >> bit) & 1) ? r : omr);
-    } else if (j - E < half) {
-        const uint64_t p = j - E;
-        tab_out[p] = gl::klerp(tab[2 * p], tab[2 * p + 1], r);
+    if (j >= a.N) {
+        const uint64_t q = j - a.N;
+        if (q < a.half) a.tab_out[q] = gl::klerp(a.tab[2 * q], a.tab[2 * q + 1], a.r);
+        return;
     }
+    const uint64_t key = a.key[j];
+    const uint32_t idx = (uint32_t)key, blk = ta_addr(key) >> (a.bit + 1);
+    const K f = ((ta_addr(key) >> a.bit) & 1) ? a.r : gl::ksub(gl::kone(), a.r);
+    a.wt[idx] = gl::kmul(a.wt[idx], f);
+    if (a.kind == 1) a.d[idx] = gl::kmul(a.d[idx], f);
+    // items before (block, item index) in the current order
+    auto lower = [&](uint32_t block, uint32_t item) {
+        uint32_t lo = 0, hi = a.N;
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            const uint64_t k = a.key[mid];
+            const uint32_t b = ta_addr(k) >> (a.bit + 1);
+            if (b < block || (b == block && (uint32_t)k < item)) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    const uint32_t sib = blk ^ 1;
+    a.key_out[j + lower(sib, idx) - lower(max(blk, sib), 0)] = key;  // the runs meet at the larger block's start
 }
 
 __global__ void scatter_init_kernel(const uint64_t* __restrict__ addr, const K* __restrict__ val, uint64_t n,
@@ -1341,9 +1553,11 @@ __global__ void scatter_init_kernel(const uint64_t* __restrict__ addr, const K* 
 struct neo_gpu_twist_addr {
     neo_gpu_ctx* ctx = nullptr;
     int kind = 0;
-    uint32_t A = 0, bit = 0, E = 0;
-    DevBuf<K> eq, hr, rv, hw, inc, wv, rpw, wpw, tab[2], partials, vals;
-    DevBuf<uint32_t> ra, wa;
+    uint32_t A = 0, bit = 0, N = 0;  // N items
+    DevBuf<uint64_t> key[2];
+    int kcur = 0;
+    DevBuf<K> wt, kc, d, tab[2], recs, vals;
+    DevBuf<uint32_t> heads, hist;
     DevBuf<unsigned int> ticket;     // ta_eval_kernel's block counter (returns to zero after every launch)
     DevBuf<K> dcols, dr, dv;         // build workspace, kept for reuse
     DevBuf<uint32_t> counts;
@@ -1359,15 +1573,18 @@ namespace {
 
 int ta_apply_fold(neo_gpu_twist_addr* o) {
     neo_gpu_ctx* ctx = o->ctx;
-    cudaStream_t S = ctx->stream;
-    // the events' address weights and the initial-memory table, one launch
     const uint64_t half = o->tab_len >> 1;
-    const uint64_t n = o->E + half;
+    const uint64_t n = o->N + half;
     if (n) {
-        ta_fold_kernel<<<ceil_div(n, 256), 256, 0, S>>>(o->ra.p, o->wa.p, o->rpw.p, o->wpw.p, o->E, o->bit, o->pending_r,
-                                                       o->kind, o->tab[o->cur].p, o->tab[o->cur ^ 1].p, half);
+        TaFold a;
+        a.N = o->N; a.bit = o->bit; a.kind = o->kind; a.r = o->pending_r;
+        a.key = o->key[o->kcur].p; a.key_out = o->key[o->kcur ^ 1].p;
+        a.wt = o->wt.p; a.d = o->d.p;
+        a.tab = o->tab[o->cur].p; a.tab_out = o->tab[o->cur ^ 1].p; a.half = half;
+        ta_fold_kernel<<<ceil_div(n, 256), 256, 0, ctx->stream>>>(a);
         NEO_LAUNCHED(ctx);
     }
+    o->kcur ^= 1;
     o->cur ^= 1;
     o->tab_len = half;
     o->bit++;
@@ -1376,7 +1593,7 @@ int ta_apply_fold(neo_gpu_twist_addr* o) {
 }
 
 // The round's values at x = 0, 1, 2 into d_dst (device), without a host sync
-// (the pending fold applied first); no events: zeros.
+// (the pending fold applied first); no items: zeros.
 int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
     neo_gpu_ctx* ctx = o->ctx;
     cudaStream_t S = ctx->stream;
@@ -1384,24 +1601,23 @@ int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
         int rc = ta_apply_fold(o);
         if (rc) return rc;
     }
-    if (o->E == 0) {
+    if (o->N == 0) {
         NEO_CK(ctx, cudaMemsetAsync(d_dst, 0, 3 * sizeof(K), S));
         return NEO_OK;
     }
-    const uint32_t nbx = ceil_div(o->E, TA_T);
-    const uint32_t nb = nbx * nbx;
-    NEO_CK(ctx, o->partials.ensure((size_t)3 * nb));
+    const uint32_t nb = ceil_div(o->N, TE_T);
     TaEval a;
     a.kind = o->kind;
-    a.E = o->E;
+    a.N = o->N;
     a.bit = o->bit;
-    a.eq = o->eq.p; a.hr = o->hr.p; a.rv = o->rv.p; a.hw = o->hw.p; a.inc = o->inc.p; a.wv = o->wv.p;
-    a.rpw = o->rpw.p; a.wpw = o->wpw.p; a.ra = o->ra.p; a.wa = o->wa.p;
+    a.key = o->key[o->kcur].p;
+    a.wt = o->wt.p; a.kc = o->kc.p; a.d = o->d.p;
     a.init_tab = o->tab[o->cur].p;
-    a.partials = o->partials.p;
+    a.recs = o->recs.p;
+    a.heads = o->heads.p;
     a.out = d_dst;
     a.ticket = o->ticket.p;
-    ta_eval_kernel<<<dim3(nbx, nbx), TA_T, 0, S>>>(a);
+    ta_eval_kernel<<<nb, TE_T, 0, S>>>(a);
     NEO_LAUNCHED(ctx);
     return NEO_OK;
 }
@@ -1438,6 +1654,7 @@ int ta_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_cycle,
     o->A = A;
     o->bit = 0;
     o->cur = 0;
+    o->kcur = 0;
     o->pending = false;
     auto fail = [&](int rc) {
         if (fresh) delete o;
@@ -1469,29 +1686,33 @@ int ta_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_cycle,
     std::vector<uint32_t> hc(nblk);
     NEO_CK(ctx, ctx_d2h(ctx, hc.data(), counts.p, nblk * 4));
     NEO_CK(ctx, ctx_sync(ctx));
-    uint64_t E = 0;
-    for (auto& c : hc) { uint32_t v = c; c = (uint32_t)E; E += v; }
-    o->E = (uint32_t)E;
-    const size_t ecap = E ? E : 1;
-    if (o->eq.ensure(ecap) || o->hr.ensure(ecap) || o->rv.ensure(ecap) || o->hw.ensure(ecap) || o->inc.ensure(ecap) ||
-        o->wv.ensure(ecap) || o->rpw.ensure(ecap) || o->wpw.ensure(ecap) ||
-        o->ra.ensure(ecap) || o->wa.ensure(ecap) || o->vals.ensure(3) || o->ticket.ensure(1) ||
+    uint64_t N = 0;
+    for (auto& c : hc) { uint32_t v = c; c = (uint32_t)N; N += v; }
+    if (N > 0x7FFFFFFFull) return fail(ctx->fail(NEO_ERR_UNSUPPORTED, "twist_addr: too many events"));
+    o->N = (uint32_t)N;
+    const size_t cap = N ? N : 1;
+    const uint32_t n_tiles = ceil_div(cap, RS_TILE), nb = ceil_div(cap, TE_T);
+    if (o->key[0].ensure(cap) || o->key[1].ensure(cap) || o->wt.ensure(cap) || o->kc.ensure(cap) ||
+        (kind == 1 && o->d.ensure(cap)) || o->recs.ensure((size_t)nb * TA_REC) || o->heads.ensure(nb) ||
+        o->hist.ensure((size_t)n_tiles * 256) || o->vals.ensure(3) || o->ticket.ensure(1) ||
         o->tab[0].ensure(P + 1) || o->tab[1].ensure(P / 2 + 1))
         return fail(ctx->fail(NEO_ERR_OOM, "twist_addr: event arrays"));
     NEO_CK(ctx, cudaMemsetAsync(o->ticket.p, 0, sizeof(unsigned int), S));
     NEO_CK(ctx, cudaMemcpyAsync(counts.p, hc.data(), nblk * 4, cudaMemcpyHostToDevice, S));
     b.r_cycle = dr.p; b.ell = ell; b.A = A; b.L = L; b.offs = counts.p;
-    b.eq = o->eq.p; b.ehr = o->hr.p; b.erv = o->rv.p; b.ehw = o->hw.p; b.einc = o->inc.p; b.ewv = o->wv.p;
-    b.era = o->ra.p; b.ewa = o->wa.p;
-    NEO_CK(ctx, cudaMemsetAsync(o->ra.p, 0, ecap * 4, S));
-    NEO_CK(ctx, cudaMemsetAsync(o->hr.p, 0, ecap * sizeof(K), S));
-    NEO_CK(ctx, cudaMemsetAsync(o->wv.p, 0, ecap * sizeof(K), S));
+    b.key = o->key[0].p; b.wt = o->wt.p; b.kc = o->kc.p; b.d = o->d.p;
     ta_build_kernel<<<nblk, TA_T, 0, S>>>(b);
     NEO_LAUNCHED(ctx);
-    // prefix weights start at one
-    std::vector<K> ones(ecap, gl::kone());
-    NEO_CK(ctx, cudaMemcpyAsync(o->rpw.p, ones.data(), ecap * sizeof(K), cudaMemcpyHostToDevice, S));
-    NEO_CK(ctx, cudaMemcpyAsync(o->wpw.p, ones.data(), ecap * sizeof(K), cudaMemcpyHostToDevice, S));
+    // round 0's order: by address bits 1..A-1, items of a run in time order
+    for (uint32_t sh = 1; sh < A && N; sh += 8) {
+        rs_hist_kernel<<<n_tiles, RS_T, 0, S>>>(o->key[o->kcur].p, o->N, (int)sh, n_tiles, o->hist.p);
+        NEO_LAUNCHED(ctx);
+        rs_scan_kernel<<<1, 1024, 0, S>>>(o->hist.p, (uint64_t)n_tiles * 256);
+        NEO_LAUNCHED(ctx);
+        rs_scatter_kernel<<<n_tiles, RS_T, 0, S>>>(o->key[o->kcur].p, o->N, (int)sh, n_tiles, o->hist.p, o->key[o->kcur ^ 1].p);
+        NEO_LAUNCHED(ctx);
+        o->kcur ^= 1;
+    }
     // initial memory as a dense table over the 2^A addresses (plus one zero pad)
     NEO_CK(ctx, cudaMemsetAsync(o->tab[0].p, 0, (P + 1) * sizeof(K), S));
     NEO_CK(ctx, cudaMemsetAsync(o->tab[1].p, 0, (P / 2 + 1) * sizeof(K), S));
