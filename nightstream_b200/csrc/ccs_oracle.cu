@@ -781,6 +781,7 @@ static int neo_gpu_ccs_oracle_create_impl_abi(neo_gpu_ctx* ctx, const neo_ccs_de
     *out = nullptr;
     if (ell_d == 0 || ell_d > 8 || ell_n < 1 || ell_n > 30) return ctx->fail(NEO_ERR_ARG, "ccs_oracle: ell_d/ell_n out of range");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     auto* o = new neo_gpu_ccs_oracle();
     std::unique_ptr<neo_gpu_ccs_oracle> guard(o);
     int rc = dev_ccs_upload(ctx, desc, o->own_ccs);
@@ -1382,6 +1383,7 @@ static int neo_gpu_ccs_oracle_evals_impl_abi(neo_gpu_ccs_oracle* o, const uint64
     if (!xs || !ys || nx == 0 || nx > 16) return ctx->fail(NEO_ERR_ARG, "evals: bad args");
     if (o->round_idx >= o->ell_n + o->ell_d) return ctx->fail(NEO_ERR_ARG, "evals: all rounds done");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     if (o->round_idx < o->ell_n) {
         if (!o->coeffs_valid) {
             int rc = row_round(o);
@@ -1425,6 +1427,7 @@ static int neo_gpu_ccs_oracle_row_rounds_device_impl_abi(neo_gpu_ccs_oracle* o, 
     if (!chals || !d_coeffs || n == 0) return ctx->fail(NEO_ERR_ARG, "row_rounds_device: bad args");
     if (o->round_idx + n > o->ell_n) return ctx->fail(NEO_ERR_ARG, "row_rounds_device: beyond the row rounds");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     const uint32_t j0 = o->round_idx;
     for (uint32_t i = 0; i < n; i++) o->row_chals.push_back(gl::kmk(gl::canon(chals[2 * i]), gl::canon(chals[2 * i + 1])));
     // every challenge of the sequence goes up once; round j reads only the first j
@@ -1454,6 +1457,7 @@ static int neo_gpu_ccs_oracle_me_outputs_impl_abi(neo_gpu_ccs_oracle* o, uint64_
     if (!y || !y_scalars) return ctx->fail(NEO_ERR_ARG, "me_outputs: null output");
     if (o->row_chals.size() != o->ell_n) return ctx->fail(NEO_ERR_ARG, "me_outputs: row challenges not finalized");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     if (!o->have_pre) {
         int rc = ajtai_precompute(o);
         if (rc) return rc;
@@ -1507,6 +1511,7 @@ static int neo_gpu_ccs_autotune_impl_abi(neo_gpu_ctx* ctx, const neo_ccs_desc* d
     if (desc->n != desc->m || (1u << ell_n) != desc->n || ell_n < 3)
         return ctx->fail(NEO_ERR_UNSUPPORTED, "ccs_autotune: needs n == m == 2^ell, ell >= 3");
     NEO_CK(ctx, cudaSetDevice(ctx->device));
+    PoolScope pool_scope(ctx);
     const uint32_t ell_d = 6, d_sc = 6;
     uint64_t seed = 0x4E454F54554E45ull;
     auto rk = [&](size_t n) {

@@ -133,7 +133,7 @@ int pp_slot(neo_gpu_ctx* ctx, uint32_t kappa, uint64_t m, PPEntry** out) {
     PPEntry* pp = slot;
     const size_t n = (size_t)kappa * m * NEO_D;
     if (pp->d_pp && pp->kappa != kappa) { cudaFree(pp->d_pp); pp->d_pp = nullptr; pp->kappa = 0; }
-    if (!pp->d_pp) NEO_CK(ctx, cudaMalloc(&pp->d_pp, n * 8));
+    if (!pp->d_pp) NEO_CK(ctx, ctx_malloc(ctx, reinterpret_cast<void**>(&pp->d_pp), n * 8));
     pp->tc = false;  // the tiles (kept allocated: their size depends on m only) are rebuilt by pp_finish
     *out = pp;
     return NEO_OK;
@@ -183,6 +183,7 @@ static int neo_gpu_commit_impl_abi(neo_gpu_ctx* ctx, const int8_t* digits, uint3
     if (!ctx) return NEO_ERR_ARG;
     if (!digits || !out || n_vec == 0 || m == 0) return ctx->fail(NEO_ERR_ARG, "commit: bad args");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     PPEntry* pp = pp_lookup(ctx->device, m);
     if (!pp || !pp->kappa) return ctx->fail(NEO_ERR_ARG, "commit: PP not loaded for this m");
     DevBuf<int8_t> dZ;

@@ -729,7 +729,7 @@ int commit_ws(neo_gpu_ctx* ctx, uint32_t n_groups, size_t acc_words, TcArgs* a, 
             ctx->commit_words = 0;
         }
         void* p = nullptr;
-        NEO_CK(ctx, pooled ? cudaMallocAsync(&p, bytes, ctx->stream) : cudaMalloc(&p, bytes));
+        NEO_CK(ctx, pooled ? cudaMallocAsync(&p, bytes, ctx->stream) : ctx_malloc(ctx, &p, bytes));
         ctx->commit_buf = p;
         NEO_CK(ctx, cudaMemsetAsync(p, 0, bytes, ctx->stream));
         ctx->commit_groups = groups;
@@ -813,7 +813,7 @@ int tc_pp_prepare(neo_gpu_ctx* ctx, PPEntry* pp) {
     if (pp->kappa * 8 > 128) return ctx->fail(NEO_ERR_UNSUPPORTED, "tensor-core commit: kappa <= 16");
     pp->tc = false;
     const uint64_t n_kb = (pp->m + 1) / 2;
-    if (!pp->d_pp_limbs) NEO_CK(ctx, cudaMalloc(&pp->d_pp_limbs, n_kb * TC_A_BYTES));  // size depends on m only
+    if (!pp->d_pp_limbs) NEO_CK(ctx, ctx_malloc(ctx, reinterpret_cast<void**>(&pp->d_pp_limbs), n_kb * TC_A_BYTES));  // size depends on m only
     pp_limbs_kernel<<<(unsigned)n_kb, 256, 0, ctx->stream>>>(pp->d_pp, pp->kappa, pp->m, pp->d_pp_limbs);
     NEO_LAUNCHED(ctx);
     NEO_CK(ctx, ctx_sync(ctx));

@@ -23,6 +23,18 @@ static int neo_gpu_ctx_create_impl_abi(int device, neo_gpu_ctx** out) {
         delete c;
         return NEO_ERR_CUDA;
     }
+    // without a pool (an old driver) the buffers come from cudaMalloc
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    if (cudaMemPoolCreate(&c->pool, &props) == cudaSuccess) {
+        uint64_t keep = CTX_POOL_KEEP;
+        cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    } else {
+        c->pool = nullptr;
+        cudaGetLastError();
+    }
     *out = c;
     return NEO_OK;
 }
@@ -31,6 +43,7 @@ extern "C" int neo_gpu_ctx_create(int device, neo_gpu_ctx** out) { NEO_ABI_GUARD
 // Stream on which DevBuf allocations of this thread are made (stream-ordered,
 // from the device's memory pool) and later freed; null: cudaMalloc / cudaFree.
 thread_local cudaStream_t g_alloc_stream = nullptr;
+thread_local PoolRef g_pool;
 
 static int neo_gpu_ctx_destroy_impl_abi(neo_gpu_ctx* ctx) {
     if (!ctx) return NEO_ERR_ARG;
@@ -40,6 +53,7 @@ static int neo_gpu_ctx_destroy_impl_abi(neo_gpu_ctx* ctx) {
     if (ctx->commit_buf) cudaFree(ctx->commit_buf);
     if (ctx->chi_cache) cudaFree(ctx->chi_cache);
     if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return NEO_OK;
@@ -81,6 +95,7 @@ static int neo_gpu_wait_probe_impl_abi(neo_gpu_ctx* ctx, uint32_t set_flag, uint
     if (!ctx) return NEO_ERR_ARG;
     if (spin_limit == 0 || spin_limit > (1u << 20)) return ctx->fail(NEO_ERR_ARG, "wait_probe: spin_limit in [1, 2^20]");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     DevBuf<uint32_t> flag;
     NEO_CK(ctx, flag.alloc(1));
     NEO_CK(ctx, cudaMemsetAsync(flag.p, 0, 4, ctx->stream));
@@ -231,6 +246,7 @@ __global__ void decomp_b2_kernel(const uint64_t* __restrict__ z, uint64_t m, int
 static int neo_gpu_decomp_b2_impl_abi(neo_gpu_ctx* ctx, const uint64_t* z, uint64_t m, int8_t* Z) {
     if (!ctx || !z || !Z || m == 0) return ctx ? ctx->fail(NEO_ERR_ARG, "decomp: bad args") : NEO_ERR_ARG;
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     DevBuf<uint64_t> dz;
     DevBuf<int8_t> dZ;
     NEO_CK(ctx, dz.alloc(m));
@@ -353,6 +369,7 @@ static int neo_gpu_rlc_mix_impl_abi(neo_gpu_ctx* ctx, const int8_t* rho_coeffs, 
     if (!ctx) return NEO_ERR_ARG;
     if (!rho_coeffs || !Zs || !Zmix || count == 0 || count > 64 || m == 0) return ctx->fail(NEO_ERR_ARG, "rlc: bad args");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     DevBuf<int8_t> dZs, drot;
     DevBuf<int32_t> dmix;
     NEO_CK(ctx, dZs.alloc((size_t)count * NEO_D * m));
@@ -433,6 +450,7 @@ static int neo_gpu_split_b_impl_abi(neo_gpu_ctx* ctx, const int32_t* Zmix, uint6
     if (!ctx) return NEO_ERR_ARG;
     if (!Zmix || !planes || !nonzero || len == 0) return ctx->fail(NEO_ERR_ARG, "split_b: bad args");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     DevBuf<int32_t> dmix;
     DevBuf<int8_t> dpl;
     DevBuf<uint32_t> dfl;
@@ -684,6 +702,7 @@ static int neo_gpu_me_y_impl_abi(neo_gpu_ctx* ctx, const neo_ccs_desc* desc, con
     if (!desc || !Z || !r || !y || !y_scalars || n_w == 0 || ell_n == 0 || ell_n > 30)
         return ctx->fail(NEO_ERR_ARG, "me_y: bad args");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     DevCcs ccs;
     int rc = dev_ccs_upload(ctx, desc, ccs);
     if (rc) return rc;

@@ -578,6 +578,7 @@ static int shard_create_impl(neo_gpu_ctx* ctx, const neo_ccs_desc* desc, uint32_
     if (!pp) return ctx->fail(NEO_ERR_ARG, "shard_create: upload PP for this m first");
     if (k_rho == 0 || k_rho > 17 || m_in == 0 || m_in > desc->m) return ctx->fail(NEO_ERR_ARG, "shard_create: k_rho/m_in");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     auto* sh = new neo_gpu_shard();
     std::unique_ptr<neo_gpu_shard> guard(sh);
     sh->ctx = ctx;
@@ -1874,6 +1875,7 @@ static int neo_gpu_shard_fold_step_impl_abi(neo_gpu_shard* sh, const uint64_t* z
     if (!sh) return NEO_ERR_ARG;
     if (!z) return sh->ctx->fail(NEO_ERR_ARG, "fold_step: null witness");
     cudaSetDevice(sh->ctx->device);
+    PoolScope pool_scope(sh->ctx);
     int rc = fold_step_impl(sh, z, nullptr);
     if (rc) return rc;
     if (proof_len) *proof_len = sh->proof.size();
@@ -1891,6 +1893,7 @@ static int neo_gpu_shard_fold_step_device_impl_abi(neo_gpu_shard* sh, const uint
     if (!sh) return NEO_ERR_ARG;
     if (!d_z) return sh->ctx->fail(NEO_ERR_ARG, "fold_step_device: null witness");
     cudaSetDevice(sh->ctx->device);
+    PoolScope pool_scope(sh->ctx);
     int rc = fold_step_impl(sh, nullptr, d_z);
     if (rc) return rc;
     if (proof_len) *proof_len = sh->proof.size();
@@ -2013,6 +2016,7 @@ static int neo_gpu_shard_fold_step_trace_impl_abi(neo_gpu_shard* sh, const uint6
     const size_t ns = sh->shout.size(), nt = sh->twist.size();
     if ((ns && !trc->shout) || (nt && !trc->twist)) return ctx->fail(NEO_ERR_ARG, "fold_step_trace: missing events");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     cudaStream_t st = ctx->stream;
     // validate and pack the events (the reference's build errors: bad flags,
     // Twist addresses outside the memory)
@@ -2517,6 +2521,7 @@ static int neo_gpu_shard_restore_impl_abi(neo_gpu_shard* sh, const uint8_t* buf,
     neo_gpu_ctx* ctx = sh->ctx;
     if (!buf) return ctx->fail(NEO_ERR_ARG, "shard_restore: null buffer");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     CkptReader r{buf, len};
     uint64_t want[14], got[14];
     ckpt_header(sh, want);

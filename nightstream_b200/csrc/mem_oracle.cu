@@ -689,6 +689,7 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
     const uint32_t deg = degree_of(kind, A, n_cols);
     if (deg > MEM_MAX_DEG) return ctx->fail(NEO_ERR_UNSUPPORTED, "mem_oracle: degree bound above 31");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
 
     // reuse: rebuild into the caller's object, keeping its device buffers
     neo_gpu_mem_oracle* o = reuse ? *out : nullptr;
@@ -756,7 +757,7 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
                 ctx->chi_cache = nullptr;
                 ctx->chi_cache_bytes = 0;
                 ctx->chi_key.clear();
-                if (cudaMalloc(&ctx->chi_cache, bytes)) return fail(ctx->fail(NEO_ERR_OOM, "mem_oracle: chi cache"));
+                if (ctx_malloc(ctx, &ctx->chi_cache, bytes)) return fail(ctx->fail(NEO_ERR_OOM, "mem_oracle: chi cache"));
                 ctx->chi_cache_bytes = bytes;
             }
             if (cudaMemcpyAsync(ctx->chi_cache, T, bytes, cudaMemcpyDeviceToDevice, S))
@@ -999,6 +1000,7 @@ static int neo_gpu_mem_oracle_evals_impl_abi(neo_gpu_mem_oracle* o, const uint64
     if (!o) return NEO_ERR_ARG;
     if ((!xs || !ys) && nx) return o->ctx->fail(NEO_ERR_ARG, "mem_oracle_evals: null buffer");
     cudaSetDevice(o->ctx->device);
+    PoolScope pool_scope(o->ctx);
     int rc = mem_round_values(o);
     if (rc) return rc;
     for (uint32_t i = 0; i < nx; i++) {
@@ -1088,6 +1090,7 @@ static int neo_gpu_addr_lookup_weights_impl_abi(neo_gpu_ctx* ctx, uint32_t ell, 
         return ctx->fail(NEO_ERR_ARG, "addr_lookup_weights: null buffer");
     if (ell > 30 || ell_addr > 30) return ctx->fail(NEO_ERR_ARG, "addr_lookup_weights: size");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     cudaStream_t S = ctx->stream;
     const uint64_t L = 1ULL << ell, P = 1ULL << ell_addr;
     DevBuf<K> dr, has, bits, w, tab;
@@ -1643,6 +1646,7 @@ int ta_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_cycle,
     for (uint64_t i = 0; i < n_init; i++)
         if (init_addr[i] >> A) return ctx->fail(NEO_ERR_ARG, "twist_addr: init address out of range");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     cudaStream_t S = ctx->stream;
     const uint64_t L = 1ULL << ell, P = 1ULL << A;
     const uint32_t n_cols = kind == 0 ? 4 + 2 * A : 3 + A;
@@ -1777,6 +1781,7 @@ static int neo_gpu_twist_addr_evals_impl_abi(neo_gpu_twist_addr* o, const uint64
     if (!o) return NEO_ERR_ARG;
     if ((!xs || !ys) && nx) return o->ctx->fail(NEO_ERR_ARG, "twist_addr_evals: null buffer");
     cudaSetDevice(o->ctx->device);
+    PoolScope pool_scope(o->ctx);
     int rc = ta_values(o);
     if (rc) return rc;
     for (uint32_t i = 0; i < nx; i++) {

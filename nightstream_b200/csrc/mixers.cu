@@ -54,6 +54,7 @@ static int neo_gpu_mix_rhos_commits_impl_abi(neo_gpu_ctx* ctx, const uint64_t* r
     if (!rhos || !cs || !out || count == 0 || kappa == 0 || count > (1u << 20))
         return ctx->fail(NEO_ERR_ARG, "mix_rhos_commits: bad args");
     NEO_CK(ctx, cudaSetDevice(ctx->device));
+    PoolScope pool_scope(ctx);
     DevBuf<uint64_t> dr, dc, dout;
     NEO_CK(ctx, dr.alloc((size_t)count * NEO_D * NEO_D));
     NEO_CK(ctx, dc.alloc((size_t)count * kappa * NEO_D));
@@ -77,6 +78,7 @@ static int neo_gpu_combine_b_pows_impl_abi(neo_gpu_ctx* ctx, const uint64_t* cs,
     if (!cs || !out || count == 0 || kappa == 0 || count > (1u << 20))
         return ctx->fail(NEO_ERR_ARG, "combine_b_pows: bad args");
     NEO_CK(ctx, cudaSetDevice(ctx->device));
+    PoolScope pool_scope(ctx);
     const uint32_t len = kappa * NEO_D;
     DevBuf<uint64_t> dc, dout;
     NEO_CK(ctx, dc.alloc((size_t)count * len));

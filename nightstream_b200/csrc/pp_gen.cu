@@ -240,6 +240,7 @@ static int neo_gpu_chacha8_sample_impl_abi(neo_gpu_ctx* ctx, const uint8_t* seed
     if (!ctx) return NEO_ERR_ARG;
     if ((n_streams && (!seeds || !counts)) || !out) return ctx->fail(NEO_ERR_ARG, "chacha8_sample: bad args");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     std::vector<uint64_t> offs(n_streams);
     uint64_t total = 0;
     for (uint32_t s = 0; s < n_streams; s++) {
@@ -263,6 +264,7 @@ static int neo_gpu_pp_generate_impl_abi(neo_gpu_ctx* ctx, const uint8_t* seed, u
     if (!seed || kappa == 0 || kappa > 64 || m == 0) return ctx->fail(NEO_ERR_ARG, "pp_generate: bad args");
     if (mode != NEO_PP_SETUP && mode != NEO_PP_SETUP_PAR) return ctx->fail(NEO_ERR_ARG, "pp_generate: bad mode");
     cudaSetDevice(ctx->device);
+    PoolScope pool_scope(ctx);
     std::vector<std::array<uint8_t, 32>> seeds;
     std::vector<uint64_t> counts, offs;
     if (mode == NEO_PP_SETUP) {
