@@ -23,6 +23,12 @@ static int neo_gpu_ctx_create_impl_abi(int device, neo_gpu_ctx** out) {
         delete c;
         return NEO_ERR_CUDA;
     }
+    if (cudaHostAlloc(&c->h_result, CTX_RESULT_BYTES, cudaHostAllocMapped) != cudaSuccess) {
+        cudaFree(c->d_err);
+        cudaStreamDestroy(c->stream);
+        delete c;
+        return NEO_ERR_OOM;
+    }
     // without a pool (an old driver) the buffers come from cudaMalloc
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
@@ -53,6 +59,7 @@ static int neo_gpu_ctx_destroy_impl_abi(neo_gpu_ctx* ctx) {
     if (ctx->commit_buf) cudaFree(ctx->commit_buf);
     if (ctx->chi_cache) cudaFree(ctx->chi_cache);
     if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->h_result) cudaFreeHost(ctx->h_result);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     cudaStreamDestroy(ctx->stream);
     delete ctx;

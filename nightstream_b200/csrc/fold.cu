@@ -171,13 +171,33 @@ __global__ void __launch_bounds__(256) child_y_kernel(const int8_t* __restrict__
     }
 }
 
+// out[i] = column id[i] of src (columns of L 16-byte entries); blockIdx.y = i.
+// Bound by memory: GATHER_PER independent 16-byte loads a thread.
+constexpr uint32_t GATHER_MAX = 128, GATHER_PER = 4;
+struct GatherIds {
+    uint32_t id[GATHER_MAX];
+};
+__global__ void __launch_bounds__(256) gather_cols_kernel(const ulonglong2* __restrict__ src, uint64_t L,
+                                                          const __grid_constant__ GatherIds g,
+                                                          ulonglong2* __restrict__ out) {
+    const uint64_t t0 = blockIdx.x * (uint64_t)(256 * GATHER_PER) + threadIdx.x;
+    const ulonglong2* s = src + (uint64_t)g.id[blockIdx.y] * L;
+    ulonglong2* d = out + (uint64_t)blockIdx.y * L;
+    ulonglong2 v[GATHER_PER];
+#pragma unroll
+    for (uint32_t e = 0; e < GATHER_PER; e++)
+        if (t0 + e * 256 < L) v[e] = s[t0 + e * 256];
+#pragma unroll
+    for (uint32_t e = 0; e < GATHER_PER; e++)
+        if (t0 + e * 256 < L) d[t0 + e * 256] = v[e];
+}
+
 // build_time_sparse_from_bus_col (memory_sidecar/cpu_bus.rs:976-1016), dense:
 // out[c][t] = z[bus_base + c*steps + (t - m_in)] for m_in <= t < m_in + steps, else 0
 __global__ void bus_decode_kernel(const uint64_t* __restrict__ z, uint32_t m_in, uint64_t bus_base, uint64_t steps,
-                                  uint32_t ncols, uint64_t L, K* __restrict__ out) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= (uint64_t)ncols * L) return;
-    const uint64_t c = i / L, t = i - c * L;
+                                  uint64_t L, K* __restrict__ out) {
+    const uint64_t c = blockIdx.y, t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, i = c * L + t;
+    if (t >= L) return;
     K v = gl::kzero();
     if (t >= m_in && t - m_in < steps) v = gl::kfq(gl::canon(z[bus_base + c * steps + (t - m_in)]));
     out[i] = v;
@@ -274,7 +294,7 @@ struct neo_gpu_shard {
     // batched sum-check rounds: every claim's round values in one device array,
     // read back with one copy per round (page-locked), and the partial sums of
     // the multi-claim memory kernels
-    DevBuf<K> d_round, d_mpart;
+    DevBuf<K> d_mpart;
     HostBuf<K> h_round;
     DevBuf<uint64_t> d_events;  // a trace chunk's packed events (neo_gpu_shard_fold_step_trace)
     HostBuf<uint64_t> h_events;
@@ -717,7 +737,7 @@ void ccs_oracle_round_set(neo_gpu_ccs_oracle* o, const K* coeffs);
 bool mem_round_multi_ok(const neo_gpu_mem_oracle* o);
 int ta_round_launch(neo_gpu_twist_addr* o, K* d_dst, bool* launched);
 int mem_claims_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* claims, DevBuf<K>& partials,
-                     DevBuf<K>& d_slots, HostBuf<K>& h_slots);
+                     HostBuf<K>& h_slots);
 int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* const* d_out,
                            DevBuf<K>& partials);
 
@@ -815,8 +835,7 @@ struct Claim {
 // Per round every claim is launched first -- the Pi_CCS claim writes its
 // coefficients, the memory claims their values at 0..deg (all of them in one
 // multi-claim fold and eval), the Twist address-lane claims theirs at 0, 1,
-// 2, into one device array -- then a single copy and sync bring the round
-// back; claims whose tables are exhausted take the per-claim path.
+// 2, into one page-locked array -- then a single sync ends the round; claims whose tables are exhausted take the per-claim path.
 static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_idx, std::vector<Claim>& cl,
                           uint32_t rounds, std::vector<K>& chals, std::vector<K>& finals, std::vector<uint64_t>& P,
                           BatchRec* rec = nullptr) {
@@ -839,7 +858,6 @@ static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_i
     }
     // slots: MAX_SLOT K values per claim
     constexpr uint32_t MAX_SLOT = 33;
-    NEO_CK(ctx, sh->d_round.ensure(cl.size() * MAX_SLOT));
     NEO_CK(ctx, sh->h_round.ensure(cl.size() * MAX_SLOT));
     chals.clear();
     std::vector<neo_gpu_mem_oracle*> mos;
@@ -851,7 +869,7 @@ static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_i
         mos.clear();
         mdst.clear();
         for (size_t i = 0; i < cl.size(); i++) {
-            K* slot = sh->d_round.p + i * MAX_SLOT;
+            K* slot = sh->h_round.p + i * MAX_SLOT;  // page-locked: the launches write the values here
             kind[i] = 0;
             if (cl[i].ccs && cl[i].deg + 1 <= MAX_SLOT) {
                 int rc = ccs_oracle_round_launch(cl[i].ccs, slot, &ncoef[i]);
@@ -874,8 +892,6 @@ static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_i
             int rc = mem_round_launch_multi(ctx, mos.data() + i0, nn, mdst.data() + i0, sh->d_mpart);
             if (rc) return rc;
         }
-        NEO_CK(ctx, cudaMemcpyAsync(sh->h_round.p, sh->d_round.p, cl.size() * MAX_SLOT * sizeof(K),
-                                    cudaMemcpyDeviceToHost, ctx->stream));
         NEO_CK(ctx, ctx_sync(ctx));
         for (size_t i = 0; i < cl.size(); i++) {
             const uint32_t np = cl[i].deg + 1;
@@ -1001,12 +1017,18 @@ static int upload_point(neo_gpu_shard* sh, const std::vector<K>& r) {
     return NEO_OK;
 }
 
-// gather bus columns (ids) of `src` into d_asm, in the given order
+// gather bus columns (ids) of `src` into d_asm, in the given order: one launch
+// (a copy per column was 130 of the step's launches, 2 us each on the device)
 static int assemble(neo_gpu_shard* sh, const K* src, const std::vector<uint32_t>& ids) {
     const uint64_t L = 1ULL << sh->ell_n;
-    for (size_t i = 0; i < ids.size(); i++)
-        NEO_CK(sh->ctx, cudaMemcpyAsync(sh->d_asm.p + i * L, src + (size_t)ids[i] * L, L * sizeof(K),
-                                        cudaMemcpyDeviceToDevice, sh->ctx->stream));
+    for (size_t i0 = 0; i0 < ids.size(); i0 += GATHER_MAX) {
+        GatherIds g;
+        const uint32_t n = (uint32_t)std::min<size_t>(GATHER_MAX, ids.size() - i0);
+        std::copy(ids.begin() + i0, ids.begin() + i0 + n, g.id);
+        gather_cols_kernel<<<dim3(ceil_div(L, 256 * GATHER_PER), n), 256, 0, sh->ctx->stream>>>(
+            reinterpret_cast<const ulonglong2*>(src), L, g, reinterpret_cast<ulonglong2*>(sh->d_asm.p + i0 * L));
+        NEO_LAUNCHED(sh->ctx);
+    }
     return NEO_OK;
 }
 
@@ -1252,8 +1274,8 @@ static int fold_step_impl(neo_gpu_shard* sh, const uint64_t* z_host, const uint6
     NEO_LAUNCHED(ctx);
     if ((rc = launch_commit(ctx, sh->Zall.p, 1, m, sh->d_commits.p, TC_DIGITS_SMALL))) return rc;  // digits in {-1, 0, 1}
     if (has_mem) {
-        bus_decode_kernel<<<ceil_div((uint64_t)nb * L, 256), 256, 0, ctx->stream>>>(d_z, sh->m_in, sh->bus_base, sh->steps,
-                                                                                    nb, L, sh->d_cols.p);
+        bus_decode_kernel<<<dim3(ceil_div(L, 256), nb), 256, 0, ctx->stream>>>(d_z, sh->m_in, sh->bus_base, sh->steps, L,
+                                                                               sh->d_cols.p);
         NEO_LAUNCHED(ctx);
     }
     MeInst mcs;
@@ -1564,7 +1586,7 @@ static int fold_step_impl(neo_gpu_shard* sh, const uint64_t* z_host, const uint6
             {  // both claims from one evaluation of round 0
                 neo_gpu_mem_oracle* g2[2] = {vo, ao};
                 K c2[2];
-                if ((rc = mem_claims_multi(ctx, g2, 2, c2, sh->d_mpart, sh->d_round, sh->h_round))) return rc;
+                if ((rc = mem_claims_multi(ctx, g2, 2, c2, sh->d_mpart, sh->h_round))) return rc;
                 vc = c2[0];
                 ac_ = c2[1];
             }
@@ -1756,7 +1778,7 @@ static int fold_step_impl(neo_gpu_shard* sh, const uint64_t* z_host, const uint6
             std::vector<K> vs(vos.size());
             for (size_t i0 = 0; i0 < vos.size(); i0 += 24) {
                 const int nn = (int)std::min<size_t>(24, vos.size() - i0);
-                if ((rc = mem_claims_multi(ctx, vos.data() + i0, nn, vs.data() + i0, sh->d_mpart, sh->d_round,
+                if ((rc = mem_claims_multi(ctx, vos.data() + i0, nn, vs.data() + i0, sh->d_mpart,
                                            sh->h_round)))
                     return rc;
             }
@@ -1850,12 +1872,10 @@ static int fold_step_impl(neo_gpu_shard* sh, const uint64_t* z_host, const uint6
     tr.append_message("fold/step_done", bidx.data(), 8);
     sh->acc.swap(children);
     if (!sh->twist.empty()) {
-        // this step becomes the rollover source of the next one
+        // this step becomes the rollover source of the next one (d_cols is written anew by every step)
         NEO_CK(ctx, cudaMemcpyAsync(sh->valwit.p + (size_t)NEO_D * m, sh->valwit.p, (size_t)NEO_D * m,
                                     cudaMemcpyDeviceToDevice, ctx->stream));
-        NEO_CK(ctx, cudaMemcpyAsync(sh->d_prev_cols.p, sh->d_cols.p, (size_t)nb * L * sizeof(K), cudaMemcpyDeviceToDevice,
-                                    ctx->stream));
-        NEO_CK(ctx, ctx_sync(ctx));
+        sh->d_prev_cols.swap(sh->d_cols);
         sh->prev_c = mcs.c;
         sh->prev_X = mcs.X;
         sh->has_prev = true;

@@ -139,6 +139,15 @@ GL_HD K ksqr(K a) {
     uint64_t x = mul(a.re, a.im);
     return kmk(add(mul(a.re, a.re), mul7(mul(a.im, a.im))), add(x, x));
 }
+// a x mod q for x < 2^26: two 32 x 32-bit products and one correction
+GL_HD uint64_t mul_tiny(uint64_t a, uint32_t x) {
+    const uint64_t p0 = (a & GL_EPS) * x, p1 = (a >> 32) * x + (p0 >> 32);
+    const uint64_t hi = p1 >> 32, t = (hi << 32) - hi;  // hi 2^64 = hi (2^32 - 1)
+    uint64_t s = ((p1 << 32) | (p0 & GL_EPS)) + t;
+    s += (uint64_t)(s < t) * GL_EPS;  // a carry leaves s < t < 2^58
+    return canon(s);
+}
+GL_HD K kscale_tiny(K a, uint32_t x) { return kmk(mul_tiny(a.re, x), mul_tiny(a.im, x)); }
 GL_HD K kscale(K a, uint64_t s) { return kmk(mul(a.re, s), mul(a.im, s)); }
 // multiply by a small signed integer |s| < 2^31
 GL_HD K kscale_small(K a, int32_t s) {

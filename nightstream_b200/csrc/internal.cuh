@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 #include "../../include/neo_gpu.h"
 #include "abi_guard.h"
@@ -21,6 +22,9 @@ struct neo_gpu_ctx {
     cudaMemPool_t pool = nullptr;    // this context's device buffers (PoolScope); keeps at most CTX_POOL_KEEP when idle
     std::string err;
     uint64_t launches = 0;
+    // page-locked, device-mapped: kernels write a round's few values here, so that a
+    // round ends with its launch instead of a copy (a call reads it before it returns)
+    void* h_result = nullptr;
     uint32_t* d_err = nullptr;       // device error word (bounded-wait timeouts); 0 = ok
     void* scratch = nullptr;         // growable per-context scratch (stream-ordered use)
     size_t scratch_bytes = 0;
@@ -43,6 +47,8 @@ struct neo_gpu_ctx {
         return code;
     }
 };
+
+constexpr size_t CTX_RESULT_BYTES = 4096;
 
 // wait for the context's stream (a spinning stream synchronization: batch
 // workers that slept in blocking waits were measured no faster)
@@ -192,6 +198,12 @@ struct DevBuf {
         s = nullptr;
         n = 0;
         cap = 0;
+    }
+    void swap(DevBuf& o) {
+        std::swap(p, o.p);
+        std::swap(n, o.n);
+        std::swap(s, o.s);
+        std::swap(cap, o.cap);
     }
     size_t bytes() const { return n * sizeof(T); }
 };

@@ -15,9 +15,9 @@
 //     extension of [u < t], so the reference's Σ inc_u·LT(u, point) is the
 //     folded exclusive prefix sum (one scan here);
 //   * LT(t, r_time) for the val-evaluation oracle.
-// A round evaluates Σ_pairs Π_f (f0 + x (f1 - f0)) at x = 0..deg (one thread
-// per (pair, x)), sums per block and then over blocks, and interpolates the
-// requested points on the host. fold(r) is one pass over every factor.
+// A round evaluates Σ_pairs Π_f (f0 + x (f1 - f0)) at x = 0..deg, the pending
+// fold of every factor inside the same launch, and interpolates the requested
+// points on the host.
 // All arithmetic is exact in F_q / K, so values equal the reference's.
 #include "internal.cuh"
 #include <algorithm>
@@ -27,7 +27,6 @@ using gl::K;
 namespace {
 
 constexpr int MEM_MAX_DEG = 31;
-constexpr int MT = 256;
 
 __device__ __forceinline__ K shfl_xor_km(K a, int o) {
     K r;
@@ -41,10 +40,15 @@ __device__ __forceinline__ K eq_bit_affine(K bit, K u) {
     return gl::kadd(gl::kmul(bit, gl::ksub(gl::kdbl(u), gl::kone())), gl::ksub(gl::kone(), u));
 }
 
-// columns b < A of [A][len], in place: col_b[t] = eq_bit_affine(col_b[t], u_b)
-__global__ void eqbit_kernel(K* __restrict__ cols, uint64_t len, uint32_t A, const K* __restrict__ u) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < len * A) cols[i] = eq_bit_affine(cols[i], u[i / len]);
+// columns b = blockIdx.y of [A][len]: out_b[t] = eq_bit_affine(cols_b[t], u_b)
+// (out may be cols).  Bound by HBM: 32 bytes an entry, and the columns are read
+// where they are instead of copied first (12 columns of 2^16: 12 copies and
+// 10.3 us of this kernel, now the latter alone).
+__global__ void eqbit_kernel(const K* cols, uint64_t len, const K* __restrict__ u, K* out) {
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (t >= len) return;
+    const uint64_t i = blockIdx.y * len + t;
+    out[i] = eq_bit_affine(cols[i], u[blockIdx.y]);
 }
 
 // inc_terms(t) = has_write(t)·inc(t)·Π_b eq_bit_affine(wa_b(t), r_addr_b)
@@ -53,8 +57,10 @@ __global__ void inc_terms_kernel(const K* __restrict__ has_w, const K* __restric
                                  uint32_t A, const K* __restrict__ r_addr, uint64_t len, K* __restrict__ out) {
     uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (t >= len) return;
-    K v = gl::kmul(has_w[t], inc[t]);
-    for (uint32_t b = 0; b < A; b++) v = gl::kmul(v, eq_bit_affine(wa[(uint64_t)b * len + t], r_addr[b]));
+    K v = has_w[t];
+    if (!gl::kiszero(v)) v = gl::kmul(v, inc[t]);
+    // rows without a write (most of the time domain) read no address bits
+    for (uint32_t b = 0; b < A && !gl::kiszero(v); b++) v = gl::kmul(v, eq_bit_affine(wa[(uint64_t)b * len + t], r_addr[b]));
     out[t] = v;
 }
 
@@ -180,68 +186,6 @@ __global__ void mem_fold_kernel(const K* __restrict__ src, uint64_t src_len, K* 
     dst[f * half + p] = gl::klerp(s[0], s[1], r);
 }
 
-struct MemEvalArgs {
-    const K* tab;       // [nf][len]
-    uint64_t len;       // current table length (>= 2)
-    uint32_t nf;
-    int bitness;        // 1: factor 0 is χ, the rest columns weighted by w
-    const K* w;         // bitness weights [nf - 1]
-    K* partials;        // [npts][gridDim.x]
-};
-
-// one thread per (pair, x); x = blockIdx.y
-__global__ void __launch_bounds__(MT) mem_eval_kernel(const MemEvalArgs a) {
-    __shared__ K s_red[MT / 32];
-    const uint64_t pairs = a.len >> 1;
-    const uint64_t p = blockIdx.x * (uint64_t)MT + threadIdx.x;
-    const uint32_t x = blockIdx.y;
-    K acc = gl::kzero();
-    if (p < pairs) {
-        // A factor that is zero on both children makes the whole product zero
-        // at every x: gate columns (has_lookup, has_read, has_write, the
-        // address weights) are zero outside the active trace rows, so most
-        // pairs stop after loading the gate (factors are ordered gate-first).
-        if (!a.bitness) {
-            K prod = gl::kone();
-            for (uint32_t f = 0; f < a.nf; f++) {
-                const K* s = a.tab + (uint64_t)f * a.len + 2 * p;
-                K f0 = s[0], f1 = s[1];
-                if (gl::kiszero(f0) && gl::kiszero(f1)) {
-                    prod = gl::kzero();
-                    break;
-                }
-                K v = gl::kadd(f0, gl::kscale_small(gl::ksub(f1, f0), (int32_t)x));
-                prod = gl::kmul(prod, v);
-            }
-            acc = prod;
-        } else {
-            const K* s = a.tab + 2 * p;
-            K sum = gl::kzero();
-            for (uint32_t f = 1; f < a.nf; f++) {
-                const K* c = a.tab + (uint64_t)f * a.len + 2 * p;
-                if (gl::kiszero(c[0]) && gl::kiszero(c[1])) continue;  // b(b - 1) = 0 at every x
-                K bx = gl::kadd(c[0], gl::kscale_small(gl::ksub(c[1], c[0]), (int32_t)x));
-                sum = gl::kadd(sum, gl::kmul(gl::kmul(a.w[f - 1], bx), gl::ksub(bx, gl::kone())));
-            }
-            if (!gl::kiszero(sum)) {
-                K chi = gl::kadd(s[0], gl::kscale_small(gl::ksub(s[1], s[0]), (int32_t)x));
-                acc = gl::kmul(chi, sum);
-            }
-        }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc = gl::kadd(acc, shfl_xor_km(acc, o));
-    if (lane == 0) s_red[warp] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        K s = gl::kzero();
-#pragma unroll
-        for (int w = 0; w < MT / 32; w++) s = gl::kadd(s, s_red[w]);
-        a.partials[(uint64_t)x * gridDim.x + blockIdx.x] = s;
-    }
-}
-
 // vals[x] = Σ_b partials[x][b]; one block per x
 __global__ void __launch_bounds__(256) mem_reduce_kernel(const K* __restrict__ partials, uint32_t nblocks,
                                                          K* __restrict__ vals) {
@@ -318,11 +262,10 @@ __global__ void __launch_bounds__(256) dot_kernel(const K* __restrict__ a, const
 // A batched round (the Route-A time claims, the val-eval batch, the address
 // pre-time batches) evaluates every claim's round polynomial at x = 0..deg
 // before the transcript draws the next challenge.  One kernel folds (the
-// pending challenge), evaluates and reduces (each claim's last block sums its
-// partials) the tables of up to MULTI_MAX claims together; the values land in
-// one device array that the host reads with a single copy.
+// pending challenge), evaluates and reduces the tables of up to MULTI_MAX claims
+// together; the values land in page-locked memory.
 constexpr int MULTI_MAX = 24;
-constexpr int MX = 8;  // evaluation points per pass (thread-local accumulators)
+constexpr uint32_t MULTI_TILES = 2 * 148;  // tiles of a launch that keep the SMs busy
 
 struct MultiClaim {
     const K* tab;      // [nf][len] current tables (written by this launch when src is set)
@@ -334,13 +277,59 @@ struct MultiClaim {
     K r;               // fold challenge
     uint32_t blk0;     // first block of this claim
     uint32_t part0;    // first partial [npts][nblk]
-    uint32_t nblk;     // partial columns per point: pair blocks of 256 pairs x column chunks
-    uint32_t ppt;      // evaluation points per thread (1, 2, 4 or MX): blocks = ceil(npts / ppt) * nblk
-    uint32_t nchunk;   // bitness: column chunks of BIT_CHUNK columns (1 otherwise)
+    uint32_t nblk;     // blocks of this claim (tiles dealt out in turn)
+    uint32_t hb;       // 1, 2, 4 or 8: warps per point set
+    uint32_t fs;       // lanes that share a pair's factors (1, 2, 4, .. 16)
+    uint32_t lpb;      // log2 of the pairs per tile, 32 hb / fs
+    uint32_t small;    // few pairs: one block per point (multi_small)
     K* out;            // values at x = 0..npts-1
     unsigned int* ticket;  // the claim's block counter (zero between launches)
 };
-constexpr uint32_t BIT_CHUNK = 4;  // bitness columns per thread
+
+// entries 2p, 2p + 1 of a table in one 32-byte load (read-only data, 32-byte aligned)
+__device__ __forceinline__ void ldg_pair(const K* p, K& a, K& b) {
+    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(a.re), "=l"(a.im), "=l"(b.re), "=l"(b.im) : "l"(p));
+}
+__device__ __forceinline__ K ldg_k(const K* p) {
+    const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p));
+    return gl::kmk(v.x, v.y);
+}
+
+// The pending folds of the claims with at least FOLD_PAIRS pairs, as a launch of
+// their own: most rows of the first rounds are outside the active trace, where the
+// fold is all there is to do and streams (dst[p] = lerp(src[2p], src[2p+1], r),
+// 48 bytes an entry; 100 factors of 2^16 entries: 20 us), while the evaluation's
+// tiles wait on barriers (116 us with the fold inside).  blockIdx.y:
+// a factor of one of the claims.
+constexpr uint64_t FOLD_PAIRS = 4096;
+constexpr uint32_t FOLD_PER = 2;
+struct MultiFold {
+    int n;
+    const K* src[MULTI_MAX];
+    K* dst[MULTI_MAX];
+    uint64_t half[MULTI_MAX];   // entries of a folded factor
+    uint32_t f0[MULTI_MAX + 1]; // first blockIdx.y
+    K r[MULTI_MAX];
+};
+__global__ void __launch_bounds__(256) mem_multi_fold_kernel(const __grid_constant__ MultiFold a) {
+    int c = 0;
+    while (blockIdx.y >= a.f0[c + 1]) c++;
+    const uint64_t half = a.half[c], f = blockIdx.y - a.f0[c];
+    const uint64_t p0 = blockIdx.x * (uint64_t)(256 * FOLD_PER) + threadIdx.x;
+    const K* s = a.src[c] + f * 2 * half;
+    K* d = a.dst[c] + f * half;
+    const K r = a.r[c];
+    K lo[FOLD_PER], hi[FOLD_PER];
+#pragma unroll
+    for (uint32_t e = 0; e < FOLD_PER; e++)
+        if (p0 + e * 256 < half) ldg_pair(s + 2 * (p0 + e * 256), lo[e], hi[e]);
+#pragma unroll
+    for (uint32_t e = 0; e < FOLD_PER; e++)
+        if (p0 + e * 256 < half) {
+            const K df = gl::ksub(hi[e], lo[e]);
+            d[p0 + e * 256] = gl::kiszero(df) ? lo[e] : gl::kadd(lo[e], gl::kmul(df, r));  // constant runs cost no product
+        }
+}
 
 struct MultiArgs {
     int n;
@@ -354,178 +343,209 @@ __device__ __forceinline__ int multi_claim_of(const MultiArgs& a, uint32_t blk) 
     return c;
 }
 
-// Factor f of pair p in the current round: (f0, f1) = the entries 2p, 2p+1.
-// With a pending fold they are lerp(src[4p], src[4p+1], r) and lerp(src[4p+2],
-// src[4p+3], r) -- computed here unless this thread wrote them already.
-__device__ __forceinline__ void multi_factor(const MultiClaim& c, uint32_t f, uint64_t p, bool from_tab, K& f0, K& f1) {
-    if (c.src && !from_tab) {
+// Factor f of pair p in the current round: (f0, f1) = the entries 2p, 2p+1; with
+// a pending fold lerp(src[4p], src[4p+1], r) and lerp(src[4p+2], src[4p+3], r),
+// written to the tables when `own`.
+__device__ __forceinline__ void multi_factor(const MultiClaim& c, uint32_t f, uint64_t p, bool own, K& f0, K& f1) {
+    if (c.src) {
         const K* o = c.src + (uint64_t)f * (2 * c.len) + 4 * p;
-        f0 = gl::klerp(o[0], o[1], c.r);
-        f1 = gl::klerp(o[2], o[3], c.r);
+        K o0, o1, o2, o3;
+        ldg_pair(o, o0, o1);
+        ldg_pair(o + 2, o2, o3);
+        f0 = gl::klerp(o0, o1, c.r);
+        f1 = gl::klerp(o2, o3, c.r);
+        if (own) {
+            K* t = const_cast<K*>(c.tab) + (uint64_t)f * c.len + 2 * p;
+            t[0] = f0;
+            t[1] = f1;
+        }
         return;
     }
-    const K* s = c.tab + (uint64_t)f * c.len + 2 * p;
-    f0 = s[0];
-    f1 = s[1];
+    ldg_pair(c.tab + (uint64_t)f * c.len + 2 * p, f0, f1);
 }
 
-// The pending fold of the factors this thread owns (point group 0: every
-// factor, or for a bitness claim its column chunk and, in chunk 0, chi).
-__device__ __forceinline__ void multi_fold_owned(const MultiClaim& c, uint64_t p, uint32_t ch) {
-    K* t = const_cast<K*>(c.tab);
-    auto one = [&](uint32_t f) {
-        const K* o = c.src + (uint64_t)f * (2 * c.len) + 4 * p;
-        t[(uint64_t)f * c.len + 2 * p] = gl::klerp(o[0], o[1], c.r);
-        t[(uint64_t)f * c.len + 2 * p + 1] = gl::klerp(o[2], o[3], c.r);
+// A claim with at most SMALL_PAIRS pairs (its last rounds): one block per point x
+// does every pair, so there is nothing to add up between blocks.  fs lanes share a
+// pair's factors and multiply (bitness: add) their parts with shuffles: the launch
+// is one dependent chain, and a thread walking 15 factors took 22 to 30 us where
+// this takes 8.  Block 0 writes the folded tables.
+constexpr uint32_t SMALL_PAIRS = 16;
+__device__ __noinline__ void multi_small(const MultiClaim& c, uint32_t x, K* s_sum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t fs = c.fs, sub = threadIdx.x & (fs - 1), p = threadIdx.x / fs;
+    const bool live = p < (uint32_t)(c.len >> 1);
+    auto value = [&](uint32_t f) {  // factor f at x
+        K f0, f1;
+        multi_factor(c, f, p, x == 0, f0, f1);
+        return gl::kadd(f0, gl::kscale_tiny(gl::ksub(f1, f0), x));
     };
+    K acc;
     if (!c.bitness) {
-        for (uint32_t f = 0; f < c.nf; f++) one(f);
-        return;
-    }
-    if (ch == 0) one(0);
-    const uint32_t f_lo = 1 + ch * BIT_CHUNK, f_hi = min(c.nf, f_lo + BIT_CHUNK);
-    for (uint32_t f = f_lo; f < f_hi; f++) one(f);
-}
-
-// Values of one pair at x = x0 .. x0 + PPT - 1: the product of the claim's
-// affine factors (a factor zero on both children zeroes every point), or for
-// a bitness claim chi(x) times the weighted b(b - 1) sum over the columns of
-// chunk ch, additions along x.  own: this thread folded its factors already.
-template <int PPT>
-__device__ __forceinline__ void multi_eval_points(const MultiClaim& c, uint64_t p, uint32_t x0, uint32_t ch, bool own,
-                                                  K* acc) {
-    if (!c.bitness) {
-#pragma unroll
-        for (int i = 0; i < PPT; i++) acc[i] = gl::kone();
-        for (uint32_t f = 0; f < c.nf; f++) {
-            K f0, f1;
-            multi_factor(c, f, p, own, f0, f1);
-            if (gl::kiszero(f0) && gl::kiszero(f1)) {
-#pragma unroll
-                for (int i = 0; i < PPT; i++) acc[i] = gl::kzero();
-                return;
-            }
-            const K d = gl::ksub(f1, f0);
-            K v = gl::kadd(f0, gl::kscale_small(d, (int32_t)x0));
-#pragma unroll
-            for (int i = 0; i < PPT; i++) {
-                acc[i] = gl::kmul(acc[i], v);
-                v = gl::kadd(v, d);
+        acc = gl::kone();
+        if (live) {
+#pragma unroll 2
+            for (uint32_t f = sub; f < c.nf; f += fs) acc = gl::kmul(acc, value(f));
+        }
+        for (uint32_t o = 1; o < fs; o <<= 1) acc = gl::kmul(acc, shfl_xor_km(acc, o));
+    } else {
+        acc = gl::kzero();
+        if (live) {
+#pragma unroll 2
+            for (uint32_t f = 1 + sub; f < c.nf; f += fs) {
+                const K v = value(f);
+                acc = gl::kadd(acc, gl::kmul(c.w[f - 1], gl::kmul(v, gl::ksub(v, gl::kone()))));
             }
         }
-        return;
+        for (uint32_t o = 1; o < fs; o <<= 1) acc = gl::kadd(acc, shfl_xor_km(acc, o));
+        if (live && sub == 0) acc = gl::kmul(acc, value(0));
     }
+    K total = live && sub == 0 ? acc : gl::kzero();
 #pragma unroll
-    for (int i = 0; i < PPT; i++) acc[i] = gl::kzero();
-    const uint32_t f_lo = 1 + ch * BIT_CHUNK, f_hi = min(c.nf, f_lo + BIT_CHUNK);
-    // the chunk's column pairs are loaded together (one memory round trip)
-    K b0[BIT_CHUNK], b1[BIT_CHUNK];
-#pragma unroll
-    for (uint32_t u = 0; u < BIT_CHUNK; u++) {
-        if (f_lo + u < f_hi) multi_factor(c, f_lo + u, p, own, b0[u], b1[u]);
-        else b0[u] = b1[u] = gl::kzero();
-    }
-    bool any = false;
-#pragma unroll
-    for (uint32_t u = 0; u < BIT_CHUNK; u++) {
-        if (gl::kiszero(b0[u]) && gl::kiszero(b1[u])) continue;  // b(b - 1) = 0 at every x
-        any = true;
-        const K d = gl::ksub(b1[u], b0[u]), w = c.w[f_lo + u - 1];
-        K v = gl::kadd(b0[u], gl::kscale_small(d, (int32_t)x0));
-#pragma unroll
-        for (int i = 0; i < PPT; i++) {
-            acc[i] = gl::kadd(acc[i], gl::kmul(w, gl::kmul(v, gl::ksub(v, gl::kone()))));
-            v = gl::kadd(v, d);
-        }
-    }
-    if (!any) return;
-    K f0, f1;
-    multi_factor(c, 0, p, own && ch == 0, f0, f1);
-    const K d = gl::ksub(f1, f0);
-    K v = gl::kadd(f0, gl::kscale_small(d, (int32_t)x0));
-#pragma unroll
-    for (int i = 0; i < PPT; i++) {
-        acc[i] = gl::kmul(acc[i], v);
-        v = gl::kadd(v, d);
+    for (int o = 16; o > 0; o >>= 1) total = gl::kadd(total, shfl_xor_km(total, o));
+    if (lane == 0) s_sum[warp] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) total = gl::kadd(total, s_sum[w]);
+        c.out[x] = total;
     }
 }
 
-// Block (point group g, partial column r) of one claim: r = ch * (pair
-// blocks) + pair block pb; thread t takes pair pb * 256 + t (bitness: its
-// column chunk ch) at the claim's ppt points x0 = g * ppt ..; each point is
-// reduced over the block into partials[x][r].  A claim with many pairs takes
-// MX points per thread (its factor pairs read once per MX points); one with
-// few pairs (the late rounds) takes fewer, so that its point groups run side
-// by side instead of one thread walking every point.
+// Larger claims: a block takes tiles of 32 hb / fs pairs, dealt out in turn so that
+// the active rows (a run at the start of the time domain) spread over the blocks.
+// Per chunk of factors the block folds the tile once (the folded tables go out, f0
+// and f1 - f0 of every pair into shared memory), then warp (x set, pair group)
+// multiplies up its points x, x + 8 / hb, .. with fs lanes per pair.  A tile whose
+// gate (factor 1: has_lookup / has_read / has_write behind chi; factor 0 where no
+// chi leads) is zero on both children of every pair adds nothing at any x; a
+// bitness column that is zero adds nothing either.  What bounds it: the arithmetic
+// of the active tiles, which is why few pairs are cut into smaller tiles (a Twist
+// read check of 15 factors and 16 points with 2^14 of 2^16 rows active: first
+// round 43 us, at 2^10 pairs 15; with one thread per pair walking the factors
+// at up to 8 points 96 and 44, with 32 pairs a tile throughout 52 and 26).
+constexpr uint32_t MF = 512;     // (factor, pair) entries per chunk
+constexpr int MPTS = 4;          // points per warp: npts <= 32, 8 / hb point sets
 __global__ void __launch_bounds__(256) mem_multi_eval_kernel(const __grid_constant__ MultiArgs a) {
-    __shared__ K s_red[256 / 32][MX];
+    __shared__ K s_f[2][MF];    // f0, f1 - f0: [factor][pair]
+    __shared__ K s_red[8][MPTS];
+    __shared__ uint8_t s_on[256];
     const int ci = multi_claim_of(a, blockIdx.x);
     const MultiClaim& c = a.c[ci];
     const uint32_t b = blockIdx.x - c.blk0;
-    const uint32_t g = b / c.nblk, pb = b % c.nblk;  // pb: the partial column
-    const uint32_t nbp = c.nblk / c.nchunk;          // pair blocks
-    const uint32_t ch = pb / nbp;
-    const uint32_t x0 = g * c.ppt;
-    const uint32_t np = min(c.ppt, c.npts - x0);
-    const uint64_t pairs = c.len >> 1;
-    const uint64_t p = (uint64_t)(pb % nbp) * 256 + threadIdx.x;
+    if (c.small) {
+        multi_small(c, b, &s_red[0][0]);
+        return;
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // a product whose gate factor (factor 1: has_lookup / has_read /
-    // has_write behind chi; factor 0 where no chi leads) is zero on both
-    // children contributes nothing at any x
-    bool live = p < pairs;
-    // a pending fold: point group 0 writes the folded tables of its pairs
-    const bool own = c.src && g == 0;
-    if (live && own) multi_fold_owned(c, p, ch);
-    if (live && !c.bitness) {
-        K a0, a1, b0, b1;
-        multi_factor(c, 0, p, own, a0, a1);
-        multi_factor(c, c.nf > 1 ? 1 : 0, p, own, b0, b1);
-        live = !(gl::kiszero(a0) && gl::kiszero(a1)) && !(gl::kiszero(b0) && gl::kiszero(b1));
-    }
-    K acc[MX];
+    const uint32_t hb = c.hb, fs = c.fs, lpb = c.lpb, pb = 1u << lpb, fch = MF >> lpb, xstep = 8 / hb;
+    const uint32_t sub = lane & (fs - 1), pl = (warp % hb) * (32 / fs) + lane / fs;  // factor share, pair of the tile
+    const uint32_t xw = warp / hb;  // first point
+    const uint64_t pairs = c.len >> 1, tiles = (pairs + pb - 1) / pb;
+    const uint32_t gate = c.nf > 1 ? 1u : 0u;
+    K total[MPTS];
 #pragma unroll
-    for (int i = 0; i < MX; i++) acc[i] = gl::kzero();
-    if (live) {
-        switch (c.ppt) {
-            case 1: multi_eval_points<1>(c, p, x0, ch, own, acc); break;
-            case 2: multi_eval_points<2>(c, p, x0, ch, own, acc); break;
-            case 4: multi_eval_points<4>(c, p, x0, ch, own, acc); break;
-            default: multi_eval_points<MX>(c, p, x0, ch, own, acc); break;
+    for (int k = 0; k < MPTS; k++) total[k] = gl::kzero();
+    // with no fold to do, 256 pairs of the block's coming tiles are looked over first
+    // (every column of a bitness claim, else the gate) and tiles without any are skipped
+    const bool scan = !c.src;
+    const uint32_t tps = 256 >> lpb;
+    for (uint64_t i = 0; b + i * c.nblk < tiles; i++) {
+        const uint64_t tile = b + i * c.nblk;
+        if (scan && i % tps == 0) {
+            __syncthreads();
+            if (threadIdx.x < tps) s_on[threadIdx.x] = 0;
+            __syncthreads();
+            const uint64_t p = (b + (i + (threadIdx.x >> lpb)) * c.nblk) * pb + (threadIdx.x & (pb - 1));
+            bool nz = false;
+            if (p < pairs) {
+                const uint32_t fl = c.bitness ? 1 : gate, fh = c.bitness ? c.nf : gate + 1;
+#pragma unroll 4
+                for (uint32_t f = fl; f < fh; f++) {
+                    K f0, f1;
+                    ldg_pair(c.tab + (uint64_t)f * c.len + 2 * p, f0, f1);
+                    nz = nz || !gl::kiszero(f0) || !gl::kiszero(f1);
+                }
+            }
+            if (nz) s_on[threadIdx.x >> lpb] = 1;
+            __syncthreads();
+        }
+        if (scan && !s_on[i % tps]) continue;  // block-uniform
+        K acc[MPTS], chi[MPTS];
+#pragma unroll
+        for (int k = 0; k < MPTS; k++) acc[k] = c.bitness ? gl::kzero() : gl::kone();
+        bool on = true;
+        for (uint32_t fb = 0; fb < c.nf; fb += fch) {
+            const uint32_t nfc = min(fch, c.nf - fb);
+            bool nz = c.bitness;
+            for (uint32_t e = threadIdx.x; e < nfc * pb; e += 256) {
+                const uint32_t f = e >> lpb;
+                const uint64_t p = tile * pb + (e & (pb - 1));
+                K f0 = gl::kzero(), f1 = gl::kzero();
+                if (p < pairs) multi_factor(c, fb + f, p, true, f0, f1);
+                if (!c.bitness && fb + f == gate) nz = nz || !gl::kiszero(f0) || !gl::kiszero(f1);
+                s_f[0][e] = f0;
+                s_f[1][e] = gl::ksub(f1, f0);
+            }
+            if (fb == 0 && !scan) on = __syncthreads_or(nz);
+            else __syncthreads();
+            if (on && xw < c.npts) {
+                for (uint32_t f = sub; f < nfc; f += fs) {
+                    const K f0 = s_f[0][(f << lpb) + pl], d = s_f[1][(f << lpb) + pl];
+                    const bool chi_f = c.bitness && fb + f == 0;
+                    if (c.bitness && !chi_f && gl::kiszero(f0) && gl::kiszero(d)) continue;
+                    K v = gl::kadd(f0, gl::kscale_tiny(d, xw));
+                    const K dx = gl::kscale_tiny(d, xstep);
+                    const K w = c.bitness && !chi_f ? ldg_k(c.w + fb + f - 1) : gl::kzero();
+#pragma unroll
+                    for (int k = 0; k < MPTS; k++) {
+                        if (xw + k * xstep >= c.npts) break;
+                        if (!c.bitness) acc[k] = gl::kmul(acc[k], v);
+                        else if (chi_f) chi[k] = v;
+                        else acc[k] = gl::kadd(acc[k], gl::kmul(w, gl::kmul(v, gl::ksub(v, gl::kone()))));
+                        v = gl::kadd(v, dx);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        if (on && xw < c.npts) {  // warp-uniform
+            const bool add = sub == 0 && tile * pb + pl < pairs;
+#pragma unroll
+            for (int k = 0; k < MPTS; k++) {
+                if (xw + k * xstep >= c.npts) break;
+                for (uint32_t o = 1; o < fs; o <<= 1) {
+                    const K other = shfl_xor_km(acc[k], o);
+                    acc[k] = c.bitness ? gl::kadd(acc[k], other) : gl::kmul(acc[k], other);
+                }
+                if (add) total[k] = gl::kadd(total[k], c.bitness ? gl::kmul(chi[k], acc[k]) : acc[k]);
+            }
         }
     }
-    const bool any = __syncthreads_or(live);
-    if (!any) {
-        if (threadIdx.x < np) a.partials[c.part0 + (uint64_t)(x0 + threadIdx.x) * c.nblk + pb] = gl::kzero();
-    } else {
 #pragma unroll
-        for (int i = 0; i < MX; i++) {
-            if ((uint32_t)i >= np) break;
-            K v = acc[i];
+    for (int k = 0; k < MPTS; k++) {
+        if (xw + k * xstep >= c.npts) break;
+        K v = total[k];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v = gl::kadd(v, shfl_xor_km(v, o));
-            if (lane == 0) s_red[warp][i] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < np) {
-            K v = gl::kzero();
-#pragma unroll
-            for (int w = 0; w < 256 / 32; w++) v = gl::kadd(v, s_red[w][threadIdx.x]);
-            a.partials[c.part0 + (uint64_t)(x0 + threadIdx.x) * c.nblk + pb] = v;
-        }
+        for (int o = 16; o > 0; o >>= 1) v = gl::kadd(v, shfl_xor_km(v, o));
+        if (lane == 0) s_red[warp][k] = v;
     }
+    __syncthreads();
+    if (threadIdx.x < c.npts) {
+        const uint32_t x = threadIdx.x;
+        K v = gl::kzero();
+        for (uint32_t g = 0; g < hb; g++) v = gl::kadd(v, s_red[(x % xstep) * hb + g][x / xstep]);
+        if (c.nblk == 1) c.out[x] = v;
+        else a.partials[c.part0 + (uint64_t)x * c.nblk + b] = v;
+    }
+    if (c.nblk == 1) return;
     // the claim's last block to finish sums its partials (ticket, no waits)
     __threadfence();
     __syncthreads();
     __shared__ unsigned int s_last;
-    const uint32_t claim_blocks = c.nblk * ((c.npts + c.ppt - 1) / c.ppt);
-    if (threadIdx.x == 0) s_last = atomicInc(c.ticket, claim_blocks - 1) == claim_blocks - 1;
+    if (threadIdx.x == 0) s_last = atomicInc(c.ticket, c.nblk - 1) == c.nblk - 1;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // one warp per point: the points' sums run side by side (a claim of the
-    // late rounds has one partial per point, so this tail is a few load
-    // latencies instead of one block-wide reduction per point)
+    // one warp per point: the points' sums run side by side
     for (uint32_t x = warp; x < c.npts; x += 256 / 32) {
         K v = gl::kzero();
 #pragma unroll 4
@@ -556,9 +576,10 @@ struct neo_gpu_mem_oracle {
     K pending_r{};
     DevBuf<K> w;          // bitness weights
     std::vector<K> hw;    // host copy of the weights
-    DevBuf<K> partials, vals;
+    DevBuf<K> partials;
     DevBuf<K> dpt, dra, tmp, sums;  // build workspace, kept for reuse
     std::vector<K> hvals;
+    bool hvals_valid = false;  // hvals holds this round's values (the claim needs round 0's)
     K claim{};
 };
 
@@ -601,57 +622,6 @@ uint32_t degree_of(int kind, uint32_t A, uint32_t n_cols) {
     return 0;
 }
 
-// round values at x = 0..deg into o->hvals (applies a pending fold first)
-int mem_round_values(neo_gpu_mem_oracle* o) {
-    neo_gpu_ctx* ctx = o->ctx;
-    if (o->pending) {
-        K* src = o->tab[o->cur].p;
-        K* dst = o->tab[o->cur ^ 1].p;
-        uint64_t tot = (o->len >> 1) * o->nf;
-        mem_fold_kernel<<<ceil_div(tot, 256), 256, 0, ctx->stream>>>(src, o->len, dst, o->nf, o->pending_r);
-        NEO_LAUNCHED(ctx);
-        o->cur ^= 1;
-        o->len >>= 1;
-        o->pending = false;
-    }
-    const uint32_t npts = o->deg + 1;
-    o->hvals.assign(npts, gl::kzero());
-    if (o->len == 1) {
-        std::vector<K> v(o->nf);
-        NEO_CK(ctx, ctx_d2h(ctx, v.data(), o->tab[o->cur].p, o->nf * sizeof(K)));
-        NEO_CK(ctx, ctx_sync(ctx));
-        K val;
-        if (o->bitness) {
-            K s = gl::kzero();
-            for (uint32_t f = 1; f < o->nf; f++)
-                s = gl::kadd(s, gl::kmul(gl::kmul(o->hw[f - 1], v[f]), gl::ksub(v[f], gl::kone())));
-            val = gl::kmul(v[0], s);
-        } else {
-            val = gl::kone();
-            for (uint32_t f = 0; f < o->nf; f++) val = gl::kmul(val, v[f]);
-        }
-        for (auto& h : o->hvals) h = val;
-        return NEO_OK;
-    }
-    const uint64_t pairs = o->len >> 1;
-    const uint32_t nb = (uint32_t)ceil_div(pairs, MT);
-    NEO_CK(ctx, o->partials.ensure((size_t)nb * npts));
-    MemEvalArgs a;
-    a.tab = o->tab[o->cur].p;
-    a.len = o->len;
-    a.nf = o->nf;
-    a.bitness = o->bitness;
-    a.w = o->w.p;
-    a.partials = o->partials.p;
-    mem_eval_kernel<<<dim3(nb, npts), MT, 0, ctx->stream>>>(a);
-    NEO_LAUNCHED(ctx);
-    mem_reduce_kernel<<<npts, 256, 0, ctx->stream>>>(o->partials.p, nb, o->vals.p);
-    NEO_LAUNCHED(ctx);
-    NEO_CK(ctx, ctx_d2h(ctx, o->hvals.data(), o->vals.p, npts * sizeof(K)));
-    NEO_CK(ctx, ctx_sync(ctx));
-    return NEO_OK;
-}
-
 // p(x) from p(0..n-1) (Lagrange on the integer nodes)
 K lagrange_at(const std::vector<K>& v, K x) {
     const int n = (int)v.size();
@@ -669,6 +639,8 @@ K lagrange_at(const std::vector<K>& v, K x) {
     }
     return acc;
 }
+
+int mem_round_values(neo_gpu_mem_oracle* o);
 
 int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point, uint32_t A, const uint64_t* r_addr,
                const uint64_t* init, uint32_t n_cols, const uint64_t* cols, bool cols_on_device,
@@ -699,6 +671,7 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
     o->bit_idx = 0;
     o->cur = 0;
     o->pending = false;
+    o->hvals_valid = false;
     o->hw.clear();
     o->kind = kind;
     o->ell = ell;
@@ -712,15 +685,17 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
         if (fresh) delete o;
         return rc;
     };
-    if (o->tab[0].ensure((size_t)o->nf * L) || o->tab[1].ensure((size_t)o->nf * (L > 1 ? L / 2 : 1)) ||
-        o->vals.ensure(deg + 1))
+    if (o->tab[0].ensure((size_t)o->nf * L) || o->tab[1].ensure((size_t)o->nf * (L > 1 ? L / 2 : 1)))
         return fail(ctx->fail(NEO_ERR_OOM, "mem_oracle: table allocation"));
     K* T = o->tab[0].p;
     cudaStream_t S = ctx->stream;
     const cudaMemcpyKind cpk = cols_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     const size_t colb = L * sizeof(K);
     auto col = [&](uint32_t c) { return reinterpret_cast<const K*>(cols) + (size_t)c * L; };
-    auto put = [&](uint32_t f, uint32_t c) { return cudaMemcpyAsync(T + (size_t)f * L, col(c), colb, cpk, S); };
+    // factors f.. = columns c.. (n of them, adjacent)
+    auto put = [&](uint32_t f, uint32_t c, uint32_t n = 1) {
+        return n ? cudaMemcpyAsync(T + (size_t)f * L, col(c), colb * n, cpk, S) : cudaSuccess;
+    };
     DevBuf<K>& dpt = o->dpt;
     DevBuf<K>& dra = o->dra;
     DevBuf<K>& tmp = o->tmp;
@@ -734,9 +709,9 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
     auto eqbits = [&](uint32_t f0, uint32_t c0) -> int {
         if (!A) return NEO_OK;
         if (!r_addr) return ctx->fail(NEO_ERR_ARG, "mem_oracle: address bits without r_addr");
-        for (uint32_t b = 0; b < A; b++)
-            if (put(f0 + b, c0 + b)) return ctx->fail(NEO_ERR_CUDA, "mem_oracle: column upload");
-        eqbit_kernel<<<ceil_div(L * A, 256), 256, 0, S>>>(T + (size_t)f0 * L, L, A, dra.p);  // all A columns at once
+        K* dst = T + (size_t)f0 * L;
+        if (!cols_on_device && put(f0, c0, A)) return ctx->fail(NEO_ERR_CUDA, "mem_oracle: column upload");
+        eqbit_kernel<<<dim3(ceil_div(L, 256), A), 256, 0, S>>>(cols_on_device ? col(c0) : dst, L, dra.p, dst);
         NEO_LAUNCHED(ctx);
         return NEO_OK;
     };
@@ -768,15 +743,14 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
     cudaError_t ce = cudaSuccess;
     switch (kind) {
         case NEO_MEM_SHOUT_VALUE:
-            ce = put(1, 0);
-            if (!ce) ce = put(2, 1);
+            ce = put(1, 0, 2);
             break;
         case NEO_MEM_SHOUT_ADAPTER:
             ce = put(1, 0);
             if (!ce) rc = eqbits(2, 1);
             break;
         case NEO_MEM_BITNESS:
-            for (uint32_t c = 0; c < n_cols && !ce; c++) ce = put(1 + c, c);
+            ce = put(1, 0, n_cols);
             for (uint32_t c = 0; c < n_cols; c++) o->hw.push_back(kload_h(weights + 2 * c));
             if (!ce && n_cols && (o->w.ensure(n_cols) ||
                         cudaMemcpyAsync(o->w.p, weights, n_cols * sizeof(K), cudaMemcpyHostToDevice, S)))
@@ -788,16 +762,18 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
             // write stream columns: has_write, inc, wa bits
             const uint32_t c_hw = rd ? 2 + A : 0, c_inc = rd ? 3 + A : 2, c_wa = rd ? 4 + A : 3;
             const uint32_t c_a = rd ? 1 : 1;  // rv (read) or wv (write)
-            if (tmp.ensure((size_t)(4 + A) * L)) { ce = cudaErrorMemoryAllocation; break; }
-            K* hw = tmp.p;
-            K* inc = tmp.p + L;
-            K* aa = tmp.p + 2 * L;
-            K* terms = tmp.p + 3 * L;
-            K* wa = tmp.p + 4 * L;
-            ce = cudaMemcpyAsync(hw, col(c_hw), colb, cpk, S);
-            if (!ce) ce = cudaMemcpyAsync(inc, col(c_inc), colb, cpk, S);
-            if (!ce) ce = cudaMemcpyAsync(aa, col(c_a), colb, cpk, S);
-            if (!ce && A) ce = cudaMemcpyAsync(wa, col(c_wa), colb * A, cpk, S);
+            // columns on the device are read where they are
+            if (tmp.ensure((cols_on_device ? 1 : (size_t)(4 + A)) * L)) { ce = cudaErrorMemoryAllocation; break; }
+            K* terms = tmp.p;
+            const K *hw = col(c_hw), *inc = col(c_inc), *aa = col(c_a), *wa = col(c_wa);
+            if (!cols_on_device) {
+                K* up = tmp.p + L;
+                ce = cudaMemcpyAsync(up, hw, colb, cpk, S);
+                if (!ce) ce = cudaMemcpyAsync(up + L, inc, colb, cpk, S);
+                if (!ce) ce = cudaMemcpyAsync(up + 2 * L, aa, colb, cpk, S);
+                if (!ce && A) ce = cudaMemcpyAsync(up + 3 * L, wa, colb * A, cpk, S);
+                hw = up; inc = up + L; aa = up + 2 * L; wa = up + 3 * L;
+            }
             if (ce) break;
             inc_terms_kernel<<<ceil_div(L, 256), 256, 0, S>>>(hw, inc, wa, A, dra.p, L, terms);
             NEO_LAUNCHED(ctx);
@@ -816,20 +792,18 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
             if (!ce) rc = eqbits(3, rd ? 2 : 3);
         } break;
         case NEO_MEM_VAL_EVAL:
-            ce = put(0, 0);
-            if (!ce) ce = put(1, 1);
+            ce = put(0, 0, 2);
             if (ce) break;
             lt_table_kernel<<<ceil_div(L, 256), 256, 0, S>>>(dpt.p, ell, T + 2 * L);
             NEO_LAUNCHED(ctx);
             rc = eqbits(3, 2);
             break;
         case NEO_MEM_TOTAL_INC:
-            ce = put(0, 0);
-            if (!ce) ce = put(1, 1);
+            ce = put(0, 0, 2);
             if (!ce) rc = eqbits(2, 2);
             break;
         case NEO_MEM_PRODUCT:
-            for (uint32_t c = 0; c < n_cols && !ce; c++) ce = put(c, c);
+            ce = put(0, 0, n_cols);
             break;
     }
     if (ce) return fail(ctx->fail(ce == cudaErrorMemoryAllocation ? NEO_ERR_OOM : NEO_ERR_CUDA, "mem_oracle: build", ce));
@@ -869,19 +843,38 @@ int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int 
     if (n > MULTI_MAX) return ctx->fail(NEO_ERR_UNSUPPORTED, "mem_round_launch_multi: too many claims");
     MultiArgs a{};
     a.n = n;
+    // a launch's blocks, shared out by what a claim reads of the inactive rows: every
+    // column of a bitness claim, the gate of a product (which gets as much as 8 columns
+    // for its products)
+    auto multi_weight = [](const neo_gpu_mem_oracle* o) -> uint64_t { return o->bitness ? o->nf : 8; };
+    uint64_t wsum = 0;
+    for (int i = 0; i < n; i++) wsum += multi_weight(os[i]);
+    MultiFold mf{};
+    uint64_t fold_len = 0;
     uint32_t blocks = 0;
     uint64_t parts = 0;
     for (int i = 0; i < n; i++) {
         neo_gpu_mem_oracle* o = os[i];
         MultiClaim& c = a.c[i];
-        c.src = nullptr;
-        if (o->pending) {  // the evaluation launch applies the fold (point group 0 writes the tables)
+        c = MultiClaim{};
+        if (o->pending) {  // a small claim's evaluation applies the fold; a large one's is a launch of its own
             c.src = o->tab[o->cur].p;
             c.r = o->pending_r;
             o->cur ^= 1;
             o->len >>= 1;
             o->pending = false;
+            if (o->len >= 2 * FOLD_PAIRS) {
+                mf.src[mf.n] = c.src;
+                mf.dst[mf.n] = o->tab[o->cur].p;
+                mf.half[mf.n] = o->len;
+                mf.r[mf.n] = c.r;
+                mf.f0[mf.n + 1] = mf.f0[mf.n] + o->nf;
+                mf.n++;
+                fold_len = std::max(fold_len, o->len);
+                c.src = nullptr;
+            }
         }
+        o->hvals_valid = false;
         if (o->len < 2) return ctx->fail(NEO_ERR_INVARIANT, "mem_round_launch_multi: no pairs left");
         c.tab = o->tab[o->cur].p;
         c.len = o->len;
@@ -890,18 +883,30 @@ int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int 
         c.bitness = o->bitness;
         c.w = o->w.p;
         c.blk0 = blocks;
-        c.nchunk = o->bitness ? std::max<uint32_t>(1, (uint32_t)ceil_div(o->nf - 1, BIT_CHUNK)) : 1;
-        c.nblk = (uint32_t)ceil_div(o->len >> 1, 256) * c.nchunk;
-        // points per thread: MX while the pairs fill the GPU, fewer for the
-        // small tables of the late rounds (their point groups run in parallel),
-        // never more than the claim's points rounded up to a power of two
-        const uint64_t pairs = o->len >> 1;
-        uint32_t ppt = pairs >= 8192 ? MX : (pairs >= 1024 ? 4 : (pairs >= 256 ? 2 : 1));
-        while (ppt > 1 && ppt / 2 >= c.npts) ppt /= 2;
-        c.ppt = ppt;
         c.part0 = (uint32_t)parts;
         c.out = d_out[i];
-        blocks += c.nblk * (uint32_t)ceil_div(c.npts, c.ppt);
+        const uint64_t pairs = o->len >> 1;
+        if (pairs <= SMALL_PAIRS) {
+            // lanes per pair: what 256 threads leave, up to 16 and to the factors there are
+            c.small = 1;
+            c.fs = 1;
+            while (c.fs < 16 && 2 * c.fs * pairs <= 256 && c.fs < c.nf - (c.bitness ? 1 : 0)) c.fs *= 2;
+            blocks += c.npts;
+            continue;
+        }
+        // eight warps cover the points; with fewer points, warps share a point's pairs
+        c.hb = 1;
+        while (c.hb < 8 && 8 / (2 * c.hb) >= c.npts) c.hb *= 2;
+        // about four blocks per SM over the launch's claims; tiles small enough
+        // for two per SM (up to 16 lanes a pair)
+        c.fs = 1;
+        while (c.fs < 16 && 2 * c.fs <= c.nf && pairs * c.fs / (32 * c.hb) < MULTI_TILES / (uint32_t)n) c.fs *= 2;
+        c.lpb = 5;
+        for (uint32_t h = 1; h < c.hb; h *= 2) c.lpb++;
+        for (uint32_t h = 1; h < c.fs; h *= 2) c.lpb--;
+        const uint64_t tiles = (pairs + (1ull << c.lpb) - 1) >> c.lpb;
+        c.nblk = (uint32_t)std::min<uint64_t>(tiles, std::max<uint64_t>(64, 4ull * 148 * multi_weight(o) / wsum));
+        blocks += c.nblk;
         parts += (uint64_t)c.npts * c.nblk;
     }
     if (parts > 0xFFFFFFFFull) return ctx->fail(NEO_ERR_UNSUPPORTED, "mem_round_launch_multi: too many partials");
@@ -918,6 +923,10 @@ int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int 
         NEO_CK(ctx, cudaMemsetAsync(tickets, 0, MULTI_TICKET_K * sizeof(K), ctx->stream));
     for (int i = 0; i < n; i++) a.c[i].ticket = tickets + i;
     a.partials = partials.p;
+    if (mf.n) {
+        mem_multi_fold_kernel<<<dim3(ceil_div(fold_len, 256 * FOLD_PER), mf.f0[mf.n]), 256, 0, ctx->stream>>>(mf);
+        NEO_LAUNCHED(ctx);
+    }
     mem_multi_eval_kernel<<<blocks, 256, 0, ctx->stream>>>(a);
     NEO_LAUNCHED(ctx);
     return NEO_OK;
@@ -925,11 +934,57 @@ int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int 
 
 
 
+namespace {
+
+// round values at x = 0..deg into o->hvals (applies a pending fold first); the
+// launch writes them into the context's host-mapped result buffer
+int mem_round_values(neo_gpu_mem_oracle* o) {
+    if (o->hvals_valid) return NEO_OK;
+    neo_gpu_ctx* ctx = o->ctx;
+    const uint32_t npts = o->deg + 1;
+    o->hvals.assign(npts, gl::kzero());
+    if (mem_round_multi_ok(o)) {
+        K* out = reinterpret_cast<K*>(ctx->h_result);
+        if (int rc = mem_round_launch_multi(ctx, &o, 1, &out, o->partials)) return rc;
+        NEO_CK(ctx, ctx_sync(ctx));
+        for (uint32_t x = 0; x < npts; x++) o->hvals[x] = out[x];
+        o->hvals_valid = true;
+        return NEO_OK;
+    }
+    if (o->pending) {
+        mem_fold_kernel<<<ceil_div((o->len >> 1) * o->nf, 256), 256, 0, ctx->stream>>>(
+            o->tab[o->cur].p, o->len, o->tab[o->cur ^ 1].p, o->nf, o->pending_r);
+        NEO_LAUNCHED(ctx);
+        o->cur ^= 1;
+        o->len >>= 1;
+        o->pending = false;
+    }
+    // one entry per factor: the final product at every x
+    std::vector<K> v(o->nf);
+    NEO_CK(ctx, ctx_d2h(ctx, v.data(), o->tab[o->cur].p, o->nf * sizeof(K)));
+    NEO_CK(ctx, ctx_sync(ctx));
+    K val;
+    if (o->bitness) {
+        K s = gl::kzero();
+        for (uint32_t f = 1; f < o->nf; f++)
+            s = gl::kadd(s, gl::kmul(gl::kmul(o->hw[f - 1], v[f]), gl::ksub(v[f], gl::kone())));
+        val = gl::kmul(v[0], s);
+    } else {
+        val = gl::kone();
+        for (uint32_t f = 0; f < o->nf; f++) val = gl::kmul(val, v[f]);
+    }
+    for (auto& h : o->hvals) h = val;
+    o->hvals_valid = true;
+    return NEO_OK;
+}
+
+}  // namespace
+
 // Claims (sums over the hypercube, p_0(0) + p_0(1)) of n lazily built oracles:
-// one multi-claim evaluation of their round 0, one copy and one sync;
+// one multi-claim evaluation of their round 0 into page-locked memory, one sync;
 // oracles the multi-claim kernel cannot take are evaluated one by one.
 int mem_claims_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* claims, DevBuf<K>& partials,
-                     DevBuf<K>& d_slots, HostBuf<K>& h_slots) {
+                     HostBuf<K>& h_slots) {
     constexpr uint32_t SLOT = MEM_MAX_DEG + 1;
     bool multi = n > 0 && n <= MULTI_MAX;
     for (int i = 0; i < n && multi; i++) multi = mem_round_multi_ok(os[i]) && !os[i]->pending && os[i]->ell > 0;
@@ -943,12 +998,10 @@ int mem_claims_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* 
         NEO_CK(ctx, ctx_sync(ctx));
         return NEO_OK;
     }
-    NEO_CK(ctx, d_slots.ensure((size_t)n * SLOT));
     NEO_CK(ctx, h_slots.ensure((size_t)n * SLOT));
     std::vector<K*> dst(n);
-    for (int i = 0; i < n; i++) dst[i] = d_slots.p + (size_t)i * SLOT;
+    for (int i = 0; i < n; i++) dst[i] = h_slots.p + (size_t)i * SLOT;
     if (int rc = mem_round_launch_multi(ctx, os, n, dst.data(), partials)) return rc;
-    NEO_CK(ctx, cudaMemcpyAsync(h_slots.p, d_slots.p, (size_t)n * SLOT * sizeof(K), cudaMemcpyDeviceToHost, ctx->stream));
     NEO_CK(ctx, ctx_sync(ctx));
     for (int i = 0; i < n; i++) {
         const K* v = h_slots.p + (size_t)i * SLOT;
@@ -1016,6 +1069,7 @@ static int neo_gpu_mem_oracle_fold_impl_abi(neo_gpu_mem_oracle* o, const uint64_
     if (!o) return NEO_ERR_ARG;
     if (!r) return o->ctx->fail(NEO_ERR_ARG, "mem_oracle_fold: null challenge");
     if (o->bit_idx >= o->ell) return NEO_OK;  // no rounds left: ignored, as in the reference
+    o->hvals_valid = false;
     if (o->pending) {
         // two folds without an evaluation in between: apply the first now
         neo_gpu_ctx* ctx = o->ctx;
@@ -1559,7 +1613,7 @@ struct neo_gpu_twist_addr {
     uint32_t A = 0, bit = 0, N = 0;  // N items
     DevBuf<uint64_t> key[2];
     int kcur = 0;
-    DevBuf<K> wt, kc, d, tab[2], recs, vals;
+    DevBuf<K> wt, kc, d, tab[2], recs;
     DevBuf<uint32_t> heads, hist;
     DevBuf<unsigned int> ticket;     // ta_eval_kernel's block counter (returns to zero after every launch)
     DevBuf<K> dcols, dr, dv;         // build workspace, kept for reuse
@@ -1628,9 +1682,11 @@ int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
 int ta_values(neo_gpu_twist_addr* o) {
     neo_gpu_ctx* ctx = o->ctx;
     o->hvals.assign(3, gl::kzero());
-    if (int rc = ta_values_launch(o, o->vals.p)) return rc;
-    NEO_CK(ctx, ctx_d2h(ctx, o->hvals.data(), o->vals.p, 3 * sizeof(K)));
+    if (o->N == 0) return o->pending ? ta_apply_fold(o) : NEO_OK;
+    K* out = reinterpret_cast<K*>(ctx->h_result);
+    if (int rc = ta_values_launch(o, out)) return rc;
     NEO_CK(ctx, ctx_sync(ctx));
+    o->hvals.assign(out, out + 3);
     return NEO_OK;
 }
 
@@ -1698,7 +1754,7 @@ int ta_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_cycle,
     const uint32_t n_tiles = ceil_div(cap, RS_TILE), nb = ceil_div(cap, TE_T);
     if (o->key[0].ensure(cap) || o->key[1].ensure(cap) || o->wt.ensure(cap) || o->kc.ensure(cap) ||
         (kind == 1 && o->d.ensure(cap)) || o->recs.ensure((size_t)nb * TA_REC) || o->heads.ensure(nb) ||
-        o->hist.ensure((size_t)n_tiles * 256) || o->vals.ensure(3) || o->ticket.ensure(1) ||
+        o->hist.ensure((size_t)n_tiles * 256) || o->ticket.ensure(1) ||
         o->tab[0].ensure(P + 1) || o->tab[1].ensure(P / 2 + 1))
         return fail(ctx->fail(NEO_ERR_OOM, "twist_addr: event arrays"));
     NEO_CK(ctx, cudaMemsetAsync(o->ticket.p, 0, sizeof(unsigned int), S));
