@@ -269,7 +269,7 @@ inline cudaError_t ctx_scratch(neo_gpu_ctx* ctx, size_t bytes, void** p) {
     *p = ctx->scratch;
     return cudaSuccess;
 }
-int dev_ccs_upload(neo_gpu_ctx* ctx, const neo_ccs_desc* desc, DevCcs& out);
+int dev_ccs_upload(neo_gpu_ctx* ctx, const neo_ccs_desc* desc, DevCcs& out, bool want_csr = true);
 
 // Kernels callable from several translation units.
 int launch_chi_table(neo_gpu_ctx* ctx, const gl::K* d_bits, uint32_t nbits, gl::K* d_out);
