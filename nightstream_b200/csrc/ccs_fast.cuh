@@ -196,23 +196,45 @@ __device__ __forceinline__ K chi_of(const K* pts, int n, uint32_t b) {
     return w;
 }
 
-// block sum of v[0..n) into rec[0..n), zeros in rec[n..REC); n <= REC
-__device__ __forceinline__ void block_sum_rec(const K* v, int n, K* rec) {
-    __shared__ K s_red[FR / 32][REC];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll 1
-    for (int d = 0; d < n; d++) {
-        K x = v[d];
+// Warp sums of v[0..N), N a power of two up to 16: halving exchange steps (a lane
+// keeps half of its values and sends the other half) and then plain ones, so N
+// values cost N - 1 + log2(32 / N) K additions instead of 5 N.  Returns the sum
+// of value `*idx`.
+template <int N>
+__device__ __forceinline__ K warp_sums(K (&v)[N], int* idx) {
+    const int lane = threadIdx.x & 31;
+    int id = 0, o = 16;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = gl::kadd(x, shfl_xor_k(x, o));
-        if (lane == 0) s_red[warp][d] = x;
+    for (int n = N / 2; n >= 1; n /= 2, o /= 2) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; i++) {
+            const K keep = up ? v[n + i] : v[i], send = up ? v[i] : v[n + i];
+            v[i] = gl::kadd(keep, shfl_xor_k(send, o));
+        }
+        if (up) id += n;
     }
+    K x = v[0];
+#pragma unroll
+    for (int q = 16 / N; q > 0; q /= 2) x = gl::kadd(x, shfl_xor_k(x, q));
+    *idx = id;
+    return x;
+}
+
+// block sum of v[0..N) into rec[0..min(N, REC)), zeros in the rest of rec
+template <int N>
+__device__ __forceinline__ void block_sum_rec(K (&v)[N], K* rec) {
+    __shared__ K s_red[FR / 32][N];
+    const int warp = threadIdx.x >> 5;
+    int idx;
+    const K x = warp_sums<N>(v, &idx);
+    s_red[warp][idx] = x;  // the lanes of a value hold the same sum
     __syncthreads();
     if (threadIdx.x < REC) {
-        K x = gl::kzero();
-        if ((int)threadIdx.x < n)
-            for (int w = 0; w < FR / 32; w++) x = gl::kadd(x, s_red[w][threadIdx.x]);
-        st_k(rec + threadIdx.x, x);
+        K y = gl::kzero();
+        if (threadIdx.x < N)
+            for (int w = 0; w < FR / 32; w++) y = gl::kadd(y, s_red[w][threadIdx.x]);
+        st_k(rec + threadIdx.x, y);
     }
 }
 
@@ -245,7 +267,7 @@ struct FastRoundArgs {
     const K* E;                  // E_j [pairs]
     uint64_t pairs;
     // NC
-    const K* chals;              // device r_0..r_{j-1}
+    K chals[32];                 // r_0..r_{j-1}
     const int8_t* Z;             // [nq][m]
     uint64_t m;
     const K* nc_in;              // T_{j-1} [nq][nc_len_in] (rounds >= 5)
@@ -318,13 +340,14 @@ __device__ __noinline__ void mom_role(const FastRoundArgs& a, uint32_t blk, K* r
             for (int d = 0; d < 4; d++) c[d] = kmul_n(h, F[d]);
         }
     }
-    block_sum_rec(c, 4, rec);
+    block_sum_rec<4>(c, rec);
 }
 
 __device__ __noinline__ void small_role(const FastRoundArgs& a, uint32_t blk, K* rec) {
-    K out[REC];
+    static_assert(REC <= 16, "a record fits the block sum");
+    K out[16];
 #pragma unroll
-    for (int d = 0; d < REC; d++) out[d] = gl::kzero();
+    for (int d = 0; d < 16; d++) out[d] = gl::kzero();
     const uint64_t t = blk * (uint64_t)FR + threadIdx.x;
     if (t < a.pairs) {
         K lo_s[2 + MAX_FVAR + 2], hi_s[2 + MAX_FVAR + 2];
@@ -388,7 +411,7 @@ __device__ __noinline__ void small_role(const FastRoundArgs& a, uint32_t blk, K*
             out[MAX_DEG + 2] = kmul_n(r1, v1);
         }
     }
-    block_sum_rec(out, REC, rec);
+    block_sum_rec<16>(out, rec);
 }
 
 // Round 3, separable part.  With lo, hi the K-linear forms of the even and
@@ -425,7 +448,7 @@ __device__ __noinline__ void sep_role(const FastRoundArgs& a, uint32_t blk, K* r
             c[3] = gl::ksub(sb3, sa3);
         }
     }
-    block_sum_rec(c, 4, rec);
+    block_sum_rec<4>(c, rec);
 }
 
 template <int MODE, bool C>
@@ -546,15 +569,15 @@ __device__ __forceinline__ void nc_role(const FastRoundArgs& a, uint32_t blk, K*
             for (int d = 0; d < 4; d++) out[d] = kmul_c<C>(e, gl::kacc_reduce(acc[d]));
         }
     }
-    block_sum_rec(out, 4, rec);
+    block_sum_rec<4>(out, rec);
 }
 
 // Sums the records of every block of the launch (run by the last block).
 __device__ __noinline__ void round_final_reduce(const FastRoundArgs& a) {
-    __shared__ K s_tot[FR / 32][REC];
-    K s[REC];
+    __shared__ K s_tot[FR / 32][16];
+    K s[16];
 #pragma unroll
-    for (int d = 0; d < REC; d++) s[d] = gl::kzero();
+    for (int d = 0; d < 16; d++) s[d] = gl::kzero();
     for (uint32_t r = threadIdx.x; r < gridDim.x; r += FR) {
         const ulonglong2* p = reinterpret_cast<const ulonglong2*>(a.partials + (uint64_t)r * REC);
 #pragma unroll
@@ -563,14 +586,10 @@ __device__ __noinline__ void round_final_reduce(const FastRoundArgs& a) {
             s[d] = gl::kadd(s[d], gl::kmk(v.x, v.y));
         }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int d = 0; d < REC; d++) {
-        K x = s[d];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = gl::kadd(x, shfl_xor_k(x, o));
-        if (lane == 0) s_tot[warp][d] = x;
-    }
+    const int warp = threadIdx.x >> 5;
+    int idx;
+    const K tot = warp_sums<16>(s, &idx);
+    s_tot[warp][idx] = tot;
     __syncthreads();
     __shared__ K s_S[REC];
     if (threadIdx.x < REC) {

@@ -721,7 +721,7 @@ struct neo_gpu_ccs_oracle {
     DevBuf<K> nc[2];
     int nc_cur = 0;
     int J = 0;
-    DevBuf<K> wg, eqw, partials, coeffs, ys, scratch_k;
+    DevBuf<K> wg, eqw, partials, ys;
     DevBuf<K> d_chals;  // row challenges on the device (prefix χ tables of the streaming rounds)
     // ternary-digit path (ccs_fast.cuh): E tables, the 8-row pattern histogram
     bool fast = false;
@@ -1003,7 +1003,6 @@ static int oracle_init(neo_gpu_ctx* ctx, neo_gpu_ccs_oracle* o, const int8_t* d_
     NEO_CK(ctx, o->d_chals.ensure(o->ell_n ? o->ell_n : 1));
     uint64_t max_blocks = (uint64_t)ceil_div(n_pad / 2, RT) * nq + 16;
     NEO_CK(ctx, o->partials.ensure(max_blocks * (o->deg_max + 1)));
-    NEO_CK(ctx, o->coeffs.ensure(MAX_DEG + 1));
     NEO_CK(ctx, o->ys.ensure(16));
     if (o->fast) {  // the pattern-histogram row rounds
         int rc2 = fast_setup(o);
@@ -1084,7 +1083,7 @@ static int fast_setup(neo_gpu_ccs_oracle* o) {
 
 // One row round on the ternary-digit path (one launch; round 0 first builds
 // the pattern histogram); leaves deg_max + 1 coefficients in coeffs_dst
-// (device).  d_chals must hold r_0..r_{j-1}.
+// (device-visible).
 static int fast_round_launch(neo_gpu_ccs_oracle* o, K* coeffs_dst) {
     neo_gpu_ctx* ctx = o->ctx;
     const uint32_t j = o->round_idx, ell = o->ell_n, nq = o->k * NEO_D;
@@ -1140,7 +1139,7 @@ static int fast_round_launch(neo_gpu_ccs_oracle* o, K* coeffs_dst) {
     a.E = o->E_all.p + (o->n_pad - (o->n_pad >> j));
     a.pairs = o->n_pad >> (j + 1);
     a.n_small = (uint32_t)ceil_div(a.pairs, FR);
-    a.chals = o->d_chals.p;
+    for (uint32_t i = 0; i < j && i < 32; i++) a.chals[i] = o->row_chals[i];
     a.Z = o->Z;
     a.m = o->m;
     a.wg = o->wg.p;
@@ -1190,8 +1189,9 @@ static int fast_round_launch(neo_gpu_ccs_oracle* o, K* coeffs_dst) {
 }
 
 // Launches row round j = round_idx (folding the previous challenge in) and
-// leaves its deg_max + 1 coefficients in coeffs_dst (device); no host sync.
-// d_chals must hold the row challenges of the rounds already bound.
+// leaves its deg_max + 1 coefficients in coeffs_dst (device-visible); no host sync.
+// Without the ternary-digit path d_chals must hold the row challenges of the
+// rounds already bound.
 static int row_round_launch(neo_gpu_ccs_oracle* o, K* coeffs_dst) {
     if (o->fast) return fast_round_launch(o, coeffs_dst);
     neo_gpu_ctx* ctx = o->ctx;
@@ -1285,14 +1285,14 @@ static int row_round_launch(neo_gpu_ccs_oracle* o, K* coeffs_dst) {
 static int row_round(neo_gpu_ccs_oracle* o) {
     neo_gpu_ctx* ctx = o->ctx;
     const uint32_t j = o->round_idx;
-    if (j > 0 && ((int)j <= o->J || o->fast))
+    if (j > 0 && (int)j <= o->J && !o->fast)
         NEO_CK(ctx, cudaMemcpyAsync(o->d_chals.p, o->row_chals.data(), j * sizeof(K), cudaMemcpyHostToDevice,
                                     ctx->stream));
-    int rc = row_round_launch(o, o->coeffs.p);
+    K* out = reinterpret_cast<K*>(ctx->h_result);  // the launch writes the coefficients there
+    int rc = row_round_launch(o, out);
     if (rc) return rc;
-    o->h_coeffs.resize(o->deg_max + 1);
-    NEO_CK(ctx, ctx_d2h(ctx, o->h_coeffs.data(), o->coeffs.p, (o->deg_max + 1) * 16));
     NEO_CK(ctx, ctx_sync(ctx));
+    o->h_coeffs.assign(out, out + o->deg_max + 1);
     o->coeffs_valid = true;
     return NEO_OK;
 }
@@ -1304,7 +1304,7 @@ int ccs_oracle_round_launch(neo_gpu_ccs_oracle* o, K* d_dst, uint32_t* ncoef) {
     neo_gpu_ctx* ctx = o->ctx;
     const uint32_t j = o->round_idx;
     if (j >= o->ell_n) return ctx->fail(NEO_ERR_ARG, "ccs round launch: not a row round");
-    if (j > 0 && ((int)j <= o->J || o->fast)) {
+    if (j > 0 && (int)j <= o->J && !o->fast) {
         NEO_CK(ctx, o->h_chals.ensure(o->ell_n));
         memcpy(o->h_chals.p, o->row_chals.data(), j * sizeof(K));
         NEO_CK(ctx, cudaMemcpyAsync(o->d_chals.p, o->h_chals.p, j * sizeof(K), cudaMemcpyHostToDevice, ctx->stream));
@@ -1366,14 +1366,15 @@ static int ajtai_round(neo_gpu_ccs_oracle* o, const uint64_t* xs, uint32_t nx, u
     for (int v = 0; v < o->n_fvar; v++) a.fvar_j[v] = o->fvar_j[v];
     a.y = o->y_eval.p;
     a.ysc = o->y_sc.p;
-    a.ys_out = o->ys.p;
+    K* out = reinterpret_cast<K*>(ctx->h_result);
+    a.ys_out = out;
     size_t smem = ((size_t)o->k * (1 + o->t) * NEO_D + (size_t)nx * o->k) * sizeof(K);
     static SmemLimit limit;
     NEO_CK(ctx, limit.at_least(ajtai_round_kernel, smem));
     ajtai_round_kernel<<<1, 512, smem, ctx->stream>>>(a);
     NEO_LAUNCHED(ctx);
-    NEO_CK(ctx, ctx_d2h(ctx, ys, o->ys.p, nx * 16));
     NEO_CK(ctx, ctx_sync(ctx));
+    memcpy(ys, out, nx * sizeof(K));
     return NEO_OK;
 }
 
@@ -1431,7 +1432,8 @@ static int neo_gpu_ccs_oracle_row_rounds_device_impl_abi(neo_gpu_ccs_oracle* o, 
     const uint32_t j0 = o->round_idx;
     for (uint32_t i = 0; i < n; i++) o->row_chals.push_back(gl::kmk(gl::canon(chals[2 * i]), gl::canon(chals[2 * i + 1])));
     // every challenge of the sequence goes up once; round j reads only the first j
-    NEO_CK(ctx, cudaMemcpyAsync(o->d_chals.p, o->row_chals.data(), (j0 + n) * sizeof(K), cudaMemcpyHostToDevice,
+    // (the ternary-digit launches carry theirs as arguments)
+    if (!o->fast) NEO_CK(ctx, cudaMemcpyAsync(o->d_chals.p, o->row_chals.data(), (j0 + n) * sizeof(K), cudaMemcpyHostToDevice,
                                 ctx->stream));
     // rounds are written at stride d_sc + 1; coefficients above deg_max are zero
     const uint32_t ncoef = o->d_sc + 1;
