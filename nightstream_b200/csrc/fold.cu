@@ -739,7 +739,7 @@ int ta_round_launch(neo_gpu_twist_addr* o, K* d_dst, bool* launched);
 int mem_claims_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* claims, DevBuf<K>& partials,
                      HostBuf<K>& h_slots);
 int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* const* d_out,
-                           DevBuf<K>& partials);
+                           DevBuf<K>& partials, bool coeffs);
 
 namespace {
 
@@ -832,9 +832,8 @@ struct Claim {
 
 // run_batched_sumcheck_prover (sumcheck.rs:350-456) inside sc_start / sc_end
 // (sumcheck_ds.rs:11-19); round polynomials appended to P in claim order.
-// Per round every claim is launched first -- the Pi_CCS claim writes its
-// coefficients, the memory claims their values at 0..deg (all of them in one
-// multi-claim fold and eval), the Twist address-lane claims theirs at 0, 1,
+// Per round every claim is launched first -- the Pi_CCS claim and the memory
+// claims (all of them in one multi-claim evaluation) write their coefficients, the Twist address-lane claims theirs at 0, 1,
 // 2, into one page-locked array -- then a single sync ends the round; claims whose tables are exhausted take the per-claim path.
 static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_idx, std::vector<Claim>& cl,
                           uint32_t rounds, std::vector<K>& chals, std::vector<K>& finals, std::vector<uint64_t>& P,
@@ -862,7 +861,8 @@ static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_i
     chals.clear();
     std::vector<neo_gpu_mem_oracle*> mos;
     std::vector<K*> mdst;
-    std::vector<uint32_t> kind(cl.size()), ncoef(cl.size());  // kind: 0 per-claim, 1 ccs, 2 multi memory
+    // kind: 0 per-claim call, 1 Pi_CCS coefficients, 2 values at 0..deg, 3 memory coefficients
+    std::vector<uint32_t> kind(cl.size()), ncoef(cl.size());
     for (uint32_t rd = 0; rd < rounds; rd++) {
         auto br = le64(rd);
         tr.append_message("batched/round_idx", br.data(), 8);
@@ -879,7 +879,7 @@ static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_i
                        mem_round_multi_ok(cl[i].mem)) {
                 mos.push_back(cl[i].mem);
                 mdst.push_back(slot);
-                kind[i] = 2;
+                kind[i] = 3;
             } else if (cl[i].ta && cl[i].deg == 2) {
                 bool launched = false;
                 int rc = ta_round_launch(cl[i].ta, slot, &launched);
@@ -889,29 +889,40 @@ static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_i
         }
         for (size_t i0 = 0; i0 < mos.size(); i0 += 24) {
             const int nn = (int)std::min<size_t>(24, mos.size() - i0);
-            int rc = mem_round_launch_multi(ctx, mos.data() + i0, nn, mdst.data() + i0, sh->d_mpart);
+            int rc = mem_round_launch_multi(ctx, mos.data() + i0, nn, mdst.data() + i0, sh->d_mpart, true);
             if (rc) return rc;
         }
         NEO_CK(ctx, ctx_sync(ctx));
         for (size_t i = 0; i < cl.size(); i++) {
             const uint32_t np = cl[i].deg + 1;
-            std::vector<K> xs(np), ys(np);
-            for (uint32_t x = 0; x < np; x++) xs[x] = gl::kfq(x);
             const K* h = sh->h_round.p + i * MAX_SLOT;
-            if (kind[i] == 1) {
-                // values at 0..deg from the coefficients (Horner, sumcheck.rs:48-60)
-                ccs_oracle_round_set(cl[i].ccs, h);
-                std::vector<K> co(h, h + ncoef[i]);
-                for (uint32_t x = 0; x < np; x++) ys[x] = poly_eval(co, xs[x]);
-            } else if (kind[i] == 2) {
-                for (uint32_t x = 0; x < np; x++) ys[x] = h[x];
+            K at01;  // p(0) + p(1)
+            if (kind[i] == 1 || kind[i] == 3) {  // the polynomial of at most np coefficients itself
+                uint32_t nc = np;
+                if (kind[i] == 1) {
+                    ccs_oracle_round_set(cl[i].ccs, h);
+                    nc = ncoef[i];
+                }
+                polys[i].assign(h, h + std::min(nc, np));
+                for (uint32_t d = np; d < nc; d++)
+                    if (!gl::kiszero(h[d])) return ctx->fail(NEO_ERR_INVARIANT, "batched sum-check: degree above the claim's bound");
+                polys[i].resize(np, gl::kzero());
+                at01 = polys[i][0];
+                for (const K& c : polys[i]) at01 = gl::kadd(at01, c);
             } else {
-                int rc = cl[i].evals(xs.data(), np, ys.data());
-                if (rc) return rc;
+                std::vector<K> xs(np), ys(np);
+                for (uint32_t x = 0; x < np; x++) xs[x] = gl::kfq(x);
+                if (kind[i] == 2) {
+                    std::copy(h, h + np, ys.begin());
+                } else {
+                    int rc = cl[i].evals(xs.data(), np, ys.data());
+                    if (rc) return rc;
+                }
+                at01 = gl::kadd(ys[0], ys[1]);
+                interpolate(xs, ys, polys[i]);
             }
-            if (!keq(gl::kadd(ys[0], ys[1]), running[i]))
+            if (!keq(at01, running[i]))
                 return ctx->fail(NEO_ERR_INVARIANT, ("batched sum-check " + cl[i].label + ": p(0)+p(1) != running sum").c_str());
-            interpolate(xs, ys, polys[i]);
         }
         for (size_t i = 0; i < cl.size(); i++) {
             tr.append_message("batched/claim_label", cl[i].label);

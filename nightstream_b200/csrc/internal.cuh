@@ -32,6 +32,7 @@ struct neo_gpu_ctx {
     void* commit_buf = nullptr;
     uint32_t commit_groups = 0;
     size_t commit_words = 0;
+    uint64_t* vinv = nullptr;        // inverse Vandermonde tables (mem_oracle.cu), once a batched round needs them
     // the last chi table a memory oracle built (the time-lane oracles of a
     // step share their point): key = ell then the point's words
     void* chi_cache = nullptr;

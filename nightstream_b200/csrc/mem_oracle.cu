@@ -282,7 +282,9 @@ struct MultiClaim {
     uint32_t fs;       // lanes that share a pair's factors (1, 2, 4, .. 16)
     uint32_t lpb;      // log2 of the pairs per tile, 32 hb / fs
     uint32_t small;    // few pairs: one block per point (multi_small)
-    K* out;            // values at x = 0..npts-1
+    const uint64_t* vinv;  // null: out gets the values at x = 0..npts-1; else the polynomial's
+                           // coefficients, through the npts x npts inverse Vandermonde matrix of 0..npts-1
+    K* out;
     unsigned int* ticket;  // the claim's block counter (zero between launches)
 };
 
@@ -364,13 +366,29 @@ __device__ __forceinline__ void multi_factor(const MultiClaim& c, uint32_t f, ui
     ldg_pair(c.tab + (uint64_t)f * c.len + 2 * p, f0, f1);
 }
 
+// The round polynomial from its values s_v[0..npts), by the whole block: eight
+// lanes per coefficient.  The sum-check driver absorbs coefficients; interpolating
+// 16 to 20 points on the host cost 60 to 100 us per claim and round.
+__device__ __forceinline__ void multi_coeffs(const MultiClaim& c, const K* s_v) {
+    const uint32_t n = c.npts, l = threadIdx.x & 7;
+    for (uint32_t d0 = 0; d0 < n; d0 += 32) {
+        const uint32_t d = d0 + (threadIdx.x >> 3);
+        K acc = gl::kzero();
+        if (d < n)
+            for (uint32_t x = l; x < n; x += 8) acc = gl::kadd(acc, gl::kscale(s_v[x], __ldg(c.vinv + d * n + x)));
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) acc = gl::kadd(acc, shfl_xor_km(acc, o));
+        if (l == 0 && d < n) c.out[d] = acc;
+    }
+}
+
 // A claim with at most SMALL_PAIRS pairs (its last rounds): one block per point x
-// does every pair, so there is nothing to add up between blocks.  fs lanes share a
+// does every pair (coefficients: the last block takes them from all points' values).  fs lanes share a
 // pair's factors and multiply (bitness: add) their parts with shuffles: the launch
 // is one dependent chain, and a thread walking 15 factors took 22 to 30 us where
 // this takes 8.  Block 0 writes the folded tables.
 constexpr uint32_t SMALL_PAIRS = 16;
-__device__ __noinline__ void multi_small(const MultiClaim& c, uint32_t x, K* s_sum) {
+__device__ __noinline__ void multi_small(const MultiClaim& c, uint32_t x, K* s_sum, K* s_v, K* partials) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t fs = c.fs, sub = threadIdx.x & (fs - 1), p = threadIdx.x / fs;
     const bool live = p < (uint32_t)(c.len >> 1);
@@ -406,8 +424,24 @@ __device__ __noinline__ void multi_small(const MultiClaim& c, uint32_t x, K* s_s
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < 8; w++) total = gl::kadd(total, s_sum[w]);
-        c.out[x] = total;
+        if (!c.vinv) c.out[x] = total;
+        else partials[c.part0 + x] = total;
     }
+    if (!c.vinv) return;
+    __shared__ unsigned int s_last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicInc(c.ticket, c.npts - 1) == c.npts - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (threadIdx.x < c.npts) {
+        const ulonglong2 u = __ldcg(reinterpret_cast<const ulonglong2*>(partials + c.part0 + threadIdx.x));
+        s_v[threadIdx.x] = gl::kmk(u.x, u.y);
+    }
+    __syncthreads();
+    multi_coeffs(c, s_v);
 }
 
 // Larger claims: a block takes tiles of 32 hb / fs pairs, dealt out in turn so that
@@ -428,11 +462,12 @@ __global__ void __launch_bounds__(256) mem_multi_eval_kernel(const __grid_consta
     __shared__ K s_f[2][MF];    // f0, f1 - f0: [factor][pair]
     __shared__ K s_red[8][MPTS];
     __shared__ uint8_t s_on[256];
+    __shared__ K s_v[MEM_MAX_DEG + 1];
     const int ci = multi_claim_of(a, blockIdx.x);
     const MultiClaim& c = a.c[ci];
     const uint32_t b = blockIdx.x - c.blk0;
     if (c.small) {
-        multi_small(c, b, &s_red[0][0]);
+        multi_small(c, b, &s_red[0][0], s_v, a.partials);
         return;
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -533,10 +568,15 @@ __global__ void __launch_bounds__(256) mem_multi_eval_kernel(const __grid_consta
         const uint32_t x = threadIdx.x;
         K v = gl::kzero();
         for (uint32_t g = 0; g < hb; g++) v = gl::kadd(v, s_red[(x % xstep) * hb + g][x / xstep]);
-        if (c.nblk == 1) c.out[x] = v;
-        else a.partials[c.part0 + (uint64_t)x * c.nblk + b] = v;
+        if (c.nblk > 1) a.partials[c.part0 + (uint64_t)x * c.nblk + b] = v;
+        else if (c.vinv) s_v[x] = v;
+        else c.out[x] = v;
     }
-    if (c.nblk == 1) return;
+    if (c.nblk == 1) {
+        __syncthreads();
+        if (c.vinv) multi_coeffs(c, s_v);
+        return;
+    }
     // the claim's last block to finish sums its partials (ticket, no waits)
     __threadfence();
     __syncthreads();
@@ -555,8 +595,37 @@ __global__ void __launch_bounds__(256) mem_multi_eval_kernel(const __grid_consta
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = gl::kadd(v, shfl_xor_km(v, o));
-        if (lane == 0) c.out[x] = v;
+        if (lane == 0) (c.vinv ? s_v : c.out)[x] = v;
     }
+    if (!c.vinv) return;
+    __syncthreads();
+    multi_coeffs(c, s_v);
+}
+
+// Inverse Vandermonde matrices of the nodes 0..n-1 for n = 2..MEM_MAX_DEG + 1, row
+// d column x: coefficient d of the x-th Lagrange basis polynomial.
+constexpr uint32_t VINV_MAX = MEM_MAX_DEG + 1;
+inline uint32_t vinv_off(uint32_t n) { return (n - 1) * n * (2 * n - 1) / 6; }  // sum of k^2, k < n
+const std::vector<uint64_t>& vinv_host() {
+    static const std::vector<uint64_t> tab = [] {
+        std::vector<uint64_t> t(vinv_off(VINV_MAX + 1));
+        for (uint32_t n = 1; n <= VINV_MAX; n++)
+            for (uint32_t x = 0; x < n; x++) {
+                std::vector<uint64_t> co(1, 1);  // prod_{j != x} (X - j)
+                uint64_t den = 1;
+                for (uint32_t j = 0; j < n; j++) {
+                    if (j == x) continue;
+                    co.push_back(0);
+                    for (size_t d = co.size(); d-- > 0;)
+                        co[d] = gl::sub(d ? co[d - 1] : 0, gl::mul(co[d], (uint64_t)j));
+                    den = gl::mul(den, x > j ? (uint64_t)(x - j) : gl::neg((uint64_t)(j - x)));
+                }
+                const uint64_t s = gl::inv(den);
+                for (uint32_t d = 0; d < n; d++) t[vinv_off(n) + d * n + x] = gl::mul(co[d], s);
+            }
+        return t;
+    }();
+    return tab;
 }
 
 
@@ -835,11 +904,16 @@ bool mem_round_multi_ok(const neo_gpu_mem_oracle* o) {
 }
 
 // The next round of n oracles: pending folds, then the values at x = 0..deg
-// of oracle i into d_out[i] (device), in one launch and without a host
-// sync.  Every oracle must satisfy mem_round_multi_ok; n <= MULTI_MAX.
+// of oracle i (coeffs: the round polynomial's coefficients) into d_out[i] (device-
+// visible), in one launch and without a host sync.  Every oracle must satisfy mem_round_multi_ok; n <= MULTI_MAX.
 int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* const* d_out,
-                           DevBuf<K>& partials) {
+                           DevBuf<K>& partials, bool coeffs) {
     if (n <= 0) return NEO_OK;
+    if (coeffs && !ctx->vinv) {
+        const std::vector<uint64_t>& t = vinv_host();
+        NEO_CK(ctx, ctx_malloc(ctx, reinterpret_cast<void**>(&ctx->vinv), t.size() * 8));
+        NEO_CK(ctx, cudaMemcpyAsync(ctx->vinv, t.data(), t.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
+    }
     if (n > MULTI_MAX) return ctx->fail(NEO_ERR_UNSUPPORTED, "mem_round_launch_multi: too many claims");
     MultiArgs a{};
     a.n = n;
@@ -885,6 +959,7 @@ int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int 
         c.blk0 = blocks;
         c.part0 = (uint32_t)parts;
         c.out = d_out[i];
+        c.vinv = coeffs ? ctx->vinv + vinv_off(c.npts) : nullptr;
         const uint64_t pairs = o->len >> 1;
         if (pairs <= SMALL_PAIRS) {
             // lanes per pair: what 256 threads leave, up to 16 and to the factors there are
@@ -892,6 +967,7 @@ int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int 
             c.fs = 1;
             while (c.fs < 16 && 2 * c.fs * pairs <= 256 && c.fs < c.nf - (c.bitness ? 1 : 0)) c.fs *= 2;
             blocks += c.npts;
+            parts += c.npts;
             continue;
         }
         // eight warps cover the points; with fewer points, warps share a point's pairs
@@ -945,7 +1021,7 @@ int mem_round_values(neo_gpu_mem_oracle* o) {
     o->hvals.assign(npts, gl::kzero());
     if (mem_round_multi_ok(o)) {
         K* out = reinterpret_cast<K*>(ctx->h_result);
-        if (int rc = mem_round_launch_multi(ctx, &o, 1, &out, o->partials)) return rc;
+        if (int rc = mem_round_launch_multi(ctx, &o, 1, &out, o->partials, false)) return rc;
         NEO_CK(ctx, ctx_sync(ctx));
         for (uint32_t x = 0; x < npts; x++) o->hvals[x] = out[x];
         o->hvals_valid = true;
@@ -1001,7 +1077,7 @@ int mem_claims_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* 
     NEO_CK(ctx, h_slots.ensure((size_t)n * SLOT));
     std::vector<K*> dst(n);
     for (int i = 0; i < n; i++) dst[i] = h_slots.p + (size_t)i * SLOT;
-    if (int rc = mem_round_launch_multi(ctx, os, n, dst.data(), partials)) return rc;
+    if (int rc = mem_round_launch_multi(ctx, os, n, dst.data(), partials, false)) return rc;
     NEO_CK(ctx, ctx_sync(ctx));
     for (int i = 0; i < n; i++) {
         const K* v = h_slots.p + (size_t)i * SLOT;
