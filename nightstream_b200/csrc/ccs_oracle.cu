@@ -1289,9 +1289,11 @@ static int row_round(neo_gpu_ccs_oracle* o) {
         NEO_CK(ctx, cudaMemcpyAsync(o->d_chals.p, o->row_chals.data(), j * sizeof(K), cudaMemcpyHostToDevice,
                                     ctx->stream));
     K* out = reinterpret_cast<K*>(ctx->h_result);  // the launch writes the coefficients there
+    const size_t words = 2 * ((size_t)o->deg_max + 1);
+    result_arm(out, words);
     int rc = row_round_launch(o, out);
     if (rc) return rc;
-    NEO_CK(ctx, ctx_sync(ctx));
+    NEO_CK(ctx, result_wait(ctx, out, words));
     o->h_coeffs.assign(out, out + o->deg_max + 1);
     o->coeffs_valid = true;
     return NEO_OK;
@@ -1371,9 +1373,10 @@ static int ajtai_round(neo_gpu_ccs_oracle* o, const uint64_t* xs, uint32_t nx, u
     size_t smem = ((size_t)o->k * (1 + o->t) * NEO_D + (size_t)nx * o->k) * sizeof(K);
     static SmemLimit limit;
     NEO_CK(ctx, limit.at_least(ajtai_round_kernel, smem));
+    result_arm(out, 2 * (size_t)nx);
     ajtai_round_kernel<<<1, 512, smem, ctx->stream>>>(a);
     NEO_LAUNCHED(ctx);
-    NEO_CK(ctx, ctx_sync(ctx));
+    NEO_CK(ctx, result_wait(ctx, out, 2 * (size_t)nx));
     memcpy(ys, out, nx * sizeof(K));
     return NEO_OK;
 }

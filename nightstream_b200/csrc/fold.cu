@@ -868,6 +868,7 @@ static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_i
         tr.append_message("batched/round_idx", br.data(), 8);
         mos.clear();
         mdst.clear();
+        result_arm(sh->h_round.p, 2 * cl.size() * MAX_SLOT);
         for (size_t i = 0; i < cl.size(); i++) {
             K* slot = sh->h_round.p + i * MAX_SLOT;  // page-locked: the launches write the values here
             kind[i] = 0;
@@ -892,7 +893,9 @@ static int run_batched_ds(neo_gpu_shard* sh, const char* domain, uint64_t inst_i
             int rc = mem_round_launch_multi(ctx, mos.data() + i0, nn, mdst.data() + i0, sh->d_mpart, true);
             if (rc) return rc;
         }
-        NEO_CK(ctx, ctx_sync(ctx));
+        for (size_t i = 0; i < cl.size(); i++)
+            if (kind[i])
+                NEO_CK(ctx, result_wait(ctx, sh->h_round.p + i * MAX_SLOT, 2 * (size_t)(kind[i] == 1 ? ncoef[i] : cl[i].deg + 1)));
         for (size_t i = 0; i < cl.size(); i++) {
             const uint32_t np = cl[i].deg + 1;
             const K* h = sh->h_round.p + i * MAX_SLOT;

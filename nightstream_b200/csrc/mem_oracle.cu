@@ -1021,8 +1021,9 @@ int mem_round_values(neo_gpu_mem_oracle* o) {
     o->hvals.assign(npts, gl::kzero());
     if (mem_round_multi_ok(o)) {
         K* out = reinterpret_cast<K*>(ctx->h_result);
+        result_arm(out, 2 * (size_t)npts);
         if (int rc = mem_round_launch_multi(ctx, &o, 1, &out, o->partials, false)) return rc;
-        NEO_CK(ctx, ctx_sync(ctx));
+        NEO_CK(ctx, result_wait(ctx, out, 2 * (size_t)npts));
         for (uint32_t x = 0; x < npts; x++) o->hvals[x] = out[x];
         o->hvals_valid = true;
         return NEO_OK;
@@ -1760,8 +1761,9 @@ int ta_values(neo_gpu_twist_addr* o) {
     o->hvals.assign(3, gl::kzero());
     if (o->N == 0) return o->pending ? ta_apply_fold(o) : NEO_OK;
     K* out = reinterpret_cast<K*>(ctx->h_result);
+    result_arm(out, 6);
     if (int rc = ta_values_launch(o, out)) return rc;
-    NEO_CK(ctx, ctx_sync(ctx));
+    NEO_CK(ctx, result_wait(ctx, out, 6));
     o->hvals.assign(out, out + 3);
     return NEO_OK;
 }
