@@ -357,18 +357,25 @@ __global__ void __launch_bounds__(256) reduce_eval_kernel(const EvalArgs a) {
 // Table build kernels
 // ---------------------------------------------------------------------------
 // z1[c] = sum_rho b^rho Z_0[rho][c]  (oracle.rs:215-243)
-__global__ void z1_kernel(const int8_t* __restrict__ Z, uint64_t m, uint32_t b, uint64_t* __restrict__ z1) {
-    uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+// The powers come as arguments and the digits as two integer sums (|z| < 2^8 times a
+// 32-bit half, 54 of them: below 2^46), so that a column is 54 independent loads and
+// 108 integer products; with the power as a running field product it took 18 us at
+// 2^16 columns, now 4.
+struct Z1Pow {
+    uint64_t pw[NEO_D];  // b^rho
+};
+__global__ void __launch_bounds__(256) z1_kernel(const int8_t* __restrict__ Z, uint64_t m, const __grid_constant__ Z1Pow b,
+                                                 uint64_t* __restrict__ z1) {
+    const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (c >= m) return;
-    uint64_t acc = 0, pw = 1;
+    int64_t lo = 0, hi = 0;
+#pragma unroll 27
     for (int rho = 0; rho < NEO_D; rho++) {
-        int z = Z[(uint64_t)rho * m + c];
-        if (z == 1) acc = gl::add(acc, pw);
-        else if (z == -1) acc = gl::sub(acc, pw);
-        else if (z) acc = gl::add(acc, gl::mul(pw, gl::from_i64(z)));
-        pw = gl::mul(pw, b);
+        const int64_t z = __ldg(Z + (uint64_t)rho * m + c);
+        lo += z * (int64_t)(uint32_t)b.pw[rho];
+        hi += z * (int64_t)(b.pw[rho] >> 32);
     }
-    z1[c] = acc;
+    z1[c] = gl::add(gl::from_i64(lo), gl::mul(gl::from_i64(hi), 1ull << 32));
 }
 
 // out[r] = (M x)[r] for base-field x (CSR), or x[r] for the identity (oracle.rs:245-285)
@@ -485,218 +492,196 @@ __global__ void eval_tbl_kernel(const uint64_t* __restrict__ row_ptr, const uint
     out[r] = acc;
 }
 
+#include "ccs_fast.cuh"
+
 // ---------------------------------------------------------------------------
-// Ajtai phase (oracle.rs:1812-1951): one block.
+// Ajtai phase (oracle.rs:1659-1953): evaluations of a round over the 54 (padded to
+// 2^ell_d) Ajtai coordinates.  Field arithmetic is exact, so the work is regrouped
+// without changing a bit:
+//  * the evaluation part is linear in the y vectors, so ajtai_pre_kernel combines
+//    all (k - 1) t of them with their gamma weights once, for every round;
+//  * the NC part of a round is a cubic in X: its four coefficients are summed over
+//    the k vectors and the tail, whatever the number of points;
+//  * the prefix fold by bits 0..j-1 is the weighted sum with the chi weights of
+//    those challenges, a warp per vector;
+//  * x-independent chains (gamma powers, equality products, F') are formed by
+//    separate warps, products by lanes and shuffles.
+// A launch is one dependent chain on one SM, bound by its latency: with the vectors
+// combined per round, the points evaluated one by one and the chains in one warp's
+// threads a round took 32 us at k = 13 and 17 at k = 1; now 12 and 11 (and 8 or 3 once).
 // ---------------------------------------------------------------------------
-struct AjtaiArgs {
-    int k, t, ell_d, ell_n, j, nx, has_inputs;
-    K xs[16];
-    K alpha[8], beta_a[8], ajtai_chals[8];
+__device__ __forceinline__ K kpow_d(K a, uint32_t e) {
+    K r = gl::kone();
+#pragma unroll 1
+    for (; e; e >>= 1) {
+        if (e & 1) r = kmul_n(r, a);
+        a = ksqr_n(a);
+    }
+    return r;
+}
+// product over the lanes of a warp, in every lane
+__device__ __forceinline__ K warp_prod(K v) {
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) v = kmul_n(v, shfl_xor_k(v, o));
+    return v;
+}
+
+// AJ_E: the 54 entries of the combined evaluation vector; AJ_EQ: eq(beta_r, r_row) and
+// eq(r_in, r_row) gamma^k; AJ_F: F'; AJ_G: gamma^1..gamma^k
+constexpr int AJ_E = 0, AJ_EQ = NEO_D, AJ_F = NEO_D + 2, AJ_G = NEO_D + 3, AJ_MAX = 160;
+struct AjtaiPre {
+    int k, t, ell_n, has_inputs;  // k (1 + t) <= AJ_MAX
     K beta_r[32], r_in[32], row_chals[32];
     K gamma;
     FTerms f;
     int fvar_j[MAX_FVAR];
     const K* y;      // [k][t][54]
     const K* ysc;    // [k][t]
-    K* ys_out;       // [nx]
+    K* out;          // [AJ_G + k]
 };
-
-__device__ K eq_lin_d(K a, K b) {
-    return gl::kadd(gl::kmul(gl::ksub(gl::kone(), a), gl::ksub(gl::kone(), b)), gl::kmul(a, b));
-}
-
-// warp-wide sum of K values (lane 0 holds the total)
-__device__ __forceinline__ K warp_ksum(K v) {
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        K o;
-        o.re = __shfl_down_sync(0xffffffffu, (unsigned long long)v.re, off);
-        o.im = __shfl_down_sync(0xffffffffu, (unsigned long long)v.im, off);
-        v = gl::kadd(v, o);
-    }
-    return v;
-}
-
-// One Ajtai-phase round (oracle.rs:1659-1953): evaluations at xs of round j
-// over the 54 (padded to 2^ell_d) Ajtai coordinates.  Field arithmetic is
-// exact, so the work is reordered for parallelism without changing a bit:
-//  * the prefix fold by bits 0..j-1 of each vector is the weighted sum with
-//    the chi weights of those challenges (one thread per folded entry);
-//  * an evaluation vector's round value is linear in x, A + (B - A) x with
-//    A, B the tail-weighted sums of its lo / hi entries, so its gamma-weighted
-//    combination is formed once per round, not once per x;
-//  * x-independent products (gamma powers, prefix and row equalities, F') are
-//    separate threads' chains, and tail sums are warp reductions.
-__global__ void __launch_bounds__(512) ajtai_round_kernel(const AjtaiArgs a) {
-    extern __shared__ K s_dyn[];          // s_y [nvec][54] folded, then s_nc [nx][k]
-    __shared__ K s_wb[128], s_wa[128], s_w[128];
-    __shared__ K s_A[160], s_B[160];
-    __shared__ K s_gp[161];               // gamma^0..gamma^k
-    __shared__ K s_gkp[160];              // (gamma^k)^0..(gamma^k)^(t-1), t < k (1 + t) <= 160
-    __shared__ K s_fixed[8];              // ebp, eap, eq_br, eq_ri, fprime, SA, SB
-    __shared__ K s_ncsum[16];
-    const int nvec = a.k * (1 + a.t);     // vector q < k: NC (y[i][0]); then eval (i, jm)
-    K* s_y = s_dyn;
-    K* s_nc = s_dyn + nvec * NEO_D;
-    const int j = a.j, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int ntail = a.ell_d - j - 1, tail_len = 1 << ntail;
-    const int hs = 1 << (j + 1), stride = 1 << j;
-
-    // ---- 1. x-independent chains and weights ----
-    if (tid == 0) {
-        K g = gl::kone();
-        s_gp[0] = g;
-        for (int i = 0; i < a.k; i++) { g = gl::kmul(g, a.gamma); s_gp[i + 1] = g; }
-        K p = gl::kone();
-        for (int jm = 0; jm < a.t; jm++) { s_gkp[jm] = p; p = gl::kmul(p, g); }
-    } else if (tid == 1 || tid == 2) {
+__global__ void __launch_bounds__(512) ajtai_pre_kernel(const __grid_constant__ AjtaiPre a) {
+    __shared__ K s_w[AJ_MAX];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nterm = (a.k - 1) * a.t;  // (i, jm), i >= 1: gamma^i (gamma^k)^jm
+    if (tid < nterm) s_w[tid] = kpow_d(a.gamma, 1 + tid / a.t + a.k * (tid % a.t));
+    if (tid >= 192 && tid < 192 + a.k) st_k(a.out + AJ_G + tid - 192, kpow_d(a.gamma, tid - 191));
+    if (warp == 12 || warp == 13) {
+        const bool in = warp == 13;
         K e = gl::kone();
-        for (int i = 0; i < j; i++) e = gl::kmul(e, eq_lin_d(a.ajtai_chals[i], tid == 1 ? a.beta_a[i] : a.alpha[i]));
-        s_fixed[tid - 1] = e;  // ebp, eap
-    } else if (tid == 3 || tid == 4) {
-        K e = gl::kone();
-        if (tid == 3 || a.has_inputs)
-            for (int i = 0; i < a.ell_n; i++) e = gl::kmul(e, eq_lin_d(a.row_chals[i], tid == 3 ? a.beta_r[i] : a.r_in[i]));
-        s_fixed[tid - 1] = e;  // eq_br, eq_ri
-    } else if (tid == 5) {
+        if (lane < a.ell_n && (!in || a.has_inputs)) e = eq_lin(a.row_chals[lane], in ? a.r_in[lane] : a.beta_r[lane]);
+        e = warp_prod(e);
+        if (lane == 0) {
+            if (in) e = a.has_inputs ? kmul_n(e, kpow_d(a.gamma, a.k)) : gl::kzero();
+            st_k(a.out + AJ_EQ + in, e);
+        }
+    } else if (warp == 14 && lane == 0) {
         // F' = f(m_vals), m_vals[j] = y_scalars[0][j] (z1 . v_j by linearity of recomposition)
         K fprime = gl::kzero();
+#pragma unroll 1
         for (int tt = 0; tt < a.f.n_terms; tt++) {
             K p = a.f.coeff[tt];
+#pragma unroll 1
             for (int vv = 0; vv < a.f.n_vars[tt]; vv++) {
-                K mv = a.ysc[a.fvar_j[a.f.var_pos[tt][vv]]];
-                for (int e = 0; e < a.f.var_exp[tt][vv]; e++) p = gl::kmul(p, mv);
+                const K mv = ld_k(a.ysc + a.fvar_j[a.f.var_pos[tt][vv]]);
+#pragma unroll 1
+                for (int e = 0; e < a.f.var_exp[tt][vv]; e++) p = kmul_n(p, mv);
             }
             fprime = gl::kadd(fprime, p);
         }
-        s_fixed[4] = fprime;
-    } else if (tid >= 32 && tid < 32 + (1 << j)) {
-        // fold weight of offset b: prod over bits of (bit ? c : 1 - c)
-        const int b = tid - 32;
-        K w = gl::kone();
-        for (int i = 0; i < j; i++) w = gl::kmul(w, ((b >> i) & 1) ? a.ajtai_chals[i] : gl::ksub(gl::kone(), a.ajtai_chals[i]));
-        s_w[b] = w;
-    } else if (tid >= 160 && tid < 160 + tail_len) {
-        // tail weights chi(beta_a[j+1..]), chi(alpha[j+1..])
-        const int tt = tid - 160;
-        K wb = gl::kone(), wa = gl::kone();
-        for (int i = 0; i < ntail; i++) {
-            int bit = (tt >> i) & 1;
-            K b = a.beta_a[j + 1 + i], al = a.alpha[j + 1 + i];
-            wb = gl::kmul(wb, bit ? b : gl::ksub(gl::kone(), b));
-            wa = gl::kmul(wa, bit ? al : gl::ksub(gl::kone(), al));
-        }
-        s_wb[tt] = wb;
-        s_wa[tt] = wa;
+        st_k(a.out + AJ_F, fprime);
     }
     __syncthreads();
-
-    // ---- 2. prefix fold by bits 0..j-1: entry i of the folded vector at s_y[q][i 2^j] ----
-    {
-        const int L = (NEO_D + stride - 1) >> j;
-        for (int w = tid; w < nvec * L; w += blockDim.x) {
-            const int q = w / L, i = w % L;
-            const K* src = q < a.k ? a.y + ((uint64_t)q * a.t + 0) * NEO_D : a.y + (uint64_t)(q - a.k) * NEO_D;
-            const int base = i << j;
-            K acc;
-            if (j == 0) {
-                acc = src[base];
-            } else {
-                acc = gl::kzero();
-                for (int b = 0; b < stride && base + b < NEO_D; b++) acc = gl::kadd(acc, gl::kmul(s_w[b], src[base + b]));
-            }
-            s_y[q * NEO_D + base] = acc;
-        }
-    }
-    __syncthreads();
-
-    // ---- 3. tail sums: `seg` lanes per item (the tail length, at most 32),
-    //         32 / seg items per warp, segment sums by width-limited shuffles ----
-    const int n_nc = a.nx * a.k, n_items = n_nc + 2 * (nvec - a.k);
-    const int seg = tail_len < 32 ? tail_len : 32, per_warp = 32 / seg;
-    const int sub = lane % seg;
-    for (int base = warp * per_warp; base < n_items; base += nwarps * per_warp) {
-        const int item = base + lane / seg;
-        K part = gl::kzero();
-        if (item < n_nc) {
-            const int xi = item / a.k, q = item % a.k;
-            const K x = a.xs[xi];
-            const K* v = s_y + q * NEO_D;
-            for (int tt = sub; tt < tail_len; tt += seg) {
-                const int idx = tt * hs;
-                if (idx >= NEO_D) continue;
-                const int i1 = idx + stride;
-                K val = gl::klerp(v[idx], i1 < NEO_D ? v[i1] : gl::kzero(), x);
-                val = gl::kmul(val, gl::ksub(gl::ksqr(val), gl::kone()));  // range product, b = 2
-                part = gl::kadd(part, gl::kmul(s_wb[tt], val));
-            }
-        } else if (item < n_items) {
-            const int e = item - n_nc, q = a.k + (e >> 1), hi_side = e & 1;
-            const K* v = s_y + q * NEO_D;
-            for (int tt = sub; tt < tail_len; tt += seg) {
-                const int idx = tt * hs;
-                if (idx >= NEO_D) continue;
-                const int pos = idx + (hi_side ? stride : 0);
-                if (pos < NEO_D) part = gl::kadd(part, gl::kmul(s_wa[tt], v[pos]));
-            }
-        }
-        for (int off = seg >> 1; off > 0; off >>= 1) {
-            K o;
-            o.re = __shfl_down_sync(0xffffffffu, (unsigned long long)part.re, off, seg);
-            o.im = __shfl_down_sync(0xffffffffu, (unsigned long long)part.im, off, seg);
-            part = gl::kadd(part, o);
-        }
-        if (sub == 0 && item < n_items) {
-            if (item < n_nc) {
-                s_nc[(item / a.k) * a.k + item % a.k] = part;
-            } else {
-                const int e = item - n_nc;
-                (e & 1 ? s_B : s_A)[a.k + (e >> 1)] = part;
-            }
-        }
-    }
-    __syncthreads();
-
-    // ---- 4. gamma-weighted combinations ----
-    if (warp == 0 || warp == 1) {
-        // S = sum_{jm, i >= 1} gamma^i (gamma^k)^jm X[k + i t + jm], X = A (warp 0) or B (warp 1)
-        const K* X = warp == 0 ? s_A : s_B;
-        const int nterm = (a.k - 1) * a.t;
-        K part = gl::kzero();
-        for (int u = lane; u < nterm; u += 32) {
-            const int i = 1 + u / a.t, jm = u % a.t;
-            part = gl::kadd(part, gl::kmul(gl::kmul(s_gp[i], s_gkp[jm]), X[a.k + i * a.t + jm]));
-        }
-        part = warp_ksum(part);
-        if (lane == 0) s_fixed[5 + warp] = part;
-    } else {
-        // nc_sum[x] = sum_i gamma^(i+1) nc[x][i], warps 2.. over the points
-        for (int xi = warp - 2; xi < a.nx; xi += nwarps - 2) {
-            K part = gl::kzero();
-            for (int i = lane; i < a.k; i += 32) part = gl::kadd(part, gl::kmul(s_gp[i + 1], s_nc[xi * a.k + i]));
-            part = warp_ksum(part);
-            if (lane == 0) s_ncsum[xi] = part;
-        }
-    }
-    __syncthreads();
-
-    // ---- 5. per evaluation point ----
-    if (tid < a.nx) {
-        const int xi = tid;
-        const K x = a.xs[xi];
-        const K gk = s_gp[a.k];
-        const K eq_beta = gl::kmul(s_fixed[2], gl::kmul(s_fixed[0], eq_lin_d(x, a.beta_a[j])));
-        const K eq_ar = a.has_inputs ? gl::kmul(s_fixed[3], gl::kmul(s_fixed[1], eq_lin_d(x, a.alpha[j]))) : gl::kzero();
-        K out = gl::kmul(eq_beta, gl::kadd(s_fixed[4], s_ncsum[xi]));
-        if (a.k >= 2 && !gl::kiszero(eq_ar)) {
-            const K inner = gl::klerp(s_fixed[5], s_fixed[6], x);
-            out = gl::kadd(out, gl::kmul(eq_ar, gl::kmul(gk, inner)));
-        }
-        a.ys_out[xi] = out;
-    }
+    // eight lanes an entry
+    const int rho = tid >> 3;
+    K acc = gl::kzero();
+    if (rho < NEO_D)
+#pragma unroll 4
+        for (int u = lane & 7; u < nterm; u += 8)
+            acc = gl::kadd(acc, gl::kmul(s_w[u], ld_k(a.y + (uint64_t)(a.t + u) * NEO_D + rho)));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) acc = gl::kadd(acc, shfl_xor_k(acc, o));
+    if ((lane & 7) == 0 && rho < NEO_D) st_k(a.out + AJ_E + rho, acc);
 }
 
-#include "ccs_fast.cuh"
+struct AjtaiArgs {
+    int k, t, ell_d, j, nx, has_inputs;
+    K xs[16];
+    K alpha[8], beta_a[8], ajtai_chals[8];
+    const K* y;      // [k][t][54]
+    const K* pre;    // ajtai_pre_kernel's
+    K* ys_out;       // [nx]
+};
+constexpr int AJ_T = 512;
+__global__ void __launch_bounds__(AJ_T) ajtai_round_kernel(const __grid_constant__ AjtaiArgs a) {
+    extern __shared__ K s_y[];            // [k + 1][54] folded: the NC vectors (y[i][0]), the combined one
+    __shared__ K s_w[128], s_wb[128], s_wa[128], s_g[AJ_MAX];
+    __shared__ K s_eq[2];                 // the x-independent factors of eq_beta and of eq_alpha gamma^k
+    __shared__ K s_red[AJ_T / 32][8], s_sum[8];
+    const int j = a.j, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ntail = a.ell_d - j - 1, tail_len = 1 << ntail;
+    const int hs = 1 << (j + 1), stride = 1 << j;
+    // ---- 1. weights: fold weights of offsets, tail weights chi(beta_a[j+1..]), chi(alpha[j+1..]) ----
+    if (tid < 128) {
+        if (tid < stride) s_w[tid] = chi_of(a.ajtai_chals, j, tid);
+    } else if (tid < 256) {
+        if (tid - 128 < tail_len) s_wb[tid - 128] = chi_of(a.beta_a + j + 1, ntail, tid - 128);
+    } else if (tid < 384) {
+        if (tid - 256 < tail_len) s_wa[tid - 256] = chi_of(a.alpha + j + 1, ntail, tid - 256);
+    } else if (warp == 12 || warp == 13) {
+        const bool in = warp == 13;
+        K e = lane < j ? eq_lin(a.ajtai_chals[lane], in ? a.alpha[lane] : a.beta_a[lane]) : gl::kone();
+        e = warp_prod(e);
+        if (lane == 0) s_eq[in] = kmul_n(e, ld_k(a.pre + AJ_EQ + in));
+    } else {
+        for (int i = tid - 448; i < a.k; i += 64) s_g[i] = ld_k(a.pre + AJ_G + i);
+    }
+    __syncthreads();
+    // ---- 2. prefix fold by bits 0..j-1: entry i of the folded vector at s_y[q][i 2^j] ----
+    for (int q = warp; q <= a.k; q += AJ_T / 32) {
+        const K* src = q < a.k ? a.y + (uint64_t)q * a.t * NEO_D : a.pre + AJ_E;
+        K* dst = s_y + q * NEO_D;
+        K v0 = ld_k(src + lane), v1 = lane + 32 < NEO_D ? ld_k(src + lane + 32) : gl::kzero();
+        if (j > 0) {
+            v0 = kmul_n(v0, s_w[lane & (stride - 1)]);
+            v1 = kmul_n(v1, s_w[(lane + 32) & (stride - 1)]);
+            for (int o = 1; o < stride && o < 32; o <<= 1) {
+                v0 = gl::kadd(v0, shfl_xor_k(v0, o));
+                v1 = gl::kadd(v1, shfl_xor_k(v1, o));
+            }
+            if (stride > 32) v0 = gl::kadd(v0, v1);
+        }
+        if ((lane & (stride - 1)) == 0) {
+            dst[lane] = v0;
+            if (stride <= 32 && lane + 32 < NEO_D) dst[lane + 32] = v1;
+        }
+    }
+    __syncthreads();
+    // ---- 3. sums over the tail: NC coefficients 0..3 of all vectors, and the combined
+    //         vector's lo and hi sums ----
+    K v[8];
+#pragma unroll
+    for (int d = 0; d < 8; d++) v[d] = gl::kzero();
+    const int nt = (NEO_D + hs - 1) / hs;
+    for (int u = tid; u < (a.k + 1) * nt; u += AJ_T) {
+        const int q = u / nt, tt = u - q * nt, idx = tt * hs, i1 = idx + stride;
+        const K lo = s_y[q * NEO_D + idx], hi = i1 < NEO_D ? s_y[q * NEO_D + i1] : gl::kzero();
+        if (q < a.k) {
+            K n[4];
+            n_coeffs<true>(lo, hi, n);  // range product, b = 2
+            const K w = kmul_n(s_wb[tt], s_g[q]);
+#pragma unroll
+            for (int d = 0; d < 4; d++) v[d] = gl::kadd(v[d], kmul_n(w, n[d]));
+        } else {
+            v[4] = gl::kadd(v[4], kmul_n(s_wa[tt], lo));
+            v[5] = gl::kadd(v[5], kmul_n(s_wa[tt], hi));
+        }
+    }
+    int idx;
+    const K tot = warp_sums<8>(v, &idx);
+    s_red[warp][idx] = tot;  // the lanes of a value hold the same sum
+    __syncthreads();
+    if (tid < 128) {  // 16 lanes a value
+        K x = s_red[tid & 15][tid >> 4];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) x = gl::kadd(x, shfl_xor_k(x, o));
+        if ((tid & 15) == 0) s_sum[tid >> 4] = x;
+    }
+    __syncthreads();
+    // ---- 4. per evaluation point ----
+    if (tid < a.nx) {
+        const K x = a.xs[tid];
+        K nc = s_sum[3];
+#pragma unroll 1
+        for (int d = 2; d >= 0; d--) nc = gl::kadd(kmul_n(nc, x), s_sum[d]);
+        const K eq_beta = kmul_n(s_eq[0], eq_lin(x, a.beta_a[j]));
+        K out = kmul_n(eq_beta, gl::kadd(ld_k(a.pre + AJ_F), nc));
+        if (a.k >= 2 && a.has_inputs) {
+            const K eq_ar = kmul_n(s_eq[1], eq_lin(x, a.alpha[j]));
+            out = gl::kadd(out, kmul_n(eq_ar, gl::kadd(s_sum[4], kmul_n(gl::ksub(s_sum[5], s_sum[4]), x))));
+        }
+        st_k(a.ys_out + tid, out);
+    }
+}
 
 }  // namespace
 
@@ -746,8 +731,8 @@ struct neo_gpu_ccs_oracle {
     bool coeffs_valid = false;
     std::vector<K> h_coeffs;
     // Ajtai-phase state
-    bool have_pre = false;
-    DevBuf<K> chi_r, vj, y_eval, y_sc;
+    bool have_pre = false, have_aj = false;
+    DevBuf<K> chi_r, vj, y_eval, y_sc, aj_pre;
     // build temporaries, kept across re-initialisations
     DevBuf<K> ws_bits, ws_w, ws_coef, ws_u, ws_upart;  // ws_upart: eval_u_pair_kernel partials
     DevBuf<unsigned int> ws_uticket;
@@ -842,7 +827,7 @@ static int oracle_init(neo_gpu_ctx* ctx, neo_gpu_ccs_oracle* o, const int8_t* d_
     o->n_small = 0; o->idx_eqrin = -1; o->idx_eval = -1;
     o->small_cur = 0; o->nc_cur = 0;
     o->row_chals.clear(); o->ajtai_chals.clear(); o->r_in.clear();
-    o->round_idx = 0; o->coeffs_valid = false; o->have_pre = false;
+    o->round_idx = 0; o->coeffs_valid = false; o->have_pre = o->have_aj = false;
     int rc = 0;
     o->t = cc.t;
     o->m = cc.m;
@@ -926,7 +911,10 @@ static int oracle_init(neo_gpu_ctx* ctx, neo_gpu_ccs_oracle* o, const int8_t* d_
     if ((rc = launch_chi_table(ctx, dbits.p, ell_n, S))) return rc;
     DevBuf<uint64_t>& z1 = o->ws_z1;
     NEO_CK(ctx, z1.ensure(m));
-    z1_kernel<<<ceil_div(m, 256), 256, 0, ctx->stream>>>(o->Z, m, b, z1.p);
+    Z1Pow zp;
+    zp.pw[0] = 1;
+    for (int rho = 1; rho < NEO_D; rho++) zp.pw[rho] = gl::mul(zp.pw[rho - 1], b);
+    z1_kernel<<<ceil_div(m, 256), 256, 0, ctx->stream>>>(o->Z, m, zp, z1.p);
     NEO_LAUNCHED(ctx);
     for (int v = 0; v < o->n_fvar; v++) {
         int j = o->fvar_j[v];
@@ -1348,33 +1336,45 @@ static int ajtai_round(neo_gpu_ccs_oracle* o, const uint64_t* xs, uint32_t nx, u
         int rc = ajtai_precompute(o);
         if (rc) return rc;
     }
-    if (nx > 16 || o->ell_n > 32 || o->ell_d > 8 || o->k * (1 + o->t) > 160)
+    if (nx > 16 || o->ell_n > 32 || o->ell_d > 8 || o->k * (1 + o->t) > AJ_MAX)
         return ctx->fail(NEO_ERR_UNSUPPORTED, "ccs_oracle: ajtai phase size limits");
+    if (!o->have_aj) {
+        NEO_CK(ctx, o->aj_pre.ensure(AJ_G + o->k));
+        AjtaiPre p{};
+        p.k = (int)o->k; p.t = (int)o->t; p.ell_n = (int)o->ell_n;
+        p.has_inputs = o->has_inputs;
+        for (uint32_t i = 0; i < o->ell_n; i++) {
+            p.beta_r[i] = o->beta_r[i];
+            p.row_chals[i] = o->row_chals[i];
+            if (o->has_inputs) p.r_in[i] = o->r_in[i];
+        }
+        p.gamma = o->gamma;
+        p.f = o->f;
+        for (int v = 0; v < o->n_fvar; v++) p.fvar_j[v] = o->fvar_j[v];
+        p.y = o->y_eval.p;
+        p.ysc = o->y_sc.p;
+        p.out = o->aj_pre.p;
+        ajtai_pre_kernel<<<1, 512, 0, ctx->stream>>>(p);
+        NEO_LAUNCHED(ctx);
+        o->have_aj = true;
+    }
     AjtaiArgs a{};
-    a.k = (int)o->k; a.t = (int)o->t; a.ell_d = (int)o->ell_d; a.ell_n = (int)o->ell_n;
+    a.k = (int)o->k; a.t = (int)o->t; a.ell_d = (int)o->ell_d;
     a.j = (int)(o->round_idx - o->ell_n);
     a.nx = (int)nx;
     a.has_inputs = o->has_inputs;
     for (uint32_t i = 0; i < nx; i++) a.xs[i] = gl::kmk(gl::canon(xs[2 * i]), gl::canon(xs[2 * i + 1]));
     for (uint32_t i = 0; i < o->ell_d; i++) { a.alpha[i] = o->alpha[i]; a.beta_a[i] = o->beta_a[i]; }
     for (size_t i = 0; i < o->ajtai_chals.size(); i++) a.ajtai_chals[i] = o->ajtai_chals[i];
-    for (uint32_t i = 0; i < o->ell_n; i++) {
-        a.beta_r[i] = o->beta_r[i];
-        a.row_chals[i] = o->row_chals[i];
-        if (o->has_inputs) a.r_in[i] = o->r_in[i];
-    }
-    a.gamma = o->gamma;
-    a.f = o->f;
-    for (int v = 0; v < o->n_fvar; v++) a.fvar_j[v] = o->fvar_j[v];
     a.y = o->y_eval.p;
-    a.ysc = o->y_sc.p;
+    a.pre = o->aj_pre.p;
     K* out = reinterpret_cast<K*>(ctx->h_result);
     a.ys_out = out;
-    size_t smem = ((size_t)o->k * (1 + o->t) * NEO_D + (size_t)nx * o->k) * sizeof(K);
+    size_t smem = ((size_t)o->k + 1) * NEO_D * sizeof(K);
     static SmemLimit limit;
     NEO_CK(ctx, limit.at_least(ajtai_round_kernel, smem));
     result_arm(out, 2 * (size_t)nx);
-    ajtai_round_kernel<<<1, 512, smem, ctx->stream>>>(a);
+    ajtai_round_kernel<<<1, AJ_T, smem, ctx->stream>>>(a);
     NEO_LAUNCHED(ctx);
     NEO_CK(ctx, result_wait(ctx, out, 2 * (size_t)nx));
     memcpy(ys, out, nx * sizeof(K));

