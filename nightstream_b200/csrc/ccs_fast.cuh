@@ -246,7 +246,8 @@ __device__ __forceinline__ void block_sum_rec(K (&v)[N], K* rec) {
 //   NC blocks (rounds >= 3): E_j(t) sum_q wg_q N(y_{q,t}(X)) over a q chunk,
 //     one thread per (pair, chunk).
 // The last block to finish (an atomic ticket) sums the records and writes the
-// round's coefficients C_j eq(beta_j, X) S(X) + gamma^k V(X).
+// round's coefficients C_j eq(beta_j, X) S(X) + gamma^k V(X) (e0 and e1 come as
+// arguments: the chain from the challenges cost the last block 2.4 us).
 struct FastRoundArgs {
     int j;
     uint32_t n_mom, n_small;     // blocks of the first two roles; the rest are NC blocks
@@ -264,6 +265,7 @@ struct FastRoundArgs {
     int idx_eqrin, idx_eval;
     FTerms f;
     int fdeg;                    // degree of f (<= MAX_DEG - 1)
+    int lanes;                   // eight lanes per pair (small_lanes_role) instead of one
     const K* E;                  // E_j [pairs]
     uint64_t pairs;
     // NC
@@ -280,9 +282,8 @@ struct FastRoundArgs {
     K* partials;                 // [gridDim.x][REC]
     unsigned int* ticket;        // zero between launches (atomicInc wraps it)
     int ncoef;
-    K beta[32];                  // beta_r
+    K e0, e1;                    // C_j eq(beta_j, X) = e0 + e1 X
     K gamma_to_k;
-    K* Cs;                       // [ell]: C_j of each round (written by round j)
     K* coeffs_out;               // [ncoef]
 };
 
@@ -412,6 +413,92 @@ __device__ __noinline__ void small_role(const FastRoundArgs& a, uint32_t blk, K*
         }
     }
     block_sum_rec<16>(out, rec);
+}
+
+// The small tables with eight lanes per pair, 32 pairs a block: the folds go over the
+// block's threads, and lane d of a pair holds coefficient d of a term, multiplied by a
+// factor a + b X with one product by a and one by b of its neighbour's coefficient.
+// A round with few pairs is one dependent chain, and a thread that walked a pair's
+// tables and terms by itself was most of it (R1CS, 2^10 rows: 16.5 us a round, with
+// the lanes 11); SMALL_LANE_PAIRS keeps the form to one block per SM, where the
+// extra partial records cost nothing.
+constexpr uint64_t SMALL_LANE_PAIRS = 148 * 32;
+__host__ __device__ constexpr uint32_t small_blocks(uint64_t pairs) {
+    return (uint32_t)(pairs <= SMALL_LANE_PAIRS ? (pairs + 31) / 32 : (pairs + FR - 1) / FR);
+}
+__device__ __noinline__ void small_lanes_role(const FastRoundArgs& a, uint32_t blk, K* rec) {
+    static_assert(MAX_DEG == 8, "a lane per coefficient of f");
+    __shared__ K s_lo[2 + MAX_FVAR + 2][32], s_df[2 + MAX_FVAR + 2][32];  // entry 2t, and entry 2t+1 minus it
+    __shared__ K s_sum[FR / 32][REC];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = tid & 7, pl = tid >> 3;
+    const uint64_t t0 = blk * 32ull, t = t0 + pl;
+    for (int e = tid; e < (a.n_small_tab - 1) * 32; e += FR) {
+        const int s = 1 + (e >> 5), p = e & 31;
+        const uint64_t tp = t0 + p;
+        if (tp >= a.pairs) continue;
+        K lo, hi;
+        if (a.fold) {
+            const K* in = a.small_in + (uint64_t)s * a.small_len_in + 4 * tp;
+            const K x0 = ld_k(in), x1 = ld_k(in + 1), x2 = ld_k(in + 2), x3 = ld_k(in + 3);
+            lo = klerp_c<true>(x0, x1, a.r);
+            hi = klerp_c<true>(x2, x3, a.r);
+            if (a.small_out) {
+                K* o = a.small_out + (uint64_t)s * a.small_len_out + 2 * tp;
+                st_k(o, lo);
+                st_k(o + 1, hi);
+            }
+        } else {
+            const K* in = a.small_in + (uint64_t)s * a.small_len_in + 2 * tp;
+            lo = ld_k(in);
+            hi = ld_k(in + 1);
+        }
+        s_lo[s][p] = lo;
+        s_df[s][p] = gl::ksub(hi, lo);
+    }
+    const bool live = t < a.pairs;
+    const K e = live ? ld_k(a.E + t) : gl::kzero();
+    __syncthreads();
+    // coefficient d of (term) (av + bv X); the lanes of a dead pair multiply zeros
+    auto times = [&](K c, K av, K bv) {
+        K below;
+        below.re = __shfl_up_sync(0xffffffffu, (unsigned long long)c.re, 1, 8);
+        below.im = __shfl_up_sync(0xffffffffu, (unsigned long long)c.im, 1, 8);
+        const K x = kmul_n(av, c), y = kmul_n(bv, below);
+        return d ? gl::kadd(x, y) : x;
+    };
+    auto at = [&](const K (*tab)[32], int s) { return live ? tab[s][pl] : gl::kzero(); };
+    K S = gl::kzero();
+#pragma unroll 1
+    for (int tt = 0; tt < a.f.n_terms; tt++) {
+        K c = d == 0 ? a.f.coeff[tt] : gl::kzero();
+#pragma unroll 1
+        for (int vv = 0; vv < a.f.n_vars[tt]; vv++) {
+            const int pos = a.f.var_pos[tt][vv];
+            const K av = at(s_lo, 1 + pos), bv = at(s_df, 1 + pos);
+#pragma unroll 1
+            for (int x = 0; x < a.f.var_exp[tt][vv]; x++) c = times(c, av, bv);
+        }
+        S = gl::kadd(S, c);
+    }
+    S = kmul_n(e, S);
+    K V = gl::kzero();
+    if (a.idx_eval >= 0) {
+        if (d < 2) V = at(d ? s_df : s_lo, a.idx_eval);
+        V = times(V, at(s_lo, a.idx_eqrin), at(s_df, a.idx_eqrin));
+    }
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {
+        S = gl::kadd(S, shfl_xor_k(S, o));
+        V = gl::kadd(V, shfl_xor_k(V, o));
+    }
+    if (lane < 8) s_sum[warp][lane] = S;
+    if (lane < 3) s_sum[warp][MAX_DEG + lane] = V;
+    __syncthreads();
+    if (tid < REC) {
+        K x = gl::kzero();
+        for (int w = 0; w < FR / 32; w++) x = gl::kadd(x, s_sum[w][tid]);
+        st_k(rec + tid, x);
+    }
 }
 
 // Round 3, separable part.  With lo, hi the K-linear forms of the even and
@@ -600,17 +687,11 @@ __device__ __noinline__ void round_final_reduce(const FastRoundArgs& a) {
     }
     __syncthreads();
     if (threadIdx.x < (unsigned)a.ncoef) {
-        // C_j eq(beta_j, X) = e0 + e1 X; coefficient d = e0 S_d + e1 S_{d-1} + gamma^k V_d
-        // C_j = C_{j-1} eq(beta_{j-1}, r_{j-1}), C_0 = 1; kept on the device per round
-        const K Cj = a.j == 0 ? gl::kone() : kmul_n(ld_k(a.Cs + a.j - 1), eq_lin(a.beta[a.j - 1], a.chals[a.j - 1]));
-        if (threadIdx.x == 0) st_k(a.Cs + a.j, Cj);
-        const K bj = a.beta[a.j];
-        const K e0 = kmul_n(Cj, gl::ksub(gl::kone(), bj));
-        const K e1 = kmul_n(Cj, gl::ksub(gl::kdbl(bj), gl::kone()));
+        // coefficient d = e0 S_d + e1 S_{d-1} + gamma^k V_d
         const int d = threadIdx.x;
         K v = gl::kzero();
-        if (d < MAX_DEG) v = kmul_n(e0, s_S[d]);
-        if (d >= 1 && d - 1 < MAX_DEG) v = gl::kadd(v, kmul_n(e1, s_S[d - 1]));
+        if (d < MAX_DEG) v = kmul_n(a.e0, s_S[d]);
+        if (d >= 1 && d - 1 < MAX_DEG) v = gl::kadd(v, kmul_n(a.e1, s_S[d - 1]));
         if (d < 3) v = gl::kadd(v, kmul_n(a.gamma_to_k, s_S[MAX_DEG + d]));
         st_k(a.coeffs_out + d, v);
     }
@@ -627,7 +708,8 @@ __global__ void __launch_bounds__(FR, 2) ccs_fast_round_kernel(const __grid_cons
         if constexpr (MODE == 3) sep_role(a, b, rec);
         else mom_role(a, b, rec);
     } else if (b < a.n_mom + a.n_small) {
-        small_role(a, b - a.n_mom, rec);
+        if (a.lanes) small_lanes_role(a, b - a.n_mom, rec);
+        else small_role(a, b - a.n_mom, rec);
     } else {
         if constexpr (MODE != 0) nc_role<MODE, C>(a, b - a.n_mom - a.n_small, rec, s_wg);
     }

@@ -715,7 +715,6 @@ struct neo_gpu_ccs_oracle {
     DevBuf<uint32_t> hist_part; // [hist blocks][8][NPAT]
     DevBuf<uint32_t> tern_flag;
     DevBuf<uint32_t> ticket;    // last-block ticket of the fused round kernel
-    DevBuf<K> Cs;               // C_j = prod_{i<j} eq(beta_i, r_i) per row round
     HostBuf<K> h_chals;         // page-locked staging of the row challenges (async upload)
     uint32_t hist_gx = 0, hist_gy = 0, hist_qc = 0;
     bool hist_split = false;
@@ -1049,12 +1048,11 @@ static int fast_setup(neo_gpu_ccs_oracle* o) {
     NEO_CK(ctx, o->hist_part.ensure((size_t)nz * o->hist_gx * o->hist_gy * NPAT * HIST_LIMBS));
     NEO_CK(ctx, o->hist64.ensure((size_t)nz * NPAT * HIST_LIMBS));
     NEO_CK(ctx, o->ticket.ensure(1));
-    NEO_CK(ctx, o->Cs.ensure(ell));
     NEO_CK(ctx, cudaMemsetAsync(o->ticket.p, 0, 4, ctx->stream));
     // partial records: the largest round
     uint64_t recs = 0;
     for (uint32_t j = 0; j < ell; j++) {
-        uint64_t r = ceil_div(o->n_pad >> (j + 1), FR);
+        uint64_t r = small_blocks(o->n_pad >> (j + 1));
         if (j <= 3) r += ceil_div(NPAT, FR);
         if (j >= 3) {
             uint32_t nc, qc, blocks;
@@ -1126,8 +1124,17 @@ static int fast_round_launch(neo_gpu_ccs_oracle* o, K* coeffs_dst) {
     a.fdeg = o->deg_max - 1;
     a.E = o->E_all.p + (o->n_pad - (o->n_pad >> j));
     a.pairs = o->n_pad >> (j + 1);
-    a.n_small = (uint32_t)ceil_div(a.pairs, FR);
-    for (uint32_t i = 0; i < j && i < 32; i++) a.chals[i] = o->row_chals[i];
+    a.n_small = small_blocks(a.pairs);
+    a.lanes = a.pairs <= SMALL_LANE_PAIRS;
+    // C_j eq(beta_j, X) = e0 + e1 X, C_j = prod_{i<j} eq(beta_i, r_i)
+    K Cj = gl::kone();
+    for (uint32_t i = 0; i < j && i < 32; i++) {
+        const K b = o->beta_r[i], r = o->row_chals[i];
+        a.chals[i] = r;
+        Cj = gl::kmul(Cj, gl::kadd(gl::kmul(gl::ksub(gl::kone(), b), gl::ksub(gl::kone(), r)), gl::kmul(b, r)));
+    }
+    a.e0 = gl::kmul(Cj, gl::ksub(gl::kone(), o->beta_r[j]));
+    a.e1 = gl::kmul(Cj, gl::ksub(gl::kdbl(o->beta_r[j]), gl::kone()));
     a.Z = o->Z;
     a.m = o->m;
     a.wg = o->wg.p;
@@ -1151,9 +1158,7 @@ static int fast_round_launch(neo_gpu_ccs_oracle* o, K* coeffs_dst) {
     a.partials = o->partials.p;
     a.ticket = o->ticket.p;
     a.ncoef = o->deg_max + 1;
-    for (uint32_t i = 0; i < ell && i < 32; i++) a.beta[i] = o->beta_r[i];
     a.gamma_to_k = o->gamma_to_k;
-    a.Cs = o->Cs.p;
     a.coeffs_out = coeffs_dst;
     const uint32_t blocks = a.n_mom + a.n_small + nc_blocks;
     const size_t wsm = j >= 3 ? (size_t)nq * sizeof(K) : 0;

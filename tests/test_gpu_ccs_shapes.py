@@ -91,3 +91,25 @@ def test_ajtai_rounds_shapes(ctx, ell_d, k, inputs):
         g.fold(r)
         o.fold(r)
     g.close()
+
+
+def test_row_rounds_across_the_pair_forms(ctx):
+    """2^14 rows: the first row round has a thread per pair, the next ones eight lanes;
+    an f of degree 7, the largest, fills every coefficient lane."""
+    ell, k = 14, 2
+    n = 1 << ell
+    rng = np.random.default_rng(14)
+    ccs = CcsStructure(n, n, [None] + [_matrix(rng, n, kd) for kd in ("uniform", "skew")],
+                       [(1, [3, 3, 1]), (Q - 5, [0, 1, 0]), (9, [1, 0, 1])])
+    Z = rng.integers(-1, 2, size=(k, 54, n)).astype(np.int8)
+    d_sc = ccs.f_degree + 1
+    args = (ccs, Z, 2, synth.uniform_k(rng, 6), synth.uniform_k(rng, 6), synth.uniform_k(rng, ell),
+            synth.uniform_k(rng, 1)[0], synth.uniform_k(rng, ell), 6, ell, d_sc)
+    g, o = gpu.GpuCcsOracle(ctx, *args), O.CcsOracle(*args)
+    xs = np.array([[x, 0] for x in range(d_sc + 1)], np.uint64)
+    for rnd in range(ell):
+        assert np.array_equal(g.evals_at(xs), o.evals_at(xs)), f"round {rnd}"
+        r = synth.uniform_k(rng, 1)[0]
+        g.fold(r)
+        o.fold(r)
+    g.close()
