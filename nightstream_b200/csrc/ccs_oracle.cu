@@ -1327,10 +1327,8 @@ static int ajtai_precompute(neo_gpu_ccs_oracle* o) {
     NEO_CK(ctx, cudaMemcpyAsync(dbits.p, o->row_chals.data(), o->ell_n * 16, cudaMemcpyHostToDevice, ctx->stream));
     int rc = launch_chi_table(ctx, dbits.p, o->ell_n, o->chi_r.p);
     if (rc) return rc;
-    rc = launch_me_y(ctx, *o->ccs, o->Z, o->k, o->m, o->chi_r.p, o->ell_n, o->b, o->vj.p, o->y_eval.p, o->y_sc.p,
-                     o->fast);  // fast: every digit checked ternary at creation
+    rc = launch_me_y(ctx, *o->ccs, o->Z, o->k, o->m, o->chi_r.p, o->ell_n, o->b, o->vj.p, o->y_eval.p, o->y_sc.p);
     if (rc) return rc;
-    NEO_CK(ctx, ctx_sync(ctx));
     o->have_pre = true;
     return NEO_OK;
 }
@@ -1382,6 +1380,7 @@ static int ajtai_round(neo_gpu_ccs_oracle* o, const uint64_t* xs, uint32_t nx, u
     ajtai_round_kernel<<<1, AJ_T, smem, ctx->stream>>>(a);
     NEO_LAUNCHED(ctx);
     NEO_CK(ctx, result_wait(ctx, out, 2 * (size_t)nx));
+    if (int rc = check_host_error(ctx)) return rc;
     memcpy(ys, out, nx * sizeof(K));
     return NEO_OK;
 }
@@ -1475,7 +1474,7 @@ static int neo_gpu_ccs_oracle_me_outputs_impl_abi(neo_gpu_ccs_oracle* o, uint64_
     NEO_CK(ctx, ctx_d2h(ctx, y, o->y_eval.p, o->y_eval.bytes()));
     NEO_CK(ctx, ctx_d2h(ctx, y_scalars, o->y_sc.p, o->y_sc.bytes()));
     NEO_CK(ctx, ctx_sync(ctx));
-    return NEO_OK;
+    return check_host_error(ctx);
 }
 extern "C" int neo_gpu_ccs_oracle_me_outputs(neo_gpu_ccs_oracle* o, uint64_t* y, uint64_t* y_scalars) { NEO_ABI_GUARD(neo_gpu_ccs_oracle_me_outputs_impl_abi(o, y, y_scalars)) }
 

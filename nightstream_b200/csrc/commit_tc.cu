@@ -44,6 +44,7 @@
 //
 // What bounds it, and what it measured, stands at commit_win_kernel.
 #include "internal.cuh"
+#include "tc.cuh"
 #include <algorithm>
 
 namespace {
@@ -53,103 +54,6 @@ constexpr int TC_BUILDERS = 128;            // warps 2..5: B builders, then the 
 constexpr int TC_TRANSPOSERS = 64;          // warps 6, 7
 constexpr int TC_MAX_KB = 512;              // K blocks per CTA (int32 overflow bound)
 constexpr uint32_t TC_MIN_KB = 4;           // K blocks per CTA worth a CTA of its own (m = 2^10: 2 and 4 14.6 us, 8 16.7)
-constexpr uint32_t TC_SPIN_LIMIT = 1u << 22;       // wait attempts (each suspends at most a hardware limit)
-constexpr uint64_t TC_WAIT_NS = 500ull * 1000 * 1000;  // 0.5 s of global time per wait
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-// bounded wait on phase parity; false on timeout.  mbarrier.try_wait suspends
-// the thread until the phase completes or a hardware time limit passes, so a
-// waiting warp does not keep polling shared memory; the wait gives up after
-// TC_WAIT_NS of global time or TC_SPIN_LIMIT attempts, whichever comes first.
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t addr = smem_u32(bar);
-    uint64_t t0 = 0;
-    for (uint32_t it = 0; it < TC_SPIN_LIMIT; it++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (done) return true;
-        const uint64_t t = globaltimer_ns();
-        if (it == 0)
-            t0 = t;
-        else if (t - t0 > TC_WAIT_NS)
-            return false;
-    }
-    return false;
-}
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-// UMMA shared-memory descriptor: K-major, 128B swizzle, 8-row atoms 1024 B apart.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);          // start address
-    d |= (uint64_t)1 << 16;                           // leading byte offset (unused for SW128 K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                 // stride byte offset: 8 rows x 128 B
-    d |= (uint64_t)1 << 46;                           // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;                           // layout: SWIZZLE_128B
-    return d;
-}
-
-// UMMA shared-memory descriptor: K-major, no swizzle: 8-row x 16-byte core
-// matrices, `lbo` bytes between core matrices along K, 128 between 8-row groups.
-__device__ __forceinline__ uint64_t ns_desc(uint32_t saddr, uint32_t lbo) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)((lbo >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((128 >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;  // descriptor version (sm_100); layout bits 61-63 = 0: no swizzle
-    return d;
-}
-
-// instruction descriptor: kind::i8, D = s32, A = u8 (K-major), B = s8 (K-major), M = 128
-__host__ __device__ constexpr uint32_t idesc_i8(int n) {
-    return (2u << 4)            // c_format = S32
-           | (0u << 7)          // a_format = unsigned 8-bit
-           | (1u << 10)         // b_format = signed 8-bit
-           | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-
 // ---------------------------------------------------------------------------
 // prep: PP -> pre-swizzled u8 limb tiles  PPL[kb][row][128 B]
 // ---------------------------------------------------------------------------
@@ -481,7 +385,7 @@ commit_win_kernel(const __grid_constant__ TcArgs a) {
     } else if (warp == 1) {
         // ---- MMA issuer: one M = 128, N = NPAD MMA per 32-byte K step ----
         if (lane == 0) {
-            const uint32_t id = idesc_i8(S::NPAD);
+            const uint32_t id = idesc_i8(S::NPAD, false, true);
             for (uint32_t it = 0; it < nkb; it++) {
                 const int sa = it % S::ASTAGES, sb = it % S::BSTAGES;
                 if (!mbar_wait(&full_a[sa], (it / S::ASTAGES) & 1) || !mbar_wait(&full_b[sb], (it / S::BSTAGES) & 1)) {

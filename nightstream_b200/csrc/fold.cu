@@ -1829,7 +1829,7 @@ static int fold_step_impl(neo_gpu_shard* sh, const uint64_t* z_host, const uint6
         if ((rc = upload_point(sh, r_val))) return rc;
         if ((rc = launch_chi_table(ctx, sh->d_r.p, ell_n, sh->d_chi.p))) return rc;
         if ((rc = launch_me_y(ctx, sh->ccs, sh->valwit.p, nv, m, sh->d_chi.p, ell_n, sh->b, sh->d_vj.p, sh->d_yv.p,
-                              sh->d_yvsc.p, true)))
+                              sh->d_yvsc.p)))
             return rc;
         std::vector<K> yv((size_t)nv * t * NEO_D), yvsc((size_t)nv * t);
         NEO_CK(ctx, ctx_d2h(ctx, yv.data(), sh->d_yv.p, yv.size() * sizeof(K)));

@@ -50,6 +50,19 @@ struct neo_gpu_ctx {
 };
 
 constexpr size_t CTX_RESULT_BYTES = 4096;
+// the last word of h_result: nonzero once a kernel's bounded wait gave up
+inline volatile uint32_t* ctx_host_err(neo_gpu_ctx* c) {
+    return reinterpret_cast<volatile uint32_t*>(static_cast<char*>(c->h_result) + CTX_RESULT_BYTES - 8);
+}
+// for a call that has waited for the launches it asks about
+inline int check_host_error(neo_gpu_ctx* c) {
+    const uint32_t e = *ctx_host_err(c);
+    if (!e) return NEO_OK;
+    *ctx_host_err(c) = 0;
+    char buf[64];
+    snprintf(buf, sizeof buf, "device wait timed out (error bits 0x%x)", e);
+    return c->fail(NEO_ERR_CUDA, buf);
+}
 
 // wait for the context's stream (a spinning stream synchronization: batch
 // workers that slept in blocking waits were measured no faster)
@@ -305,8 +318,8 @@ int launch_chi_table(neo_gpu_ctx* ctx, const gl::K* d_bits, uint32_t nbits, gl::
 int launch_suffix_chi_tables(neo_gpu_ctx* ctx, const gl::K* d_bits, uint32_t nbits, gl::K* d_out);
 int launch_me_y(neo_gpu_ctx* ctx, const DevCcs& ccs, const int8_t* d_Z, uint32_t n_w, uint64_t m,
                 const gl::K* d_chi, uint32_t ell_n, uint32_t b, gl::K* d_vj_scratch, gl::K* d_y,
-                gl::K* d_ysc, bool ternary = false);
-// y[row][j] = sum_c Z[row][c] v[j][c] of R ternary digit rows (y layout [w][t][54]); *done = false
+                gl::K* d_ysc);
+// y[row][j] = sum_c Z[row][c] v[j][c] of R int8 digit rows (y layout [w][t][54]); *done = false
 // (nothing launched) when m % 64 != 0 or t > 4
 int launch_zrows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t R, uint64_t m, uint32_t t, const gl::K* d_v,
                  gl::K* d_y, bool* done);
