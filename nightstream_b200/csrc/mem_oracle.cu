@@ -265,7 +265,10 @@ __global__ void __launch_bounds__(256) dot_kernel(const K* __restrict__ a, const
 // pending challenge), evaluates and reduces the tables of up to MULTI_MAX claims
 // together; the values land in page-locked memory.
 constexpr int MULTI_MAX = 24;
-constexpr uint32_t MULTI_TILES = 2 * 148;  // tiles of a launch that keep the SMs busy
+// tiles of a launch below which a pair's factors are shared by more lanes: the active rows
+// are often a quarter of all, so three times what two blocks per SM need (2^16 rows, 15
+// factors, us per round 1 to 3: 28, 19, 15 with two tiles per SM, 20, 16, 14 with six)
+constexpr uint32_t MULTI_TILES = 6 * 148;
 
 struct MultiClaim {
     const K* tab;      // [nf][len] current tables (written by this launch when src is set)
@@ -286,7 +289,13 @@ struct MultiClaim {
                            // coefficients, through the npts x npts inverse Vandermonde matrix of 0..npts-1
     K* out;
     unsigned int* ticket;  // the claim's block counter (zero between launches)
+    // [MULTI_COPIES][MEM_MAX_DEG + 1][4] sums of the tiles' values, as 32-bit halves of re
+    // and im (zero between launches).  Blocks add to them without waiting; with a partial
+    // per block and point, the last block read 592 x 17 of them, 10 us of a round.  The
+    // blocks take turns over the copies, so that an address sees a quarter of the adds.
+    unsigned long long* acc;
 };
+constexpr uint32_t MULTI_COPIES = 4;
 
 // entries 2p, 2p + 1 of a table in one 32-byte load (read-only data, 32-byte aligned)
 __device__ __forceinline__ void ldg_pair(const K* p, K& a, K& b) {
@@ -568,8 +577,13 @@ __global__ void __launch_bounds__(256) mem_multi_eval_kernel(const __grid_consta
         const uint32_t x = threadIdx.x;
         K v = gl::kzero();
         for (uint32_t g = 0; g < hb; g++) v = gl::kadd(v, s_red[(x % xstep) * hb + g][x / xstep]);
-        if (c.nblk > 1) a.partials[c.part0 + (uint64_t)x * c.nblk + b] = v;
-        else if (c.vinv) s_v[x] = v;
+        if (c.nblk > 1) {
+            unsigned long long* acc = c.acc + ((b % MULTI_COPIES) * (MEM_MAX_DEG + 1) + x) * 4;
+            atomicAdd(acc, (unsigned long long)(uint32_t)v.re);
+            atomicAdd(acc + 1, (unsigned long long)(v.re >> 32));
+            atomicAdd(acc + 2, (unsigned long long)(uint32_t)v.im);
+            atomicAdd(acc + 3, (unsigned long long)(v.im >> 32));
+        } else if (c.vinv) s_v[x] = v;
         else c.out[x] = v;
     }
     if (c.nblk == 1) {
@@ -577,7 +591,7 @@ __global__ void __launch_bounds__(256) mem_multi_eval_kernel(const __grid_consta
         if (c.vinv) multi_coeffs(c, s_v);
         return;
     }
-    // the claim's last block to finish sums its partials (ticket, no waits)
+    // the claim's last block to finish reduces the sums (ticket, no waits) and clears them
     __threadfence();
     __syncthreads();
     __shared__ unsigned int s_last;
@@ -585,18 +599,24 @@ __global__ void __launch_bounds__(256) mem_multi_eval_kernel(const __grid_consta
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // one warp per point: the points' sums run side by side
-    for (uint32_t x = warp; x < c.npts; x += 256 / 32) {
-        K v = gl::kzero();
-#pragma unroll 4
-        for (uint32_t r = lane; r < c.nblk; r += 32) {
-            const ulonglong2 u = __ldcg(reinterpret_cast<const ulonglong2*>(a.partials + c.part0 + (uint64_t)x * c.nblk + r));
-            v = gl::kadd(v, gl::kmk(u.x, u.y));
-        }
+    const bool on = threadIdx.x < 4 * c.npts;  // a thread per point and half word
+    unsigned long long t[MULTI_COPIES] = {}, v = 0;
+    if (on) {
+        unsigned long long* acc = c.acc + threadIdx.x;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = gl::kadd(v, shfl_xor_km(v, o));
-        if (lane == 0) (c.vinv ? s_v : c.out)[x] = v;
+        for (uint32_t i = 0; i < MULTI_COPIES; i++) t[i] = __ldcg(acc + i * (MEM_MAX_DEG + 1) * 4);
+#pragma unroll
+        for (uint32_t i = 0; i < MULTI_COPIES; i++) {
+            v += t[i];
+            acc[i * (MEM_MAX_DEG + 1) * 4] = 0;
+        }
     }
+    // lo + 2^32 hi (each below 2^64: fewer than 2^32 blocks), then the component two lanes up
+    uint64_t w = gl::canon(v);
+    if (threadIdx.x & 1) w = gl::mul(w, 1ull << 32);
+    w = gl::add(w, __shfl_down_sync(0xffffffffu, (unsigned long long)w, 1));
+    const uint64_t im = __shfl_down_sync(0xffffffffu, (unsigned long long)w, 2);
+    if (on && (threadIdx.x & 3) == 0) (c.vinv ? s_v : c.out)[threadIdx.x >> 2] = gl::kmk(w, im);
     if (!c.vinv) return;
     __syncthreads();
     multi_coeffs(c, s_v);
@@ -973,31 +993,36 @@ int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int 
         // eight warps cover the points; with fewer points, warps share a point's pairs
         c.hb = 1;
         while (c.hb < 8 && 8 / (2 * c.hb) >= c.npts) c.hb *= 2;
-        // about four blocks per SM over the launch's claims; tiles small enough
-        // for two per SM (up to 16 lanes a pair)
+        // the blocks that are resident, two per SM, over the launch's claims (with four
+        // per SM the first rounds of a fold step's 100 columns took 31 to 43 us, now 24 to
+        // 28); tiles small enough (up to 16 lanes a pair)
         c.fs = 1;
         while (c.fs < 16 && 2 * c.fs <= c.nf && pairs * c.fs / (32 * c.hb) < MULTI_TILES / (uint32_t)n) c.fs *= 2;
         c.lpb = 5;
         for (uint32_t h = 1; h < c.hb; h *= 2) c.lpb++;
         for (uint32_t h = 1; h < c.fs; h *= 2) c.lpb--;
         const uint64_t tiles = (pairs + (1ull << c.lpb) - 1) >> c.lpb;
-        c.nblk = (uint32_t)std::min<uint64_t>(tiles, std::max<uint64_t>(64, 4ull * 148 * multi_weight(o) / wsum));
+        c.nblk = (uint32_t)std::min<uint64_t>(tiles, std::max<uint64_t>(64, 2ull * 148 * multi_weight(o) / wsum));
         blocks += c.nblk;
-        parts += (uint64_t)c.npts * c.nblk;
     }
     if (parts > 0xFFFFFFFFull) return ctx->fail(NEO_ERR_UNSUPPORTED, "mem_round_launch_multi: too many partials");
-    // the claims' tickets sit behind the partials (MULTI_MAX counters in
-    // MULTI_TICKET_K entries); they return to zero after every launch, so
-    // they are cleared only when the buffer is (re)allocated
-    constexpr size_t MULTI_TICKET_K = (MULTI_MAX * sizeof(unsigned int) + sizeof(K) - 1) / sizeof(K);
+    // the claims' sums and tickets (MULTI_MAX of each, in MULTI_TICKET_K entries) sit
+    // behind the partials of the small claims; they return to zero after every launch,
+    // so they are cleared only when the buffer is (re)allocated
+    constexpr size_t ACC_WORDS = (size_t)MULTI_COPIES * (MEM_MAX_DEG + 1) * 4;
+    constexpr size_t MULTI_ACC_K = MULTI_MAX * ACC_WORDS * 8 / sizeof(K);
+    constexpr size_t MULTI_TICKET_K = MULTI_ACC_K + (MULTI_MAX * sizeof(unsigned int) + sizeof(K) - 1) / sizeof(K);
     const K* before = partials.p;
     const size_t cap_before = partials.cap;
     NEO_CK(ctx, partials.ensure(std::max<uint64_t>(parts, cap_before > MULTI_TICKET_K ? cap_before - MULTI_TICKET_K : 0) +
                                 MULTI_TICKET_K));
-    unsigned int* tickets = reinterpret_cast<unsigned int*>(partials.p + (partials.cap - MULTI_TICKET_K));
+    K* tail = partials.p + (partials.cap - MULTI_TICKET_K);
     if (partials.p != before || partials.cap != cap_before)
-        NEO_CK(ctx, cudaMemsetAsync(tickets, 0, MULTI_TICKET_K * sizeof(K), ctx->stream));
-    for (int i = 0; i < n; i++) a.c[i].ticket = tickets + i;
+        NEO_CK(ctx, cudaMemsetAsync(tail, 0, MULTI_TICKET_K * sizeof(K), ctx->stream));
+    for (int i = 0; i < n; i++) {
+        a.c[i].acc = reinterpret_cast<unsigned long long*>(tail) + i * ACC_WORDS;
+        a.c[i].ticket = reinterpret_cast<unsigned int*>(tail + MULTI_ACC_K) + i;
+    }
     a.partials = partials.p;
     if (mf.n) {
         mem_multi_fold_kernel<<<dim3(ceil_div(fold_len, 256 * FOLD_PER), mf.f0[mf.n]), 256, 0, ctx->stream>>>(mf);
