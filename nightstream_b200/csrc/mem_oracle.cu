@@ -1487,14 +1487,98 @@ struct TaEval {
     int kind;  // 0 read, 1 write
     uint32_t N, bit;
     const uint64_t* key;    // sorted by (addr >> (bit + 1), item)
-    const K *wt, *kc, *d;
-    const K* init_tab;      // folded initial memory, >= 2 entries
+    uint64_t* key_next;     // the same items for the next round: by (addr >> (bit + 2), item)
+    K *wt, *d;
+    const K* kc;
+    const K* init_tab;      // initial memory, >= 2 entries; before the fold when pending
+    int pending;            // bind the previous bit to r first
+    K r;
+    K* tab_out;             // pending: the folded initial memory, `half` entries
+    uint64_t half;
     K* recs;                // [gridDim.x][TA_REC]
     uint32_t* heads;        // [gridDim.x] 1: a run starts inside the block
     K* out;                 // the round's values at x = 0, 1, 2
     unsigned int* ticket;
 };
 constexpr int TA_REC = 8;   // S0..S2, U0..U2, T0, T1
+
+// the last block: the carries into the blocks, and the round's values
+__device__ __forceinline__ void ta_carries(const TaEval& a, K (*s_red)[6]) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __threadfence();
+    // carries: inclusive segmented scan of (T0, T1, head) over the blocks, TE_T at a time
+    auto ldk = [](const K* q) {
+        const ulonglong2 u = __ldcg(reinterpret_cast<const ulonglong2*>(q));
+        return gl::kmk(u.x, u.y);
+    };
+    K sum[3] = {gl::kzero(), gl::kzero(), gl::kzero()};
+    K in0 = gl::kzero(), in1 = gl::kzero();  // carried into this batch of blocks
+    __shared__ K s_c[2][TE_T];
+    __shared__ uint32_t s_f[TE_T];
+    for (uint32_t base = 0; base < gridDim.x; base += TE_T) {
+        const uint32_t blk = base + tid;
+        const bool on = blk < gridDim.x;
+        const K* r = a.recs + (uint64_t)(on ? blk : 0) * TA_REC;
+        K y0 = on ? ldk(r + 6) : gl::kzero(), y1 = on ? ldk(r + 7) : gl::kzero();
+        uint32_t f = on ? __ldcg(a.heads + blk) : 0;
+        if (tid == 0 && !f) { y0 = gl::kadd(y0, in0); y1 = gl::kadd(y1, in1); }
+        const uint32_t live_n = min((uint32_t)TE_T, gridDim.x - base);
+        for (uint32_t o = 1; o < live_n; o <<= 1) {
+            s_c[0][tid] = y0; s_c[1][tid] = y1; s_f[tid] = f;
+            __syncthreads();
+            if ((uint32_t)tid >= o && !f) {
+                y0 = gl::kadd(y0, s_c[0][tid - o]);
+                y1 = gl::kadd(y1, s_c[1][tid - o]);
+                f = s_f[tid - o];
+            }
+            __syncthreads();
+        }
+        s_c[0][tid] = y0; s_c[1][tid] = y1;
+        __syncthreads();
+        const K c0 = tid ? s_c[0][tid - 1] : in0, c1 = tid ? s_c[1][tid - 1] : in1;
+        if (on) {
+            sum[0] = gl::kadd(sum[0], gl::kadd(ldk(r), gl::kmul(ldk(r + 3), c0)));
+            sum[1] = gl::kadd(sum[1], gl::kadd(ldk(r + 1), gl::kmul(ldk(r + 4), c1)));
+            sum[2] = gl::kadd(sum[2], gl::kadd(ldk(r + 2), gl::kmul(ldk(r + 5), gl::ksub(gl::kdbl(c1), c0))));
+        }
+        in0 = s_c[0][TE_T - 1];
+        in1 = s_c[1][TE_T - 1];
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        K v = sum[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v = gl::kadd(v, shfl_xor_km(v, o));
+        if (lane == 0) s_red[warp][i] = v;
+    }
+    __syncthreads();
+    if (tid < 3) {
+        K v = gl::kzero();
+        for (int i = 0; i < TE_T / 32; i++) v = gl::kadd(v, s_red[i][tid]);
+        a.out[tid] = a.kind == 0 ? v : gl::kneg(v);
+    }
+}
+
+// positions of the items in the order by (addr >> (bit + 2), item), from the one by
+// (addr >> (bit + 1), item): an item moves by the sibling run's items that come before
+// it in time
+__device__ __forceinline__ uint32_t ta_merged(const uint64_t* key, uint32_t N, uint32_t bit, uint32_t j, uint64_t k) {
+    // items before (block, item index) in the current order
+    auto lower = [&](uint32_t block, uint32_t item) {
+        uint32_t lo = 0, hi = N;
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            const uint64_t x = key[mid];
+            const uint32_t b = ta_addr(x) >> (bit + 1);
+            if (b < block || (b == block && (uint32_t)x < item)) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo;
+    };
+    const uint32_t blk = ta_addr(k) >> (bit + 1), sib = blk ^ 1;
+    return j + lower(sib, (uint32_t)k) - lower(max(blk, sib), 0);  // the runs meet at the larger block's start
+}
 
 // Blocks of TE_T sorted items.  A query's contribution at x = 0, 1, 2 is w times
 //   child 0:  v0 − k,  0,  −(2 v1 − v0 − k);   child 1:  0,  v1 − k,  2 (2 v1 − v0 − k)
@@ -1503,6 +1587,12 @@ constexpr int TA_REC = 8;   // S0..S2, U0..U2, T0, T1
 // factors U of the two sums carried in (S0 += U0 c0, S1 += U1 c1, S2 += U2 (2 c1
 // − c0)) and its own last run's sums T; the last block to finish (ticket, no
 // waits) scans the carries over the blocks and adds everything up.
+// A round is this one launch: a pending challenge is bound as the weights and the
+// initial values are read, and what only the next round reads is written once a
+// block's part of the values is out (the folded initial memory; the next order, which
+// no challenge enters: two binary searches an item).  The launch is one chain of
+// dependent steps, and with the fold as a launch before it a round's two took 13.1 and
+// 6.5 us (2^15 items); now 13 until the values are out and 17 in all.
 __global__ void __launch_bounds__(TE_T) ta_eval_kernel(const TaEval a) {
     __shared__ K s_e[2][TE_T];              // exclusive prefix sums over the block (children 0, 1)
     __shared__ K s_w[2][TE_T / 32];
@@ -1518,14 +1608,30 @@ __global__ void __launch_bounds__(TE_T) ta_eval_kernel(const TaEval a) {
     bool head = p == 0;
     if (live && p) head = (ta_addr(a.key[p - 1]) >> (a.bit + 1)) != seg;
     const bool is_q = live && (a.kind == 1 || !(key >> 63)), is_w = live && (a.kind == 1 || (key >> 63));
-    const K w = live ? a.wt[idx] : gl::kzero();
-    const K dl = !is_w ? gl::kzero() : a.kind == 1 ? a.d[idx] : w;
+    K w = live ? a.wt[idx] : gl::kzero();
+    K dl = live && a.kind == 1 ? a.d[idx] : gl::kzero();
     K kc = gl::kzero(), i0 = gl::kzero(), i1 = gl::kzero();
     if (is_q) {
         kc = a.kc[idx];
-        i0 = a.init_tab[2 * (uint64_t)seg];
-        i1 = a.init_tab[2 * (uint64_t)seg + 1];
+        if (a.pending) {
+            const K* t = a.init_tab + 4 * (uint64_t)seg;
+            i0 = gl::klerp(t[0], t[1], a.r);
+            if (a.half > 1) i1 = gl::klerp(t[2], t[3], a.r);  // one entry left: only x = 0 counts
+        } else {
+            i0 = a.init_tab[2 * (uint64_t)seg];
+            i1 = a.init_tab[2 * (uint64_t)seg + 1];
+        }
     }
+    if (a.pending && live) {  // an item is one thread's
+        const K f = ((addr >> (a.bit - 1)) & 1) ? a.r : gl::ksub(gl::kone(), a.r);
+        w = gl::kmul(w, f);
+        a.wt[idx] = w;
+        if (a.kind == 1) {
+            dl = gl::kmul(dl, f);
+            a.d[idx] = dl;
+        }
+    }
+    dl = !is_w ? gl::kzero() : a.kind == 1 ? dl : w;
     // inclusive scans of the two children's deltas and of the last head's position
     K x0 = child ? gl::kzero() : dl, x1 = child ? dl : gl::kzero();
     const K own0 = x0, own1 = x1;
@@ -1602,66 +1708,17 @@ __global__ void __launch_bounds__(TE_T) ta_eval_kernel(const TaEval a) {
     __syncthreads();
     if (tid == 0) s_last = atomicInc(a.ticket, gridDim.x - 1) == gridDim.x - 1;
     __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    // carries: inclusive segmented scan of (T0, T1, head) over the blocks, TE_T at a time
-    auto ldk = [](const K* q) {
-        const ulonglong2 u = __ldcg(reinterpret_cast<const ulonglong2*>(q));
-        return gl::kmk(u.x, u.y);
-    };
-    K sum[3] = {gl::kzero(), gl::kzero(), gl::kzero()};
-    K in0 = gl::kzero(), in1 = gl::kzero();  // carried into this batch of blocks
-    __shared__ K s_c[2][TE_T];
-    __shared__ uint32_t s_f[TE_T];
-    for (uint32_t base = 0; base < gridDim.x; base += TE_T) {
-        const uint32_t blk = base + tid;
-        const bool on = blk < gridDim.x;
-        const K* r = a.recs + (uint64_t)(on ? blk : 0) * TA_REC;
-        K y0 = on ? ldk(r + 6) : gl::kzero(), y1 = on ? ldk(r + 7) : gl::kzero();
-        uint32_t f = on ? __ldcg(a.heads + blk) : 0;
-        if (tid == 0 && !f) { y0 = gl::kadd(y0, in0); y1 = gl::kadd(y1, in1); }
-        const uint32_t live_n = min((uint32_t)TE_T, gridDim.x - base);
-        for (uint32_t o = 1; o < live_n; o <<= 1) {
-            s_c[0][tid] = y0; s_c[1][tid] = y1; s_f[tid] = f;
-            __syncthreads();
-            if ((uint32_t)tid >= o && !f) {
-                y0 = gl::kadd(y0, s_c[0][tid - o]);
-                y1 = gl::kadd(y1, s_c[1][tid - o]);
-                f = s_f[tid - o];
-            }
-            __syncthreads();
-        }
-        s_c[0][tid] = y0; s_c[1][tid] = y1;
-        __syncthreads();
-        const K c0 = tid ? s_c[0][tid - 1] : in0, c1 = tid ? s_c[1][tid - 1] : in1;
-        if (on) {
-            sum[0] = gl::kadd(sum[0], gl::kadd(ldk(r), gl::kmul(ldk(r + 3), c0)));
-            sum[1] = gl::kadd(sum[1], gl::kadd(ldk(r + 1), gl::kmul(ldk(r + 4), c1)));
-            sum[2] = gl::kadd(sum[2], gl::kadd(ldk(r + 2), gl::kmul(ldk(r + 5), gl::ksub(gl::kdbl(c1), c0))));
-        }
-        in0 = s_c[0][TE_T - 1];
-        in1 = s_c[1][TE_T - 1];
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        K v = sum[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = gl::kadd(v, shfl_xor_km(v, o));
-        if (lane == 0) s_red[warp][i] = v;
-    }
-    __syncthreads();
-    if (tid < 3) {
-        K v = gl::kzero();
-        for (int i = 0; i < TE_T / 32; i++) v = gl::kadd(v, s_red[i][tid]);
-        a.out[tid] = a.kind == 0 ? v : gl::kneg(v);
-    }
+    if (s_last) ta_carries(a, s_red);
+    // what the next round reads
+    if (live && a.key_next) a.key_next[ta_merged(a.key, a.N, a.bit, p, key)] = key;
+    if (a.pending)
+        for (uint64_t q = p; q < a.half; q += (uint64_t)gridDim.x * TE_T)
+            a.tab_out[q] = gl::klerp(a.init_tab[2 * q], a.init_tab[2 * q + 1], a.r);
 }
 
-// One fold of the address lane: item j's weights by its own bit, the
-// initial-memory table on its low address bit, and the items' order from
-// (addr >> (bit + 1), item) to (addr >> (bit + 2), item): an item moves by the
-// sibling run's items that come before it in time.
+// One fold of the address lane by itself (a second fold without an evaluation in
+// between, or no items): item j's weights by its own bit, the initial-memory table on
+// its low address bit, and the items' order.
 struct TaFold {
     uint32_t N, bit;
     int kind;
@@ -1681,24 +1738,11 @@ __global__ void __launch_bounds__(256) ta_fold_kernel(const TaFold a) {
         return;
     }
     const uint64_t key = a.key[j];
-    const uint32_t idx = (uint32_t)key, blk = ta_addr(key) >> (a.bit + 1);
+    const uint32_t idx = (uint32_t)key;
     const K f = ((ta_addr(key) >> a.bit) & 1) ? a.r : gl::ksub(gl::kone(), a.r);
     a.wt[idx] = gl::kmul(a.wt[idx], f);
     if (a.kind == 1) a.d[idx] = gl::kmul(a.d[idx], f);
-    // items before (block, item index) in the current order
-    auto lower = [&](uint32_t block, uint32_t item) {
-        uint32_t lo = 0, hi = a.N;
-        while (lo < hi) {
-            const uint32_t mid = lo + (hi - lo) / 2;
-            const uint64_t k = a.key[mid];
-            const uint32_t b = ta_addr(k) >> (a.bit + 1);
-            if (b < block || (b == block && (uint32_t)k < item)) lo = mid + 1;
-            else hi = mid;
-        }
-        return lo;
-    };
-    const uint32_t sib = blk ^ 1;
-    a.key_out[j + lower(sib, idx) - lower(max(blk, sib), 0)] = key;  // the runs meet at the larger block's start
+    a.key_out[ta_merged(a.key, a.N, a.bit, (uint32_t)j, key)] = key;
 }
 
 __global__ void scatter_init_kernel(const uint64_t* __restrict__ addr, const K* __restrict__ val, uint64_t n,
@@ -1724,6 +1768,7 @@ struct neo_gpu_twist_addr {
     uint64_t tab_len = 0;
     int cur = 0;
     bool pending = false;
+    bool next_order = false;         // key[kcur ^ 1] holds the order after the next fold
     K pending_r{};
     std::vector<K> hvals;
 };
@@ -1748,6 +1793,7 @@ int ta_apply_fold(neo_gpu_twist_addr* o) {
     o->tab_len = half;
     o->bit++;
     o->pending = false;
+    o->next_order = false;
     return NEO_OK;
 }
 
@@ -1756,7 +1802,9 @@ int ta_apply_fold(neo_gpu_twist_addr* o) {
 int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
     neo_gpu_ctx* ctx = o->ctx;
     cudaStream_t S = ctx->stream;
-    if (o->pending) {
+    // the launch binds the challenge itself once the order is there
+    const bool fused = o->pending && o->next_order && o->N;
+    if (o->pending && !fused) {
         int rc = ta_apply_fold(o);
         if (rc) return rc;
     }
@@ -1765,11 +1813,20 @@ int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
         return NEO_OK;
     }
     const uint32_t nb = ceil_div(o->N, TE_T);
-    TaEval a;
+    TaEval a{};
+    if (fused) {
+        a.pending = 1;
+        a.r = o->pending_r;
+        a.half = o->tab_len >> 1;
+        a.tab_out = o->tab[o->cur ^ 1].p;
+        o->kcur ^= 1;
+        o->bit++;
+    }
     a.kind = o->kind;
     a.N = o->N;
     a.bit = o->bit;
     a.key = o->key[o->kcur].p;
+    a.key_next = o->bit < o->A ? o->key[o->kcur ^ 1].p : nullptr;
     a.wt = o->wt.p; a.kc = o->kc.p; a.d = o->d.p;
     a.init_tab = o->tab[o->cur].p;
     a.recs = o->recs.p;
@@ -1778,6 +1835,12 @@ int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
     a.ticket = o->ticket.p;
     ta_eval_kernel<<<nb, TE_T, 0, S>>>(a);
     NEO_LAUNCHED(ctx);
+    if (fused) {
+        o->cur ^= 1;
+        o->tab_len >>= 1;
+        o->pending = false;
+    }
+    o->next_order = a.key_next != nullptr;
     return NEO_OK;
 }
 
@@ -1818,7 +1881,7 @@ int ta_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_cycle,
     o->bit = 0;
     o->cur = 0;
     o->kcur = 0;
-    o->pending = false;
+    o->pending = o->next_order = false;
     auto fail = [&](int rc) {
         if (fresh) delete o;
         return rc;

@@ -53,3 +53,27 @@ def test_twist_addr_shapes_match_oracle(ctx, kind, ell, A, active, pattern):
             g.fold(r)
             ref.fold(r)
     g.close()
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("A,active", [(1, 5), (6, 300), (11, 1000)])
+def test_rounds_in_any_call_order(ctx, kind, A, active):
+    """Values asked twice, folds without values in between (the order of the next round is
+    then not there yet), and a fold as the last call."""
+    rng = np.random.default_rng(A * 10 + kind)
+    ell = 10
+    cols = columns(kind, ell, A, active, "uniform", rng)
+    r_cycle = rand_k(rng, ell)
+    init = [(int(a), tuple(int(x) for x in rand_k(rng, 1)[0])) for a in sorted({0, (1 << A) - 1})]
+    ref = oracle.TwistAddrOracle(kind, cols, r_cycle, A, init)
+    g = gpu.GpuTwistAddrOracle(ctx, kind, cols, r_cycle, A, init)
+    xs = np.array([[0, 0], [1, 0], [2, 0], [5, 6]], np.uint64)
+    for rnd in range(A):
+        if rnd % 4 != 1:
+            for _ in range(1 + rnd % 3):
+                assert np.array_equal(g.evals_at(xs), ref.evals_at(xs)), f"round {rnd}"
+        r = rand_k(rng, 1)[0]
+        g.fold(r)
+        ref.fold(r)
+    assert np.array_equal(g.evals_at(xs), ref.evals_at(xs))
+    g.close()
