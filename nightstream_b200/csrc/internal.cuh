@@ -312,10 +312,23 @@ inline cudaError_t ctx_scratch(neo_gpu_ctx* ctx, size_t bytes, void** p) {
 }
 int dev_ccs_upload(neo_gpu_ctx* ctx, const neo_ccs_desc* desc, DevCcs& out, bool want_csr = true);
 
-// Kernels callable from several translation units.
+// A point of up to 32 coordinates as a kernel argument: it rides in the launch, where a
+// small copy from pageable memory cost the host 6 to 8 us and the stream 1.5.
+struct KPoint {
+    gl::K x[32];
+};
+inline KPoint make_point(const gl::K* h, uint32_t n) {
+    KPoint p{};
+    for (uint32_t i = 0; i < n && i < 32; i++) p.x[i] = h[i];
+    return p;
+}
+
+// Kernels callable from several translation units.  chi(point) over 2^nbits entries, the
+// point on the host or on the device
+int launch_chi_point(neo_gpu_ctx* ctx, const gl::K* h_point, uint32_t nbits, gl::K* d_out);
 int launch_chi_table(neo_gpu_ctx* ctx, const gl::K* d_bits, uint32_t nbits, gl::K* d_out);
 // chi(bits[j+1..nbits)) for every j < nbits, table j at 2^nbits - 2^(nbits-j), in one launch
-int launch_suffix_chi_tables(neo_gpu_ctx* ctx, const gl::K* d_bits, uint32_t nbits, gl::K* d_out);
+int launch_suffix_chi_tables(neo_gpu_ctx* ctx, const gl::K* h_point, uint32_t nbits, gl::K* d_out);
 int launch_me_y(neo_gpu_ctx* ctx, const DevCcs& ccs, const int8_t* d_Z, uint32_t n_w, uint64_t m,
                 const gl::K* d_chi, uint32_t ell_n, uint32_t b, gl::K* d_vj_scratch, gl::K* d_y,
                 gl::K* d_ysc);

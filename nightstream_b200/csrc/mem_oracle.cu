@@ -44,23 +44,23 @@ __device__ __forceinline__ K eq_bit_affine(K bit, K u) {
 // (out may be cols).  Bound by HBM: 32 bytes an entry, and the columns are read
 // where they are instead of copied first (12 columns of 2^16: 12 copies and
 // 10.3 us of this kernel, now the latter alone).
-__global__ void eqbit_kernel(const K* cols, uint64_t len, const K* __restrict__ u, K* out) {
+__global__ void eqbit_kernel(const K* cols, uint64_t len, const __grid_constant__ KPoint u, K* out) {
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (t >= len) return;
     const uint64_t i = blockIdx.y * len + t;
-    out[i] = eq_bit_affine(cols[i], u[blockIdx.y]);
+    out[i] = eq_bit_affine(cols[i], u.x[blockIdx.y]);
 }
 
 // inc_terms(t) = has_write(t)·inc(t)·Π_b eq_bit_affine(wa_b(t), r_addr_b)
 // (build_inc_terms_at_r_addr, twist_oracle.rs:351-378)
 __global__ void inc_terms_kernel(const K* __restrict__ has_w, const K* __restrict__ inc, const K* __restrict__ wa,
-                                 uint32_t A, const K* __restrict__ r_addr, uint64_t len, K* __restrict__ out) {
+                                 uint32_t A, const __grid_constant__ KPoint r_addr, uint64_t len, K* __restrict__ out) {
     uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (t >= len) return;
     K v = has_w[t];
     if (!gl::kiszero(v)) v = gl::kmul(v, inc[t]);
     // rows without a write (most of the time domain) read no address bits
-    for (uint32_t b = 0; b < A && !gl::kiszero(v); b++) v = gl::kmul(v, eq_bit_affine(wa[(uint64_t)b * len + t], r_addr[b]));
+    for (uint32_t b = 0; b < A && !gl::kiszero(v); b++) v = gl::kmul(v, eq_bit_affine(wa[(uint64_t)b * len + t], r_addr.x[b]));
     out[t] = v;
 }
 
@@ -159,31 +159,55 @@ __global__ void __launch_bounds__(SCAN_T) scan_final_kernel(const K* __restrict_
     }
 }
 
-// LT(t, r) for Boolean t (twist_oracle.rs:320-334)
-__global__ void lt_table_kernel(const K* __restrict__ r, uint32_t ell, K* __restrict__ out) {
-    uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t >= (1ULL << ell)) return;
-    K suffix = gl::kone(), acc = gl::kzero();
-    for (int i = (int)ell - 1; i >= 0; i--) {
-        K ri = r[i];
+// LT(t, r) for Boolean t (twist_oracle.rs:320-334): from the top bit down,
+// acc += suffix r_i where t_i = 0, suffix *= chi_i.  The low 8 bits' (acc, suffix = 1)
+// is a thread's, the high bits' a warp leader's, and LT = acc_hi + suffix_hi acc_lo
+// (2^18 entries: 51 us with every bit in every thread, now 9).
+__device__ __forceinline__ void lt_bits(const KPoint& r, int hi, int lo, uint64_t t, K& acc, K& suffix) {
+    acc = gl::kzero();
+    suffix = gl::kone();
+#pragma unroll 1
+    for (int i = hi - 1; i >= lo; i--) {
+        const K x = gl::kmul(r.x[i], suffix);
         if (((t >> i) & 1) == 0) {
-            acc = gl::kadd(acc, gl::kmul(ri, suffix));
-            suffix = gl::kmul(suffix, gl::ksub(gl::kone(), ri));
+            acc = gl::kadd(acc, x);
+            suffix = gl::ksub(suffix, x);
         } else {
-            suffix = gl::kmul(suffix, ri);
+            suffix = x;
         }
     }
-    out[t] = acc;
+}
+constexpr uint32_t LT_HIGH = 8;
+__global__ void __launch_bounds__(256) lt_table_kernel(const __grid_constant__ KPoint r, uint32_t ell, K* __restrict__ out) {
+    __shared__ K s_acc[LT_HIGH], s_suf[LT_HIGH];
+    const uint32_t low = min(ell, 8u), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t n_hi = 1ull << (ell - low), h0 = blockIdx.x * (uint64_t)LT_HIGH;
+    K acc, suffix;
+    if (lane == 0) {
+        lt_bits(r, (int)ell, (int)low, (h0 + warp) << low, acc, suffix);
+        s_acc[warp] = acc;
+        s_suf[warp] = suffix;
+    }
+    lt_bits(r, (int)low, 0, threadIdx.x, acc, suffix);
+    __syncthreads();
+    if (threadIdx.x >> low) return;
+#pragma unroll
+    for (uint32_t v = 0; v < LT_HIGH; v++)
+        if (h0 + v < n_hi) out[((h0 + v) << low) + threadIdx.x] = gl::kadd(s_acc[v], gl::kmul(s_suf[v], acc));
 }
 
 // fold every factor on variable 0: dst[f][p] = src[f][2p] + r (src[f][2p+1] − src[f][2p])
-__global__ void mem_fold_kernel(const K* __restrict__ src, uint64_t src_len, K* __restrict__ dst, uint32_t nf, K r) {
+// (host, unless null: page-locked copy of the last entries, one per factor)
+__global__ void mem_fold_kernel(const K* __restrict__ src, uint64_t src_len, K* __restrict__ dst, uint32_t nf, K r,
+                                K* host) {
     const uint64_t half = src_len >> 1;
     uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= half * nf) return;
     uint64_t f = i / half, p = i - f * half;
     const K* s = src + f * src_len + 2 * p;
-    dst[f * half + p] = gl::klerp(s[0], s[1], r);
+    const K v = gl::klerp(s[0], s[1], r);
+    dst[f * half + p] = v;
+    if (host) host[f] = v;
 }
 
 // vals[x] = Σ_b partials[x][b]; one block per x
@@ -666,7 +690,7 @@ struct neo_gpu_mem_oracle {
     DevBuf<K> w;          // bitness weights
     std::vector<K> hw;    // host copy of the weights
     DevBuf<K> partials;
-    DevBuf<K> dpt, dra, tmp, sums;  // build workspace, kept for reuse
+    DevBuf<K> tmp, sums;  // build workspace, kept for reuse
     std::vector<K> hvals;
     bool hvals_valid = false;  // hvals holds this round's values (the claim needs round 0's)
     K claim{};
@@ -785,22 +809,15 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
     auto put = [&](uint32_t f, uint32_t c, uint32_t n = 1) {
         return n ? cudaMemcpyAsync(T + (size_t)f * L, col(c), colb * n, cpk, S) : cudaSuccess;
     };
-    DevBuf<K>& dpt = o->dpt;
-    DevBuf<K>& dra = o->dra;
     DevBuf<K>& tmp = o->tmp;
-    if (r_point && dpt.ensure(ell ? ell : 1)) return fail(ctx->fail(NEO_ERR_OOM, "mem_oracle: point"));
-    if (r_point && ell && cudaMemcpyAsync(dpt.p, r_point, ell * sizeof(K), cudaMemcpyHostToDevice, S))
-        return fail(ctx->fail(NEO_ERR_CUDA, "mem_oracle: point upload"));
-    if (A && r_addr) {
-        if (dra.ensure(A) || cudaMemcpyAsync(dra.p, r_addr, A * sizeof(K), cudaMemcpyHostToDevice, S))
-            return fail(ctx->fail(NEO_ERR_OOM, "mem_oracle: r_addr"));
-    }
+    // (the kinds that read r_addr have A <= 31 by the degree bound)
+    const KPoint addr_pt = A && r_addr ? make_point(reinterpret_cast<const K*>(r_addr), A) : KPoint{};
     auto eqbits = [&](uint32_t f0, uint32_t c0) -> int {
         if (!A) return NEO_OK;
         if (!r_addr) return ctx->fail(NEO_ERR_ARG, "mem_oracle: address bits without r_addr");
         K* dst = T + (size_t)f0 * L;
         if (!cols_on_device && put(f0, c0, A)) return ctx->fail(NEO_ERR_CUDA, "mem_oracle: column upload");
-        eqbit_kernel<<<dim3(ceil_div(L, 256), A), 256, 0, S>>>(cols_on_device ? col(c0) : dst, L, dra.p, dst);
+        eqbit_kernel<<<dim3(ceil_div(L, 256), A), 256, 0, S>>>(cols_on_device ? col(c0) : dst, L, addr_pt, dst);
         NEO_LAUNCHED(ctx);
         return NEO_OK;
     };
@@ -813,7 +830,7 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
             if (cudaMemcpyAsync(T, ctx->chi_cache, bytes, cudaMemcpyDeviceToDevice, S))
                 return fail(ctx->fail(NEO_ERR_CUDA, "mem_oracle: chi copy"));
         } else {
-            rc = launch_chi_table(ctx, dpt.p, ell, T);
+            rc = launch_chi_point(ctx, reinterpret_cast<const K*>(r_point), ell, T);
             if (rc) return fail(rc);
             if (ctx->chi_cache_bytes < bytes) {
                 cudaStreamSynchronize(S);  // the old cache may still be read by an earlier copy
@@ -864,7 +881,7 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
                 hw = up; inc = up + L; aa = up + 2 * L; wa = up + 3 * L;
             }
             if (ce) break;
-            inc_terms_kernel<<<ceil_div(L, 256), 256, 0, S>>>(hw, inc, wa, A, dra.p, L, terms);
+            inc_terms_kernel<<<ceil_div(L, 256), 256, 0, S>>>(hw, inc, wa, A, addr_pt, L, terms);
             NEO_LAUNCHED(ctx);
             const uint32_t nblk = (uint32_t)ceil_div(L, SCAN_BLK);
             DevBuf<K>& sums = o->sums;
@@ -883,7 +900,8 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
         case NEO_MEM_VAL_EVAL:
             ce = put(0, 0, 2);
             if (ce) break;
-            lt_table_kernel<<<ceil_div(L, 256), 256, 0, S>>>(dpt.p, ell, T + 2 * L);
+            lt_table_kernel<<<ceil_div(std::max<uint64_t>(L >> 8, 1), LT_HIGH), 256, 0, S>>>(
+                make_point(reinterpret_cast<const K*>(r_point), ell), ell, T + 2 * L);
             NEO_LAUNCHED(ctx);
             rc = eqbits(3, 2);
             break;
@@ -1053,18 +1071,28 @@ int mem_round_values(neo_gpu_mem_oracle* o) {
         o->hvals_valid = true;
         return NEO_OK;
     }
+    // one entry per factor: the final product at every x
+    std::vector<K> v(o->nf);
+    bool have = false;
     if (o->pending) {
+        K* out = reinterpret_cast<K*>(ctx->h_result);
+        have = o->len == 2 && o->nf <= 128;  // fits h_result
+        if (have) result_arm(out, 2 * (size_t)o->nf);
         mem_fold_kernel<<<ceil_div((o->len >> 1) * o->nf, 256), 256, 0, ctx->stream>>>(
-            o->tab[o->cur].p, o->len, o->tab[o->cur ^ 1].p, o->nf, o->pending_r);
+            o->tab[o->cur].p, o->len, o->tab[o->cur ^ 1].p, o->nf, o->pending_r, have ? out : nullptr);
         NEO_LAUNCHED(ctx);
         o->cur ^= 1;
         o->len >>= 1;
         o->pending = false;
+        if (have) {
+            NEO_CK(ctx, result_wait(ctx, out, 2 * (size_t)o->nf));
+            std::copy(out, out + o->nf, v.begin());
+        }
     }
-    // one entry per factor: the final product at every x
-    std::vector<K> v(o->nf);
-    NEO_CK(ctx, ctx_d2h(ctx, v.data(), o->tab[o->cur].p, o->nf * sizeof(K)));
-    NEO_CK(ctx, ctx_sync(ctx));
+    if (!have) {
+        NEO_CK(ctx, ctx_d2h(ctx, v.data(), o->tab[o->cur].p, o->nf * sizeof(K)));
+        NEO_CK(ctx, ctx_sync(ctx));
+    }
     K val;
     if (o->bitness) {
         K s = gl::kzero();
@@ -1178,7 +1206,7 @@ static int neo_gpu_mem_oracle_fold_impl_abi(neo_gpu_mem_oracle* o, const uint64_
         cudaSetDevice(ctx->device);
         uint64_t tot = (o->len >> 1) * o->nf;
         mem_fold_kernel<<<ceil_div(tot, 256), 256, 0, ctx->stream>>>(o->tab[o->cur].p, o->len, o->tab[o->cur ^ 1].p,
-                                                                     o->nf, o->pending_r);
+                                                                     o->nf, o->pending_r, nullptr);
         NEO_LAUNCHED(ctx);
         o->cur ^= 1;
         o->len >>= 1;

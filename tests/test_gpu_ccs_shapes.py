@@ -113,3 +113,16 @@ def test_row_rounds_across_the_pair_forms(ctx):
         g.fold(r)
         o.fold(r)
     g.close()
+
+
+@pytest.mark.parametrize("order", ["MIM", "IMMI", "MMI", "IIM"])
+def test_identities_between_matrices(ctx, order):
+    """The column pointers go up in one copy per run of matrices."""
+    ell = 6
+    n = 1 << ell
+    rng = np.random.default_rng(len(order))
+    ccs = CcsStructure(n, n, [None if c == "I" else _matrix(rng, n, "uniform") for c in order], [(1, [1] * len(order))])
+    Z = rng.integers(-1, 2, size=(54, n)).astype(np.int8)
+    r = synth.uniform_k(rng, ell)
+    for a, b in zip(ctx.me_y(ccs, Z, r), O.me_y_at_r(ccs, Z, ell, r)):
+        assert np.array_equal(a, b)
