@@ -336,6 +336,10 @@ int launch_me_y(neo_gpu_ctx* ctx, const DevCcs& ccs, const int8_t* d_Z, uint32_t
 // (nothing launched) when m % 64 != 0 or t > 4
 int launch_zrows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t R, uint64_t m, uint32_t t, const gl::K* d_v,
                  gl::K* d_y, bool* done);
+// bus openings y[w][c][rho] = sum_j Z[w 54 + rho][base + c steps + j] v[j]; *done = false
+// (nothing launched) unless m, base and steps are multiples of 16
+int launch_bus_rows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t n_w, uint64_t m, uint64_t base, uint64_t steps,
+                    uint32_t ncols, const gl::K* d_v, gl::K* d_y, bool* done);
 // What the caller knows about the digits of a commitment: any int8
 // (TC_DIGITS_ANY: the cyclic tensor-core form), |digit| <= 63 by construction
 // (TC_DIGITS_SMALL: the small-digit form, a violation is reported through the

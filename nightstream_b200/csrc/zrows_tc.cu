@@ -32,16 +32,20 @@ constexpr uint64_t ZT_MAX_COLS = 1u << 16;
 constexpr uint32_t ZT_TMEM = 64;  // columns: 16 t, a power of two
 static_assert(ZT_A % 1024 == 0 && ZT_B % 1024 == 0, "swizzle atoms are 1024-byte aligned");
 
+// Row r = (w ncols + c) 54 + rho is n bytes at Z + (w 54 + rho) m + base + c n (whole
+// digit rows: ncols = 1, base = 0, n = m)
 struct ZrowsArgs {
-    const int8_t* Z;   // [R][m]
+    const int8_t* Z;
+    uint64_t m, base;
+    uint32_t ncols;
     uint32_t R, t;
-    uint64_t m;        // a multiple of 64
-    const K* v;        // [t][m]
+    uint64_t n;        // columns, a multiple of 16; every row begins on 16 bytes
+    const K* v;        // [t][n]
     uint64_t cols;     // columns per block, a multiple of ZT_COLS
     unsigned long long* acc_lo;  // [R][t][2], zero
     unsigned int* acc_wrap;      // [R][t][2], zero
     unsigned int* tickets;       // [row groups], zero
-    K* y;              // [R / 54][t][54]
+    K* y;              // [R / 54][t][54], R a multiple of 54
     volatile uint32_t* err;  // page-locked: set when a wait gives up
 };
 
@@ -58,7 +62,7 @@ __global__ void __launch_bounds__(ZT_T, 3) zrows_tc_kernel(const ZrowsArgs a) {
     uint8_t* stages = s_raw + ((1024 - (smem_u32(s_raw) & 1023)) & 1023);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t row0 = blockIdx.x * ZT_ROWS, t = a.t;
-    const uint64_t c_lo = blockIdx.y * a.cols, c_hi = min(a.m, c_lo + a.cols);
+    const uint64_t c_lo = blockIdx.y * a.cols, c_hi = min(a.n, c_lo + a.cols);
     const uint32_t n = (uint32_t)((c_hi - c_lo + ZT_COLS - 1) / ZT_COLS);
     if (tid == 0) {
         mbar_init(&s_done[0], 1);
@@ -80,19 +84,23 @@ __global__ void __launch_bounds__(ZT_T, 3) zrows_tc_kernel(const ZrowsArgs a) {
     uint4 za[4];
     uint4 vb[4];
     const uint32_t ak = (tid & 7) * 16, ar = tid >> 3;
+    const int8_t* zr[4];  // null: no such row
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const uint32_t r = row0 + ar + 32 * e, q = r / NEO_D;
+        zr[e] = r < a.R ? a.Z + ((uint64_t)(q / a.ncols) * NEO_D + r % NEO_D) * a.m + a.base + (uint64_t)(q % a.ncols) * a.n : nullptr;
+    }
     auto fetch = [&](uint32_t i) {
         const uint64_t c = c_lo + (uint64_t)i * ZT_COLS;
 #pragma unroll
         for (int e = 0; e < 4; e++) {
-            const uint32_t r = row0 + ar + 32 * e;
-            za[e] = r < a.R && c + ak < c_hi ? __ldg(reinterpret_cast<const uint4*>(a.Z + (uint64_t)r * a.m + c + ak))
-                                             : make_uint4(0, 0, 0, 0);
+            za[e] = zr[e] && c + ak < c_hi ? __ldg(reinterpret_cast<const uint4*>(zr[e] + c + ak)) : make_uint4(0, 0, 0, 0);
         }
         if (warp < (int)t) {
             const uint64_t cv = c + 4 * lane;
 #pragma unroll
             for (int e = 0; e < 4; e++)
-                vb[e] = cv < c_hi ? __ldg(reinterpret_cast<const uint4*>(a.v + (uint64_t)warp * a.m + cv + e)) : make_uint4(0, 0, 0, 0);
+                vb[e] = cv < c_hi ? __ldg(reinterpret_cast<const uint4*>(a.v + (uint64_t)warp * a.n + cv + e)) : make_uint4(0, 0, 0, 0);
         }
     };
     if (n) fetch(0);
@@ -193,6 +201,31 @@ __global__ void __launch_bounds__(ZT_T, 3) zrows_tc_kernel(const ZrowsArgs a) {
     }
 }
 
+static int zrows_launch(neo_gpu_ctx* ctx, ZrowsArgs a) {
+    const uint32_t groups = (a.R + ZT_ROWS - 1) / ZT_ROWS;
+    const uint64_t chunks = (a.n + ZT_COLS - 1) / ZT_COLS;
+    // three blocks per SM, as many as are resident
+    uint64_t splits = std::min<uint64_t>(chunks, std::max<uint64_t>(1, 3 * 148 / groups));
+    a.cols = std::min<uint64_t>((chunks + splits - 1) / splits * ZT_COLS, ZT_MAX_COLS);
+    splits = (a.n + a.cols - 1) / a.cols;
+    // accumulators and tickets, cleared together
+    const size_t n_acc = (size_t)a.R * a.t * 2, lo_bytes = n_acc * 8, wrap_bytes = n_acc * 4;
+    void* scratch = nullptr;
+    NEO_CK(ctx, ctx_scratch(ctx, lo_bytes + wrap_bytes + groups * sizeof(unsigned int), &scratch));
+    uint8_t* sb = reinterpret_cast<uint8_t*>(scratch);
+    NEO_CK(ctx, cudaMemsetAsync(sb, 0, lo_bytes + wrap_bytes + groups * sizeof(unsigned int), ctx->stream));
+    a.acc_lo = reinterpret_cast<unsigned long long*>(sb);
+    a.acc_wrap = reinterpret_cast<unsigned int*>(sb + lo_bytes);
+    a.tickets = reinterpret_cast<unsigned int*>(sb + lo_bytes + wrap_bytes);
+    a.err = ctx_host_err(ctx);
+    constexpr size_t smem = 2 * ZT_STAGE + 1024;
+    static SmemLimit limit;
+    NEO_CK(ctx, limit.at_least(zrows_tc_kernel, smem));
+    zrows_tc_kernel<<<dim3(groups, (uint32_t)splits), ZT_T, smem, ctx->stream>>>(a);
+    NEO_LAUNCHED(ctx);
+    return NEO_OK;
+}
+
 }  // namespace
 
 // y of R digit rows (layout [w][t][54], row = w * 54 + rho); *done = false when the
@@ -203,35 +236,37 @@ int launch_zrows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t R, uint64_t m, ui
     *done = false;
     if (t == 0 || t > ZT_TMAX || m % 64 || m == 0 || R == 0) return NEO_OK;
     if ((reinterpret_cast<uintptr_t>(d_Z) & 15) || (reinterpret_cast<uintptr_t>(d_v) & 15)) return NEO_OK;
-    const uint32_t groups = (R + ZT_ROWS - 1) / ZT_ROWS;
-    const uint64_t chunks = (m + ZT_COLS - 1) / ZT_COLS;
-    // three blocks per SM, as many as are resident
-    uint64_t splits = std::min<uint64_t>(chunks, std::max<uint64_t>(1, 3 * 148 / groups));
-    const uint64_t cols = std::min<uint64_t>((chunks + splits - 1) / splits * ZT_COLS, ZT_MAX_COLS);
-    splits = (m + cols - 1) / cols;
-    // accumulators and tickets, cleared together
-    const size_t n_acc = (size_t)R * t * 2, lo_bytes = n_acc * 8, wrap_bytes = n_acc * 4;
-    void* scratch = nullptr;
-    NEO_CK(ctx, ctx_scratch(ctx, lo_bytes + wrap_bytes + groups * sizeof(unsigned int), &scratch));
-    uint8_t* sb = reinterpret_cast<uint8_t*>(scratch);
-    NEO_CK(ctx, cudaMemsetAsync(sb, 0, lo_bytes + wrap_bytes + groups * sizeof(unsigned int), ctx->stream));
     ZrowsArgs a{};
     a.Z = d_Z;
+    a.m = a.n = m;
+    a.ncols = 1;
     a.R = R;
     a.t = t;
-    a.m = m;
     a.v = d_v;
-    a.cols = cols;
-    a.acc_lo = reinterpret_cast<unsigned long long*>(sb);
-    a.acc_wrap = reinterpret_cast<unsigned int*>(sb + lo_bytes);
-    a.tickets = reinterpret_cast<unsigned int*>(sb + lo_bytes + wrap_bytes);
     a.y = d_y;
-    a.err = ctx_host_err(ctx);
-    constexpr size_t smem = 2 * ZT_STAGE + 1024;
-    static SmemLimit limit;
-    NEO_CK(ctx, limit.at_least(zrows_tc_kernel, smem));
-    zrows_tc_kernel<<<dim3(groups, (uint32_t)splits), ZT_T, smem, ctx->stream>>>(a);
-    NEO_LAUNCHED(ctx);
     *done = true;
-    return NEO_OK;
+    return zrows_launch(ctx, a);
+}
+
+// Bus openings y[w][c][rho] = sum_j Z[w 54 + rho][base + c steps + j] v[j] of n_w
+// witnesses and ncols chunks of `steps` digits; *done = false when a chunk does not
+// begin on 16 bytes in every row
+int launch_bus_rows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t n_w, uint64_t m, uint64_t base, uint64_t steps,
+                    uint32_t ncols, const K* d_v, K* d_y, bool* done) {
+    *done = false;
+    if (steps == 0 || ncols == 0 || m % 16 || base % 16 || steps % 16) return NEO_OK;
+    if ((reinterpret_cast<uintptr_t>(d_Z) & 15) || (reinterpret_cast<uintptr_t>(d_v) & 15)) return NEO_OK;
+    if ((uint64_t)n_w * ncols * NEO_D > 0x7FFFFFFFull) return NEO_OK;
+    ZrowsArgs a{};
+    a.Z = d_Z;
+    a.m = m;
+    a.base = base;
+    a.ncols = ncols;
+    a.n = steps;
+    a.R = n_w * ncols * NEO_D;
+    a.t = 1;
+    a.v = d_v;
+    a.y = d_y;
+    *done = true;
+    return zrows_launch(ctx, a);
 }
