@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libneo_gpu.so")
 OBJDIR = os.path.join(HERE, "_build")
-SOURCES = ["core.cu", "commit.cu", "commit_tc.cu", "zrows_tc.cu", "ccs_oracle.cu", "fold.cu", "batch.cu",
+SOURCES = ["core.cu", "commit.cu", "commit_tc.cu", "zrows_tc.cu", "rlc_tc.cu", "ccs_oracle.cu", "fold.cu", "batch.cu",
            "mem_oracle.cu", "mixers.cu", "pp_gen.cu", "tune.cu", "transcript.cpp", "transcript_capi.cpp"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -336,6 +336,8 @@ int launch_me_y(neo_gpu_ctx* ctx, const DevCcs& ccs, const int8_t* d_Z, uint32_t
 // (nothing launched) when m % 64 != 0 or t > 4
 int launch_zrows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t R, uint64_t m, uint32_t t, const gl::K* d_v,
                  gl::K* d_y, bool* done);
+// the RLC mix on the tensor cores (d_rot: [count][54][RLC_ROT_ROW], 16-byte aligned)
+int launch_rlc_mix(neo_gpu_ctx* ctx, const int8_t* d_rot, const int8_t* d_Zs, uint32_t count, uint64_t m, int32_t* d_Zmix);
 // bus openings y[w][c][rho] = sum_j Z[w 54 + rho][base + c steps + j] v[j]; *done = false
 // (nothing launched) unless m, base and steps are multiples of 16
 int launch_bus_rows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t n_w, uint64_t m, uint64_t base, uint64_t steps,

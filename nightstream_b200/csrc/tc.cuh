@@ -102,4 +102,9 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
+// byte offset of byte k of row `row` in a 128B-swizzled K-major tile
+__device__ __forceinline__ uint32_t sw128_at(uint32_t row, uint32_t k) {
+    return row * 128 + ((((k >> 4) ^ (row & 7)) << 4) | (k & 15));
+}
+
 }  // namespace

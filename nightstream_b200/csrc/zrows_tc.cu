@@ -49,11 +49,6 @@ struct ZrowsArgs {
     volatile uint32_t* err;  // page-locked: set when a wait gives up
 };
 
-// byte offset of byte k of row `row` in a 128B-swizzled K-major tile
-__device__ __forceinline__ uint32_t sw128_at(uint32_t row, uint32_t k) {
-    return row * 128 + ((((k >> 4) ^ (row & 7)) << 4) | (k & 15));
-}
-
 __global__ void __launch_bounds__(ZT_T, 3) zrows_tc_kernel(const ZrowsArgs a) {
     extern __shared__ uint8_t s_raw[];
     __shared__ __align__(8) uint64_t s_done[2];  // MMAs of a stage complete

@@ -1,4 +1,4 @@
-"""Parts of a fold step at the edges of their shapes: the digit split at whole and ragged
+"""Parts of a fold step at the edges of their shapes: the RLC mix, the digit split at whole and ragged
 eights over its ranges, and bus openings of chunks that begin at any byte, and of
 aligned ones with a short last tile."""
 import numpy as np
@@ -10,6 +10,15 @@ from nightstream_b200 import gpu, synth
 
 pytestmark = pytest.mark.gpu
 Q = (1 << 64) - (1 << 32) + 1
+
+
+@pytest.mark.parametrize("count,m", [(1, 1), (1, 128), (2, 4), (3, 101), (13, 127), (13, 129), (12, 260), (64, 1022), (5, 16383)])
+def test_rlc_mix_shapes(ctx, count, m):
+    """Column tiles with a remainder, rows on any byte, an odd witness out, full int8."""
+    rng = np.random.default_rng(count * 1000 + m)
+    rho = rng.integers(-2, 3, size=(count, 54)).astype(np.int8)
+    Zs = rng.integers(-128, 128, size=(count, 54, m)).astype(np.int8)
+    assert np.array_equal(ctx.rlc_mix(rho, Zs), O.rlc_mix(rho, Zs))
 
 
 @pytest.mark.parametrize("n,k,b", [(8, 1, 2), (8, 12, 2), (2056, 12, 2), (4097, 12, 2), (4100, 30, 2), (4096, 31, 2),
