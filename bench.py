@@ -170,10 +170,10 @@ class Clocks:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-# DRAM bytes (read + write) of one 12-plane commit_p8_kernel<4> launch per
-# witness column, from an ncu capture at m = 2^14 (182.1 MB / 16384: the PP
-# limb tiles once plus the window sequences once); the tiles scale with m.
-COMMIT_TRAFFIC_PER_M = 182.1e6 / 16384
+# DRAM bytes (read + write) of one 12-plane commitment per witness column, from an
+# ncu capture at m = 2^14 (commit_win_kernel<4> 161.6 MB, the PP limb tiles once plus
+# the sequences, and win_seq_kernel 11.1 MB); the tiles scale with m.
+COMMIT_TRAFFIC_PER_M = 172.7e6 / 16384
 
 
 # DRAM bytes (read + write) of the 18 launches of one 16-round Pi_CCS sequence
@@ -280,12 +280,13 @@ def commit_roofline(ctx, m, stream, n_vec=12, reps=5):
     peak, peak_src = int8_peak_tops()
     achieved = ops / (commit_ms * 1e-3) / 1e12
     nv = 4 if n_vec > 1 else 1
-    return {"kernel": f"Ajtai commit, {n_vec} digit plane(s) per call, small-digit form (p8_seq_kernel + "
-                      f"commit_p8_kernel<{nv}>: tcgen05 kind::i8, N = {64 * nv}, + commit_p8_reduce_kernel<{nv}>)",
+    return {"kernel": f"Ajtai commit, {n_vec} digit plane(s) per call, small-digit form ("
+                      f"{'win_seq_kernel + ' if nv == 4 else ''}commit_win_kernel<{nv}>: tcgen05 kind::i8, "
+                      f"{nv} vector(s) per CTA)",
             "bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TOPS", "frac": achieved / peak,
             "traffic": COMMIT_TRAFFIC_PER_M * m if m >= 1 << 14 and n_vec == 12 else None,
-            "traffic_source": "ncu dram__bytes_read+write of one 12-plane commit_p8_kernel<4> launch at "
-                              "m = 2^14, scaled by m",
+            "traffic_source": "ncu dram__bytes_read+write of one 12-plane commitment (win_seq_kernel, "
+                              "commit_win_kernel<4>) at m = 2^14, scaled by m",
             "launch_ms": commit_ms, "peak_source": peak_src, "algorithmic_ops_per_launch": ops,
             "frac_of_datasheet": achieved / INT8_DATASHEET_TOPS,
             "datasheet_peak": INT8_DATASHEET_TOPS}

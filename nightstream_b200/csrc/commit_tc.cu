@@ -14,11 +14,11 @@
 //      h(x) = -z[x + 27] (-27 <= x < 0),  z[x] - z[x + 27] (0 <= x < 27),  z[x] (27 <= x < 54)
 //    (X^54 = -X^27 - 1, X^81 = 1 mod Phi_81).  So the 54 output rows are the
 //    windows o = 0..53 of G[w] = h(80 - w): row r = 80 - o for o >= 27, and
-//    r = 26 - o with the finished sum negated for o < 27.  64 rows and
+//    r = 26 - o with the finished sum negated for o < 27.  56 rows and
 //    128 sequence bytes per vector, 7 chunks of 16 bytes per phase.
 //  * Any int8 digit (cyclic): the product mod X^81 - 1, G[w] = z[(80 - w) mod 81]
 //    (z[x] = 0 for x >= 54), rows o = 0..80, output row 80 - o, folded 81 -> 54
-//    with X^54 = -X^27 - 1 when the sum is finished.  96 rows and 160 bytes per
+//    with X^54 = -X^27 - 1 when the sum is finished.  88 rows and 160 bytes per
 //    vector, 9 chunks.
 //
 // Accumulation is int32 in TMEM; a CTA covers at most 512 K blocks, so
@@ -696,9 +696,9 @@ int launch_win(neo_gpu_ctx* ctx, TcArgs a) {
     return launch_gemm<NV, CYC, true>(ctx, a);
 }
 
-// Vectors per CTA.  Small digits: 4 (N = 256) reads each A tile from shared
+// Vectors per CTA.  Small digits: 4 (N = 224) reads each A tile from shared
 // memory once per four vectors; one or two vectors alone take their own size
-// instead of padding.  Any digit: 2 (N = 192), the most that leaves TMEM and
+// instead of padding.  Any digit: 2 (N = 176), the most that leaves TMEM and
 // shared memory for two CTAs per SM.
 int launch_small(neo_gpu_ctx* ctx, const TcArgs& a) {
     if (a.n_vec == 1) return launch_win<1, false>(ctx, a);
@@ -708,7 +708,7 @@ int launch_small(neo_gpu_ctx* ctx, const TcArgs& a) {
 int launch_any(neo_gpu_ctx* ctx, const TcArgs& a) {
     return a.n_vec == 1 ? launch_win<1, true>(ctx, a) : launch_win<2, true>(ctx, a);
 }
-size_t acc_words(uint32_t n_vec) { return ((size_t)n_vec + 3) / 4 * 4 * 32 * 96; }  // both forms: at most 96 rows a vector
+size_t acc_words(uint32_t n_vec) { return ((size_t)n_vec + 3) / 4 * 4 * 32 * 96; }  // both forms: at most 88 rows, with room a vector
 
 }  // namespace
 
