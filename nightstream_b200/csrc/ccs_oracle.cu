@@ -379,11 +379,18 @@ __global__ void __launch_bounds__(256) z1_kernel(const int8_t* __restrict__ Z, u
 }
 
 // out[r] = (M x)[r] for base-field x (CSR), or x[r] for the identity (oracle.rs:245-285)
+// (blockIdx.y: the f variable's matrix)
 __global__ void spmv_fq_kernel(const uint64_t* __restrict__ row_ptr, const uint32_t* __restrict__ col,
-                               const uint64_t* __restrict__ val, int is_identity, uint32_t n, uint32_t m,
+                               const uint64_t* __restrict__ val, const __grid_constant__ MatSel sel, uint32_t n, uint32_t m,
                                const uint64_t* __restrict__ x, uint64_t n_pad, K* __restrict__ out) {
     uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (r >= n_pad) return;
+    const uint32_t q = blockIdx.y;
+    row_ptr += (uint64_t)sel.j[q] * ((uint64_t)n + 1);
+    col += sel.off[q];
+    val += sel.off[q];
+    out += (uint64_t)q * n_pad;
+    const bool is_identity = sel.id[q];
     uint64_t acc = 0;
     if (r < n) {
         if (is_identity) {
@@ -928,12 +935,10 @@ static int oracle_init(neo_gpu_ctx* ctx, neo_gpu_ccs_oracle* o, const int8_t* d_
     for (int rho = 1; rho < NEO_D; rho++) zp.pw[rho] = gl::mul(zp.pw[rho - 1], b);
     z1_kernel<<<ceil_div(m, 256), 256, 0, ctx->stream>>>(o->Z, m, zp, z1.p);
     NEO_LAUNCHED(ctx);
-    for (int v = 0; v < o->n_fvar; v++) {
-        int j = o->fvar_j[v];
-        spmv_fq_kernel<<<ceil_div(n_pad, 256), 256, 0, ctx->stream>>>(
-            o->ccs->csr_ptr.p + (size_t)j * (desc->n + 1), o->ccs->csr_col.p + o->ccs->nnz_off[j],
-            o->ccs->csr_val.p + o->ccs->nnz_off[j], o->ccs->is_identity[j], desc->n, desc->m, z1.p, n_pad,
-            S + (size_t)(1 + v) * n_pad);
+    if (o->n_fvar) {
+        spmv_fq_kernel<<<dim3(ceil_div(n_pad, 256), o->n_fvar), 256, 0, ctx->stream>>>(
+            o->ccs->csr_ptr.p, o->ccs->csr_col.p, o->ccs->csr_val.p, mat_sel(*o->ccs, o->fvar_j, o->n_fvar), desc->n, desc->m,
+            z1.p, n_pad, S + n_pad);
         NEO_LAUNCHED(ctx);
     }
     o->gamma_to_k = gl::kone();

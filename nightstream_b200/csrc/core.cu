@@ -599,13 +599,20 @@ extern "C" int neo_gpu_split_b(neo_gpu_ctx* ctx, const int32_t* Zmix, uint64_t l
 // ME evaluations: v_j = M_j^T chi_r (CSC), y[w][j][rho] = sum_c Z_w[rho][c] v_j[c]
 // (crates/neo-reductions/src/common.rs:582-650; oracle.rs:1694-1768)
 // ---------------------------------------------------------------------------
+// blockIdx.y: the matrix.  Bound by the latency of the dependent loads pointer -> row ->
+// chi, so all matrices go in one launch (four at 2^10 columns: 18 us one by one, 6 together; at 2^18 69 and 54).
 __global__ void matT_chi_kernel(const uint64_t* __restrict__ csc_ptr, const uint32_t* __restrict__ csc_row,
-                                const uint64_t* __restrict__ csc_val, int is_identity, uint32_t n, uint32_t m,
-                                uint64_t n_sz, const K* __restrict__ chi, K* __restrict__ v) {
+                                const uint64_t* __restrict__ csc_val, const __grid_constant__ MatSel sel, uint32_t n,
+                                uint32_t m, uint64_t n_sz, const K* __restrict__ chi, K* __restrict__ v) {
     uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (c >= m) return;
+    const uint32_t q = blockIdx.y;
+    csc_ptr += (uint64_t)sel.j[q] * ((uint64_t)m + 1);
+    csc_row += sel.off[q];
+    csc_val += sel.off[q];
+    v += (uint64_t)q * m;
     uint64_t n_eff = n < n_sz ? n : n_sz;
-    if (is_identity) {
+    if (sel.id[q]) {
         v[c] = c < n_eff ? chi[c] : gl::kzero();
         return;
     }
@@ -682,12 +689,9 @@ __global__ void __launch_bounds__(128) y_scalars_kernel(const K* __restrict__ y,
 int launch_me_y(neo_gpu_ctx* ctx, const DevCcs& ccs, const int8_t* d_Z, uint32_t n_w, uint64_t m, const K* d_chi,
                 uint32_t ell_n, uint32_t b, K* d_vj, K* d_y, K* d_ysc) {
     uint64_t n_sz = 1ULL << ell_n;
-    for (uint32_t j = 0; j < ccs.t; j++) {
-        matT_chi_kernel<<<ceil_div(m, 256), 256, 0, ctx->stream>>>(
-            ccs.csc_ptr.p + (size_t)j * (m + 1), ccs.csc_row.p + ccs.nnz_off[j], ccs.csc_val.p + ccs.nnz_off[j],
-            ccs.is_identity[j], ccs.n, (uint32_t)m, n_sz, d_chi, d_vj + (size_t)j * m);
-        NEO_LAUNCHED(ctx);
-    }
+    matT_chi_kernel<<<dim3(ceil_div(m, 256), ccs.t), 256, 0, ctx->stream>>>(
+        ccs.csc_ptr.p, ccs.csc_row.p, ccs.csc_val.p, mat_sel(ccs, nullptr, ccs.t), ccs.n, (uint32_t)m, n_sz, d_chi, d_vj);
+    NEO_LAUNCHED(ctx);
     bool done = false;
     if (int rc = launch_zrows(ctx, d_Z, n_w * NEO_D, m, ccs.t, d_vj, d_y, &done)) return rc;
     if (!done) {

@@ -311,6 +311,21 @@ inline cudaError_t ctx_scratch(neo_gpu_ctx* ctx, size_t bytes, void** p) {
     return cudaSuccess;
 }
 int dev_ccs_upload(neo_gpu_ctx* ctx, const neo_ccs_desc* desc, DevCcs& out, bool want_csr = true);
+// matrices of one launch (blockIdx.y): index, first nonzero, identity
+struct MatSel {
+    uint64_t off[16];
+    uint8_t j[16], id[16];
+};
+inline MatSel mat_sel(const DevCcs& c, const int* js, uint32_t n) {  // js null: matrices 0..n-1
+    MatSel s{};
+    for (uint32_t q = 0; q < n && q < 16; q++) {
+        const uint32_t j = js ? (uint32_t)js[q] : q;
+        s.j[q] = (uint8_t)j;
+        s.off[q] = c.nnz_off[j];
+        s.id[q] = c.is_identity[j];
+    }
+    return s;
+}
 
 // A point of up to 32 coordinates as a kernel argument: it rides in the launch, where a
 // small copy from pageable memory cost the host 6 to 8 us and the stream 1.5.
