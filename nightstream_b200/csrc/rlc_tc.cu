@@ -45,11 +45,7 @@ __global__ void __launch_bounds__(MT_T, 3) rlc_mix_tc_kernel(const MixArgs a) {
         mbar_init(&s_done[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "n"(MT_TMEM)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
+    if (warp == 0) tmem_alloc<MT_TMEM>(&s_tmem);
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
@@ -151,13 +147,7 @@ __global__ void __launch_bounds__(MT_T, 3) rlc_mix_tc_kernel(const MixArgs a) {
     for (uint32_t r0 = (warp >> 2) * 32; r0 < (okw ? (warp >> 2) * 32 + 32 : 0); r0 += 16) {
         int x[16];
         const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + r0;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]),
-              "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        tmem_ld(taddr, x);
 #pragma unroll
         for (int e = 0; e < 16; e++)
             if (cc < a.m && r0 + e < NEO_D) a.out[(uint64_t)(r0 + e) * a.m + cc] = x[e];
@@ -166,7 +156,7 @@ __global__ void __launch_bounds__(MT_T, 3) rlc_mix_tc_kernel(const MixArgs a) {
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(MT_TMEM));
+        tmem_dealloc<MT_TMEM>(tmem);
     }
 }
 

@@ -64,11 +64,7 @@ __global__ void __launch_bounds__(ZT_T, 3) zrows_tc_kernel(const ZrowsArgs a) {
         mbar_init(&s_done[1], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "n"(ZT_TMEM)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-    }
+    if (warp == 0) tmem_alloc<ZT_TMEM>(&s_tmem);
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
@@ -147,13 +143,7 @@ __global__ void __launch_bounds__(ZT_T, 3) zrows_tc_kernel(const ZrowsArgs a) {
     for (uint32_t j = warp >> 2; j < (okw && n ? t : 0); j += 2) {
         int x[16];
         const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 16 * j;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]), "=r"(x[4]), "=r"(x[5]), "=r"(x[6]), "=r"(x[7]), "=r"(x[8]),
-              "=r"(x[9]), "=r"(x[10]), "=r"(x[11]), "=r"(x[12]), "=r"(x[13]), "=r"(x[14]), "=r"(x[15])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        tmem_ld(taddr, x);
         if (row >= a.R) continue;
 #pragma unroll
         for (int e = 0; e < 2; e++) {
@@ -176,7 +166,7 @@ __global__ void __launch_bounds__(ZT_T, 3) zrows_tc_kernel(const ZrowsArgs a) {
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(ZT_TMEM));
+        tmem_dealloc<ZT_TMEM>(tmem);
     }
     if (tid == 0) s_last = atomicInc(a.tickets + blockIdx.x, gridDim.y - 1) == gridDim.y - 1;
     __syncthreads();
