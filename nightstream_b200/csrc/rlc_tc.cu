@@ -11,6 +11,7 @@
 // By dp4a, which issues slowly here, 13 witnesses of 2^10 columns took 29 us, of 2^14 40
 // (three threads a column, each reading it all) and of 2^16 69; now 9.5, 10 and 26.
 #include "internal.cuh"
+#include "mix_words.h"
 #include "tc.cuh"
 
 namespace {
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(MT_T, 3) rlc_mix_tc_kernel(const MixArgs a) {
     // a lane one quad and the K quads kq = lane / 8 + 4 e (rows 4 kq .. 4 kq + 3 of 54)
     const uint32_t h = warp >> 2, cq = (warp & 3) * 8 + (lane & 7), kl = lane >> 3;
     const uint64_t c = c0 + 4 * cq;
+    const MixRows rows = {a.Z, a.m, (uint64_t)a.count * NEO_D * a.m, a.count};
     uint32_t z[4][4], zn[4][4];  // zn: the words after (rows on any byte)
     uint4 rb[2];
     auto fetch = [&](uint32_t i) {
@@ -70,14 +72,7 @@ __global__ void __launch_bounds__(MT_T, 3) rlc_mix_tc_kernel(const MixArgs a) {
                 if constexpr (WORDS) {
                     z[e][b] = in ? __ldg(reinterpret_cast<const uint32_t*>(zw + (uint64_t)k * a.m)) : 0u;
                 } else {
-                    // the words that hold the quad (the second only if the row reaches into it;
-                    // columns past the row's end are not stored), shifted when they are used:
-                    // branch-free, so that all the loads are in flight
-                    const int8_t* p = in ? zw + (uint64_t)k * a.m : a.Z;
-                    const uint32_t off = (uint32_t)(reinterpret_cast<uintptr_t>(p) & 3);
-                    const uint32_t* w = reinterpret_cast<const uint32_t*>(p - off);
-                    z[e][b] = __ldg(w);
-                    zn[e][b] = __ldg(in && off && c + 4 - off < a.m ? w + 1 : w);
+                    mix_fetch(rows, w, k, c, z[e][b], zn[e][b]);  // shifted when they are used
                 }
             }
 #pragma unroll
@@ -102,12 +97,7 @@ __global__ void __launch_bounds__(MT_T, 3) rlc_mix_tc_kernel(const MixArgs a) {
             const uint32_t k = 64 * h + 4 * (kl + 4 * e);
             if constexpr (!WORDS) {
 #pragma unroll
-                for (int b = 0; b < 4; b++) {
-                    const uint32_t kr = 4 * (kl + 4 * e) + b, wi = 2 * i + h;
-                    const bool in = wi < a.count && c < a.m && kr < NEO_D;
-                    const uint64_t at = reinterpret_cast<uintptr_t>(a.Z) + ((uint64_t)wi * NEO_D + kr) * a.m + c;
-                    z[e][b] = in ? __funnelshift_r(z[e][b], zn[e][b], 8 * (uint32_t)(at & 3)) : 0u;
-                }
+                for (int b = 0; b < 4; b++) z[e][b] = mix_quad(rows, 2 * i + h, 4 * (kl + 4 * e) + b, c, z[e][b], zn[e][b]);
             }
             const uint32_t l01 = __byte_perm(z[e][0], z[e][1], 0x5140), l23 = __byte_perm(z[e][2], z[e][3], 0x5140);
             const uint32_t h01 = __byte_perm(z[e][0], z[e][1], 0x7362), h23 = __byte_perm(z[e][2], z[e][3], 0x7362);
