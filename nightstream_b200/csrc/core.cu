@@ -136,6 +136,7 @@ extern "C" int neo_gpu_synchronize(neo_gpu_ctx* ctx) { NEO_ABI_GUARD(neo_gpu_syn
 // ---------------------------------------------------------------------------
 struct CcsRanges {  // the nonzeros of each matrix (none for an identity)
     uint64_t lo[16], hi[16];
+    uint64_t first[16];  // the first that belongs to a column
 };
 // blockIdx.y = matrix: values made canonical in place, entries per row at ptr[row + 1] (ptr may be null)
 __global__ void csr_count_kernel(const __grid_constant__ CcsRanges g, const uint32_t* __restrict__ row,
@@ -144,7 +145,7 @@ __global__ void csr_count_kernel(const __grid_constant__ CcsRanges g, const uint
     const uint64_t k = g.lo[j] + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (k >= g.hi[j]) return;
     val[k] = gl::canon(val[k]);
-    if (ptr) atomicAdd(ptr + (uint64_t)j * (n + 1) + row[k] + 1, 1ull);
+    if (ptr && k >= g.first[j]) atomicAdd(ptr + (uint64_t)j * (n + 1) + row[k] + 1, 1ull);
 }
 
 // Inclusive scan of each matrix's n + 1 counters (blockIdx.y), two launches: blocks
@@ -212,10 +213,10 @@ __global__ void csr_fill_kernel(const __grid_constant__ CcsRanges g, const uint6
     const uint32_t j = blockIdx.y;
     const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (c >= m) return;
-    const uint64_t base = g.lo[j], cnt = g.hi[j] - base;
+    if (g.hi[j] == g.lo[j]) return;  // an identity's column pointers are not there
+    const uint64_t base = g.lo[j];
     const uint64_t* cp = csc_ptr + (uint64_t)j * (m + 1);
-    const uint64_t k1 = min(cp[c + 1], cnt);
-    for (uint64_t k = cp[c]; k < k1; k++) {
+    for (uint64_t k = cp[c]; k < cp[c + 1]; k++) {
         const uint64_t pos = base + atomicAdd(cursor + (uint64_t)j * (n + 1) + row[base + k], 1ull);
         csr_col[pos] = (uint32_t)c;
         csr_val[pos] = val[base + k];
@@ -235,11 +236,18 @@ int dev_ccs_upload(neo_gpu_ctx* ctx, const neo_ccs_desc* d, DevCcs& o, bool want
     CcsRanges g{};
     for (uint32_t j = 0; j < d->t; j++) {
         if (o.is_identity[j]) continue;
-        g.lo[j] = o.nnz_off[j];
-        g.hi[j] = o.nnz_off[j + 1];
+        // what the kernels index with: a matrix's range inside the nonzeros, columns one after the
+        // other inside the range (entries before the first column belong to none), rows below n
+        const uint64_t base = o.nnz_off[j], end = o.nnz_off[j + 1], cnt = end - base;
+        if (base > end || end > nnz) return ctx->fail(NEO_ERR_ARG, "ccs: nnz_off decreases");
         const uint64_t* cp = d->col_ptr + (size_t)j * (d->m + 1);
-        const uint64_t base = o.nnz_off[j], cnt = o.nnz_off[j + 1] - base;
         if (cp[d->m] != cnt) return ctx->fail(NEO_ERR_ARG, "ccs: col_ptr inconsistent with nnz_off");
+        uint64_t down = 0;
+        for (uint32_t c = 0; c < d->m; c++) down |= (uint64_t)(cp[c] > cp[c + 1]);
+        if (down) return ctx->fail(NEO_ERR_ARG, "ccs: col_ptr decreases");
+        g.lo[j] = base;
+        g.hi[j] = end;
+        g.first[j] = base + cp[0];
         uint32_t top = 0;
         for (uint64_t k = 0; k < cnt; k++) top = std::max(top, d->row_idx[base + k]);
         if (cnt && top >= d->n) return ctx->fail(NEO_ERR_ARG, "ccs: row index out of range");
