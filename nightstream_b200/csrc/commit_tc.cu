@@ -366,9 +366,17 @@ commit_win_kernel(const __grid_constant__ TcArgs a) {
         return __shfl_sync(0xffffffffu, st, 0);
     };
 
+    // a producer's last copies have landed before the CTA ends, also after another role gave
+    // up (bounded waits; when nobody did, the MMAs have waited for them already)
+    auto drain = [&](uint64_t* full, uint32_t stages, uint32_t issued) {
+        for (uint32_t it = issued > stages ? issued - stages : 0; it < issued; it++)
+            if (!mbar_wait(&full[it % stages], (it / stages) & 1)) break;
+    };
+
     if (warp == 0) {
         // ---- producer: A tiles ----
         if (lane == 0) {
+            uint32_t issued = 0;
             for (uint32_t it = 0; it < nkb; it++) {
                 const int s = it % S::ASTAGES;
                 const uint32_t ph = (it / S::ASTAGES) & 1;
@@ -376,7 +384,9 @@ commit_win_kernel(const __grid_constant__ TcArgs a) {
                 if (s_abort) break;
                 mbar_expect_tx(&full_a[s], TC_A_BYTES);
                 bulk_g2s(sA + s * TC_A_BYTES, a.ppl + (uint64_t)(kb0 + it) * TC_A_BYTES, TC_A_BYTES, &full_a[s]);
+                issued++;
             }
+            drain(full_a, S::ASTAGES, issued);
         }
     } else if (warp == 1) {
         // ---- MMA issuer: one M = 128, N = NPAD MMA per 32-byte K step ----
@@ -404,13 +414,16 @@ commit_win_kernel(const __grid_constant__ TcArgs a) {
     } else if (!FUSED && warp >= 2 + TC_BUILDERS / 32) {
         // ---- second producer: the records of G (one thread of the last two warps) ----
         if (lane == 0 && warp == 2 + TC_BUILDERS / 32) {
+            uint32_t issued = 0;
             for (uint32_t it = 0; it < nkb; it++) {
                 const int s = it % S::GSTAGES;
                 if (it >= S::GSTAGES && !mbar_wait(&empty_g[s], ((it / S::GSTAGES) & 1) ^ 1)) { atomicOr(a.err, 0x20u); s_abort = 1; break; }
                 if (s_abort) break;
                 mbar_expect_tx(&full_g[s], S::G_BYTES);
                 bulk_g2s(sG + s * S::G_BYTES, a.G + ((uint64_t)group * a.n_kb + kb0 + it) * S::G_BYTES, S::G_BYTES, &full_g[s]);
+                issued++;
             }
+            drain(full_g, S::GSTAGES, issued);
         }
     } else if (FUSED && warp >= 2 + TC_BUILDERS / 32) {
         // ---- transposers: thread (column, vector) of a G tile ----
@@ -505,7 +518,9 @@ commit_win_kernel(const __grid_constant__ TcArgs a) {
     // of 8 limbs into one column per lane, as L + 2^32 H with L and H the sums of
     // its low and high four limbs (|.| < 2^56) ----
     uint32_t okw = 0;  // lane 0 waits for the warp
-    if (lane == 0) okw = (nkb > 0 && !s_abort && mbar_wait(done, 0)) ? 1u : 0u;
+    // the issuer's last commit covers every MMA of the CTA: waited for after an abort too,
+    // before the TMEM and the shared memory go back
+    if (lane == 0) okw = (nkb > 0 && mbar_wait(done, 0) && !s_abort) ? 1u : 0u;
     const bool ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
     if (nkb > 0 && !ok && lane == 0) atomicOr(a.err, 8u);
     asm volatile("tcgen05.fence::after_thread_sync;");
