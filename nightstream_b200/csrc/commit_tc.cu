@@ -231,8 +231,9 @@ __global__ void __launch_bounds__(SEQ_T) win_seq_kernel(const int8_t* __restrict
     constexpr int NV = 4;
     constexpr int PITCH = S::SEQ + 16;  // per column; a thread's four columns are SEQ_T apart in the stage
     __shared__ __align__(16) uint8_t s_out[SEQ_COLS * PITCH];
-    const uint32_t v = blockIdx.y, tid = threadIdx.x;
-    const uint64_t j0 = (uint64_t)blockIdx.x * SEQ_COLS, j = j0 + 4 * tid;
+    // (vector, columns): a grid of one dimension, as the vectors may be more than 65535
+    const uint32_t per = (n_kb + SEQ_COLS / 2 - 1) / (SEQ_COLS / 2), v = blockIdx.x / per, tid = threadIdx.x;
+    const uint64_t j0 = (uint64_t)(blockIdx.x % per) * SEQ_COLS, j = j0 + 4 * tid;
     const int8_t* zv = digits + (uint64_t)v * NEO_D * m;
     uint32_t z[NEO_D];
     if constexpr (V4) {  // m % 4 == 0: a word is inside the row or past it
@@ -686,7 +687,9 @@ int launch_win(neo_gpu_ctx* ctx, TcArgs a) {
             NEO_CK(ctx, ctx_scratch(ctx, (size_t)a.n_groups * a.n_kb * Win<4, false, false>::G_BYTES, &G));
             uint8_t* g = reinterpret_cast<uint8_t*>(G);
             a.G = g;
-            const dim3 grid((a.n_kb + SEQ_COLS / 2 - 1) / (SEQ_COLS / 2), a.n_vec);
+            const uint64_t grid64 = (uint64_t)((a.n_kb + SEQ_COLS / 2 - 1) / (SEQ_COLS / 2)) * a.n_vec;
+            if (grid64 > 0x7FFFFFFFull) return ctx->fail(NEO_ERR_UNSUPPORTED, "commit: too many vectors for one launch");
+            const unsigned grid = (unsigned)grid64;
             if (a.m % 4 == 0 && reinterpret_cast<uintptr_t>(a.digits) % 4 == 0)
                 win_seq_kernel<true><<<grid, SEQ_T, 0, ctx->stream>>>(a.digits, a.m, a.n_kb, g, a.bad);
             else
