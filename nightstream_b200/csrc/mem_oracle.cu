@@ -334,7 +334,7 @@ __device__ __forceinline__ K ldg_k(const K* p) {
 // their own: most rows of the first rounds are outside the active trace, where the
 // fold is all there is to do and streams (dst[p] = lerp(src[2p], src[2p+1], r),
 // 48 bytes an entry; 100 factors of 2^16 entries: 20 us), while the evaluation's
-// tiles wait on barriers (116 us with the fold inside).  blockIdx.y:
+// tiles wait on barriers (116 us with the fold inside).  blockIdx.y, z:
 // a factor of one of the claims.
 constexpr uint64_t FOLD_PAIRS = 4096;
 constexpr uint32_t FOLD_PER = 2;
@@ -348,8 +348,10 @@ struct MultiFold {
 };
 __global__ void __launch_bounds__(256) mem_multi_fold_kernel(const __grid_constant__ MultiFold a) {
     int c = 0;
-    while (blockIdx.y >= a.f0[c + 1]) c++;
-    const uint64_t half = a.half[c], f = blockIdx.y - a.f0[c];
+    const uint32_t y = blockIdx.y + gridDim.y * blockIdx.z;  // a bitness claim may have more than 65535 columns
+    if (y >= a.f0[a.n]) return;
+    while (y >= a.f0[c + 1]) c++;
+    const uint64_t half = a.half[c], f = y - a.f0[c];
     const uint64_t p0 = blockIdx.x * (uint64_t)(256 * FOLD_PER) + threadIdx.x;
     const K* s = a.src[c] + f * 2 * half;
     K* d = a.dst[c] + f * half;
@@ -1043,7 +1045,8 @@ int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int 
     }
     a.partials = partials.p;
     if (mf.n) {
-        mem_multi_fold_kernel<<<dim3(ceil_div(fold_len, 256 * FOLD_PER), mf.f0[mf.n]), 256, 0, ctx->stream>>>(mf);
+        const uint32_t gy = std::min(mf.f0[mf.n], 65535u);
+        mem_multi_fold_kernel<<<dim3(ceil_div(fold_len, 256 * FOLD_PER), gy, ceil_div(mf.f0[mf.n], gy)), 256, 0, ctx->stream>>>(mf);
         NEO_LAUNCHED(ctx);
     }
     mem_multi_eval_kernel<<<blocks, 256, 0, ctx->stream>>>(a);
