@@ -63,6 +63,10 @@ const char* neo_gpu_last_error(const neo_gpu_ctx* ctx);
  * the context left usable -- the same path the commitment kernel's bounded
  * mbarrier waits report through. */
 int neo_gpu_wait_probe(neo_gpu_ctx* ctx, uint32_t set_flag, uint32_t spin_limit);
+/* The same wait on a flag that nothing sets, left in flight: it runs out during
+ * the calls that follow, as a wait of their own launches would, and the first of
+ * them that looks for device-side errors returns NEO_ERR_CUDA. */
+int neo_gpu_wait_probe_async(neo_gpu_ctx* ctx, uint32_t spin_limit);
 /* Number of kernels this context has launched so far (instrumentation). */
 uint64_t neo_gpu_kernel_launches(const neo_gpu_ctx* ctx);
 /* The context's CUDA stream (a cudaStream_t), for event timing by callers. */

@@ -1336,6 +1336,14 @@ static int ajtai_precompute(neo_gpu_ccs_oracle* o) {
     return NEO_OK;
 }
 
+// The error word of the launches a call has waited for.  ME outputs whose launch gave up are
+// not whole, so the next call forms them again.
+static int check_pre(neo_gpu_ccs_oracle* o) {
+    const int rc = check_host_error(o->ctx);
+    if (rc) o->have_pre = o->have_aj = false;
+    return rc;
+}
+
 static int ajtai_round(neo_gpu_ccs_oracle* o, const uint64_t* xs, uint32_t nx, uint64_t* ys) {
     neo_gpu_ctx* ctx = o->ctx;
     if (!o->have_pre) {
@@ -1383,7 +1391,7 @@ static int ajtai_round(neo_gpu_ccs_oracle* o, const uint64_t* xs, uint32_t nx, u
     ajtai_round_kernel<<<1, AJ_T, smem, ctx->stream>>>(a);
     NEO_LAUNCHED(ctx);
     NEO_CK(ctx, result_wait(ctx, out, 2 * (size_t)nx));
-    if (int rc = check_host_error(ctx)) return rc;
+    if (int rc = check_pre(o)) return rc;
     memcpy(ys, out, nx * sizeof(K));
     return NEO_OK;
 }
@@ -1477,7 +1485,7 @@ static int neo_gpu_ccs_oracle_me_outputs_impl_abi(neo_gpu_ccs_oracle* o, uint64_
     NEO_CK(ctx, ctx_d2h(ctx, y, o->y_eval.p, o->y_eval.bytes()));
     NEO_CK(ctx, ctx_d2h(ctx, y_scalars, o->y_sc.p, o->y_sc.bytes()));
     NEO_CK(ctx, ctx_sync(ctx));
-    return check_host_error(ctx);
+    return check_pre(o);
 }
 extern "C" int neo_gpu_ccs_oracle_me_outputs(neo_gpu_ccs_oracle* o, uint64_t* y, uint64_t* y_scalars) { NEO_ABI_GUARD(neo_gpu_ccs_oracle_me_outputs_impl_abi(o, y, y_scalars)) }
 

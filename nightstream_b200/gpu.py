@@ -81,6 +81,7 @@ SIGNATURES = {
     "neo_gpu_batch_job_error": [P, U64, P, U64],
     "neo_gpu_batch_cancel": [P, U64],
     "neo_gpu_wait_probe": [P, U32, U32],
+    "neo_gpu_wait_probe_async": [P, U32],
     "neo_gpu_batch_kernel_launches": [P],
     "neo_gpu_batch_destroy": [P],
     "neo_transcript_new": [ctypes.c_char_p, P],
@@ -213,6 +214,11 @@ class Context:
         """Bounded device wait on a flag (neo_gpu_wait_probe); raises NeoGpuError
         (NEO_ERR_CUDA) when the wait runs out."""
         self.check(self.lib.neo_gpu_wait_probe(self.h, 1 if set_flag else 0, spin_limit))
+
+    def wait_probe_async(self, spin_limit: int = 1000):
+        """A bounded wait that runs out during the calls that follow
+        (neo_gpu_wait_probe_async)."""
+        self.check(self.lib.neo_gpu_wait_probe_async(self.h, spin_limit))
 
     def commit_device(self, d_digits: int, n_vec: int, m: int, d_out: int, small_digits: bool = False):
         """Asynchronous commitment of device digits; small_digits: the caller

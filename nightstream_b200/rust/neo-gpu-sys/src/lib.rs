@@ -121,6 +121,7 @@ extern "C" {
     pub fn neo_gpu_ctx_destroy(ctx: *mut neo_gpu_ctx) -> c_int;
     pub fn neo_gpu_last_error(ctx: *const neo_gpu_ctx) -> *const c_char;
     pub fn neo_gpu_wait_probe(ctx: *mut neo_gpu_ctx, set_flag: u32, spin_limit: u32) -> c_int;
+    pub fn neo_gpu_wait_probe_async(ctx: *mut neo_gpu_ctx, spin_limit: u32) -> c_int;
     pub fn neo_gpu_ctx_stream(ctx: *const neo_gpu_ctx, stream: *mut *mut c_void) -> c_int;
     pub fn neo_gpu_synchronize(ctx: *mut neo_gpu_ctx) -> c_int;
     pub fn neo_gpu_pp_upload(ctx: *mut neo_gpu_ctx, kappa: u32, m: u64, coeffs: *const u64) -> c_int;
