@@ -77,6 +77,7 @@ int check_device_error(neo_gpu_ctx* ctx) {
     NEO_CK(ctx, ctx_sync(ctx));
     if (e) {
         NEO_CK(ctx, cudaMemsetAsync(ctx->d_err, 0, 4, ctx->stream));
+        *ctx_host_err(ctx) = 0;  // the same call's error, not the next one's
         char buf[128];
         if (e == (1u << 16)) {  // set by the small-digit commitment form only
             snprintf(buf, sizeof buf, "commitment digits outside [-63, 63] on the small-digit path");

@@ -36,3 +36,11 @@ def test_me_outputs_are_formed_again_after_an_error(ctx, call):
     for a, b in zip(again, run(o)):
         assert np.array_equal(a, b)
     g.close()
+
+
+def test_one_report_clears_both_error_words(ctx):
+    ctx.wait_probe_async(1000)
+    with pytest.raises(gpu.NeoGpuError):
+        ctx.wait_probe(False, spin_limit=1000)  # both words are set by then
+    ctx.wait_probe(True)
+    ctx.synchronize()
