@@ -92,7 +92,9 @@ inline cudaError_t result_wait(neo_gpu_ctx* c, const void* p, size_t words) {
         __builtin_ia32_pause();
 #endif
     }
-    return ctx_sync(c);
+    // words still missing behind a good synchronization: a launch that did not write them
+    const cudaError_t e = ctx_sync(c);
+    return e != cudaSuccess || result_ready(p, words) ? e : cudaErrorNotReady;
 }
 
 // device -> host copy on the context's stream
