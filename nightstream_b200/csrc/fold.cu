@@ -735,7 +735,7 @@ int ccs_oracle_dev_vj(neo_gpu_ccs_oracle* o, const K** vj);
 int ccs_oracle_round_launch(neo_gpu_ccs_oracle* o, K* d_dst, uint32_t* ncoef);
 void ccs_oracle_round_set(neo_gpu_ccs_oracle* o, const K* coeffs);
 bool mem_round_multi_ok(const neo_gpu_mem_oracle* o);
-int ta_round_launch(neo_gpu_twist_addr* o, K* d_dst, bool* launched);
+int ta_round_launch(neo_gpu_twist_addr* o, K* dst, bool* launched);
 int mem_claims_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* claims, DevBuf<K>& partials,
                      HostBuf<K>& h_slots);
 int mem_round_launch_multi(neo_gpu_ctx* ctx, neo_gpu_mem_oracle* const* os, int n, K* const* d_out,

@@ -1828,9 +1828,10 @@ int ta_apply_fold(neo_gpu_twist_addr* o) {
     return NEO_OK;
 }
 
-// The round's values at x = 0, 1, 2 into d_dst (device), without a host sync
-// (the pending fold applied first); no items: zeros.
-int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
+// The round's values at x = 0, 1, 2 into dst (page-locked host memory that the caller
+// polls, so every word is one store), without a host sync (the pending fold applied
+// first); no items: zeros, by the host.
+int ta_values_launch(neo_gpu_twist_addr* o, K* dst) {
     neo_gpu_ctx* ctx = o->ctx;
     cudaStream_t S = ctx->stream;
     // the launch binds the challenge itself once the order is there
@@ -1840,7 +1841,7 @@ int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
         if (rc) return rc;
     }
     if (o->N == 0) {
-        NEO_CK(ctx, cudaMemsetAsync(d_dst, 0, 3 * sizeof(K), S));
+        for (int x = 0; x < 3; x++) dst[x] = gl::kzero();
         return NEO_OK;
     }
     const uint32_t nb = ceil_div(o->N, TE_T);
@@ -1862,7 +1863,7 @@ int ta_values_launch(neo_gpu_twist_addr* o, K* d_dst) {
     a.init_tab = o->tab[o->cur].p;
     a.recs = o->recs.p;
     a.heads = o->heads.p;
-    a.out = d_dst;
+    a.out = dst;
     a.ticket = o->ticket.p;
     ta_eval_kernel<<<nb, TE_T, 0, S>>>(a);
     NEO_LAUNCHED(ctx);
@@ -2018,14 +2019,14 @@ extern "C" int neo_gpu_twist_addr_create_device(neo_gpu_ctx* ctx, int kind, uint
                                                 const uint64_t* init_val, const uint64_t* d_cols,
                                                 neo_gpu_twist_addr** out) { NEO_ABI_GUARD(neo_gpu_twist_addr_create_device_impl_abi(ctx, kind, ell, r_cycle, ell_addr, n_init, init_addr, init_val, d_cols, out)) }
 
-// The next round of a Twist address-lane oracle into d_dst[0..3) (device),
+// The next round of a Twist address-lane oracle into dst[0..3) (page-locked),
 // without a host sync; false (nothing launched) once every address bit is
 // bound, when the value no longer depends on x.
-int ta_round_launch(neo_gpu_twist_addr* o, K* d_dst, bool* launched) {
+int ta_round_launch(neo_gpu_twist_addr* o, K* dst, bool* launched) {
     *launched = false;
     if (o->bit + (o->pending ? 1 : 0) >= o->A) return NEO_OK;
     cudaSetDevice(o->ctx->device);
-    if (int rc = ta_values_launch(o, d_dst)) return rc;
+    if (int rc = ta_values_launch(o, dst)) return rc;
     *launched = true;
     return NEO_OK;
 }
