@@ -1526,8 +1526,9 @@ struct TaEval {
     K r;
     K* tab_out;             // pending: the folded initial memory, `half` entries
     uint64_t half;
-    K* recs;                // [gridDim.x][TA_REC]
-    uint32_t* heads;        // [gridDim.x] 1: a run starts inside the block
+    uint32_t nb;            // evaluation blocks; the others make the next round's order and memory
+    K* recs;                // [nb][TA_REC]
+    uint32_t* heads;        // [nb] 1: a run starts inside the block
     K* out;                 // the round's values at x = 0, 1, 2
     unsigned int* ticket;
 };
@@ -1546,14 +1547,14 @@ __device__ __forceinline__ void ta_carries(const TaEval& a, K (*s_red)[6]) {
     K in0 = gl::kzero(), in1 = gl::kzero();  // carried into this batch of blocks
     __shared__ K s_c[2][TE_T];
     __shared__ uint32_t s_f[TE_T];
-    for (uint32_t base = 0; base < gridDim.x; base += TE_T) {
+    for (uint32_t base = 0; base < a.nb; base += TE_T) {
         const uint32_t blk = base + tid;
-        const bool on = blk < gridDim.x;
+        const bool on = blk < a.nb;
         const K* r = a.recs + (uint64_t)(on ? blk : 0) * TA_REC;
         K y0 = on ? ldk(r + 6) : gl::kzero(), y1 = on ? ldk(r + 7) : gl::kzero();
         uint32_t f = on ? __ldcg(a.heads + blk) : 0;
         if (tid == 0 && !f) { y0 = gl::kadd(y0, in0); y1 = gl::kadd(y1, in1); }
-        const uint32_t live_n = min((uint32_t)TE_T, gridDim.x - base);
+        const uint32_t live_n = min((uint32_t)TE_T, a.nb - base);
         for (uint32_t o = 1; o < live_n; o <<= 1) {
             s_c[0][tid] = y0; s_c[1][tid] = y1; s_f[tid] = f;
             __syncthreads();
@@ -1611,6 +1612,16 @@ __device__ __forceinline__ uint32_t ta_merged(const uint64_t* key, uint32_t N, u
     return j + lower(sib, (uint32_t)k) - lower(max(blk, sib), 0);  // the runs meet at the larger block's start
 }
 
+// a block's part of the round is written; the last of all blocks makes the values
+__device__ __forceinline__ void ta_finish(const TaEval& a, K (*s_red)[6]) {
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicInc(a.ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (s_last) ta_carries(a, s_red);
+}
+
 // Blocks of TE_T sorted items.  A query's contribution at x = 0, 1, 2 is w times
 //   child 0:  v0 − k,  0,  −(2 v1 − v0 − k);   child 1:  0,  v1 − k,  2 (2 v1 − v0 − k)
 // (negated for the write check), with v0, v1 the initial values plus the prefix
@@ -1619,18 +1630,30 @@ __device__ __forceinline__ uint32_t ta_merged(const uint64_t* key, uint32_t N, u
 // − c0)) and its own last run's sums T; the last block to finish (ticket, no
 // waits) scans the carries over the blocks and adds everything up.
 // A round is this one launch: a pending challenge is bound as the weights and the
-// initial values are read, and what only the next round reads is written once a
-// block's part of the values is out (the folded initial memory; the next order, which
-// no challenge enters: two binary searches an item).  The launch is one chain of
-// dependent steps, and with the fold as a launch before it a round's two took 13.1 and
-// 6.5 us (2^15 items); now 13 until the values are out and 17 in all.
+// initial values are read, and what only the next round reads (the folded initial
+// memory; the next order, which no challenge enters: two binary searches an item) is
+// the work of further blocks beside the evaluation.  The last block of all writes the
+// values, so nothing of the round is left when they are there.  The launch is one chain
+// of dependent steps, and with the fold as a launch before it a round's two took 13.1
+// and 6.5 us (2^15 items).
 __global__ void __launch_bounds__(TE_T) ta_eval_kernel(const TaEval a) {
     __shared__ K s_e[2][TE_T];              // exclusive prefix sums over the block (children 0, 1)
     __shared__ K s_w[2][TE_T / 32];
     __shared__ int s_h[TE_T / 32];
     __shared__ K s_red[TE_T / 32][6];
-    __shared__ bool s_last;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (blockIdx.x >= a.nb) {
+        const uint32_t x = (blockIdx.x - a.nb) * TE_T + tid;
+        if (a.key_next && x < a.N) {
+            const uint64_t key = a.key[x];
+            a.key_next[ta_merged(a.key, a.N, a.bit, x, key)] = key;
+        }
+        if (a.pending)
+            for (uint64_t q = x; q < a.half; q += (uint64_t)(gridDim.x - a.nb) * TE_T)
+                a.tab_out[q] = gl::klerp(a.init_tab[2 * q], a.init_tab[2 * q + 1], a.r);
+        ta_finish(a, s_red);
+        return;
+    }
     const uint32_t p = blockIdx.x * TE_T + tid;
     const bool live = p < a.N;
     const uint64_t key = live ? a.key[p] : ~0ull;
@@ -1735,16 +1758,7 @@ __global__ void __launch_bounds__(TE_T) ta_eval_kernel(const TaEval a) {
     } else if (tid == 8) {
         a.heads[blockIdx.x] = last_head >= 0;
     }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) s_last = atomicInc(a.ticket, gridDim.x - 1) == gridDim.x - 1;
-    __syncthreads();
-    if (s_last) ta_carries(a, s_red);
-    // what the next round reads
-    if (live && a.key_next) a.key_next[ta_merged(a.key, a.N, a.bit, p, key)] = key;
-    if (a.pending)
-        for (uint64_t q = p; q < a.half; q += (uint64_t)gridDim.x * TE_T)
-            a.tab_out[q] = gl::klerp(a.init_tab[2 * q], a.init_tab[2 * q + 1], a.r);
+    ta_finish(a, s_red);
 }
 
 // One fold of the address lane by itself (a second fold without an evaluation in
@@ -1865,7 +1879,11 @@ int ta_values_launch(neo_gpu_twist_addr* o, K* dst) {
     a.heads = o->heads.p;
     a.out = dst;
     a.ticket = o->ticket.p;
-    ta_eval_kernel<<<nb, TE_T, 0, S>>>(a);
+    a.nb = nb;
+    // blocks of the next order (an item a thread) and of the folded memory
+    uint32_t extra = a.key_next ? nb : 0;
+    if (a.pending) extra = std::max(extra, (uint32_t)std::min<uint64_t>(ceil_div(a.half, TE_T), 148));
+    ta_eval_kernel<<<nb + extra, TE_T, 0, S>>>(a);
     NEO_LAUNCHED(ctx);
     if (fused) {
         o->cur ^= 1;
