@@ -1896,6 +1896,7 @@ static int fold_step_impl(neo_gpu_shard* sh, const uint64_t* z_host, const uint6
         // this step becomes the rollover source of the next one (d_cols is written anew by every step)
         NEO_CK(ctx, cudaMemcpyAsync(sh->valwit.p + (size_t)NEO_D * m, sh->valwit.p, (size_t)NEO_D * m,
                                     cudaMemcpyDeviceToDevice, ctx->stream));
+        NEO_CK(ctx, ctx_sync(ctx));  // nothing of the step is left when the call returns
         sh->d_prev_cols.swap(sh->d_cols);
         sh->prev_c = mcs.c;
         sh->prev_X = mcs.X;
