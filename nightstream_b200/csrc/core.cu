@@ -58,7 +58,6 @@ static int neo_gpu_ctx_destroy_impl_abi(neo_gpu_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->scratch) cudaFree(ctx->scratch);
     if (ctx->commit_buf) cudaFree(ctx->commit_buf);
-    if (ctx->chi_cache) cudaFree(ctx->chi_cache);
     if (ctx->vinv) cudaFree(ctx->vinv);
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->h_result) cudaFreeHost(ctx->h_result);

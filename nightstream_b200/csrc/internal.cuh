@@ -33,11 +33,6 @@ struct neo_gpu_ctx {
     uint32_t commit_groups = 0;
     size_t commit_words = 0;
     uint64_t* vinv = nullptr;        // inverse Vandermonde tables (mem_oracle.cu), once a batched round needs them
-    // the last chi table a memory oracle built (the time-lane oracles of a
-    // step share their point): key = ell then the point's words
-    void* chi_cache = nullptr;
-    size_t chi_cache_bytes = 0;
-    std::vector<uint64_t> chi_key;
     int fail(int code, const char* what, cudaError_t e = cudaSuccess) {
         char buf[512];
         if (e != cudaSuccess)

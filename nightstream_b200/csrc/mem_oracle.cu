@@ -824,29 +824,9 @@ int mem_create(neo_gpu_ctx* ctx, int kind, uint32_t ell, const uint64_t* r_point
         return NEO_OK;
     };
     int rc = NEO_OK;
-    if (chi) {  // factor 0 = χ_{r_cycle}, copied when the previous oracle built it for the same point
-        std::vector<uint64_t> key(1, ell);
-        key.insert(key.end(), r_point, r_point + 2 * (size_t)ell);
-        const size_t bytes = L * sizeof(K);
-        if (ctx->chi_cache && ctx->chi_key == key && ctx->chi_cache_bytes >= bytes) {
-            if (cudaMemcpyAsync(T, ctx->chi_cache, bytes, cudaMemcpyDeviceToDevice, S))
-                return fail(ctx->fail(NEO_ERR_CUDA, "mem_oracle: chi copy"));
-        } else {
-            rc = launch_chi_point(ctx, reinterpret_cast<const K*>(r_point), ell, T);
-            if (rc) return fail(rc);
-            if (ctx->chi_cache_bytes < bytes) {
-                cudaStreamSynchronize(S);  // the old cache may still be read by an earlier copy
-                if (ctx->chi_cache) cudaFree(ctx->chi_cache);
-                ctx->chi_cache = nullptr;
-                ctx->chi_cache_bytes = 0;
-                ctx->chi_key.clear();
-                if (ctx_malloc(ctx, &ctx->chi_cache, bytes)) return fail(ctx->fail(NEO_ERR_OOM, "mem_oracle: chi cache"));
-                ctx->chi_cache_bytes = bytes;
-            }
-            if (cudaMemcpyAsync(ctx->chi_cache, T, bytes, cudaMemcpyDeviceToDevice, S))
-                return fail(ctx->fail(NEO_ERR_CUDA, "mem_oracle: chi cache copy"));
-            ctx->chi_key = key;
-        }
+    if (chi) {  // factor 0 = χ_{r_cycle}
+        rc = launch_chi_point(ctx, reinterpret_cast<const K*>(r_point), ell, T);
+        if (rc) return fail(rc);
     }
     cudaError_t ce = cudaSuccess;
     switch (kind) {
