@@ -1492,8 +1492,10 @@ extern "C" int neo_gpu_ccs_oracle_me_outputs(neo_gpu_ccs_oracle* o, uint64_t* y,
 static int neo_gpu_ccs_oracle_destroy_impl_abi(neo_gpu_ccs_oracle* o) {
     if (!o) return NEO_ERR_ARG;
     cudaSetDevice(o->ctx->device);
-    cudaStreamSynchronize(o->ctx->stream);
+    neo_gpu_ctx* ctx = o->ctx;
+    cudaStreamSynchronize(ctx->stream);
     delete o;
+    pool_trim(ctx);
     return NEO_OK;
 }
 extern "C" int neo_gpu_ccs_oracle_destroy(neo_gpu_ccs_oracle* o) { NEO_ABI_GUARD(neo_gpu_ccs_oracle_destroy_impl_abi(o)) }

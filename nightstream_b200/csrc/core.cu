@@ -36,7 +36,7 @@ static int neo_gpu_ctx_create_impl_abi(int device, neo_gpu_ctx** out) {
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
     if (cudaMemPoolCreate(&c->pool, &props) == cudaSuccess) {
-        uint64_t keep = CTX_POOL_KEEP;
+        uint64_t keep = ~0ull;  // what it keeps is bounded by pool_trim
         cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     } else {
         c->pool = nullptr;
@@ -51,6 +51,20 @@ extern "C" int neo_gpu_ctx_create(int device, neo_gpu_ctx** out) { NEO_ABI_GUARD
 // from the device's memory pool) and later freed; null: cudaMalloc / cudaFree.
 thread_local cudaStream_t g_alloc_stream = nullptr;
 thread_local PoolRef g_pool;
+thread_local uint64_t g_pool_frees = 0;
+
+// Unused memory above `keep` bytes goes back to the device.  A free counts once its
+// stream position has been seen to pass, so the stream is waited for, where there is
+// something to give back at all.
+void pool_trim(const neo_gpu_ctx* ctx, uint64_t keep) {
+    uint64_t held = 0, used = 0;
+    if (!ctx->pool || cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) || held <= keep) return;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &st) || st != cudaStreamCaptureStatusNone) return;
+    if (cudaStreamSynchronize(ctx->stream)) return;
+    if (!cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) && held > used + keep)
+        cudaMemPoolTrimTo(ctx->pool, used + keep);
+}
 
 static int neo_gpu_ctx_destroy_impl_abi(neo_gpu_ctx* ctx) {
     if (!ctx) return NEO_ERR_ARG;

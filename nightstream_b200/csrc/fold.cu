@@ -716,11 +716,13 @@ extern "C" int neo_gpu_shard_create_mem(neo_gpu_ctx* ctx, const neo_ccs_desc* de
 static int neo_gpu_shard_destroy_impl_abi(neo_gpu_shard* sh) {
     if (!sh) return NEO_ERR_ARG;
     cudaSetDevice(sh->ctx->device);
-    cudaStreamSynchronize(sh->ctx->stream);
+    neo_gpu_ctx* ctx = sh->ctx;
+    cudaStreamSynchronize(ctx->stream);
     if (sh->orc) neo_gpu_ccs_oracle_destroy(sh->orc);
     for (auto* o : sh->mem_slots) neo_gpu_mem_oracle_destroy(o);
     for (auto* o : sh->ta_slots) neo_gpu_twist_addr_destroy(o);
     delete sh;
+    pool_trim(ctx);
     return NEO_OK;
 }
 extern "C" int neo_gpu_shard_destroy(neo_gpu_shard* sh) { NEO_ABI_GUARD(neo_gpu_shard_destroy_impl_abi(sh)) }

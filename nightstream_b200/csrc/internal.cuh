@@ -19,7 +19,7 @@ constexpr int RLC_ROT_ROW = 64;
 struct neo_gpu_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
-    cudaMemPool_t pool = nullptr;    // this context's device buffers (PoolScope); keeps at most CTX_POOL_KEEP when idle
+    cudaMemPool_t pool = nullptr;    // this context's device buffers (PoolScope)
     std::string err;
     uint64_t launches = 0;
     // page-locked, device-mapped: kernels write a round's few values here, so that a
@@ -140,23 +140,34 @@ extern thread_local cudaStream_t g_alloc_stream;
 // The buffers of calls on a context come from the context's own memory pool,
 // ordered on its stream: cudaMalloc and cudaFree cost 10 to 200 us each here and
 // wait for the whole device, and an oracle's life has 15 to 36 of them (2.3 of
-// 2.8 ms of a 2^16-row Twist oracle's, 10 of 26 ms of a 2^16-row Pi_CCS oracle's;
-// the same oracles now take 0.95 and 15 ms).  What is freed stays with the pool up to
-// CTX_POOL_KEEP bytes and goes back to the device at the next synchronisation
-// above that, and altogether when the context is destroyed.  A PoolScope is open
-// for the duration of an entry point, on its thread only.
+// 2.8 ms of a 2^16-row Twist oracle's, 10 of 26 ms of a 2^16-row Pi_CCS oracle's).
+// A PoolScope is open for the duration of an entry point, on its thread only.
+//
+// What is freed stays with the pool, up to CTX_POOL_KEEP bytes beside those in use:
+// the calls that free buffers (the destructions, and entry points with temporaries)
+// give the rest back before they return (pool_trim).  The pool's own release
+// threshold is no such bound: it counts the bytes in use too, so a context with more
+// than that alive would keep nothing and map every buffer anew, and it acts at the
+// next synchronization, which may be a later call's.
 constexpr uint64_t CTX_POOL_KEEP = 1ull << 30;
 struct PoolRef {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
 };
 extern thread_local PoolRef g_pool;
+extern thread_local uint64_t g_pool_frees;  // buffers this thread gave to a pool
+void pool_trim(const neo_gpu_ctx* ctx, uint64_t keep = CTX_POOL_KEEP);
 struct PoolScope {
     PoolRef prev;
-    explicit PoolScope(const neo_gpu_ctx* ctx) : prev(g_pool) {
+    const neo_gpu_ctx* ctx;
+    uint64_t frees;
+    explicit PoolScope(const neo_gpu_ctx* c) : prev(g_pool), ctx(c), frees(g_pool_frees) {
         if (!g_alloc_stream && ctx->pool) g_pool = {ctx->pool, ctx->stream};
     }
-    ~PoolScope() { g_pool = prev; }
+    ~PoolScope() {  // behind the frees of the entry point's own buffers
+        g_pool = prev;
+        if (!prev.pool && frees != g_pool_frees) pool_trim(ctx);
+    }
     PoolScope(const PoolScope&) = delete;
     PoolScope& operator=(const PoolScope&) = delete;
 };
@@ -229,8 +240,12 @@ struct DevBuf {
     }
     void release() {
         if (p) {
-            if (s) cudaFreeAsync(p, s);
-            else cudaFree(p);
+            if (s) {
+                cudaFreeAsync(p, s);
+                g_pool_frees++;
+            } else {
+                cudaFree(p);
+            }
         }
         p = nullptr;
         s = nullptr;

@@ -1207,8 +1207,10 @@ extern "C" uint32_t neo_gpu_mem_oracle_degree_bound(const neo_gpu_mem_oracle* o)
 static int neo_gpu_mem_oracle_destroy_impl_abi(neo_gpu_mem_oracle* o) {
     if (!o) return NEO_OK;
     cudaSetDevice(o->ctx->device);
-    cudaStreamSynchronize(o->ctx->stream);
+    neo_gpu_ctx* ctx = o->ctx;
+    cudaStreamSynchronize(ctx->stream);
     delete o;
+    pool_trim(ctx);
     return NEO_OK;
 }
 extern "C" int neo_gpu_mem_oracle_destroy(neo_gpu_mem_oracle* o) { NEO_ABI_GUARD(neo_gpu_mem_oracle_destroy_impl_abi(o)) }
@@ -2070,8 +2072,10 @@ extern "C" uint32_t neo_gpu_twist_addr_degree_bound(const neo_gpu_twist_addr* o)
 static int neo_gpu_twist_addr_destroy_impl_abi(neo_gpu_twist_addr* o) {
     if (!o) return NEO_OK;
     cudaSetDevice(o->ctx->device);
-    cudaStreamSynchronize(o->ctx->stream);
+    neo_gpu_ctx* ctx = o->ctx;
+    cudaStreamSynchronize(ctx->stream);
     delete o;
+    pool_trim(ctx);
     return NEO_OK;
 }
 extern "C" int neo_gpu_twist_addr_destroy(neo_gpu_twist_addr* o) { NEO_ABI_GUARD(neo_gpu_twist_addr_destroy_impl_abi(o)) }
