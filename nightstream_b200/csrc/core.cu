@@ -493,7 +493,7 @@ static int neo_gpu_rlc_mix_impl_abi(neo_gpu_ctx* ctx, const int8_t* rho_coeffs, 
     PoolScope pool_scope(ctx);
     DevBuf<int8_t> dZs, drot;
     DevBuf<int32_t> dmix;
-    NEO_CK(ctx, dZs.alloc((size_t)count * NEO_D * m));
+    NEO_CK(ctx, dZs.alloc((size_t)count * NEO_D * m, MIX_PAD));
     NEO_CK(ctx, drot.alloc((size_t)count * NEO_D * RLC_ROT_ROW));
     NEO_CK(ctx, dmix.alloc((size_t)NEO_D * m));
     NEO_CK(ctx, cudaMemcpyAsync(dZs.p, Zs, dZs.bytes(), cudaMemcpyHostToDevice, ctx->stream));

@@ -678,14 +678,14 @@ static int shard_create_impl(neo_gpu_ctx* ctx, const neo_ccs_desc* desc, uint32_
         NEO_CK(ctx, sh->d_vj.alloc((size_t)sh->t * m));
         NEO_CK(ctx, sh->d_yv.alloc((size_t)std::max<uint32_t>(k_rho, 2) * sh->t * NEO_D));
         NEO_CK(ctx, sh->d_yvsc.alloc((size_t)std::max<uint32_t>(k_rho, 2) * sh->t));
-        NEO_CK(ctx, sh->valwit.alloc((size_t)2 * NEO_D * m));
+        NEO_CK(ctx, sh->valwit.alloc((size_t)2 * NEO_D * m, MIX_PAD));
         NEO_CK(ctx, sh->valplanes.alloc((size_t)k_rho * NEO_D * m));
         for (auto& s : sh->shout) (void)s;
         size_t wmax = 1;
         for (auto& s : sh->shout) wmax = std::max<size_t>(wmax, 1ULL << s->ea);
         NEO_CK(ctx, sh->d_w.alloc(wmax));
     }
-    NEO_CK(ctx, sh->Zall.alloc((size_t)(1 + k_rho) * NEO_D * m));
+    NEO_CK(ctx, sh->Zall.alloc((size_t)(1 + k_rho) * NEO_D * m, MIX_PAD));
     NEO_CK(ctx, sh->d_z.alloc(m));
     NEO_CK(ctx, sh->d_mix.alloc((size_t)NEO_D * m));
     NEO_CK(ctx, sh->d_rot.alloc((size_t)(1 + k_rho) * NEO_D * RLC_ROT_ROW));

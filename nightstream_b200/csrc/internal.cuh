@@ -11,6 +11,7 @@
 #include "../../include/neo_gpu.h"
 #include "abi_guard.h"
 #include "gl.cuh"
+#include "mix_words.h"
 
 #define NEO_D 54
 // bytes per rot(a) row in the RLC mix scratch: 54 int8 entries, zero padded
@@ -208,7 +209,8 @@ struct DevBuf {
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     size_t cap = 0;
-    cudaError_t alloc(size_t count) {
+    // pad: entries behind the buffer that may be read too
+    cudaError_t alloc(size_t count, size_t pad = 0) {
         release();
         n = count;
         cap = count;
@@ -216,12 +218,12 @@ struct DevBuf {
         s = g_alloc_stream;
         cudaError_t e;
         if (s) {
-            e = cudaMallocAsync(reinterpret_cast<void**>(&p), count * sizeof(T), s);
+            e = cudaMallocAsync(reinterpret_cast<void**>(&p), (count + pad) * sizeof(T), s);
         } else if (g_pool.pool) {
             s = g_pool.stream;
-            e = pool_alloc(reinterpret_cast<void**>(&p), count * sizeof(T));
+            e = pool_alloc(reinterpret_cast<void**>(&p), (count + pad) * sizeof(T));
         } else {
-            e = cudaMalloc(&p, count * sizeof(T));
+            e = cudaMalloc(&p, (count + pad) * sizeof(T));
         }
         if (e != cudaSuccess) {
             p = nullptr;
@@ -363,7 +365,8 @@ int launch_me_y(neo_gpu_ctx* ctx, const DevCcs& ccs, const int8_t* d_Z, uint32_t
 // (nothing launched) when m % 64 != 0 or t > 4
 int launch_zrows(neo_gpu_ctx* ctx, const int8_t* d_Z, uint32_t R, uint64_t m, uint32_t t, const gl::K* d_v,
                  gl::K* d_y, bool* done);
-// the RLC mix on the tensor cores (d_rot: [count][54][RLC_ROT_ROW], 16-byte aligned)
+// the RLC mix on the tensor cores (d_rot: [count][54][RLC_ROT_ROW], 16-byte aligned; d_Zs on
+// four bytes, with MIX_PAD readable bytes behind the digits)
 int launch_rlc_mix(neo_gpu_ctx* ctx, const int8_t* d_rot, const int8_t* d_Zs, uint32_t count, uint64_t m, int32_t* d_Zmix);
 // bus openings y[w][c][rho] = sum_j Z[w 54 + rho][base + c steps + j] v[j]; *done = false
 // (nothing launched) unless m, base and steps are multiples of 16

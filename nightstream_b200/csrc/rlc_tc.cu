@@ -11,7 +11,6 @@
 // By dp4a, which issues slowly here, 13 witnesses of 2^10 columns took 29 us, of 2^14 40
 // (three threads a column, each reading it all) and of 2^16 69; now 9.5, 10 and 26.
 #include "internal.cuh"
-#include "mix_words.h"
 #include "tc.cuh"
 
 namespace {
@@ -23,7 +22,7 @@ static_assert(RLC_ROT_ROW == 64, "a witness is 64 bytes of K");
 
 struct MixArgs {
     const int8_t* rot;  // [count][54][RLC_ROT_ROW]
-    const int8_t* Z;    // [count][54][m]
+    const int8_t* Z;    // [count][54][m], and MIX_PAD bytes more
     uint32_t count;
     uint64_t m;
     int32_t* out;       // [54][m]
@@ -56,7 +55,7 @@ __global__ void __launch_bounds__(MT_T, 3) rlc_mix_tc_kernel(const MixArgs a) {
     // a lane one quad and the K quads kq = lane / 8 + 4 e (rows 4 kq .. 4 kq + 3 of 54)
     const uint32_t h = warp >> 2, cq = (warp & 3) * 8 + (lane & 7), kl = lane >> 3;
     const uint64_t c = c0 + 4 * cq;
-    const MixRows rows = {a.Z, a.m, (uint64_t)a.count * NEO_D * a.m, a.count};
+    const MixRows rows = {a.Z, a.m, a.count};
     uint32_t z[4][4], zn[4][4];  // zn: the words after (rows on any byte)
     uint4 rb[2];
     auto fetch = [&](uint32_t i) {
@@ -153,6 +152,7 @@ __global__ void __launch_bounds__(MT_T, 3) rlc_mix_tc_kernel(const MixArgs a) {
 }  // namespace
 
 int launch_rlc_mix(neo_gpu_ctx* ctx, const int8_t* d_rot, const int8_t* d_Zs, uint32_t count, uint64_t m, int32_t* d_Zmix) {
+    if (reinterpret_cast<uintptr_t>(d_Zs) & 3) return ctx->fail(NEO_ERR_ARG, "rlc: digits must begin on four bytes");
     MixArgs a{};
     a.rot = d_rot;
     a.Z = d_Zs;
@@ -168,6 +168,6 @@ int launch_rlc_mix(neo_gpu_ctx* ctx, const int8_t* d_rot, const int8_t* d_Zs, ui
         return NEO_OK;
     };
     static SmemLimit words, bytes;
-    if (m % 4 == 0 && !(reinterpret_cast<uintptr_t>(d_Zs) & 3)) return launch(rlc_mix_tc_kernel<true>, words);
+    if (m % 4 == 0) return launch(rlc_mix_tc_kernel<true>, words);
     return launch(rlc_mix_tc_kernel<false>, bytes);
 }
