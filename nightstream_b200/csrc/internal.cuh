@@ -21,6 +21,7 @@ struct neo_gpu_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;    // this context's device buffers (PoolScope)
+    uint64_t pool_live = 0;          // their bytes
     std::string err;
     uint64_t launches = 0;
     // page-locked, device-mapped: kernels write a round's few values here, so that a
@@ -154,6 +155,7 @@ constexpr uint64_t CTX_POOL_KEEP = 1ull << 30;
 struct PoolRef {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
+    uint64_t* live = nullptr;  // the context's pool_live
 };
 extern thread_local PoolRef g_pool;
 extern thread_local uint64_t g_pool_frees;  // buffers this thread gave to a pool
@@ -162,8 +164,8 @@ struct PoolScope {
     PoolRef prev;
     const neo_gpu_ctx* ctx;
     uint64_t frees;
-    explicit PoolScope(const neo_gpu_ctx* c) : prev(g_pool), ctx(c), frees(g_pool_frees) {
-        if (!g_alloc_stream && ctx->pool) g_pool = {ctx->pool, ctx->stream};
+    explicit PoolScope(neo_gpu_ctx* c) : prev(g_pool), ctx(c), frees(g_pool_frees) {
+        if (!g_alloc_stream && ctx->pool) g_pool = {ctx->pool, ctx->stream, &c->pool_live};
     }
     ~PoolScope() {  // behind the frees of the entry point's own buffers
         g_pool = prev;
@@ -204,6 +206,8 @@ struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
     cudaStream_t s = nullptr;  // stream the allocation was ordered on (null: cudaMalloc); outlives the buffer
+    uint64_t* live = nullptr;  // count of bytes the allocation is part of (a context's pool_live), or null
+    size_t live_bytes = 0;
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -222,6 +226,10 @@ struct DevBuf {
         } else if (g_pool.pool) {
             s = g_pool.stream;
             e = pool_alloc(reinterpret_cast<void**>(&p), (count + pad) * sizeof(T));
+            if (e == cudaSuccess) {
+                live = g_pool.live;
+                *live += live_bytes = (count + pad) * sizeof(T);
+            }
         } else {
             e = cudaMalloc(&p, (count + pad) * sizeof(T));
         }
@@ -245,12 +253,14 @@ struct DevBuf {
             if (s) {
                 cudaFreeAsync(p, s);
                 g_pool_frees++;
+                if (live) *live -= live_bytes;
             } else {
                 cudaFree(p);
             }
         }
         p = nullptr;
         s = nullptr;
+        live = nullptr;
         n = 0;
         cap = 0;
     }
@@ -258,6 +268,8 @@ struct DevBuf {
         std::swap(p, o.p);
         std::swap(n, o.n);
         std::swap(s, o.s);
+        std::swap(live, o.live);
+        std::swap(live_bytes, o.live_bytes);
         std::swap(cap, o.cap);
     }
     size_t bytes() const { return n * sizeof(T); }
