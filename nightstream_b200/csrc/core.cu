@@ -53,19 +53,20 @@ thread_local cudaStream_t g_alloc_stream = nullptr;
 thread_local PoolRef g_pool;
 thread_local uint64_t g_pool_frees = 0;
 
-// Unused memory above `keep` bytes goes back to the device.  A free counts once its
-// stream position has been seen to pass, so the stream is waited for, where there is
-// something to give back by the bytes of the buffers alive (waiting whenever more than
-// `keep` was held added 10 us to a small oracle's 270 beside 2 GB).
-void pool_trim(const neo_gpu_ctx* ctx, uint64_t keep) {
+// Unused memory above CTX_POOL_KEEP bytes goes back to the device.  A free counts once
+// the stream has been seen to pass it, so the stream is waited for, but only where there
+// is something to give back or to show (waiting whenever more than the bound was held
+// added 10 us to a small oracle's 270 beside 2 GB).
+void pool_trim(neo_gpu_ctx* ctx) {
     uint64_t held = 0, used = 0;
-    if (!ctx->pool || cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) || held <= ctx->pool_live + keep)
-        return;
+    if (!ctx->pool || cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held)) return;
+    if (held <= ctx->pool_live + CTX_POOL_KEEP && ctx->pool_unseen <= POOL_UNSEEN) return;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &st) || st != cudaStreamCaptureStatusNone) return;
     if (cudaStreamSynchronize(ctx->stream)) return;
-    if (!cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) && held > used + keep)
-        cudaMemPoolTrimTo(ctx->pool, used + keep);
+    ctx->pool_unseen = 0;
+    if (!cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) && held > used + CTX_POOL_KEEP)
+        cudaMemPoolTrimTo(ctx->pool, used + CTX_POOL_KEEP);
 }
 
 static int neo_gpu_ctx_destroy_impl_abi(neo_gpu_ctx* ctx) {

@@ -22,6 +22,7 @@ struct neo_gpu_ctx {
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;    // this context's device buffers (PoolScope)
     uint64_t pool_live = 0;          // their bytes
+    uint64_t pool_unseen = 0;        // bytes freed since pool_trim last waited for the stream
     std::string err;
     uint64_t launches = 0;
     // page-locked, device-mapped: kernels write a round's few values here, so that a
@@ -151,21 +152,25 @@ extern thread_local cudaStream_t g_alloc_stream;
 // threshold is no such bound: it counts the bytes in use too, so a context with more
 // than that alive would keep nothing and map every buffer anew, and it acts at the
 // next synchronization, which may be a later call's.
-constexpr uint64_t CTX_POOL_KEEP = 1ull << 30;
+//
+// An allocation anywhere else in the process that would fail takes unused memory from
+// the pools (the driver does that), but only what a wait on the stream has seen freed:
+// such a wait follows once POOL_UNSEEN bytes were.
+constexpr uint64_t CTX_POOL_KEEP = 1ull << 30, POOL_UNSEEN = 64ull << 20;
 struct PoolRef {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
-    uint64_t* live = nullptr;  // the context's pool_live
+    neo_gpu_ctx* ctx = nullptr;  // whose bytes the allocations count to
 };
 extern thread_local PoolRef g_pool;
 extern thread_local uint64_t g_pool_frees;  // buffers this thread gave to a pool
-void pool_trim(const neo_gpu_ctx* ctx, uint64_t keep = CTX_POOL_KEEP);
+void pool_trim(neo_gpu_ctx* ctx);
 struct PoolScope {
     PoolRef prev;
-    const neo_gpu_ctx* ctx;
+    neo_gpu_ctx* ctx;
     uint64_t frees;
     explicit PoolScope(neo_gpu_ctx* c) : prev(g_pool), ctx(c), frees(g_pool_frees) {
-        if (!g_alloc_stream && ctx->pool) g_pool = {ctx->pool, ctx->stream, &c->pool_live};
+        if (!g_alloc_stream && ctx->pool) g_pool = {c->pool, c->stream, c};
     }
     ~PoolScope() {  // behind the frees of the entry point's own buffers
         g_pool = prev;
@@ -206,8 +211,8 @@ struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
     cudaStream_t s = nullptr;  // stream the allocation was ordered on (null: cudaMalloc); outlives the buffer
-    uint64_t* live = nullptr;  // count of bytes the allocation is part of (a context's pool_live), or null
-    size_t live_bytes = 0;
+    neo_gpu_ctx* owner = nullptr;  // the context of whose pool the allocation is, or null
+    size_t owned = 0;
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
@@ -227,8 +232,8 @@ struct DevBuf {
             s = g_pool.stream;
             e = pool_alloc(reinterpret_cast<void**>(&p), (count + pad) * sizeof(T));
             if (e == cudaSuccess) {
-                live = g_pool.live;
-                *live += live_bytes = (count + pad) * sizeof(T);
+                owner = g_pool.ctx;
+                owner->pool_live += owned = (count + pad) * sizeof(T);
             }
         } else {
             e = cudaMalloc(&p, (count + pad) * sizeof(T));
@@ -253,14 +258,17 @@ struct DevBuf {
             if (s) {
                 cudaFreeAsync(p, s);
                 g_pool_frees++;
-                if (live) *live -= live_bytes;
+                if (owner) {
+                    owner->pool_live -= owned;
+                    owner->pool_unseen += owned;
+                }
             } else {
                 cudaFree(p);
             }
         }
         p = nullptr;
         s = nullptr;
-        live = nullptr;
+        owner = nullptr;
         n = 0;
         cap = 0;
     }
@@ -268,8 +276,8 @@ struct DevBuf {
         std::swap(p, o.p);
         std::swap(n, o.n);
         std::swap(s, o.s);
-        std::swap(live, o.live);
-        std::swap(live_bytes, o.live_bytes);
+        std::swap(owner, o.owner);
+        std::swap(owned, o.owned);
         std::swap(cap, o.cap);
     }
     size_t bytes() const { return n * sizeof(T); }

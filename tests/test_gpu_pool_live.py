@@ -43,3 +43,25 @@ def test_destruction_gives_back_before_it_returns():
     assert now >= before - KEEP - SLACK
     c.close()
     assert _free() >= before - SLACK
+
+
+@pytest.mark.parametrize("who", ["context", "torch"])
+def test_others_can_have_what_a_destroyed_oracle_used(who):
+    """Memory is short; the first context has destroyed an oracle of 0.9 GB and makes no call after it."""
+    import torch
+    a, b = gpu.Context(0), gpu.Context(0)
+    _oracle(b, 1).close()  # the kernels are loaded before memory gets short
+    b.synchronize()
+    o = _oracle(a, 9)
+    fill = torch.empty(_free() - (700 << 20), dtype=torch.uint8, device="cuda")
+    o.close()
+    assert torch.cuda.mem_get_info()[0] < 800 << 20  # the context keeps it
+    if who == "context":
+        _oracle(b, 10).close()  # 1 GB of tables
+    else:
+        del_me = torch.empty(960 << 20, dtype=torch.uint8, device="cuda")
+        del del_me
+    del fill
+    torch.cuda.empty_cache()
+    a.close()
+    b.close()
