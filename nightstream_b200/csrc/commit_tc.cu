@@ -722,7 +722,17 @@ int tc_pp_prepare(neo_gpu_ctx* ctx, PPEntry* pp) {
     if (pp->kappa * 8 > 128) return ctx->fail(NEO_ERR_UNSUPPORTED, "tensor-core commit: kappa <= 16");
     pp->tc = false;
     const uint64_t n_kb = (pp->m + 1) / 2;
-    if (!pp->d_pp_limbs) NEO_CK(ctx, ctx_malloc(ctx, reinterpret_cast<void**>(&pp->d_pp_limbs), n_kb * TC_A_BYTES));  // size depends on m only
+    if (!pp->d_pp_limbs) {  // size depends on m only
+        const cudaError_t e = ctx_malloc(ctx, reinterpret_cast<void**>(&pp->d_pp_limbs), n_kb * TC_A_BYTES);
+        if (e == cudaErrorMemoryAllocation && pp->m % 2) {
+            // 8 KB of tiles a column beside 8 kappa 54 bytes of PP: an odd column count, which the
+            // CUDA-core kernels serve too, does without them
+            cudaGetLastError();
+            pp->d_pp_limbs = nullptr;
+            return NEO_OK;
+        }
+        NEO_CK(ctx, e);
+    }
     pp_limbs_kernel<<<(unsigned)n_kb, 256, 0, ctx->stream>>>(pp->d_pp, pp->kappa, pp->m, pp->d_pp_limbs);
     NEO_LAUNCHED(ctx);
     NEO_CK(ctx, ctx_sync(ctx));
