@@ -1576,22 +1576,31 @@ __device__ __forceinline__ void ta_carries(const TaEval& a, K (*s_red)[6]) {
 
 // positions of the items in the order by (addr >> (bit + 2), item), from the one by
 // (addr >> (bit + 1), item): an item moves by the sibling run's items that come before
-// it in time
+// it in time.  Its two binary searches (the items before it in the sibling run, and the
+// larger block's start, where the runs meet) go side by side, each step's loads in flight
+// together: one after the other, a round's values waited for them (an oracle of 2^14 steps
+// and 16 address bits: 640 us, now 628).
 __device__ __forceinline__ uint32_t ta_merged(const uint64_t* key, uint32_t N, uint32_t bit, uint32_t j, uint64_t k) {
-    // items before (block, item index) in the current order
-    auto lower = [&](uint32_t block, uint32_t item) {
-        uint32_t lo = 0, hi = N;
-        while (lo < hi) {
-            const uint32_t mid = lo + (hi - lo) / 2;
-            const uint64_t x = key[mid];
-            const uint32_t b = ta_addr(x) >> (bit + 1);
-            if (b < block || (b == block && (uint32_t)x < item)) lo = mid + 1;
-            else hi = mid;
-        }
-        return lo;
-    };
+    auto order = [&](uint64_t x) { return (uint64_t)(ta_addr(x) >> (bit + 1)) << 32 | (uint32_t)x; };
     const uint32_t blk = ta_addr(k) >> (bit + 1), sib = blk ^ 1;
-    return j + lower(sib, (uint32_t)k) - lower(max(blk, sib), 0);  // the runs meet at the larger block's start
+    const uint64_t at[2] = {(uint64_t)sib << 32 | (uint32_t)k, (uint64_t)max(blk, sib) << 32};
+    uint32_t lo[2] = {0, 0}, hi[2] = {N, N};
+    while (lo[0] < hi[0] || lo[1] < hi[1]) {
+        uint32_t mid[2];
+        uint64_t x[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            mid[i] = lo[i] + (hi[i] - lo[i]) / 2;
+            x[i] = key[min(mid[i], N - 1)];
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            if (lo[i] == hi[i]) continue;
+            if (order(x[i]) < at[i]) lo[i] = mid[i] + 1;
+            else hi[i] = mid[i];
+        }
+    }
+    return j + lo[0] - lo[1];
 }
 
 // a block's part of the round is written; the last of all blocks makes the values
