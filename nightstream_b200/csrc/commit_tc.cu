@@ -35,9 +35,9 @@
 //
 // One launch per call.  Warp roles of a CTA: a bulk-copy producer (A tiles,
 // stored in HBM in the 128B-swizzled K-major layout, 16 KB per K block), the
-// MMA issuer, four builder warps that are the epilogue later, and two
-// transposer warps that read the digit rows (16 to 64 columns at a time) and write
-// G straight into shared memory.  The epilogue recombines the 8 limbs of every
+// MMA issuer, four builder warps, and two transposer warps that read the digit
+// rows (16 to 64 columns at a time) and write G straight into shared memory.  All
+// eight warps are the epilogue then: it recombines the 8 limbs of every
 // (i, column) mod q in registers and adds the value's 32-bit halves into 64-bit
 // accumulators in L2 (exact and order-free); the last CTA of a vector group
 // (ticket) reduces them, writes the commitments and leaves the accumulators zero.
@@ -50,7 +50,7 @@
 namespace {
 
 constexpr int TC_A_BYTES = 128 * 128;       // 16 KB
-constexpr int TC_BUILDERS = 128;            // warps 2..5: B builders, then the epilogue (one TMEM lane group each)
+constexpr int TC_BUILDERS = 128;            // warps 2..5: B builders
 constexpr int TC_TRANSPOSERS = 64;          // warps 6, 7
 constexpr int TC_MAX_KB = 512;              // K blocks per CTA (int32 overflow bound)
 constexpr uint32_t TC_MIN_KB = 4;           // K blocks per CTA worth a CTA of its own (m = 2^10: 2 and 4 14.6 us, 8 16.7)
@@ -297,6 +297,13 @@ __global__ void __launch_bounds__(SEQ_T) win_seq_kernel(const int8_t* __restrict
 }
 static_assert(SEQ_T == 32, "win_seq_kernel: one warp, synchronised as one");
 
+// A producer's last copies have landed before its CTA ends, also after another role gave up
+// (bounded waits; when nobody did, the MMAs have waited for them already).
+__device__ __noinline__ void drain(uint64_t* full, uint32_t stages, uint32_t issued) {
+    for (uint32_t it = issued > stages ? issued - stages : 0; it < issued; it++)
+        if (!mbar_wait(&full[it % stages], (it / stages) & 1)) break;
+}
+
 // What bounds it.  One vector: HBM (537 MB of tiles at m = 2^16: 88 us = 6.1 TB/s;
 // before, with separate sequence and reduce launches and 112-byte sequences per
 // half of the rows, 127 us).  Groups of four: shared memory.  Per K block the MMAs
@@ -367,27 +374,19 @@ commit_win_kernel(const __grid_constant__ TcArgs a) {
         return __shfl_sync(0xffffffffu, st, 0);
     };
 
-    // a producer's last copies have landed before the CTA ends, also after another role gave
-    // up (bounded waits; when nobody did, the MMAs have waited for them already)
-    auto drain = [&](uint64_t* full, uint32_t stages, uint32_t issued) {
-        for (uint32_t it = issued > stages ? issued - stages : 0; it < issued; it++)
-            if (!mbar_wait(&full[it % stages], (it / stages) & 1)) break;
-    };
-
     if (warp == 0) {
         // ---- producer: A tiles ----
         if (lane == 0) {
-            uint32_t issued = 0;
-            for (uint32_t it = 0; it < nkb; it++) {
+            uint32_t it = 0;
+            for (; it < nkb; it++) {
                 const int s = it % S::ASTAGES;
                 const uint32_t ph = (it / S::ASTAGES) & 1;
                 if (it >= S::ASTAGES && !mbar_wait(&empty_a[s], ph ^ 1)) { atomicOr(a.err, 1u); s_abort = 1; break; }
                 if (s_abort) break;
                 mbar_expect_tx(&full_a[s], TC_A_BYTES);
                 bulk_g2s(sA + s * TC_A_BYTES, a.ppl + (uint64_t)(kb0 + it) * TC_A_BYTES, TC_A_BYTES, &full_a[s]);
-                issued++;
             }
-            drain(full_a, S::ASTAGES, issued);
+            drain(full_a, S::ASTAGES, it);
         }
     } else if (warp == 1) {
         // ---- MMA issuer: one M = 128, N = NPAD MMA per 32-byte K step ----
@@ -415,16 +414,15 @@ commit_win_kernel(const __grid_constant__ TcArgs a) {
     } else if (!FUSED && warp >= 2 + TC_BUILDERS / 32) {
         // ---- second producer: the records of G (one thread of the last two warps) ----
         if (lane == 0 && warp == 2 + TC_BUILDERS / 32) {
-            uint32_t issued = 0;
-            for (uint32_t it = 0; it < nkb; it++) {
+            uint32_t it = 0;
+            for (; it < nkb; it++) {
                 const int s = it % S::GSTAGES;
                 if (it >= S::GSTAGES && !mbar_wait(&empty_g[s], ((it / S::GSTAGES) & 1) ^ 1)) { atomicOr(a.err, 0x20u); s_abort = 1; break; }
                 if (s_abort) break;
                 mbar_expect_tx(&full_g[s], S::G_BYTES);
                 bulk_g2s(sG + s * S::G_BYTES, a.G + ((uint64_t)group * a.n_kb + kb0 + it) * S::G_BYTES, S::G_BYTES, &full_g[s]);
-                issued++;
             }
-            drain(full_g, S::GSTAGES, issued);
+            drain(full_g, S::GSTAGES, it);
         }
     } else if (FUSED && warp >= 2 + TC_BUILDERS / 32) {
         // ---- transposers: thread (column, vector) of a G tile ----
