@@ -53,7 +53,7 @@ constexpr int TC_A_BYTES = 128 * 128;       // 16 KB
 constexpr int TC_BUILDERS = 128;            // warps 2..5: B builders
 constexpr int TC_TRANSPOSERS = 64;          // warps 6, 7
 constexpr int TC_MAX_KB = 512;              // K blocks per CTA (int32 overflow bound)
-constexpr uint32_t TC_MIN_KB = 4;           // K blocks per CTA worth a CTA of its own (m = 2^10: 2 and 4 14.6 us, 8 16.7)
+constexpr uint32_t TC_MIN_KB = 4;           // K blocks per CTA worth a CTA of its own (1 vector, m = 2^10: 12.3 us with 2, 11.8 with 4, 12.3 with 8)
 // ---------------------------------------------------------------------------
 // prep: PP -> pre-swizzled u8 limb tiles  PPL[kb][row][128 B]
 // ---------------------------------------------------------------------------
@@ -304,17 +304,17 @@ __device__ __noinline__ void drain(uint64_t* full, uint32_t stages, uint32_t iss
         if (!mbar_wait(&full[it % stages], (it / stages) & 1)) break;
 }
 
-// What bounds it.  One vector: HBM (537 MB of tiles at m = 2^16: 88 us = 6.1 TB/s;
-// before, with separate sequence and reduce launches and 112-byte sequences per
-// half of the rows, 127 us).  Groups of four: shared memory.  Per K block the MMAs
+// What bounds it (calls back to back, us).  One vector: HBM (537 MB of tiles at m = 2^16:
+// 87 = 6.2 TB/s; before, with separate sequence and reduce launches and 112-byte sequences
+// per half of the rows, 127).  Groups of four: shared memory.  Per K block the MMAs
 // read 352 wavefronts of 128 bytes, the builders store 91 and load 68, the A tile
 // and G arrive with 136, against 478 cycles of MMA (N = 224; MMAs alone reach 4.5
-// POPS): 12 ternary vectors at m = 2^16 take 290 us (361 before), of which the
-// sequence launch 33; m = 2^14 85 (119), m = 2^10 23 (43).  Windows of one
+// POPS): 12 ternary vectors at m = 2^16 take 290 (361 before), of which the
+// sequence launch 34; m = 2^14 87 (119), m = 2^10 23 (43).  Windows of one
 // 81-periodic sequence need 7 chunks a phase where one sequence per half of the
-// rows needed 10.  One launch instead of four: 1 vector at m = 2^10 10.4 us (26).
-// Any digit: 5 vectors at m = 10006 49 us (94); an odd m, which ran on CUDA cores,
-// 1 vector at m = 5001 19 us (806).
+// rows needed 10.  One launch instead of four: 1 vector at m = 2^10 11.4 (26), of which
+// 9.7 the kernel.  Any digit: 5 vectors at m = 10006 50 (94); an odd m, which ran on CUDA
+// cores, 1 vector at m = 5001 17 (806).
 template <int NV, bool CYC, bool FUSED>
 __global__ void __launch_bounds__(Win<NV, CYC, FUSED>::THREADS, Win<NV, CYC, FUSED>::CTAS)
 commit_win_kernel(const __grid_constant__ TcArgs a) {
@@ -650,9 +650,10 @@ int commit_ws(neo_gpu_ctx* ctx, uint32_t n_groups, size_t acc_words, TcArgs* a, 
 // K blocks per CTA up to which a group of four small-digit vectors is fused: one
 // launch less, but the transposers read the digit rows 16 bytes at a time, which
 // costs more than win_seq_kernel once that hides behind enough K blocks (12
-// vectors: m = 2^14 98.6 us fused, 96.6 apart; 2^16 306 and 291).  One and two
-// vectors, and any digits, are fused at every size (1 vector at m = 2^16: 91 us
-// fused, 104 apart).
+// vectors, L2 flushed before a call: m = 2^14 100.4 us fused, 96.9 apart; 2^15 168 and
+// 169, 2^16 308 and 309; on new digits without the flush 2^16 345 and 341).  One and two
+// vectors, and any digits, are fused at every size (1 vector at m = 2^16, when it was
+// built apart too: 91 us fused, 104 apart).
 constexpr uint32_t FUSED_KB = 64;
 
 template <int NV, bool CYC, bool FUSED>

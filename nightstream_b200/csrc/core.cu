@@ -164,7 +164,7 @@ extern "C" int neo_gpu_synchronize(neo_gpu_ctx* ctx) { NEO_ABI_GUARD(neo_gpu_syn
 // ---------------------------------------------------------------------------
 // CCS upload: CSC as given, plus a CSR copy made on the device (a row's entries in
 // any order: every use sums them in F_q exactly).  On the host the transposition
-// of 590 k nonzeros and its copies took 7 of a 2^16-row Pi_CCS oracle's 15 ms;
+// of 590 k nonzeros and its copies took 7 ms of a 2^16-row Pi_CCS oracle's life;
 // these kernels, bound by their scattered 8- and 4-byte accesses, take 28 us.
 // ---------------------------------------------------------------------------
 struct CcsRanges {  // the nonzeros of each matrix (none for an identity)

@@ -69,13 +69,16 @@ inline cudaError_t ctx_sync(neo_gpu_ctx* c) { return cudaStreamSynchronize(c->st
 // A launch's few field elements in page-locked memory (h_result and the like) are
 // awaited word by word: `result_arm` fills the words with a value that no field
 // element has, and `result_wait` looks until the launch has overwritten every one.
-// The words leave by the launch's last block, which has seen all others finish, so
-// nothing of the launch is outstanding that the caller could notice.  A stream
-// synchronization learns of the end only when the launch has retired, about 4.5 us
-// later: 16 rounds of a memory oracle took 610 us with it and take 535 us, the 16
-// rounds of a small Pi_CCS call 800 and 746 us.  Polling is bounded (about a
-// millisecond), then the stream is synchronized, which also is how an error of the
-// launch is found; a launch under capture ends there too.
+// The words are a launch's last stores: they leave by its last block (a ticket), which
+// has seen all others finish; or by every block or thread for its own words, behind what
+// else it stores (multi_small's points, mem_fold_kernel's factors), and are waited for
+// all.  So nothing of the launch is left to do when they are there, and what it stored
+// is read by later launches of the stream only.  A stream synchronization learns of the
+// end when the launch has retired, about 4.5 us later: a Twist read oracle of 2^16 rows
+// takes 518 us with it and 450 without, a bitness oracle of 2^12 321 and 274, Pi_CCS of
+// 2^10 rows 675 and 621.  Polling is bounded (about a millisecond), then the stream is
+// synchronized, which also is how an error of the launch is found; a launch under
+// capture ends there too.
 inline void result_arm(void* p, size_t words) { memset(p, 0xFF, words * 8); }
 inline bool result_ready(const void* p, size_t words) {
     const uint64_t* w = static_cast<const uint64_t*>(p);
@@ -142,8 +145,10 @@ extern thread_local cudaStream_t g_alloc_stream;
 
 // The buffers of calls on a context come from the context's own memory pool,
 // ordered on its stream: cudaMalloc and cudaFree cost 10 to 200 us each here and
-// wait for the whole device, and an oracle's life has 15 to 36 of them (2.3 of
-// 2.8 ms of a 2^16-row Twist oracle's, 10 of 26 ms of a 2^16-row Pi_CCS oracle's).
+// wait for the whole device, and an oracle's life has 15 to 36 of them (a Twist read
+// oracle of 2^16 rows takes 1.8 ms with them and 0.45 from the pool, Pi_CCS of 2^16 rows
+// and 13 witnesses 20 to 50 ms and 6.9, the mix and split of 13 witnesses of 2^14
+// columns 5.5 ms and 2.1).
 // A PoolScope is open for the duration of an entry point, on its thread only.
 //
 // What is freed stays with the pool, up to CTX_POOL_KEEP bytes beside those in use:

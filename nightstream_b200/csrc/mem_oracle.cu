@@ -1302,8 +1302,8 @@ extern "C" int neo_gpu_addr_lookup_weights(neo_gpu_ctx* ctx, uint32_t ell, const
 // radix sort makes the order of round 0; a fold merges each pair of sibling
 // runs by time.  Degree 2: values at x = 0, 1, 2, interpolated on the host.
 // (One thread per query summing every earlier write of its block took 653 us a
-// round at 2^14 events, each a read and a write, and 12.6 us at 2^10; now
-// 12.5 and 11.)
+// round at 2^14 events, each a read and a write, and 12.6 us at 2^10 beside the fold's
+// launch; now 14.8 and 13.3 with the fold and the next order in it.)
 // ===========================================================================
 namespace {
 
@@ -1626,7 +1626,7 @@ __device__ __forceinline__ void ta_finish(const TaEval& a, K (*s_red)[6]) {
 // the work of further blocks beside the evaluation.  The last block of all writes the
 // values, so nothing of the round is left when they are there.  The launch is one chain
 // of dependent steps, and with the fold as a launch before it a round's two took 13.1
-// and 6.5 us (2^15 items).
+// and 6.5 us (2^15 items); in one 14.8, of which the next order 0.7.
 __global__ void __launch_bounds__(TE_T) ta_eval_kernel(const TaEval a) {
     __shared__ K s_e[2][TE_T];              // exclusive prefix sums over the block (children 0, 1)
     __shared__ K s_w[2][TE_T / 32];
