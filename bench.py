@@ -177,14 +177,15 @@ COMMIT_TRAFFIC_PER_M = 172.7e6 / 16384
 
 
 # DRAM bytes (read + write) of the 18 launches of one 16-round Pi_CCS sequence
-# (k = 13), per row, from an ncu capture at 2^16 rows (248.5 MB / 65536).
-ROUNDS_TRAFFIC_PER_ROW = 248.5e6 / 65536
+# (k = 13), per row, from an ncu capture at 2^16 rows (216.4 MB / 65536).
+ROUNDS_TRAFFIC_PER_ROW = 216.4e6 / 65536
 
 # Integer-ALU ceiling of the sequence's largest launch (round 3, the cross
-# terms), from ncu --set full at 2^16 rows, k = 13: ALU pipe and issue-slot
+# terms), from ncu at 2^16 rows, k = 13: ALU pipe and issue-slot
 # utilisation.
-ROUNDS_ALU = {"kernel": "ccs_fast_round_kernel<3,0> (round 3)", "alu_pipe_frac": 0.669, "issue_active_frac": 0.579,
-              "source": "ncu --set full -k regex:ccs_fast_round_kernel -s 3 -c 1 on bench.py --mode rounds --ell 16"}
+ROUNDS_ALU = {"kernel": "ccs_fast_round_kernel<3,0> (round 3)", "alu_pipe_frac": 0.571, "issue_active_frac": 0.561,
+              "source": "ncu -k regex:ccs_fast_round_kernel -s 19 -c 1 (sm__inst_executed_pipe_alu, sm__issue_active) on "
+                        "bench.py --mode rounds --ell 16"}
 
 
 def measured_peaks():
@@ -254,7 +255,7 @@ def rounds_roofline(ctx, ccs, z, ell, stream, reps=3):
             "launch_ms": ms / ell, "sequence_ms": ms, "peak_source": src,
             "algorithmic_bytes_per_sequence": B,
             "note": "integer-ALU bound (alu): rounds 0..4 read int8 digit planes and the whole sequence moves "
-                    "0.16x B_ccs"}
+                    "0.14x B_ccs"}
 
 
 def commit_roofline(ctx, m, stream, n_vec=12, reps=5):
